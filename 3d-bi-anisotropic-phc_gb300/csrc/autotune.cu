@@ -122,7 +122,7 @@ static int autotune_prec(Plan& P, int nvec, int reps, TuneEntry* best_out) {
   if (e == cudaSuccess && P.opt_plane_split && plane_split(P.n) > 0) {
     std::vector<int> lanes;
     if (!ds) lanes.push_back(0);  // one thread per pencil (not compiled in double-single)
-    for (int i = 1; i < kPlaneLanesMax; ++i)
+    for (int i = ds ? 1 : 0; i < kPlaneLanesMax; ++i)
       if (plane_lanes_alt(P.n, i) > 0) lanes.push_back(plane_lanes_alt(P.n, i));
     const TuneEntry base = best;
     for (int g : lanes) {

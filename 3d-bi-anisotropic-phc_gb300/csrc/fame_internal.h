@@ -109,6 +109,7 @@ struct Plan {
   int nk = 0;        // k-point instances
   int nphase = 0;
   int device = 0;
+  int sms = 152;     // SMs of that device
   cudaStream_t stream = nullptr;
   // options (fame_set_option)
   int opt_precond = 1;                // CG on B preconditioned by the averaged-medium B0^{-1}

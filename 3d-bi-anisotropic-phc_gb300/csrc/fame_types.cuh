@@ -95,6 +95,11 @@ template <class R> using cx = typename cx_of<R>::type;
 
 template <class R> FAME_HD cx<R> mk(R a, R b) { cx<R> z; z.x = a; z.y = b; return z; }
 template <class R> FAME_HD cx<R> zero() { return mk<R>(R(0), R(0)); }
+// a * b + c in one rounding where the type has the instruction (float, double).
+FAME_HD float rfma(float a, float b, float c) { return fmaf(a, b, c); }
+FAME_HD double rfma(double a, double b, double c) { return fma(a, b, c); }
+FAME_HD ff rfma(ff a, ff b, ff c) { return a * b + c; }
+
 template <class V> FAME_HD V cadd(V a, V b) { a.x += b.x; a.y += b.y; return a; }
 template <class V> FAME_HD V csub(V a, V b) { a.x -= b.x; a.y -= b.y; return a; }
 template <class V> FAME_HD V cneg(V a) { a.x = -a.x; a.y = -a.y; return a; }
@@ -107,13 +112,34 @@ template <class V> FAME_HD V cmulc(V a, V b) {
   V z; z.x = a.x * b.x + a.y * b.y; z.y = a.x * b.y - a.y * b.x; return z;
 }
 template <class V, class R> FAME_HD V cscale(V a, R s) { a.x *= s; a.y *= s; return a; }
-// a + b*c
+// a + s*b (real s)
+template <class V, class R> FAME_HD V caxpy(R s, V b, V a) {
+  a.x = rfma(s, b.x, a.x); a.y = rfma(s, b.y, a.y); return a;
+}
+// a + i*s*b (real s)
+template <class V, class R> FAME_HD V caxpyi(R s, V b, V a) {
+  a.x = rfma(-s, b.y, a.x); a.y = rfma(s, b.x, a.y); return a;
+}
+// a + b*c and a + conj(b)*c: four fused multiply-adds (written out, because
+// a + (b.x*c.x - b.y*c.y) contracts to a product, one FMA and an addition:
+// six instructions where the FP64 pipe bounds the kernel)
 template <class V> FAME_HD V cfma(V b, V c, V a) {
+  a.x = rfma(b.x, c.x, rfma(-b.y, c.y, a.x)); a.y = rfma(b.x, c.y, rfma(b.y, c.x, a.y)); return a;
+}
+template <class V> FAME_HD V cfmac(V b, V c, V a) {
+  a.x = rfma(b.x, c.x, rfma(b.y, c.y, a.x)); a.y = rfma(b.x, c.y, rfma(-b.y, c.x, a.y)); return a;
+}
+FAME_HD cff cfma(cff b, cff c, cff a) {
   a.x += b.x * c.x - b.y * c.y; a.y += b.x * c.y + b.y * c.x; return a;
 }
-// a + conj(b)*c
-template <class V> FAME_HD V cfmac(V b, V c, V a) {
+FAME_HD cff cfmac(cff b, cff c, cff a) {
   a.x += b.x * c.x + b.y * c.y; a.y += b.x * c.y - b.y * c.x; return a;
+}
+// a + i*b (s > 0) or a - i*b (s < 0)
+template <int S, class V> FAME_HD V caddi(V a, V b) {
+  V z;
+  if (S > 0) { z.x = a.x - b.y; z.y = a.y + b.x; } else { z.x = a.x + b.y; z.y = a.y - b.x; }
+  return z;
 }
 // multiply by +i (s>0) or -i (s<0)
 template <int S, class V> FAME_HD V cmul_i(V a) {
@@ -121,6 +147,33 @@ template <int S, class V> FAME_HD V cmul_i(V a) {
   if (S > 0) { z.x = -a.y; z.y = a.x; } else { z.x = a.y; z.y = -a.x; }
   return z;
 }
+#if defined(__CUDA_ARCH__)
+// complex64 on the device: both components in one packed FP32 instruction
+// (the FP32 pipe takes the same time for it as for two scalar ones, but it
+// costs one issue slot, and the complex64 kernels are bound by issue).
+// Forms that swap the components stay scalar: a packed operand would have to
+// be assembled by register moves first.
+FAME_HD float2 cadd(float2 a, float2 b) { return __fadd2_rn(a, b); }
+FAME_HD float2 csub(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.0f, -1.0f), a); }
+FAME_HD float2 cscale(float2 a, float s) { return __fmul2_rn(a, make_float2(s, s)); }
+FAME_HD float2 caxpy(float s, float2 b, float2 a) { return __ffma2_rn(make_float2(s, s), b, a); }
+FAME_HD float2 cfma(float2 b, float2 c, float2 a) {
+  a = __ffma2_rn(make_float2(b.x, b.x), c, a);
+  a.x = fmaf(-b.y, c.y, a.x); a.y = fmaf(b.y, c.x, a.y); return a;
+}
+FAME_HD float2 cfmac(float2 b, float2 c, float2 a) {
+  a = __ffma2_rn(make_float2(b.x, b.x), c, a);
+  a.x = fmaf(b.y, c.y, a.x); a.y = fmaf(-b.y, c.x, a.y); return a;
+}
+FAME_HD float2 cmul(float2 a, float2 b) {
+  float2 z = __fmul2_rn(make_float2(a.x, a.x), b);
+  z.x = fmaf(-a.y, b.y, z.x); z.y = fmaf(a.y, b.x, z.y); return z;
+}
+FAME_HD float2 cmulc(float2 a, float2 b) {
+  float2 z = __fmul2_rn(make_float2(a.x, a.x), b);
+  z.x = fmaf(a.y, b.y, z.x); z.y = fmaf(-a.y, b.x, z.y); return z;
+}
+#endif
 template <class V> FAME_HD double cabs2d(V a) { return double(a.x) * a.x + double(a.y) * a.y; }
 
 template <class D, class S> FAME_HD cx<D> cvt(S a) { return mk<D>(D(a.x), D(a.y)); }
@@ -145,6 +198,12 @@ template <int B, int E, class F> FAME_HD void static_for(F&& f) {
 // ---------------------------------------------------------------------------
 constexpr double kPi = 3.141592653589793238462643383279502884;
 
+// sqrt of a positive integer, by Newton's iteration (compile time)
+FAME_HD constexpr double csqrt_int(int n) {
+  double r = double(n);
+  for (int k = 0; k < 64; ++k) r = 0.5 * (r + double(n) / r);
+  return r;
+}
 FAME_HD constexpr double taylor_sin(double x) {
   double x2 = x * x, term = x, sum = x;
   for (int k = 1; k < 16; ++k) {

@@ -71,11 +71,11 @@ FAME_HD cx<R> twiddle(cx<R> v) {
     constexpr double s0 = (o == 1 || o == 3) ? h : -h;
     constexpr double s = S * s0;
     // (vx + i vy)(c + i s)
-    return mk<R>(R(c) * v.x - R(s) * v.y, R(c) * v.y + R(s) * v.x);
+    return cmul(mk<R>(R(c), R(s)), v);
   } else {
     constexpr double c = cs2pi(e, N, 0);
     constexpr double s = S * cs2pi(e, N, 1);
-    return mk<R>(R(c) * v.x - R(s) * v.y, R(c) * v.y + R(s) * v.x);
+    return cmul(mk<R>(R(c), R(s)), v);
   }
 }
 
@@ -89,13 +89,17 @@ FAME_HD void dft_small(cx<R> (&a)[P]) {
     a[1] = csub(t, a[1]);
   } else if constexpr (P == 4) {
     cx<R> s02 = cadd(a[0], a[2]), d02 = csub(a[0], a[2]);
-    cx<R> s13 = cadd(a[1], a[3]), d13 = cmul_i<S>(csub(a[1], a[3]));
+    cx<R> s13 = cadd(a[1], a[3]), d13 = csub(a[1], a[3]);
     a[0] = cadd(s02, s13);
     a[2] = csub(s02, s13);
-    a[1] = cadd(d02, d13);
-    a[3] = csub(d02, d13);
+    a[1] = caddi<S>(d02, d13);
+    a[3] = caddi<-S>(d02, d13);
   } else {
-    // odd P: pair symmetric terms t_n = a_n + a_{P-n}, d_n = a_n - a_{P-n}
+    // odd P: pair symmetric terms t_n = a_n + a_{P-n}, d_n = a_n - a_{P-n};
+    //   X[k], X[P-k] = re_k +- S*i*sin_k1 * f_k,
+    //   re_k = a_0 + sum cos_kn t_n,  f_k = d_1 + sum_{n>1} (sin_kn / sin_k1) d_n,
+    // so that the last product is fused with the last addition (32 instead of
+    // 36 operations at P = 5, 12 instead of 14 at P = 3).
     constexpr int H = (P - 1) / 2;
     cx<R> t[H + 1], d[H + 1];
     static_for<1, H + 1>([&](auto nc) {
@@ -109,20 +113,25 @@ FAME_HD void dft_small(cx<R> (&a)[P]) {
     a[0] = sum;
     static_for<1, H + 1>([&](auto kc) {
       constexpr int k = decltype(kc)::value;
-      cx<R> re = a0, im = zero<R>();
+      constexpr double s1 = cs2pi(k, P, 1);
+      cx<R> re = a0, f = d[1];
       static_for<1, H + 1>([&](auto nc) {
         constexpr int n = decltype(nc)::value;
         constexpr double c = cs2pi((long long)n * k, P, 0);
-        constexpr double s = cs2pi((long long)n * k, P, 1);
-        re.x += R(c) * t[n].x;
-        re.y += R(c) * t[n].y;
-        im.x += R(s) * d[n].x;
-        im.y += R(s) * d[n].y;
+        re = caxpy(R(c), t[n], re);
+        if constexpr (n > 1) {
+          constexpr double r = cs2pi((long long)n * k, P, 1) / s1;
+          f = caxpy(R(r), d[n], f);
+        }
       });
-      // X[k] = re + S*i*im ; X[P-k] = re - S*i*im
-      cx<R> iim = cmul_i<S>(im);
-      a[k] = cadd(re, iim);
-      a[P - k] = csub(re, iim);
+      if constexpr (std::is_same<R, ff>::value) {  // no fused form: one product for both outputs
+        f = cscale(f, R(s1));
+        a[k] = caddi<S>(re, f);
+        a[P - k] = caddi<-S>(re, f);
+      } else {
+        a[k] = caxpyi(R(S * s1), f, re);
+        a[P - k] = caxpyi(R(-S * s1), f, re);
+      }
     });
   }
 }

@@ -117,8 +117,12 @@ __device__ __forceinline__ PiBlock<R> pi_at(const PlanData<R>& d, int inst, int 
   return pi_block<R>(lam[i1], lam[N + i2], lz);
 }
 
-template <class R> __device__ __forceinline__ R rsqrt_n3(int n) {
-  return R(1) / sqrt(R(n) * R(n) * R(n));
+// Scale of a unitary 3D DFT, n^{-3/2}.  The S-free transforms of fncB put all of
+// it on the plane kernels' frequency side (two blocks per voxel and side), so
+// the z pass multiplies by nothing.
+template <class R, int N> __device__ __forceinline__ R scale3() {
+  constexpr double s = 1.0 / (double(N) * csqrt_int(N));
+  return R(s);
 }
 
 // Operator input / output of the split plane kernels.  The double-single
@@ -158,8 +162,8 @@ template <class R> struct DirUpd {
 //   side 0 (Pr):  p = -conj(Pi2) a + conj(Pi1) b      (Pi.Pr, SVD_Matrix_curl.m:64)
 //   side 1 (Qr):  q =  Pi1 a + Pi2 b                  (Pi.Qr, SVD_Matrix_curl.m:63)
 // else copy 3 components.  Then inverse DFT along x (rows, via shared
-// memory) and y (columns, straight to global), scale by 1/n, and multiply by
-// S_x S_y when WITH_S.
+// memory) and y (columns, straight to global); WITH_S multiplies by S_x S_y / n
+// there, PREP without S scales its input by n^{-3/2} (scale3).
 // ---------------------------------------------------------------------------
 template <class R, int N, bool PREP, bool WITH_S>
 __global__ void __launch_bounds__(((3 * N + 31) / 32) * 32, sizeof(R) == 4 ? 2 : 1)
@@ -223,7 +227,11 @@ k_plane_inv(const cx<R>* __restrict__ x, cx<R>* __restrict__ out, PlanData<R> d,
         cx<R> v0, v1, v2;
         if constexpr (PREP) {
           PiBlock<R> P = pi_at<R, N>(d, inst, k3, e, lam, i1, i2, lam[2 * N + k3]);
-          const cx<R> a = in[it][0], b = in[it][1];
+          cx<R> a = in[it][0], b = in[it][1];
+          if constexpr (!WITH_S) {
+            a = cscale(a, scale3<R, N>());
+            b = cscale(b, scale3<R, N>());
+          }
           if (side == 0) {
             v0 = cfmac(P.p1[0], b, cneg(cmulc(P.p2[0], a)));
             v1 = cfmac(P.p1[1], b, cneg(cmulc(P.p2[1], a)));
@@ -262,14 +270,13 @@ k_plane_inv(const cx<R>* __restrict__ x, cx<R>* __restrict__ out, PlanData<R> d,
 #pragma unroll
     for (int i = 0; i < N; ++i) v[i] = sm[(c * N + i) * LD + i1];
     fft<R, N, +1>(v);
-    const R scale = R(1) / R(N);
     cx<R> sx = mk<R>(R(1), R(0));
     const cx<R>* S = d.sxyz + (long long)inst * 3 * N;
-    if constexpr (WITH_S) sx = S[i1];
+    if constexpr (WITH_S) sx = cscale(S[i1], R(1.0 / N));
     cx<R>* o = out + vec * out_stride + (long long)(blockIdx.y * 3 + c) * Nq + (long long)k3 * N * N + i1;
 #pragma unroll
     for (int i2 = 0; i2 < N; ++i2) {
-      cx<R> r = cscale(v[i2], scale);
+      cx<R> r = v[i2];
       if constexpr (WITH_S) r = cmul(r, cmul(sx, S[N + i2]));
       o[(long long)i2 * N] = r;
     }
@@ -279,7 +286,7 @@ k_plane_inv(const cx<R>* __restrict__ x, cx<R>* __restrict__ out, PlanData<R> d,
 // ---------------------------------------------------------------------------
 // plane_fwd: one CTA per (k3 plane, side, vector); 3N threads.
 // Forward DFT along y (columns, straight from global) and x (rows, shared
-// memory), scale 1/n; WITH_S multiplies conj(S_x S_y) first.  POST applies
+// memory); WITH_S multiplies conj(S_x S_y) / n first.  POST applies
 // the Pi^H blocks of one side (SVD_Matrix_curl.m:63-64, handles Prs/Qrs):
 //   side 0 (Prs): a = -sum_c Pi2_c u_c,  b = sum_c Pi1_c u_c
 //   side 1 (Qrs): a = sum_c conj(Pi1_c) v_c, b = sum_c conj(Pi2_c) v_c
@@ -305,7 +312,7 @@ k_plane_fwd(const cx<R>* __restrict__ w, cx<R>* __restrict__ y, PlanData<R> d, V
     const cx<R>* src = w + vec * w_stride + (long long)(blockIdx.y * 3 + c) * Nq + (long long)k3 * N * N + i1;
     cx<R> v[N];
     cx<R> sx = mk<R>(R(1), R(0));
-    if constexpr (WITH_S) sx = S[i1];
+    if constexpr (WITH_S) sx = cscale(S[i1], R(1.0 / N));
 #pragma unroll
     for (int i2 = 0; i2 < N; ++i2) {
       v[i2] = src[(long long)i2 * N];
@@ -323,9 +330,8 @@ k_plane_fwd(const cx<R>* __restrict__ w, cx<R>* __restrict__ y, PlanData<R> d, V
 #pragma unroll
     for (int i = 0; i < N; ++i) v[i] = row[i];
     fft<R, N, -1>(v);
-    const R scale = R(1) / R(N);
 #pragma unroll
-    for (int i = 0; i < N; ++i) row[i] = cscale(v[i], scale);
+    for (int i = 0; i < N; ++i) row[i] = v[i];
   }
   __syncthreads();
   const cx<R>* lam = d.lam + (long long)inst * 3 * N;
@@ -346,6 +352,10 @@ k_plane_fwd(const cx<R>* __restrict__ w, cx<R>* __restrict__ y, PlanData<R> d, V
       } else {
         a = cfmac(P.p1[2], u2, cfmac(P.p1[1], u1, cmulc(P.p1[0], u0)));
         b = cfmac(P.p2[2], u2, cfmac(P.p2[1], u1, cmulc(P.p2[0], u0)));
+      }
+      if constexpr (!WITH_S) {
+        a = cscale(a, scale3<R, N>());
+        b = cscale(b, scale3<R, N>());
       }
       o[e] = a;
       o[Nq + e] = b;
@@ -447,8 +457,8 @@ k_plane_inv2(const cx<R>* __restrict__ x, cx<R>* __restrict__ out, PlanData<R> d
   const cx<R>* lam = d.lam + (long long)inst * 3 * N;
   const cx<R>* xin = x + vec * in_stride + blockIdx.y * in_side_stride + (long long)k3 * N * N;
   const int tid = threadIdx.x;
-  // Pi blocks (frequency voxel -> 3 components of this side), scaled by 1/n
-  // for the two inverse DFTs; all loads of a thread issued together.
+  // Pi blocks (frequency voxel -> 3 components of this side), scaled for the
+  // three inverse DFTs; all loads of a thread issued together.
   {
     constexpr int ITEMS = (N * N + T - 1) / T;
     cx<R> in[ITEMS][2];
@@ -478,7 +488,7 @@ k_plane_inv2(const cx<R>* __restrict__ x, cx<R>* __restrict__ out, PlanData<R> d
         }
       }
     }
-    const R sc = R(1) / R(N);
+    const R sc = scale3<R, N>();
     const cx<R> lz = lam[2 * N + k3];
 #pragma unroll
     for (int it = 0; it < ITEMS; ++it) {
@@ -600,11 +610,11 @@ k_plane_fwd2(const cx<R>* __restrict__ w, cx<R>* __restrict__ y, PlanData<R> d, 
       with_g<G>(g, [&](auto gc) { split_pass_b_store<R, N, G, 1, decltype(gc)::value>(sm + (c * N + p) * LD, z); });
   }
   __syncthreads();
-  // Pi^H blocks of this side, scaled by 1/n for the two forward DFTs
+  // Pi^H blocks of this side, scaled for the three forward DFTs
   const cx<R>* lam = d.lam + (long long)inst * 3 * N;
   cx<R>* o = y + vec * out_stride + blockIdx.y * out_side_stride + (long long)k3 * N * N;
   const cx<R> lz = lam[2 * N + k3];
-  const R sc = R(1) / R(N);
+  const R sc = scale3<R, N>();
   for (int e = tid; e < N * N; e += SP::TB) {
     const int i2 = e / N, i1 = e - i2 * N;
     const cx<R> u0 = sm[(0 * N + i2) * LD + i1];
@@ -627,7 +637,7 @@ k_plane_fwd2(const cx<R>* __restrict__ w, cx<R>* __restrict__ y, PlanData<R> d, 
 // ---------------------------------------------------------------------------
 // col: DFT along z of every (i1, i2) column, in place; one thread per column.
 // SMODE 1: multiply S_z(i3) after (inverse); 2: multiply conj(S_z(i3)) before
-// (forward).  Scale 1/sqrt(n).
+// (forward), both scaled by 1/sqrt(n); 0: neither (scale3).
 // ---------------------------------------------------------------------------
 template <class R, int N, int DIR, int SMODE>
 __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 3 : 1)
@@ -647,10 +657,11 @@ k_col(cx<R>* __restrict__ w, PlanData<R> d, VecCtx ctx, long long stride) {
     if constexpr (SMODE == 2) v[i] = cmulc(Sz[i], v[i]);
   }
   fft<R, N, DIR>(v);
-  const R scale = R(1) / sqrt(R(N));
+  constexpr double scale = 1.0 / csqrt_int(N);
 #pragma unroll
   for (int i = 0; i < N; ++i) {
-    cx<R> r = cscale(v[i], scale);
+    cx<R> r = v[i];
+    if constexpr (SMODE != 0) r = cscale(r, R(scale));
     if constexpr (SMODE == 1) r = cmul(Sz[i], r);
     p[(long long)i * N * N] = r;
   }
@@ -669,6 +680,17 @@ template <class R, int N> inline int plane_lanes(const Plan& P, int tuned) {
   for (int i = 0; i < kPlaneLanesMax; ++i)
     if (tuned > 0 && plane_lanes_alt(N, i) == tuned) return tuned;
   return plane_split(N);
+}
+
+// The split an untuned fncB of nvec vectors takes (as a tuned value).  In
+// complex64: one thread per pencil once the 2 N nvec CTAs give every SM its
+// two resident ones (it needs a quarter fewer instructions and half the
+// shared-memory traffic: fncB of 4 vectors at n = 40 60 -> 50 us, 8 at n = 48
+// 116 -> 106, 10 at n = 60 260 -> 246), the size's split below that, where
+// the extra warps hide latency (one vector at n = 48 41.5 -> 37.5 us, n = 60
+// 52 -> 49).  nvec is the whole batch, so sub-batches do not change a result.
+template <class R, int N> inline int default_lanes(const Plan& P, int nvec) {
+  return std::is_same<R, float>::value && N * nvec >= P.sms ? 0 : -1;
 }
 
 // f(integral_constant<G>) for the compiled lane count G == lanes of size N.
@@ -771,7 +793,7 @@ cudaError_t plane_fwd(const Plan& P, const PlanData<R>& d, const cx<R>* w, cx<R>
 // memory with coalesced row loads, G threads per column do the length-G
 // passes in place, then each the length-M DFT of its sub-pencil in
 // registers, written straight back to global (consecutive threads hold
-// consecutive x).  Scale 1/sqrt(n), no S multiply.
+// consecutive x).  No scale (scale3), no S multiply.
 // ---------------------------------------------------------------------------
 template <class R, int N, int DIR>
 __global__ void __launch_bounds__(((N * plane_split(N) + 31) / 32) * 32)
@@ -800,9 +822,6 @@ k_col2(cx<R>* __restrict__ w, VecCtx ctx, long long stride) {
     cx<R> z[M];
     with_g<G>(g, [&](auto gc) { split_pass_b_load<R, N, G, LD, decltype(gc)::value>(sm + p, z); });
     fft<R, M, DIR>(z);
-    const R scale = R(1) / sqrt(R(N));
-#pragma unroll
-    for (int i = 0; i < M; ++i) z[i] = cscale(z[i], scale);
     with_g<G>(g, [&](auto gc) { split_pass_b_store<R, N, G, (int)(N * N), decltype(gc)::value>(base + p, z); });
   }
 }
@@ -850,6 +869,7 @@ cudaError_t fncB_n(const Plan& P, const cx<R>* x, cx<R>* y, int nvec, const VecC
   const long long Nq = P.Nq;
   const TuneEntry tn = tune_for(P, tune_prec<R>(), nvec);
   const int chunk = (tn.chunk > 0 && tn.chunk < nvec) ? tn.chunk : nvec;
+  const int lanes = tn.lanes >= 0 ? tn.lanes : default_lanes<R, N>(P, nvec);
   for (int v0 = 0; v0 < nvec; v0 += chunk) {
     const int nv = std::min(chunk, nvec - v0);
     const VecCtx c = sub_ctx(ctx, v0);
@@ -861,7 +881,7 @@ cudaError_t fncB_n(const Plan& P, const cx<R>* x, cx<R>* y, int nvec, const VecC
       upd.z = pupd_z + (size_t)v0 * 4 * Nq;
       upd.beta = pupd_beta + v0;
     }
-    e = plane_inv<R, N, true, false>(P, d, xs, w0, nv, 2, 0, 4 * Nq, 2 * Nq, 6 * Nq, c, st, upd, tn.lanes);
+    e = plane_inv<R, N, true, false>(P, d, xs, w0, nv, 2, 0, 4 * Nq, 2 * Nq, 6 * Nq, c, st, upd, lanes);
     if (e != cudaSuccess) return e;
     e = col<R, N, +1, 0>(d, w0, 6, nv, 6 * Nq, c, st);
     if (e != cudaSuccess) return e;
@@ -876,7 +896,7 @@ cudaError_t fncB_n(const Plan& P, const cx<R>* x, cx<R>* y, int nvec, const VecC
     if (e != cudaSuccess) return e;
     e = col<R, N, -1, 0>(d, wm, 6, nv, 6 * Nq, c, st);
     if (e != cudaSuccess) return e;
-    e = plane_fwd<R, N, true, false>(P, d, wm, ys, nv, 2, 0, 6 * Nq, 4 * Nq, 2 * Nq, c, st, tn.lanes);
+    e = plane_fwd<R, N, true, false>(P, d, wm, ys, nv, 2, 0, 6 * Nq, 4 * Nq, 2 * Nq, c, st, lanes);
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
