@@ -159,6 +159,7 @@ int upload_field(Plan& P, PlanData<R>& d, const std::vector<double>& abg) {
   for (size_t i = 0; i < abg.size(); ++i) h[i] = R(abg[i]);
   cudaError_t e = cudaMemcpy(d.fld, h.data(), sizeof(R) * h.size(), cudaMemcpyHostToDevice);
   if (e != cudaSuccess) return cuda_fail(&P, e, "field upload");
+  d.kind = kMatField;
   for (int i = 0; i < 3; ++i)
     for (int j = 0; j < 3; ++j) {
       double g = 0.0;  // G = A^T A, A with the primitive vectors as columns

@@ -141,31 +141,61 @@ int upload_tables(Plan& P) {
       tau[k * 3 + ax] = mk<R>(R(t.real()), R(t.imag()));
     }
   }
-  // material table: Herm(N) | Herm(M) | J per (instance, phase)
-  std::vector<cx<R>> mat((size_t)nk * P.nphase * 27);
-  for (size_t t = 0; t < (size_t)nk * P.nphase; ++t) {
+  // vertex tensors of the material stencil per (instance, phase), in the order
+  // and with the scale factors its kernels read (fncb_material.cuh)
+  using cd = std::complex<double>;
+  const size_t nt = (size_t)nk * P.nphase;
+  auto tensor = [&](size_t t, int blk, int i, int j) {  // Herm(N) | Herm(M) | J
     const double* src = &P.mat_host[t * 54];
-    auto at = [&](int blk, int i, int j) {
-      return std::complex<double>(src[(blk * 9 + i * 3 + j) * 2], src[(blk * 9 + i * 3 + j) * 2 + 1]);
-    };
-    for (int blk = 0; blk < 3; ++blk)
-      for (int i = 0; i < 3; ++i)
-        for (int j = 0; j < 3; ++j) {
-          std::complex<double> v = at(blk, i, j);
-          if (blk < 2) v = 0.5 * (v + std::conj(at(blk, j, i)));
-          mat[t * 27 + blk * 9 + i * 3 + j] = mk<R>(R(v.real()), R(v.imag()));
+    auto at = [&](int r, int c) { return cd(src[(blk * 9 + r * 3 + c) * 2], src[(blk * 9 + r * 3 + c) * 2 + 1]); };
+    return blk < 2 ? 0.5 * (at(i, j) + std::conj(at(j, i))) : at(i, j);
+  };
+  bool chiral = true;
+  for (size_t t = 0; t < nt && chiral; ++t)
+    for (int i = 0; i < 3; ++i)
+      for (int j = 0; j < 3; ++j)
+        chiral = chiral && tensor(t, 0, i, j).imag() == 0.0 && tensor(t, 1, i, j).imag() == 0.0 &&
+                 tensor(t, 2, i, j).real() == 0.0;
+  d.kind = chiral ? kMatChiral : kMatGeneral;
+  const int ts = stn_size(d.kind);
+  std::vector<R> stn(nt * ts, R(0));
+  for (size_t t = 0; t < nt; ++t) {
+    R* o = &stn[t * ts];
+    const int off[3][2] = {{0, 1}, {0, 2}, {1, 2}};
+    for (int i = 0; i < 3; ++i) {
+      o[i] = R(tensor(t, 1, i, i).real() * 0.25);
+      o[3 + i] = R(tensor(t, 0, i, i).real() * 0.5);
+      const cd m = tensor(t, 1, off[i][0], off[i][1]) * 0.0625, q = tensor(t, 0, off[i][0], off[i][1]) * 0.25;
+      if (chiral) {
+        o[6 + i] = R(m.real());
+        o[9 + i] = R(q.real());
+      } else {
+        o[6 + 2 * i] = R(m.real());
+        o[7 + 2 * i] = R(m.imag());
+        o[12 + 2 * i] = R(q.real());
+        o[13 + 2 * i] = R(q.imag());
+      }
+      for (int j = 0; j < 3; ++j) {
+        const cd c = tensor(t, 2, i, j) * 0.125;
+        if (chiral) {
+          o[12 + i * 3 + j] = R(c.imag());
+        } else {
+          o[18 + 2 * (i * 3 + j)] = R(c.real());
+          o[19 + 2 * (i * 3 + j)] = R(c.imag());
         }
+      }
+    }
   }
   cudaError_t e;
   e = cudaMalloc(&d.lam, sizeof(cx<R>) * lam.size());
   if (e == cudaSuccess) e = cudaMalloc(&d.tau, sizeof(cx<R>) * tau.size());
   if (e == cudaSuccess) e = cudaMalloc(&d.sxyz, sizeof(cx<R>) * sx.size());
-  if (e == cudaSuccess) e = cudaMalloc(&d.mat, sizeof(cx<R>) * mat.size());
+  if (e == cudaSuccess) e = cudaMalloc(&d.stn, sizeof(R) * stn.size());
   if (e != cudaSuccess) return cuda_fail(&P, e, "plan tables");
   e = cudaMemcpy(d.lam, lam.data(), sizeof(cx<R>) * lam.size(), cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(d.tau, tau.data(), sizeof(cx<R>) * tau.size(), cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(d.sxyz, sx.data(), sizeof(cx<R>) * sx.size(), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(d.mat, mat.data(), sizeof(cx<R>) * mat.size(), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = cudaMemcpy(d.stn, stn.data(), sizeof(R) * stn.size(), cudaMemcpyHostToDevice);
   if (e != cudaSuccess) return cuda_fail(&P, e, "plan tables upload");
   // Pi table for complex128 only: there the transform kernels are bound by
   // GB300's FP64 rate and reading Pi (96 B per voxel) beats evaluating it
@@ -183,7 +213,7 @@ template <class R> void free_tables(PlanData<R>& d) {
   cudaFree(d.lam);
   cudaFree(d.tau);
   cudaFree(d.sxyz);
-  cudaFree(d.mat);
+  cudaFree(d.stn);
   cudaFree(d.pc);
   cudaFree(d.pi);
   cudaFree(d.fld);

@@ -79,12 +79,18 @@ struct TuneEntry {
   double us = 0.0;       // measured time of one fncB on the batch
 };
 
+// Kinds of vertex tensors and their stored sizes in reals (fncb_material.cuh).
+constexpr int kMatGeneral = 0, kMatChiral = 1, kMatField = 2;
+constexpr int kStnGeneral = 36, kStnChiral = 24;
+FAME_HD constexpr int stn_size(int kind) { return kind == kMatChiral ? kStnChiral : kStnGeneral; }
+
 // Device-side data of one precision.
 template <class R> struct PlanData {
   cx<R>* lam = nullptr;  // [nk][3n]  lambda_x | lambda_y | lambda_z  (QP symbols, delta = 1/n)
   cx<R>* tau = nullptr;  // [nk][3]   exp(i*theta_d/n): Bloch phase of one periodic shift
   cx<R>* sxyz = nullptr; // [nk][3n]  S_sDFT per axis (the MtxVecMul_FFT phase)
-  cx<R>* mat = nullptr;  // [nk][nphase][27]: Herm(N) | Herm(M) | J, row-major 3x3 each
+  R* stn = nullptr;      // [nk][nphase][stn_size(kind)] vertex tensors of the material stencil
+  int kind = kMatGeneral;
   cx<R>* pc = nullptr;   // [nk][8][Nq] CG preconditioner: inverse 4x4 Hermitian blocks, diagonal packed (lazy)
   cx<R>* pi = nullptr;   // [nk][Nq][6] Pi1 | Pi2 per frequency voxel (SVD_Matrix_curl.m:45-57); complex128 plans data only
   // Field mode (per-vertex isotropic chiral medium eps(r) I, mu = I,
@@ -165,6 +171,8 @@ struct Plan {
   std::vector<TuneEntry> tune;
 };
 
+// Vectors per launch sequence of a batch of nvec.
+inline int sub_batch(const TuneEntry& t, int nvec) { return t.chunk > 0 && t.chunk < nvec ? t.chunk : nvec; }
 // Tuned launch parameters for (prec, nvec), or the defaults.
 TuneEntry tune_for(const Plan& P, int prec, int nvec);
 // The tuning key of an arithmetic type (FAME_C64, FAME_C128, FAME_C128_DS).
@@ -228,11 +236,13 @@ cudaError_t launch_transform(const Plan& P, int trans, const cx<R>* x, cx<R>* y,
 template <class R>
 cudaError_t launch_handle(const Plan& P, int which, const cx<R>* x, cx<R>* y, int nvec,
                           const VecCtx& ctx, cx<R>* w0, cudaStream_t st);
-// Material stencil in place on periodic-frame 6-field vectors w (stride 6*Nq),
-// scratch h of the same size: w <- [M J^H; J N] w.
+// Material stencil on 6-field vectors (stride 6*Nq): out <- [M J^H; J N] w in
+// the periodic frame, or in the Bloch frame (bloch); out may be w, scratch h of
+// the same size.
 template <class R>
-cudaError_t launch_stencil(const Plan& P, cx<R>* w, cx<R>* h, int nvec, const VecCtx& ctx, cudaStream_t st);
-// Material operator alone on spatial 6-field vectors (periodic frame, no S):
+cudaError_t launch_stencil(const Plan& P, const cx<R>* w, cx<R>* out, cx<R>* h, int nvec, const VecCtx& ctx,
+                           cudaStream_t st, bool bloch = false);
+// Material operator alone on spatial 6-field vectors (Bloch frame):
 // [u'; v'] = [M J^H; J N] [u; v], the middle factor of fncB.
 template <class R>
 cudaError_t launch_material(const Plan& P, const cx<R>* uv, cx<R>* out, int nvec,

@@ -852,7 +852,7 @@ cudaError_t col(const PlanData<R>& d, cx<R>* w, int nfield, int nvec, long long 
 // kernels run with tpb threads per block.  Both come from fame_autotune.
 //
 // pq (may be null): with the single-pass stencil, per-CTA partial sums of
-// Re(x^H B x) (sweep_partials per vector, vector-major).  The curl-SVD
+// Re(x^H B x) (sweep_partials_n per vector, vector-major).  The curl-SVD
 // transforms are unitary and Pi has orthonormal columns, so x^H B x equals
 // w^H [M J^H; J N] w for the spatial fields w the stencil reads; the stencil
 // pass accumulates it while it writes its output.
@@ -868,7 +868,8 @@ cudaError_t fncB_n(const Plan& P, const cx<R>* x, cx<R>* y, int nvec, const VecC
   if (!P.opt_pi_table) d.pi = nullptr;  // evaluate Pi in the plane kernels instead
   const long long Nq = P.Nq;
   const TuneEntry tn = tune_for(P, tune_prec<R>(), nvec);
-  const int chunk = (tn.chunk > 0 && tn.chunk < nvec) ? tn.chunk : nvec;
+  const int chunk = sub_batch(tn, nvec);
+  const int tz = sweep_planes<R, N>(P, chunk);
   const int lanes = tn.lanes >= 0 ? tn.lanes : default_lanes<R, N>(P, nvec);
   for (int v0 = 0; v0 < nvec; v0 += chunk) {
     const int nv = std::min(chunk, nvec - v0);
@@ -888,10 +889,10 @@ cudaError_t fncB_n(const Plan& P, const cx<R>* x, cx<R>* y, int nvec, const VecC
     // material stencil: single pass w0 -> w1, or the two-kernel form in place on w0
     cx<R>* wm = w0;
     if (tn.stencil_tpb == 0) {
-      e = sweep_n<R, N>(P, w0, w1, nv, c, st, pq ? pq + (size_t)v0 * sweep_partials_n<R, N>() : nullptr);
+      e = sweep_n<R, N>(P, w0, w1, nv, c, st, tz, pq ? pq + (size_t)v0 * sweep_partials_n<R, N>(tz) : nullptr);
       wm = w1;
     } else {
-      e = stencil_n<R, N>(P, w0, w1, nv, c, st, tn.stencil_tpb);
+      e = stencil_n<R, N>(P, w0, w0, w1, nv, c, st, tn.stencil_tpb, false);
     }
     if (e != cudaSuccess) return e;
     e = col<R, N, -1, 0>(d, wm, 6, nv, 6 * Nq, c, st);
@@ -961,8 +962,8 @@ cudaError_t handle_n(const Plan& P, int which, const cx<R>* x, cx<R>* y, int nve
 #define FAME_SIZE_SIGS(PFX, R, NN)                                                                                 \
   PFX cudaError_t fame::detail::fncB_n<R, NN>(const Plan&, const cx<R>*, cx<R>*, int, const VecCtx&, cx<R>*,       \
                                               cx<R>*, cudaStream_t, double2*, const cx<R>*, const double*);       \
-  PFX cudaError_t fame::detail::stencil_n<R, NN>(const Plan&, cx<R>*, cx<R>*, int, const VecCtx&, cudaStream_t,    \
-                                                 int);                                                             \
+  PFX cudaError_t fame::detail::stencil_n<R, NN>(const Plan&, const cx<R>*, cx<R>*, cx<R>*, int, const VecCtx&,    \
+                                                 cudaStream_t, int, bool);                                         \
   PFX cudaError_t fame::detail::fields_inv_n<R, NN>(const Plan&, const cx<R>*, cx<R>*, int, const VecCtx&,         \
                                                     cudaStream_t);                                                 \
   PFX cudaError_t fame::detail::transform_n<R, NN>(const Plan&, int, const cx<R>*, cx<R>*, int, const VecCtx&,     \

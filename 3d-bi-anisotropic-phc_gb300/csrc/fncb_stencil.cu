@@ -7,24 +7,6 @@ namespace fame {
 namespace detail {
 
 
-// Multiply each 3Nq component block by S (conj when CONJ), in place.
-template <class R, bool CONJ>
-__global__ void k_phase(cx<R>* __restrict__ v, PlanData<R> d, VecCtx ctx, int n, int nfield,
-                        long long stride) {
-  const long long Nq = (long long)n * n * n;
-  const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const int vec = blockIdx.y;
-  if (idx >= Nq) return;
-  if (ctx.active && !ctx.active[vec]) return;
-  const int i1 = int(idx % n), i2 = int((idx / n) % n), i3 = int(idx / ((long long)n * n));
-  const cx<R>* S = d.sxyz + (long long)vec_inst(ctx, vec) * 3 * n;
-  cx<R> s = cmul(cmul(S[i1], S[n + i2]), S[2 * n + i3]);
-  for (int c = 0; c < nfield; ++c) {
-    cx<R>* p = v + vec * stride + (long long)c * Nq + idx;
-    *p = CONJ ? cmulc(s, *p) : cmul(s, *p);
-  }
-}
-
 // fncA.m:3-4: y = [ i/Sigma .* x2 ; -i/Sigma .* x1 ], Sigma = [sqrt(Lq); sqrt(Lq)].
 template <class R>
 __global__ void k_fncA(const cx<R>* __restrict__ x, cx<R>* __restrict__ y, PlanData<R> d, VecCtx ctx,
@@ -82,17 +64,16 @@ namespace fame {
 namespace detail {
 
 template <class R>
-cudaError_t stencil(const Plan& P, cx<R>* w, cx<R>* h, int nvec, const VecCtx& ctx, cudaStream_t st) {
+cudaError_t stencil(const Plan& P, const cx<R>* w, cx<R>* out, cx<R>* h, int nvec, const VecCtx& ctx, cudaStream_t st,
+                    bool bloch) {
   switch (P.n) {
-#define FAME_CASE(NN) case NN: return stencil_n<R, NN>(P, w, h, nvec, ctx, st, 256);
+#define FAME_CASE(NN) case NN: return stencil_n<R, NN>(P, w, out, h, nvec, ctx, st, 256, bloch);
     FAME_FOR_EACH_N(FAME_CASE)
 #undef FAME_CASE
     default: return cudaErrorInvalidValue;
   }
 }
 
-template cudaError_t stencil<float>(const Plan&, cx<float>*, cx<float>*, int, const VecCtx&, cudaStream_t);
-template cudaError_t stencil<double>(const Plan&, cx<double>*, cx<double>*, int, const VecCtx&, cudaStream_t);
 
 }  // namespace detail
 using namespace detail;
@@ -155,6 +136,19 @@ cudaError_t copy_to_ds(const double2* src, cff** dst, long long n, cudaStream_t 
   k_to_ds<<<dim3(conv_grid(n), 1), 256, 0, st>>>(src, *dst, n, nullptr);
   return cudaGetLastError();
 }
+cudaError_t copy_real_to_ds(const double* src, ff** dst, long long n, cudaStream_t st) {
+  if (!src) return cudaSuccess;
+  if (!*dst) {
+    cudaError_t e = cudaMalloc(dst, sizeof(ff) * (size_t)n);
+    if (e != cudaSuccess) {
+      *dst = nullptr;
+      return e;
+    }
+  }
+  FAME_LAUNCHED(1);
+  k_real_to_ds<<<conv_grid(n), 256, 0, st>>>(src, *dst, n);
+  return cudaGetLastError();
+}
 }  // namespace
 
 bool ds_supported(int n) {
@@ -176,16 +170,11 @@ int upload_tables_ds(Plan& P) {
   cudaError_t e = copy_to_ds(s.lam, &d.lam, (long long)P.nk * 3 * P.n, st);
   if (e == cudaSuccess) e = copy_to_ds(s.tau, &d.tau, (long long)P.nk * 3, st);
   if (e == cudaSuccess) e = copy_to_ds(s.sxyz, &d.sxyz, (long long)P.nk * 3 * P.n, st);
-  if (e == cudaSuccess) e = copy_to_ds(s.mat, &d.mat, (long long)P.nk * P.nphase * 27, st);
   if (e == cudaSuccess) e = copy_to_ds(s.pi, &d.pi, (long long)P.nk * 6 * P.Nq, st);
-  if (e == cudaSuccess && s.fld) {
-    if (!d.fld) e = cudaMalloc(&d.fld, sizeof(ff) * 3 * (size_t)P.Nq);
-    if (e == cudaSuccess) {
-      FAME_LAUNCHED(1);
-      k_real_to_ds<<<conv_grid(3 * P.Nq), 256, 0, st>>>(s.fld, d.fld, 3 * P.Nq);
-      e = cudaGetLastError();
-    }
-  }
+  if (e == cudaSuccess && s.kind != kMatField)
+    e = copy_real_to_ds(s.stn, &d.stn, (long long)P.nk * P.nphase * stn_size(s.kind), st);
+  if (e == cudaSuccess) e = copy_real_to_ds(s.fld, &d.fld, 3 * P.Nq, st);
+  d.kind = s.kind;
   for (int i = 0; i < 9; ++i) d.gram[i] = ff(s.gram[i]);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   return e == cudaSuccess ? FAME_OK : cuda_fail(&P, e, "double-single tables");
@@ -213,9 +202,10 @@ cudaError_t launch_fncB_ds(const Plan& P, const double2* x, double2* y, int nvec
 // 0 when the tuned form of that batch does not produce them.
 template <class R>
 int fncB_pq_partials(const Plan& P, int nvec) {
-  if (tune_for(P, tune_prec<R>(), nvec).stencil_tpb != 0) return 0;
+  const TuneEntry tn = tune_for(P, tune_prec<R>(), nvec);
+  if (tn.stencil_tpb != 0) return 0;
   switch (P.n) {
-#define FAME_CASE(NN) case NN: return sweep_partials_n<R, NN>();
+#define FAME_CASE(NN) case NN: return sweep_partials_n<R, NN>(sweep_planes<R, NN>(P, sub_batch(tn, nvec)));
     FAME_FOR_EACH_N(FAME_CASE)
 #undef FAME_CASE
     default: return 0;
@@ -252,9 +242,10 @@ cudaError_t launch_fncA(const Plan& P, const cx<R>* x, cx<R>* y, int nvec, const
 }
 
 template <class R>
-cudaError_t launch_stencil(const Plan& P, cx<R>* w, cx<R>* h, int nvec, const VecCtx& ctx, cudaStream_t st) {
+cudaError_t launch_stencil(const Plan& P, const cx<R>* w, cx<R>* out, cx<R>* h, int nvec, const VecCtx& ctx,
+                           cudaStream_t st, bool bloch) {
   if (nvec <= 0) return cudaSuccess;
-  return stencil<R>(P, w, h, nvec, ctx, st);
+  return stencil<R>(P, w, out, h, nvec, ctx, st, bloch);
 }
 
 template <class R>
@@ -296,22 +287,11 @@ cudaError_t launch_handle(const Plan& P, int which, const cx<R>* x, cx<R>* y, in
 template <class R>
 cudaError_t launch_material(const Plan& P, const cx<R>* uv, cx<R>* out, int nvec, const VecCtx& ctx, cx<R>* w1,
                             cudaStream_t st) {
-  // Bloch frame in and out: strip S, apply the periodic-frame stencil, restore S.
-  if (nvec <= 0) return cudaSuccess;
-  const long long s6 = 6 * P.Nq;
-  cudaError_t e;
-  if (out != uv) {
-    e = cudaMemcpyAsync(out, uv, sizeof(cx<R>) * s6 * nvec, cudaMemcpyDeviceToDevice, st);
-    if (e != cudaSuccess) return e;
-  }
-  const PlanData<R>& d = pdata<R>(P);
-  FAME_LAUNCHED(1);
-  k_phase<R, true><<<grid_pts1(P.Nq, nvec, 256), 256, 0, st>>>(out, d, ctx, P.n, 6, s6);
-  e = stencil<R>(P, out, w1, nvec, ctx, st);
-  if (e != cudaSuccess) return e;
-  FAME_LAUNCHED(1);
-  k_phase<R, false><<<grid_pts1(P.Nq, nvec, 256), 256, 0, st>>>(out, d, ctx, P.n, 6, s6);
-  return cudaGetLastError();
+  // The Bloch-frame operator is the same stencil with its phases at the wraps
+  // (the diagonal S that relates the frames cancels between neighbours), so S
+  // is never applied: two passes, against a copy, two phase passes and the
+  // stencil.
+  return launch_stencil<R>(P, uv, out, w1, nvec, ctx, st, true);
 }
 
 #define FAME_INST(R)                                                                                      \
@@ -322,7 +302,8 @@ cudaError_t launch_material(const Plan& P, const cx<R>* uv, cx<R>* out, int nvec
                                       cudaStream_t);                                                      \
   template cudaError_t launch_fields_inv<R>(const Plan&, const cx<R>*, cx<R>*, int, const VecCtx&,       \
                                             cudaStream_t);                                                \
-  template cudaError_t launch_stencil<R>(const Plan&, cx<R>*, cx<R>*, int, const VecCtx&, cudaStream_t); \
+  template cudaError_t launch_stencil<R>(const Plan&, const cx<R>*, cx<R>*, cx<R>*, int, const VecCtx&,  \
+                                         cudaStream_t, bool);                                             \
   template cudaError_t launch_transform<R>(const Plan&, int, const cx<R>*, cx<R>*, int, const VecCtx&,   \
                                            cudaStream_t);                                                 \
   template cudaError_t launch_handle<R>(const Plan&, int, const cx<R>*, cx<R>*, int, const VecCtx&,      \

@@ -178,7 +178,7 @@ extern "C" int fame_restore(fame_plan_t h, int nvec, const int* inst, const void
     if (e_ != cudaSuccess) return cuda_fail(&P, e_, what); \
   } while (0)
   RS_CK(launch_fields_inv<double>(P, (const double2*)x, w0, nvec, ctx, st), "fame_restore fields");
-  RS_CK(launch_stencil<double>(P, w0, w1, nvec, ctx, st), "fame_restore material");
+  RS_CK(launch_stencil<double>(P, w0, w0, w1, nvec, ctx, st), "fame_restore material");
   FAME_LAUNCHED(1);
   k_restore_fields<<<g, kT, 0, st>>>(w0, eh, Nq);
   RS_CK(cudaGetLastError(), "k_restore_fields");
@@ -190,7 +190,7 @@ extern "C" int fame_restore(fame_plan_t h, int nvec, const int* inst, const void
     FAME_LAUNCHED(1);
     k_curl_pair<<<g, kT, 0, st>>>(eh, w0, P.d64, ctx, P.n);
     RS_CK(cudaGetLastError(), "k_curl_pair");
-    RS_CK(launch_stencil<double>(P, w0, w1, nvec, ctx, st), "fame_restore residual material");
+    RS_CK(launch_stencil<double>(P, w0, w0, w1, nvec, ctx, st), "fame_restore residual material");
     const int nblk = 152;
     double* part = (double*)workspace(P, 48, sizeof(double) * 3 * nblk * nvec, &e);
     RS_CK(e, "fame_restore partials");
