@@ -25,9 +25,12 @@ TuneEntry tune_for(const Plan& P, int prec, int nvec) {
   TuneEntry d;
   d.prec = prec;
   d.nvec = nvec;
-  // complex64: single pass (two CTAs per SM); complex128 stages twice the
-  // bytes per plane and keeps the two-kernel form unless tuned otherwise
-  d.stencil_tpb = prec == FAME_C64 ? 0 : 256;
+  // complex64: single pass (bound by shared memory and latency); complex128
+  // and double-single are bound by arithmetic, and the two-kernel form does
+  // the least of it (no halo rows), in small blocks that spread evenly over
+  // the SMs (two vectors at n = 30, complex128: 143 us with blocks of 256,
+  // 136 with 128)
+  d.stencil_tpb = prec == FAME_C64 ? 0 : 128;
   return d;
 }
 

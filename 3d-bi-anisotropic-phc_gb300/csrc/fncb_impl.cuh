@@ -827,7 +827,7 @@ k_col2(cx<R>* __restrict__ w, VecCtx ctx, long long stride) {
 }
 
 template <class R, int N, int DIR, int SMODE>
-cudaError_t col(const PlanData<R>& d, cx<R>* w, int nfield, int nvec, long long stride, const VecCtx& ctx,
+cudaError_t col(const Plan& P, const PlanData<R>& d, cx<R>* w, int nfield, int nvec, long long stride, const VecCtx& ctx,
                 cudaStream_t st) {
   if constexpr (std::is_same<R, ff>::value && SMODE == 0 && plane_split(N) > 0) {
     constexpr int G = plane_split(N);
@@ -839,9 +839,14 @@ cudaError_t col(const PlanData<R>& d, cx<R>* w, int nfield, int nvec, long long 
     kfn<<<dim3(N, nfield, nvec), ((N * G + 31) / 32) * 32, sm, st>>>(w, ctx, stride);
     return cudaGetLastError();
   } else {
-    dim3 g((N * N + 127) / 128, nfield, nvec);
+    // One warp per CTA in complex128 and for small complex64 batches: the work
+    // of a launch is then spread over the SMs warp by warp (two vectors at
+    // n = 30 are 96 CTAs of four warps, up to four warps on an SM where the
+    // even share is 2.2: 23 -> 16 us), 128 threads where there are plenty.
+    const int tpb = sizeof(R) == 8 || (long long)N * N * nfield * nvec < 128LL * 6 * P.sms ? 32 : 128;
+    dim3 g((N * N + tpb - 1) / tpb, nfield, nvec);
     FAME_LAUNCHED(1);
-    k_col<R, N, DIR, SMODE><<<g, 128, 0, st>>>(w, d, ctx, stride);
+    k_col<R, N, DIR, SMODE><<<g, tpb, 0, st>>>(w, d, ctx, stride);
     return cudaGetLastError();
   }
 }
@@ -884,7 +889,7 @@ cudaError_t fncB_n(const Plan& P, const cx<R>* x, cx<R>* y, int nvec, const VecC
     }
     e = plane_inv<R, N, true, false>(P, d, xs, w0, nv, 2, 0, 4 * Nq, 2 * Nq, 6 * Nq, c, st, upd, lanes);
     if (e != cudaSuccess) return e;
-    e = col<R, N, +1, 0>(d, w0, 6, nv, 6 * Nq, c, st);
+    e = col<R, N, +1, 0>(P, d, w0, 6, nv, 6 * Nq, c, st);
     if (e != cudaSuccess) return e;
     // material stencil: single pass w0 -> w1, or the two-kernel form in place on w0
     cx<R>* wm = w0;
@@ -895,7 +900,7 @@ cudaError_t fncB_n(const Plan& P, const cx<R>* x, cx<R>* y, int nvec, const VecC
       e = stencil_n<R, N>(P, w0, w0, w1, nv, c, st, tn.stencil_tpb, false);
     }
     if (e != cudaSuccess) return e;
-    e = col<R, N, -1, 0>(d, wm, 6, nv, 6 * Nq, c, st);
+    e = col<R, N, -1, 0>(P, d, wm, 6, nv, 6 * Nq, c, st);
     if (e != cudaSuccess) return e;
     e = plane_fwd<R, N, true, false>(P, d, wm, ys, nv, 2, 0, 6 * Nq, 4 * Nq, 2 * Nq, c, st, lanes);
     if (e != cudaSuccess) return e;
@@ -909,7 +914,7 @@ cudaError_t fields_inv_n(const Plan& P, const cx<R>* x, cx<R>* w, int nvec, cons
   const long long Nq = P.Nq;
   cudaError_t e = plane_inv<R, N, true, false>(P, d, x, w, nvec, 2, 0, 4 * Nq, 2 * Nq, 6 * Nq, ctx, st);
   if (e != cudaSuccess) return e;
-  return col<R, N, +1, 0>(d, w, 6, nvec, 6 * Nq, ctx, st);
+  return col<R, N, +1, 0>(P, d, w, 6, nvec, 6 * Nq, ctx, st);
 }
 
 template <class R, int N>
@@ -921,14 +926,14 @@ cudaError_t transform_n(const Plan& P, int trans, const cx<R>* x, cx<R>* y, int 
   if (trans == 0) {
     e = plane_inv<R, N, false, true>(P, d, x, y, nvec, 1, 0, 3 * Nq, 0, 3 * Nq, ctx, st);
     if (e != cudaSuccess) return e;
-    return col<R, N, +1, 1>(d, y, 3, nvec, 3 * Nq, ctx, st);
+    return col<R, N, +1, 1>(P, d, y, 3, nvec, 3 * Nq, ctx, st);
   }
   // transpose: z first (conj(S_z) before), then y, x with conj(S_x S_y) before.
   if (x != y) {
     e = cudaMemcpyAsync(y, x, sizeof(cx<R>) * 3 * Nq * nvec, cudaMemcpyDeviceToDevice, st);
     if (e != cudaSuccess) return e;
   }
-  e = col<R, N, -1, 2>(d, y, 3, nvec, 3 * Nq, ctx, st);
+  e = col<R, N, -1, 2>(P, d, y, 3, nvec, 3 * Nq, ctx, st);
   if (e != cudaSuccess) return e;
   return plane_fwd<R, N, false, true>(P, d, y, y, nvec, 1, 0, 3 * Nq, 3 * Nq, 0, ctx, st);
 }
@@ -942,12 +947,12 @@ cudaError_t handle_n(const Plan& P, int which, const cx<R>* x, cx<R>* y, int nve
   if (which == 0 || which == 1) {  // Pr / Qr : 2Nq -> 3Nq
     e = plane_inv<R, N, true, true>(P, d, x, y, nvec, 1, which, 2 * Nq, 0, 3 * Nq, ctx, st);
     if (e != cudaSuccess) return e;
-    return col<R, N, +1, 1>(d, y, 3, nvec, 3 * Nq, ctx, st);
+    return col<R, N, +1, 1>(P, d, y, 3, nvec, 3 * Nq, ctx, st);
   }
   // Prs / Qrs : 3Nq -> 2Nq through the 3Nq scratch w0
   e = cudaMemcpyAsync(w0, x, sizeof(cx<R>) * 3 * Nq * nvec, cudaMemcpyDeviceToDevice, st);
   if (e != cudaSuccess) return e;
-  e = col<R, N, -1, 2>(d, w0, 3, nvec, 3 * Nq, ctx, st);
+  e = col<R, N, -1, 2>(P, d, w0, 3, nvec, 3 * Nq, ctx, st);
   if (e != cudaSuccess) return e;
   return plane_fwd<R, N, true, true>(P, d, w0, y, nvec, 1, which - 2, 3 * Nq, 2 * Nq, 0, ctx, st);
 }

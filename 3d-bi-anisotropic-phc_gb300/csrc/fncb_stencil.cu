@@ -67,7 +67,7 @@ template <class R>
 cudaError_t stencil(const Plan& P, const cx<R>* w, cx<R>* out, cx<R>* h, int nvec, const VecCtx& ctx, cudaStream_t st,
                     bool bloch) {
   switch (P.n) {
-#define FAME_CASE(NN) case NN: return stencil_n<R, NN>(P, w, out, h, nvec, ctx, st, 256, bloch);
+#define FAME_CASE(NN) case NN: return stencil_n<R, NN>(P, w, out, h, nvec, ctx, st, 128, bloch);
     FAME_FOR_EACH_N(FAME_CASE)
 #undef FAME_CASE
     default: return cudaErrorInvalidValue;

@@ -33,27 +33,16 @@ enum WsId {
     if (e_ != cudaSuccess) return cuda_fail(&P, e_, where); \
   } while (0)
 
-static int device_sms(int dev) {
-  static std::atomic<int> cache[64];
-  if (dev < 0 || dev >= 64) dev = 0;
-  int v = cache[dev].load(std::memory_order_relaxed);
-  if (v <= 0) {
-    if (cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v <= 0) v = 152;
-    cache[dev].store(v, std::memory_order_relaxed);
-  }
-  return v;
-}
-
 // CTAs per vector of the grid-stride reduction and update kernels: together
 // at most four per SM (one wave at four resident CTAs, two at two), so that
-// no CTA of a batch waits for a partial last wave.
+// no CTA of a batch waits for a partial last wave, and no more than one
+// element per thread.  (A floor of eight elements per thread left 28 CTAs for
+// two vectors at n = 30, and the complex128 update at 71 us of a 290 us CG
+// iteration; one element per thread: 25 us.)
 static int dot_blocks(const Plan& P, long long len, int nvec) {
-  long long target = std::max(1, 4 * device_sms(P.device) / std::max(1, nvec));
-  long long maxb = (len + 2047) / 2048;
-  long long b = std::min(target, maxb);
-  if (b < 1) b = 1;
-  if (b > 512) b = 512;
-  return int(b);
+  const long long target = std::max(1, 4 * P.sms / std::max(1, nvec));
+  const long long b = std::min(target, (len + 255) / 256);
+  return (int)std::max(1LL, std::min(512LL, b));
 }
 
 // Device scalars of the batched CG, carved from one workspace.
