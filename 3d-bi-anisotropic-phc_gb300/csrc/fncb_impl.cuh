@@ -117,6 +117,106 @@ __device__ __forceinline__ PiBlock<R> pi_at(const PlanData<R>& d, int inst, int 
   return pi_block<R>(lam[i1], lam[N + i2], lz);
 }
 
+// Pi of the voxels of one frequency plane (k3 fixed) in complex64, where the
+// plane kernels evaluate it.  With m = L x w (w = (1,2,3)/sqrt(14)) and
+// q = m x conj(L):
+//   Pi1 = conj(m)/|m|,  Pi2 = q/(|m| |L|),
+// and m_0, m_1, their products with conj(L) and the squared norms depend on
+// one of (i2, k3), (i1, k3) only: a row table in shared memory (PiRow) and
+// registers of a thread that stays in one column (PiCol) hold them, which
+// leaves 16 operations and two reciprocal square roots per voxel before the
+// products with the vectors (the blocks took about 100, 40 % of the kernels'
+// instructions; at n = 60, 10 vectors, k_plane_inv 26.3 -> 19.4 M warp
+// instructions, 58 -> 47 us).  |m|^2 as a sum of squares also has no
+// cancellation: fncB's error against 64 bits 3.5e-7 -> 2.2e-7.
+//
+// Side 0 (Pr) takes the same formulas with conj(L) for L and the two blocks
+// swapped:  side 1: v = conj(m) X + q Y with X = a/|m|, Y = b/(|m||L|);
+//           side 0: the same with X = b/|m|, Y = -a/(|m||L|).
+struct PiRow {
+  float2 ly, m0, t1, t2;  // L_y, m_0, m_0 conj(L_z), m_0 conj(L_y)
+  float lq, n1;           // |L_y|^2, |m_0|^2
+  float2 pad;
+};
+struct PiCol {
+  float2 w2lx, lx, m1, k1, k2;  // w_2 L_x, L_x, m_1, m_1 conj(L_z), m_1 conj(L_x)
+  float lq, n1;                 // |L_x|^2 + |L_z|^2, |m_1|^2
+};
+struct PiVox {
+  float2 m0, m1, m2, q0, q1, q2;
+  float inv1, i01;  // 1/|m|, 1/(|m||L|)
+};
+__device__ __forceinline__ float2 side_conj(float2 v, int side) { return side ? v : cconj(v); }
+template <int N>
+__device__ __forceinline__ void pi_row_fill(PiRow* rows, const float2* lam, int k3, int side, int i2) {
+  const float2 lz = side_conj(lam[2 * N + k3], side), ly = side_conj(lam[N + i2], side);
+  const float w2 = float(2 * kInvSqrt14), w3 = float(3 * kInvSqrt14);
+  PiRow r;
+  r.ly = ly;
+  r.m0 = caxpy(-w2, lz, cscale(ly, w3));
+  r.t1 = cmulc(lz, r.m0);
+  r.t2 = cmulc(ly, r.m0);
+  r.lq = ly.x * ly.x + ly.y * ly.y;
+  r.n1 = r.m0.x * r.m0.x + r.m0.y * r.m0.y;
+  r.pad = make_float2(0.f, 0.f);
+  rows[i2] = r;
+}
+template <int N> __device__ __forceinline__ PiCol pi_col(const float2* lam, int k3, int side, int i1) {
+  const float2 lz = side_conj(lam[2 * N + k3], side);
+  const float w1 = float(1 * kInvSqrt14), w2 = float(2 * kInvSqrt14), w3 = float(3 * kInvSqrt14);
+  PiCol c;
+  c.lx = side_conj(lam[i1], side);
+  c.w2lx = cscale(c.lx, w2);
+  c.m1 = caxpy(-w3, c.lx, cscale(lz, w1));
+  c.k1 = cmulc(lz, c.m1);
+  c.k2 = cmulc(c.lx, c.m1);
+  c.lq = c.lx.x * c.lx.x + c.lx.y * c.lx.y + lz.x * lz.x + lz.y * lz.y;
+  c.n1 = c.m1.x * c.m1.x + c.m1.y * c.m1.y;
+  return c;
+}
+__device__ __forceinline__ PiVox pi_vox(const PiRow* row, const PiCol& c) {
+  const float4* q = reinterpret_cast<const float4*>(row);
+  const float4 a = q[0], b = q[1], n = q[2];
+  const float2 ly = make_float2(a.x, a.y), t1 = make_float2(b.x, b.y), t2 = make_float2(b.z, b.w);
+  PiVox v;
+  v.m0 = make_float2(a.z, a.w);
+  v.m1 = c.m1;
+  v.m2 = caxpy(-float(kInvSqrt14), ly, c.w2lx);
+  v.q0 = csub(c.k1, cmulc(ly, v.m2));
+  v.q1 = csub(cmulc(c.lx, v.m2), t1);
+  v.q2 = csub(t2, c.k2);
+  const float n1 = fmaf(v.m2.x, v.m2.x, fmaf(v.m2.y, v.m2.y, n.y + c.n1));
+  v.inv1 = rsqrtf(n1);
+  v.i01 = v.inv1 * rsqrtf(n.x + c.lq);
+  return v;
+}
+// (a, b) of one side -> the three frequency components (Pi.Pr / Pi.Qr)
+__device__ __forceinline__ void pi_prep(const PiVox& P, int side, float2 a, float2 b, float sc, float2 (&v)[3]) {
+  const float s1 = P.inv1 * sc, s2 = P.i01 * sc;
+  const float2 X = cscale(side ? a : b, s1), Y = cscale(side ? b : a, side ? s2 : -s2);
+  v[0] = cfma(P.q0, Y, cmulc(P.m0, X));
+  v[1] = cfma(P.q1, Y, cmulc(P.m1, X));
+  v[2] = cfma(P.q2, Y, cmulc(P.m2, X));
+}
+// the adjoint: three components -> (a, b)
+__device__ __forceinline__ void pi_post(const PiVox& P, int side, const float2 (&u)[3], float sc, float2& a, float2& b) {
+  const float s1 = P.inv1 * sc, s2 = P.i01 * sc;
+  const float2 X = cscale(cfma(P.m2, u[2], cfma(P.m1, u[1], cmul(P.m0, u[0]))), s1);
+  const float2 Y = cscale(cfmac(P.q2, u[2], cfmac(P.q1, u[1], cmulc(P.q0, u[0]))), side ? s2 : -s2);
+  a = side ? X : Y;
+  b = side ? Y : X;
+}
+
+// Bytes of shared memory of the plane kernels: three padded fields, and the
+// row table in complex64.
+template <class R, int N> constexpr size_t plane_smem() {
+  return sizeof(cx<R>) * 3 * N * (N + 1) + (sizeof(R) == 4 ? sizeof(PiRow) * N : 0);
+}
+// The row table's place behind the fields (16-byte aligned: N is even).
+template <class R, int N> __device__ __forceinline__ PiRow* pi_rows(cx<R>* sm) {
+  return reinterpret_cast<PiRow*>(sm + 3 * N * (N + 1));
+}
+
 // Scale of a unitary 3D DFT, n^{-3/2}.  The S-free transforms of fncB put all of
 // it on the plane kernels' frequency side (two blocks per voxel and side), so
 // the z pass multiplies by nothing.
@@ -182,23 +282,29 @@ k_plane_inv(const cx<R>* __restrict__ x, cx<R>* __restrict__ out, PlanData<R> d,
   const cx<R>* xin = x + vec * in_stride + blockIdx.y * in_side_stride + (long long)k3 * N * N;
   const int tid = threadIdx.x;
 
-  // Input plane -> shared memory.  The global loads of PF elements per thread
-  // are issued together before any is used, so a CTA waits for one memory
-  // round trip per batch instead of one per element.
-  constexpr int T = ((3 * N + 31) / 32) * 32;
-  constexpr int ITEMS = (N * N + T - 1) / T;
+  // Input plane -> shared memory: thread (column i1, row group) takes rows
+  // grp, grp + 3, ...  The global loads of PF rows are issued together before
+  // any is used, so a CTA waits for one memory round trip per batch.
+  constexpr bool PIV = PREP && sizeof(R) == 4;
+  const int grp = tid / N, i1 = tid - grp * N;
+  const bool act = tid < 3 * N;
+  if constexpr (PIV) {
+    if (tid < N) pi_row_fill<N>(pi_rows<R, N>(sm), lam, k3, side, tid);
+  }
+  constexpr int ITEMS = (N + 2) / 3;
   constexpr int NB = PREP ? 2 : 3;                        // input blocks
-  constexpr int PF0 = (sizeof(R) == 4 ? 24 : 12) / NB;   // elements in flight per thread
-  constexpr int PF = PF0 < ITEMS ? PF0 : ITEMS;
-  static_for<0, (ITEMS + PF - 1) / PF>([&](auto bc) {
+  constexpr int PF0 = (sizeof(R) == 4 ? 24 : 12) / NB;   // rows in flight per thread
+  constexpr int NBATCH = (ITEMS + PF0 - 1) / PF0;
+  constexpr int PF = (ITEMS + NBATCH - 1) / NBATCH;
+  static_for<0, NBATCH>([&](auto bc) {
     constexpr int base = decltype(bc)::value * PF;
     cx<R> in[PF][NB];
 #pragma unroll
     for (int it = 0; it < PF; ++it) {
-      const int e = tid + (base + it) * T;
-      if (base + it < ITEMS && e < N * N) {
+      const int i2 = grp + 3 * (base + it);
+      if (act && i2 < N) {
 #pragma unroll
-        for (int c = 0; c < NB; ++c) in[it][c] = xin[c * Nq + e];
+        for (int c = 0; c < NB; ++c) in[it][c] = xin[c * Nq + i2 * N + i1];
       }
     }
     if (PREP && upd.z) {  // p = z + beta p, written back
@@ -206,49 +312,74 @@ k_plane_inv(const cx<R>* __restrict__ x, cx<R>* __restrict__ out, PlanData<R> d,
       const cx<R>* zin = upd.z + off;
       cx<R>* xw = const_cast<cx<R>*>(x) + off;
       const R bt = R(upd.beta[vec]);
+      cx<R> zz[PF][NB];
 #pragma unroll
       for (int it = 0; it < PF; ++it) {
-        const int e = tid + (base + it) * T;
-        if (base + it < ITEMS && e < N * N) {
+        const int i2 = grp + 3 * (base + it);
+        if (act && i2 < N) {
+#pragma unroll
+          for (int c = 0; c < NB; ++c) zz[it][c] = zin[c * Nq + i2 * N + i1];
+        }
+      }
+#pragma unroll
+      for (int it = 0; it < PF; ++it) {
+        const int i2 = grp + 3 * (base + it);
+        if (act && i2 < N) {
 #pragma unroll
           for (int c = 0; c < NB; ++c) {
-            const cx<R> zz = zin[c * Nq + e];
-            in[it][c] = mk<R>(zz.x + bt * in[it][c].x, zz.y + bt * in[it][c].y);
-            xw[c * Nq + e] = in[it][c];
+            in[it][c] = caxpy(bt, in[it][c], zz[it][c]);
+            xw[c * Nq + i2 * N + i1] = in[it][c];
           }
         }
       }
     }
+    if constexpr (PIV && decltype(bc)::value == 0) __syncthreads();  // the row table
+    if (act) {
+      if constexpr (PIV) {
+        const PiCol pc = pi_col<N>(lam, k3, side, i1);
 #pragma unroll
-    for (int it = 0; it < PF; ++it) {
-      const int e = tid + (base + it) * T;
-      if (base + it < ITEMS && e < N * N) {
-        const int i2 = e / N, i1 = e - i2 * N;
-        cx<R> v0, v1, v2;
-        if constexpr (PREP) {
-          PiBlock<R> P = pi_at<R, N>(d, inst, k3, e, lam, i1, i2, lam[2 * N + k3]);
-          cx<R> a = in[it][0], b = in[it][1];
-          if constexpr (!WITH_S) {
-            a = cscale(a, scale3<R, N>());
-            b = cscale(b, scale3<R, N>());
+        for (int it = 0; it < PF; ++it) {
+          const int i2 = grp + 3 * (base + it);
+          if (i2 < N) {
+            cx<R> v[3];
+            pi_prep(pi_vox(pi_rows<R, N>(sm) + i2, pc), side, in[it][0], in[it][1],
+                    WITH_S ? R(1) : scale3<R, N>(), v);
+#pragma unroll
+            for (int c = 0; c < 3; ++c) sm[(c * N + i2) * LD + i1] = v[c];
           }
-          if (side == 0) {
-            v0 = cfmac(P.p1[0], b, cneg(cmulc(P.p2[0], a)));
-            v1 = cfmac(P.p1[1], b, cneg(cmulc(P.p2[1], a)));
-            v2 = cfmac(P.p1[2], b, cneg(cmulc(P.p2[2], a)));
-          } else {
-            v0 = cfma(P.p2[0], b, cmul(P.p1[0], a));
-            v1 = cfma(P.p2[1], b, cmul(P.p1[1], a));
-            v2 = cfma(P.p2[2], b, cmul(P.p1[2], a));
-          }
-        } else {
-          v0 = in[it][0];
-          v1 = in[it][1];
-          v2 = in[it][NB - 1];
         }
-        sm[(0 * N + i2) * LD + i1] = v0;
-        sm[(1 * N + i2) * LD + i1] = v1;
-        sm[(2 * N + i2) * LD + i1] = v2;
+      } else {
+#pragma unroll
+        for (int it = 0; it < PF; ++it) {
+          const int i2 = grp + 3 * (base + it);
+          if (i2 < N) {
+            cx<R> v0, v1, v2;
+            if constexpr (PREP) {
+              PiBlock<R> P = pi_at<R, N>(d, inst, k3, i2 * N + i1, lam, i1, i2, lam[2 * N + k3]);
+              cx<R> a = in[it][0], b = in[it][1];
+              if constexpr (!WITH_S) {
+                a = cscale(a, scale3<R, N>());
+                b = cscale(b, scale3<R, N>());
+              }
+              if (side == 0) {
+                v0 = cfmac(P.p1[0], b, cneg(cmulc(P.p2[0], a)));
+                v1 = cfmac(P.p1[1], b, cneg(cmulc(P.p2[1], a)));
+                v2 = cfmac(P.p1[2], b, cneg(cmulc(P.p2[2], a)));
+              } else {
+                v0 = cfma(P.p2[0], b, cmul(P.p1[0], a));
+                v1 = cfma(P.p2[1], b, cmul(P.p1[1], a));
+                v2 = cfma(P.p2[2], b, cmul(P.p1[2], a));
+              }
+            } else {
+              v0 = in[it][0];
+              v1 = in[it][1];
+              v2 = in[it][NB - 1];
+            }
+            sm[(0 * N + i2) * LD + i1] = v0;
+            sm[(1 * N + i2) * LD + i1] = v1;
+            sm[(2 * N + i2) * LD + i1] = v2;
+          }
+        }
       }
     }
   });
@@ -307,6 +438,10 @@ k_plane_fwd(const cx<R>* __restrict__ w, cx<R>* __restrict__ y, PlanData<R> d, V
   const long long Nq = (long long)N * N * N;
   const int tid = threadIdx.x;
   const cx<R>* S = d.sxyz + (long long)inst * 3 * N;
+  const cx<R>* lam = d.lam + (long long)inst * 3 * N;
+  if constexpr (POST && sizeof(R) == 4) {
+    if (tid < N) pi_row_fill<N>(pi_rows<R, N>(sm), lam, k3, side, tid);
+  }
   if (tid < 3 * N) {  // y columns
     const int c = tid / N, i1 = tid - c * N;
     const cx<R>* src = w + vec * w_stride + (long long)(blockIdx.y * 3 + c) * Nq + (long long)k3 * N * N + i1;
@@ -334,35 +469,48 @@ k_plane_fwd(const cx<R>* __restrict__ w, cx<R>* __restrict__ y, PlanData<R> d, V
     for (int i = 0; i < N; ++i) row[i] = v[i];
   }
   __syncthreads();
-  const cx<R>* lam = d.lam + (long long)inst * 3 * N;
   cx<R>* o = y + vec * out_stride + blockIdx.y * out_side_stride + (long long)k3 * N * N;
-  constexpr int T = ((3 * N + 31) / 32) * 32;
+  if (tid < 3 * N) {
+    const int grp = tid / N, i1 = tid - grp * N;
+    if constexpr (POST && sizeof(R) == 4) {
+      const PiCol pc = pi_col<N>(lam, k3, side, i1);
 #pragma unroll 4
-  for (int e = tid; e < N * N; e += T) {
-    const int i2 = e / N, i1 = e - i2 * N;
-    cx<R> u0 = sm[(0 * N + i2) * LD + i1];
-    cx<R> u1 = sm[(1 * N + i2) * LD + i1];
-    cx<R> u2 = sm[(2 * N + i2) * LD + i1];
-    if constexpr (POST) {
-      PiBlock<R> P = pi_at<R, N>(d, inst, k3, e, lam, i1, i2, lam[2 * N + k3]);
-      cx<R> a, b;
-      if (side == 0) {
-        a = cneg(cfma(P.p2[2], u2, cfma(P.p2[1], u1, cmul(P.p2[0], u0))));
-        b = cfma(P.p1[2], u2, cfma(P.p1[1], u1, cmul(P.p1[0], u0)));
-      } else {
-        a = cfmac(P.p1[2], u2, cfmac(P.p1[1], u1, cmulc(P.p1[0], u0)));
-        b = cfmac(P.p2[2], u2, cfmac(P.p2[1], u1, cmulc(P.p2[0], u0)));
+      for (int i2 = grp; i2 < N; i2 += 3) {
+        const cx<R> u[3] = {sm[(0 * N + i2) * LD + i1], sm[(1 * N + i2) * LD + i1], sm[(2 * N + i2) * LD + i1]};
+        cx<R> a, b;
+        pi_post(pi_vox(pi_rows<R, N>(sm) + i2, pc), side, u, WITH_S ? R(1) : scale3<R, N>(), a, b);
+        o[i2 * N + i1] = a;
+        o[Nq + i2 * N + i1] = b;
       }
-      if constexpr (!WITH_S) {
-        a = cscale(a, scale3<R, N>());
-        b = cscale(b, scale3<R, N>());
-      }
-      o[e] = a;
-      o[Nq + e] = b;
     } else {
-      o[e] = u0;
-      o[Nq + e] = u1;
-      o[2 * Nq + e] = u2;
+#pragma unroll 4
+      for (int i2 = grp; i2 < N; i2 += 3) {
+        const int e = i2 * N + i1;
+        cx<R> u0 = sm[(0 * N + i2) * LD + i1];
+        cx<R> u1 = sm[(1 * N + i2) * LD + i1];
+        cx<R> u2 = sm[(2 * N + i2) * LD + i1];
+        if constexpr (POST) {
+          PiBlock<R> P = pi_at<R, N>(d, inst, k3, e, lam, i1, i2, lam[2 * N + k3]);
+          cx<R> a, b;
+          if (side == 0) {
+            a = cneg(cfma(P.p2[2], u2, cfma(P.p2[1], u1, cmul(P.p2[0], u0))));
+            b = cfma(P.p1[2], u2, cfma(P.p1[1], u1, cmul(P.p1[0], u0)));
+          } else {
+            a = cfmac(P.p1[2], u2, cfmac(P.p1[1], u1, cmulc(P.p1[0], u0)));
+            b = cfmac(P.p2[2], u2, cfmac(P.p2[1], u1, cmulc(P.p2[0], u0)));
+          }
+          if constexpr (!WITH_S) {
+            a = cscale(a, scale3<R, N>());
+            b = cscale(b, scale3<R, N>());
+          }
+          o[e] = a;
+          o[Nq + e] = b;
+        } else {
+          o[e] = u0;
+          o[Nq + e] = u1;
+          o[2 * Nq + e] = u2;
+        }
+      }
     }
   }
 }
@@ -458,16 +606,22 @@ k_plane_inv2(const cx<R>* __restrict__ x, cx<R>* __restrict__ out, PlanData<R> d
   const cx<R>* xin = x + vec * in_stride + blockIdx.y * in_side_stride + (long long)k3 * N * N;
   const int tid = threadIdx.x;
   // Pi blocks (frequency voxel -> 3 components of this side), scaled for the
-  // three inverse DFTs; all loads of a thread issued together.
+  // three inverse DFTs: thread (column i1, row group) takes every NG-th row;
+  // all loads of a thread issued together.
   {
-    constexpr int ITEMS = (N * N + T - 1) / T;
+    constexpr int NG = 3 * G;
+    constexpr int ITEMS = (N + NG - 1) / NG;
+    const int grp = tid / N, i1 = tid - grp * N;
+    if constexpr (sizeof(R) == 4) {
+      if (tid < N) pi_row_fill<N>(pi_rows<R, N>(sm), lam, k3, side, tid);
+    }
     cx<R> in[ITEMS][2];
 #pragma unroll
     for (int it = 0; it < ITEMS; ++it) {
-      const int e = tid + it * T;
-      if (tid < T && e < N * N) {
-        in[it][0] = load_io<R>(xin + e);
-        in[it][1] = load_io<R>(xin + Nq + e);
+      const int i2 = grp + it * NG;
+      if (tid < T && i2 < N) {
+        in[it][0] = load_io<R>(xin + i2 * N + i1);
+        in[it][1] = load_io<R>(xin + Nq + i2 * N + i1);
       }
     }
     if constexpr (UPD) {  // p = z + beta p, written back (UPD: upd.z set)
@@ -477,39 +631,54 @@ k_plane_inv2(const cx<R>* __restrict__ x, cx<R>* __restrict__ out, PlanData<R> d
       const R bt = R(upd.beta[vec]);
 #pragma unroll
       for (int it = 0; it < ITEMS; ++it) {
-        const int e = tid + it * T;
-        if (tid < T && e < N * N) {
+        const int i2 = grp + it * NG;
+        if (tid < T && i2 < N) {
 #pragma unroll
           for (int c = 0; c < 2; ++c) {
-            const cx<R> zz = zin[c * Nq + e];
-            in[it][c] = mk<R>(zz.x + bt * in[it][c].x, zz.y + bt * in[it][c].y);
-            xw[c * Nq + e] = in[it][c];
+            in[it][c] = caxpy(bt, in[it][c], zin[c * Nq + i2 * N + i1]);
+            xw[c * Nq + i2 * N + i1] = in[it][c];
           }
         }
       }
     }
     const R sc = scale3<R, N>();
-    const cx<R> lz = lam[2 * N + k3];
+    if constexpr (sizeof(R) == 4) {
+      __syncthreads();  // the row table
+      if (tid < T) {
+        const PiCol pc = pi_col<N>(lam, k3, side, i1);
 #pragma unroll
-    for (int it = 0; it < ITEMS; ++it) {
-      const int e = tid + it * T;
-      if (tid < T && e < N * N) {
-        const int i2 = e / N, i1 = e - i2 * N;
-        PiBlock<R> P = pi_at<R, N>(d, inst, k3, e, lam, i1, i2, lz);
-        const cx<R> a = cscale(in[it][0], sc), b = cscale(in[it][1], sc);
-        cx<R> v0, v1, v2;
-        if (side == 0) {
-          v0 = cfmac(P.p1[0], b, cneg(cmulc(P.p2[0], a)));
-          v1 = cfmac(P.p1[1], b, cneg(cmulc(P.p2[1], a)));
-          v2 = cfmac(P.p1[2], b, cneg(cmulc(P.p2[2], a)));
-        } else {
-          v0 = cfma(P.p2[0], b, cmul(P.p1[0], a));
-          v1 = cfma(P.p2[1], b, cmul(P.p1[1], a));
-          v2 = cfma(P.p2[2], b, cmul(P.p1[2], a));
+        for (int it = 0; it < ITEMS; ++it) {
+          const int i2 = grp + it * NG;
+          if (i2 < N) {
+            cx<R> v[3];
+            pi_prep(pi_vox(pi_rows<R, N>(sm) + i2, pc), side, in[it][0], in[it][1], sc, v);
+#pragma unroll
+            for (int c = 0; c < 3; ++c) sm[(c * N + i2) * LD + i1] = v[c];
+          }
         }
-        sm[(0 * N + i2) * LD + i1] = v0;
-        sm[(1 * N + i2) * LD + i1] = v1;
-        sm[(2 * N + i2) * LD + i1] = v2;
+      }
+    } else {
+      const cx<R> lz = lam[2 * N + k3];
+#pragma unroll
+      for (int it = 0; it < ITEMS; ++it) {
+        const int i2 = grp + it * NG;
+        if (tid < T && i2 < N) {
+          PiBlock<R> P = pi_at<R, N>(d, inst, k3, i2 * N + i1, lam, i1, i2, lz);
+          const cx<R> a = cscale(in[it][0], sc), b = cscale(in[it][1], sc);
+          cx<R> v0, v1, v2;
+          if (side == 0) {
+            v0 = cfmac(P.p1[0], b, cneg(cmulc(P.p2[0], a)));
+            v1 = cfmac(P.p1[1], b, cneg(cmulc(P.p2[1], a)));
+            v2 = cfmac(P.p1[2], b, cneg(cmulc(P.p2[2], a)));
+          } else {
+            v0 = cfma(P.p2[0], b, cmul(P.p1[0], a));
+            v1 = cfma(P.p2[1], b, cmul(P.p1[1], a));
+            v2 = cfma(P.p2[2], b, cmul(P.p1[2], a));
+          }
+          sm[(0 * N + i2) * LD + i1] = v0;
+          sm[(1 * N + i2) * LD + i1] = v1;
+          sm[(2 * N + i2) * LD + i1] = v2;
+        }
       }
     }
   }
@@ -562,6 +731,10 @@ k_plane_fwd2(const cx<R>* __restrict__ w, cx<R>* __restrict__ y, PlanData<R> d, 
   const int cp = tid - g * (3 * N);
   const int c = cp / N, p = cp - c * N;
   const bool act = tid < T;
+  const cx<R>* lam = d.lam + (long long)inst * 3 * N;
+  if constexpr (sizeof(R) == 4) {
+    if (tid < N) pi_row_fill<N>(pi_rows<R, N>(sm), lam, k3, side, tid);
+  }
   // y columns, pass A straight from global (pencil p = column i1 of field c)
   if (act) {
     const cx<R>* src = w + vec * w_stride + (long long)(blockIdx.y * 3 + c) * Nq + (long long)k3 * N * N + p;
@@ -611,26 +784,39 @@ k_plane_fwd2(const cx<R>* __restrict__ w, cx<R>* __restrict__ y, PlanData<R> d, 
   }
   __syncthreads();
   // Pi^H blocks of this side, scaled for the three forward DFTs
-  const cx<R>* lam = d.lam + (long long)inst * 3 * N;
   cx<R>* o = y + vec * out_stride + blockIdx.y * out_side_stride + (long long)k3 * N * N;
-  const cx<R> lz = lam[2 * N + k3];
   const R sc = scale3<R, N>();
-  for (int e = tid; e < N * N; e += SP::TB) {
-    const int i2 = e / N, i1 = e - i2 * N;
-    const cx<R> u0 = sm[(0 * N + i2) * LD + i1];
-    const cx<R> u1 = sm[(1 * N + i2) * LD + i1];
-    const cx<R> u2 = sm[(2 * N + i2) * LD + i1];
-    PiBlock<R> P = pi_at<R, N>(d, inst, k3, e, lam, i1, i2, lz);
-    cx<R> a, b;
-    if (side == 0) {
-      a = cneg(cfma(P.p2[2], u2, cfma(P.p2[1], u1, cmul(P.p2[0], u0))));
-      b = cfma(P.p1[2], u2, cfma(P.p1[1], u1, cmul(P.p1[0], u0)));
-    } else {
-      a = cfmac(P.p1[2], u2, cfmac(P.p1[1], u1, cmulc(P.p1[0], u0)));
-      b = cfmac(P.p2[2], u2, cfmac(P.p2[1], u1, cmulc(P.p2[0], u0)));
+  if (!act) return;
+  const int grp = tid / N, i1 = tid - grp * N;
+  if constexpr (sizeof(R) == 4) {
+    const PiCol pc = pi_col<N>(lam, k3, side, i1);
+#pragma unroll 2
+    for (int i2 = grp; i2 < N; i2 += 3 * G) {
+      const cx<R> u[3] = {sm[(0 * N + i2) * LD + i1], sm[(1 * N + i2) * LD + i1], sm[(2 * N + i2) * LD + i1]};
+      cx<R> a, b;
+      pi_post(pi_vox(pi_rows<R, N>(sm) + i2, pc), side, u, sc, a, b);
+      o[i2 * N + i1] = a;
+      o[Nq + i2 * N + i1] = b;
     }
-    store_io<R>(o + e, cscale(a, sc));
-    store_io<R>(o + Nq + e, cscale(b, sc));
+  } else {
+    const cx<R> lz = lam[2 * N + k3];
+    for (int i2 = grp; i2 < N; i2 += 3 * G) {
+      const int e = i2 * N + i1;
+      const cx<R> u0 = sm[(0 * N + i2) * LD + i1];
+      const cx<R> u1 = sm[(1 * N + i2) * LD + i1];
+      const cx<R> u2 = sm[(2 * N + i2) * LD + i1];
+      PiBlock<R> P = pi_at<R, N>(d, inst, k3, e, lam, i1, i2, lz);
+      cx<R> a, b;
+      if (side == 0) {
+        a = cneg(cfma(P.p2[2], u2, cfma(P.p2[1], u1, cmul(P.p2[0], u0))));
+        b = cfma(P.p1[2], u2, cfma(P.p1[1], u1, cmul(P.p1[0], u0)));
+      } else {
+        a = cfmac(P.p1[2], u2, cfmac(P.p1[1], u1, cmulc(P.p1[0], u0)));
+        b = cfmac(P.p2[2], u2, cfmac(P.p2[1], u1, cmulc(P.p2[0], u0)));
+      }
+      store_io<R>(o + e, cscale(a, sc));
+      store_io<R>(o + Nq + e, cscale(b, sc));
+    }
   }
 }
 
@@ -710,7 +896,7 @@ cudaError_t plane_inv(const Plan& P, const PlanData<R>& d, const cx<R>* x, cx<R>
                       int nside, int side0, long long in_stride, long long in_side_stride,
                       long long out_stride, const VecCtx& ctx, cudaStream_t st, DirUpd<R> upd = DirUpd<R>(),
                       int tuned_lanes = -1) {
-  const size_t sm = sizeof(cx<R>) * 3 * N * (N + 1);
+  constexpr size_t sm = plane_smem<R, N>();
   if constexpr (PREP && !WITH_S && plane_split(N) > 0) {
     const int lanes = plane_lanes<R, N>(P, tuned_lanes);
     if (lanes > 0) {
@@ -753,7 +939,7 @@ template <class R, int N, bool POST, bool WITH_S>
 cudaError_t plane_fwd(const Plan& P, const PlanData<R>& d, const cx<R>* w, cx<R>* y, int nvec, int nside,
                       int side0, long long w_stride, long long out_stride, long long out_side_stride,
                       const VecCtx& ctx, cudaStream_t st, int tuned_lanes = -1) {
-  const size_t sm = sizeof(cx<R>) * 3 * N * (N + 1);
+  constexpr size_t sm = plane_smem<R, N>();
   if constexpr (POST && !WITH_S && plane_split(N) > 0) {
     const int lanes = plane_lanes<R, N>(P, tuned_lanes);
     if (lanes > 0) {
