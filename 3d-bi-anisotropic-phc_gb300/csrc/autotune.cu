@@ -7,11 +7,7 @@
 //                CTAs better than others;
 //   stencil_tpb  the material stencil's form: 0 the single-pass k_sweep,
 //                128/256/512 threads per block of the two-kernel form;
-//   lanes        the plane kernels' split of each pencil: threads per pencil
-//                of the prime-factor split (every count compiled for the
-//                size, plane_lanes_alt) or 0, one thread per pencil.
-// chunk x stencil_tpb are timed with the size's default split, then every
-// split with the best of those.  No counterpart in the reference.
+// No counterpart in the reference.
 #include <algorithm>
 #include <vector>
 
@@ -121,21 +117,6 @@ static int autotune_prec(Plan& P, int nvec, int reps, TuneEntry* best_out) {
       e = time_one(t);
       if (e == cudaSuccess && t.us < best.us) best = t;
     }
-  // the plane kernels' split, with the best chunk and stencil form
-  if (e == cudaSuccess && P.opt_plane_split && plane_split(P.n) > 0) {
-    std::vector<int> lanes;
-    if (!ds) lanes.push_back(0);  // one thread per pencil (not compiled in double-single)
-    for (int i = ds ? 1 : 0; i < kPlaneLanesMax; ++i)
-      if (plane_lanes_alt(P.n, i) > 0) lanes.push_back(plane_lanes_alt(P.n, i));
-    const TuneEntry base = best;
-    for (int g : lanes) {
-      TuneEntry t = base;
-      t.lanes = g;
-      e = time_one(t);
-      if (e != cudaSuccess) break;
-      if (t.us < best.us) best = t;
-    }
-  }
   cudaEventDestroy(ev[0]);
   cudaEventDestroy(ev[1]);
   if (e != cudaSuccess) {

@@ -412,9 +412,7 @@ int fame_set_option(fame_plan_t h, int option, double value) {
       if (!(value > 0.0 && value < 1.0)) return fail(&P, FAME_ERR_BAD_ARG, "fame_set_option: refine tol in (0, 1)");
       P.opt_refine_tol = value;
       return FAME_OK;
-    case FAME_OPT_PLANE_SPLIT:
-      P.opt_plane_split = value != 0.0;
-      free_graphs(P);  // captured sequences hold the old kernels
+    case FAME_OPT_PLANE_SPLIT:  // one form per size and precision is compiled
       return FAME_OK;
     case FAME_OPT_ITOL_FLOOR:
       if (!(value > 0.0 && value < 1.0)) return fail(&P, FAME_ERR_BAD_ARG, "fame_set_option: itol floor in (0, 1)");

@@ -53,20 +53,11 @@ inline VecCtx sub_ctx(const VecCtx& c, int v0) {
   return s;
 }
 
-// Threads per pencil of the split-pencil plane kernels of fncB for size n
-// (0: none compiled, one thread per pencil).
-FAME_HD constexpr int plane_split(int n) {
-  return n == 60 ? 3 : n == 48 ? 3 : n == 40 ? 5 : n == 36 ? 4 : n == 30 ? 3 : n == 24 ? 3 : n == 20 ? 4
-       : n == 12 ? 3 : 0;
+// Threads per FFT pencil of the complex128 / double-single kernels for size n.
+FAME_HD constexpr int field_split(int n) {
+  return n == 64 ? 8 : n == 60 ? 4 : n == 50 ? 2 : n == 48 ? 3 : n == 40 ? 5 : n == 36 ? 4 : n == 32 ? 4 : n == 30 ? 3
+       : n == 24 ? 3 : n == 20 ? 4 : n == 18 ? 2 : n == 16 ? 4 : n == 12 ? 3 : n == 10 ? 2 : n == 8 ? 2 : n == 6 ? 2 : 1;
 }
-
-// Lane counts compiled for size n (i = 0 the default, 0 past the last): the
-// autotuner's choices of the split.  n = 60 also has 60 = 4 * 15 and 5 * 12
-// (720 / 900 threads per CTA, 15 / 12 values per thread).
-FAME_HD constexpr int plane_lanes_alt(int n, int i) {
-  return i == 0 ? plane_split(n) : n == 60 ? (i == 1 ? 4 : i == 2 ? 5 : 0) : 0;
-}
-constexpr int kPlaneLanesMax = 3;
 
 // Launch parameters of the fncB sequence picked by fame_autotune for one
 // (precision, batch width): vectors per launch sequence and the material
@@ -75,7 +66,7 @@ struct TuneEntry {
   int prec = 0, nvec = 0;
   int chunk = 0;         // 0: whole batch
   int stencil_tpb = 0;   // 0: single-pass k_sweep; 128/256/512: two-kernel form
-  int lanes = -1;        // threads per pencil of the plane kernels: -1 the size's default, 0 one
+  int lanes = -1;        // kept for its callers (fame_set_tune_lanes); the kernels take one split per size
   double us = 0.0;       // measured time of one fncB on the batch
 };
 
@@ -92,7 +83,7 @@ template <class R> struct PlanData {
   R* stn = nullptr;      // [nk][nphase][stn_size(kind)] vertex tensors of the material stencil
   int kind = kMatGeneral;
   cx<R>* pc = nullptr;   // [nk][8][Nq] CG preconditioner: inverse 4x4 Hermitian blocks, diagonal packed (lazy)
-  cx<R>* pi = nullptr;   // [nk][Nq][6] Pi1 | Pi2 per frequency voxel (SVD_Matrix_curl.m:45-57); complex128 plans data only
+  cx<R>* pi = nullptr;   // [nk][6][Nq] n^{-3/2} (Pi1 | Pi2) per frequency voxel (SVD_Matrix_curl.m:45-57); not in complex64
   // Field mode (per-vertex isotropic chiral medium eps(r) I, mu = I,
   // xi = -zeta = i gamma(r) I): vertex tensors N = a G, M = b G, J = -i g G with
   // a = 1/(eps - gamma^2), b = eps a, g = gamma a and G = A^T A the lattice
@@ -126,7 +117,6 @@ struct Plan {
   int opt_c64_round = 1;              // mixed B^{-1}: second round's B x update in complex64 (0: exact apply)
   int opt_graph = 2;                  // CG from CUDA graphs: 1 blocks of iterations, 2 the whole loop
   double opt_itol_floor = 1e-13;      // mixed form: floor of the spread-scaled inner tolerance
-  int opt_plane_split = 1;            // fncB plane kernels with several threads per pencil where compiled
   int opt_pi_table = 1;               // complex128 fncB reads Pi from the plan's table (else evaluates it)
   int opt_sira_nearest = 0;           // SIRA Ritz choice: 0 'CL' (above the target), 1 nearest either side
   int opt_refine = 1;                 // mixed form: FP64 refinement sweep of the Ritz pairs

@@ -25,17 +25,23 @@
 //
 // Pipeline (one launch each):
 //   plane_inv  : Pi blocks per frequency voxel + inverse DFT along x and y
+//                (complex64: k_plane_inv, three fields of a plane per CTA;
+//                complex128 and double-single: k_field_inv, one field)
 //   col        : inverse DFT along z (in place)
 //   sweep      : u', v' in one pass into the second buffer (fncb_material.cuh),
 //                or the two-kernel form: vertex (U, V, Hu, Hv at every vertex
 //                into scratch) then faceedge (u', v' in place)
 //   col        : forward DFT along z
-//   plane_fwd  : forward DFT along y and x + Pi^H blocks
+//   plane_fwd  : forward DFT along y and x + Pi^H blocks (k_plane_fwd, k_field_fwd)
+// The curl transforms and the handles use the same kernels; S is applied in
+// the z pass.
 //
 // This header holds the size-templated kernels; fncb_inst_*.cu instantiate
 // them per precision and grid size so the size list compiles in parallel,
 // and fncb_stencil.cu holds the size-independent kernels and the dispatch.
 #pragma once
+
+#include <cooperative_groups.h>
 
 #include "fame_internal.h"
 #include "fft_reg.cuh"
@@ -46,6 +52,17 @@ namespace detail {
 
 
 constexpr double kInvSqrt14 = 0.26726124191242438468455348087975;
+
+// conj(v) if keep is 0, v otherwise, by the sign bits (no arithmetic).
+__device__ __forceinline__ double2 conj_unless(double2 v, int keep) {
+  const int m = keep ? 0 : (int)0x80000000;
+  return make_double2(v.x, __hiloint2double(__double2hiint(v.y) ^ m, __double2loint(v.y)));
+}
+__device__ __forceinline__ cff conj_unless(cff v, int keep) {
+  const int m = keep ? 0 : (int)0x80000000;
+  v.y = ff(__int_as_float(__float_as_int(v.y.hi) ^ m), __int_as_float(__float_as_int(v.y.lo) ^ m), true);
+  return v;
+}
 
 template <class R> struct PiBlock {
   cx<R> p1[3], p2[3];
@@ -77,44 +94,33 @@ __device__ __forceinline__ PiBlock<R> pi_block(cx<R> lx, cx<R> ly, cx<R> lz) {
   return P;
 }
 
-// Pi1 | Pi2 of one voxel from the plan's table (6 complex; three 16-byte
-// loads in complex64).
-template <class R>
-__device__ __forceinline__ PiBlock<R> pi_load(const cx<R>* p) {
-  PiBlock<R> P;
-  if constexpr (sizeof(R) == 4) {
-    const float4* q = reinterpret_cast<const float4*>(p);
-    const float4 a = __ldg(q), b = __ldg(q + 1), c = __ldg(q + 2);
-    P.p1[0] = mk<R>(a.x, a.y);
-    P.p1[1] = mk<R>(a.z, a.w);
-    P.p1[2] = mk<R>(b.x, b.y);
-    P.p2[0] = mk<R>(b.z, b.w);
-    P.p2[1] = mk<R>(c.x, c.y);
-    P.p2[2] = mk<R>(c.z, c.w);
-  } else if constexpr (std::is_same<R, double>::value) {
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-      P.p1[i] = __ldg(p + i);
-      P.p2[i] = __ldg(p + 3 + i);
-    }
-  } else {
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-      P.p1[i] = p[i];
-      P.p2[i] = p[3 + i];
-    }
-  }
-  P.sig = R(0);
-  return P;
+// Scale of a unitary 3D DFT, n^{-3/2}.  Pi carries all of it (two blocks per
+// voxel and side), so neither the plane kernels nor the z pass multiply by it.
+template <class R, int N> __device__ __forceinline__ R scale3() {
+  constexpr double s = 1.0 / (double(N) * csqrt_int(N));
+  return R(s);
 }
 
-// Pi of voxel (i1, i2, k3) of instance inst: from the table when the plan has
-// one (voxel index k3*N*N + e, e = i2*N + i1), else evaluated.
+// Component c of Pi1 and Pi2 at a frequency voxel (index vox = k3 n^2 + i2 n +
+// i1) of instance inst, times n^{-3/2}: from the plan's table [6][n^3] when it
+// has one, else evaluated.
+template <class R> struct PiComp {
+  cx<R> p1, p2;
+};
 template <class R, int N>
-__device__ __forceinline__ PiBlock<R> pi_at(const PlanData<R>& d, int inst, int k3, int e, const cx<R>* lam, int i1,
-                                            int i2, cx<R> lz) {
-  if (d.pi) return pi_load<R>(d.pi + ((size_t)inst * N * N * N + (size_t)k3 * N * N + e) * 6);
-  return pi_block<R>(lam[i1], lam[N + i2], lz);
+__device__ __forceinline__ PiComp<R> pi_comp(const PlanData<R>& d, int inst, int c, int vox, const cx<R>* lam) {
+  constexpr int Nq = N * N * N;
+  PiComp<R> P;
+  if (d.pi) {
+    const cx<R>* t = d.pi + (size_t)inst * 6 * Nq + vox;
+    P.p1 = t[(size_t)c * Nq];
+    P.p2 = t[(size_t)(3 + c) * Nq];
+  } else {
+    const PiBlock<R> B = pi_block<R>(lam[vox % N], lam[N + (vox / N) % N], lam[2 * N + vox / (N * N)]);
+    P.p1 = cscale(c == 0 ? B.p1[0] : c == 1 ? B.p1[1] : B.p1[2], scale3<R, N>());
+    P.p2 = cscale(c == 0 ? B.p2[0] : c == 1 ? B.p2[1] : B.p2[2], scale3<R, N>());
+  }
+  return P;
 }
 
 // Pi of the voxels of one frequency plane (k3 fixed) in complex64, where the
@@ -128,7 +134,9 @@ __device__ __forceinline__ PiBlock<R> pi_at(const PlanData<R>& d, int inst, int 
 // products with the vectors (the blocks took about 100, 40 % of the kernels'
 // instructions; at n = 60, 10 vectors, k_plane_inv 26.3 -> 19.4 M warp
 // instructions, 58 -> 47 us).  |m|^2 as a sum of squares also has no
-// cancellation: fncB's error against 64 bits 3.5e-7 -> 2.2e-7.
+// cancellation where L is nearly parallel to w, which |L|^2 - |L.w|^2 has:
+// fncB's error against 64 bits 3.5e-7 -> 2.2e-7 of the norm, its worst element
+// (220 batches at n = 40 to 64) 3.3e-4 -> 1.6e-6.
 //
 // Side 0 (Pr) takes the same formulas with conj(L) for L and the two blocks
 // swapped:  side 1: v = conj(m) X + q Y with X = a/|m|, Y = b/(|m||L|);
@@ -207,25 +215,15 @@ __device__ __forceinline__ void pi_post(const PiVox& P, int side, const float2 (
   b = side ? Y : X;
 }
 
-// Bytes of shared memory of the plane kernels: three padded fields, and the
-// row table in complex64.
-template <class R, int N> constexpr size_t plane_smem() {
-  return sizeof(cx<R>) * 3 * N * (N + 1) + (sizeof(R) == 4 ? sizeof(PiRow) * N : 0);
-}
+// Bytes of shared memory of the complex64 plane kernels: three padded fields
+// and the row table.
+template <int N> constexpr size_t plane_smem() { return sizeof(float2) * 3 * N * (N + 1) + sizeof(PiRow) * N; }
 // The row table's place behind the fields (16-byte aligned: N is even).
-template <class R, int N> __device__ __forceinline__ PiRow* pi_rows(cx<R>* sm) {
+template <int N> __device__ __forceinline__ PiRow* pi_rows(float2* sm) {
   return reinterpret_cast<PiRow*>(sm + 3 * N * (N + 1));
 }
 
-// Scale of a unitary 3D DFT, n^{-3/2}.  The S-free transforms of fncB put all of
-// it on the plane kernels' frequency side (two blocks per voxel and side), so
-// the z pass multiplies by nothing.
-template <class R, int N> __device__ __forceinline__ R scale3() {
-  constexpr double s = 1.0 / (double(N) * csqrt_int(N));
-  return R(s);
-}
-
-// Operator input / output of the split plane kernels.  The double-single
+// Operator input / output of the field kernels.  The double-single
 // operator reads and writes complex128 vectors (the caller's), converting
 // on load and store, so it needs no conversion passes; the conversions run
 // on the FP64 pipe, which its float-float arithmetic leaves idle.
@@ -257,48 +255,53 @@ template <class R> struct DirUpd {
 };
 
 // ---------------------------------------------------------------------------
-// plane_inv: one CTA per (k3 plane, side, vector); 3N threads.
-// PREP: build the 3 frequency components of one side from (a, b):
+// complex64 plane kernels: one CTA per (k3 plane, side, vector), 3N threads,
+// one thread per pencil (N <= 64 complex values in registers).
+//
+// k_plane_inv: PREP builds the three frequency components of one side from
+// (a, b), else it copies three components; then the inverse DFT along x
+// (rows, via shared memory) and y (columns, straight to global).
 //   side 0 (Pr):  p = -conj(Pi2) a + conj(Pi1) b      (Pi.Pr, SVD_Matrix_curl.m:64)
 //   side 1 (Qr):  q =  Pi1 a + Pi2 b                  (Pi.Qr, SVD_Matrix_curl.m:63)
-// else copy 3 components.  Then inverse DFT along x (rows, via shared
-// memory) and y (columns, straight to global); WITH_S multiplies by S_x S_y / n
-// there, PREP without S scales its input by n^{-3/2} (scale3).
+// Latency-bound: at n = 60 two CTAs of six warps fit an SM (88 KB of shared
+// memory each) and issue 40 % of the cycles.  A prime-factor split of each
+// pencil over three threads (34 warps per SM) needed twice the shared-memory
+// traffic and a third more instructions, and was slower at every size and
+// batch (n = 60, warm, one vector 9.4 against 8.6 us, ten 58 against 47).
 // ---------------------------------------------------------------------------
-template <class R, int N, bool PREP, bool WITH_S>
-__global__ void __launch_bounds__(((3 * N + 31) / 32) * 32, sizeof(R) == 4 ? 2 : 1)
-k_plane_inv(const cx<R>* __restrict__ x, cx<R>* __restrict__ out, PlanData<R> d, VecCtx ctx,
-            long long in_stride, long long in_side_stride, long long out_stride, int side0, DirUpd<R> upd) {
+template <int N, bool PREP>
+__global__ void __launch_bounds__(((3 * N + 31) / 32) * 32, 2)
+k_plane_inv(const float2* __restrict__ x, float2* __restrict__ out, PlanData<float> d, VecCtx ctx,
+            long long in_stride, long long in_side_stride, long long out_stride, int side0, DirUpd<float> upd) {
   constexpr int LD = N + 1;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  cx<R>* sm = reinterpret_cast<cx<R>*>(smem_raw);  // [3][N][LD]
+  float2* sm = reinterpret_cast<float2*>(smem_raw);  // [3][N][LD]
   const int k3 = blockIdx.x;
   const int vec = blockIdx.z;
   if (ctx.active && !ctx.active[vec]) return;
   const int inst = vec_inst(ctx, vec);
   const int side = side0 + blockIdx.y;
   const long long Nq = (long long)N * N * N;
-  const cx<R>* lam = d.lam + (long long)inst * 3 * N;
-  const cx<R>* xin = x + vec * in_stride + blockIdx.y * in_side_stride + (long long)k3 * N * N;
+  const float2* lam = d.lam + (long long)inst * 3 * N;
+  const long long off = vec * in_stride + blockIdx.y * in_side_stride + (long long)k3 * N * N;
+  const float2* xin = x + off;
   const int tid = threadIdx.x;
 
   // Input plane -> shared memory: thread (column i1, row group) takes rows
   // grp, grp + 3, ...  The global loads of PF rows are issued together before
   // any is used, so a CTA waits for one memory round trip per batch.
-  constexpr bool PIV = PREP && sizeof(R) == 4;
   const int grp = tid / N, i1 = tid - grp * N;
   const bool act = tid < 3 * N;
-  if constexpr (PIV) {
-    if (tid < N) pi_row_fill<N>(pi_rows<R, N>(sm), lam, k3, side, tid);
+  if constexpr (PREP) {
+    if (tid < N) pi_row_fill<N>(pi_rows<N>(sm), lam, k3, side, tid);
   }
   constexpr int ITEMS = (N + 2) / 3;
   constexpr int NB = PREP ? 2 : 3;                        // input blocks
-  constexpr int PF0 = (sizeof(R) == 4 ? 24 : 12) / NB;   // rows in flight per thread
-  constexpr int NBATCH = (ITEMS + PF0 - 1) / PF0;
-  constexpr int PF = (ITEMS + NBATCH - 1) / NBATCH;
+  constexpr int NBATCH = (ITEMS * NB + 23) / 24;
+  constexpr int PF = (ITEMS + NBATCH - 1) / NBATCH;       // rows in flight per thread
   static_for<0, NBATCH>([&](auto bc) {
     constexpr int base = decltype(bc)::value * PF;
-    cx<R> in[PF][NB];
+    float2 in[PF][NB];
 #pragma unroll
     for (int it = 0; it < PF; ++it) {
       const int i2 = grp + 3 * (base + it);
@@ -308,11 +311,10 @@ k_plane_inv(const cx<R>* __restrict__ x, cx<R>* __restrict__ out, PlanData<R> d,
       }
     }
     if (PREP && upd.z) {  // p = z + beta p, written back
-      const long long off = vec * in_stride + blockIdx.y * in_side_stride + (long long)k3 * N * N;
-      const cx<R>* zin = upd.z + off;
-      cx<R>* xw = const_cast<cx<R>*>(x) + off;
-      const R bt = R(upd.beta[vec]);
-      cx<R> zz[PF][NB];
+      const float2* zin = upd.z + off;
+      float2* xw = const_cast<float2*>(x) + off;
+      const float bt = float(upd.beta[vec]);
+      float2 zz[PF][NB];
 #pragma unroll
       for (int it = 0; it < PF; ++it) {
         const int i2 = grp + 3 * (base + it);
@@ -333,103 +335,62 @@ k_plane_inv(const cx<R>* __restrict__ x, cx<R>* __restrict__ out, PlanData<R> d,
         }
       }
     }
-    if constexpr (PIV && decltype(bc)::value == 0) __syncthreads();  // the row table
+    if constexpr (PREP && decltype(bc)::value == 0) __syncthreads();  // the row table
     if (act) {
-      if constexpr (PIV) {
-        const PiCol pc = pi_col<N>(lam, k3, side, i1);
+      PiCol pc;
+      if constexpr (PREP) pc = pi_col<N>(lam, k3, side, i1);
 #pragma unroll
-        for (int it = 0; it < PF; ++it) {
-          const int i2 = grp + 3 * (base + it);
-          if (i2 < N) {
-            cx<R> v[3];
-            pi_prep(pi_vox(pi_rows<R, N>(sm) + i2, pc), side, in[it][0], in[it][1],
-                    WITH_S ? R(1) : scale3<R, N>(), v);
+      for (int it = 0; it < PF; ++it) {
+        const int i2 = grp + 3 * (base + it);
+        if (i2 < N) {
+          float2 v[3];
+          if constexpr (PREP) {
+            pi_prep(pi_vox(pi_rows<N>(sm) + i2, pc), side, in[it][0], in[it][1], scale3<float, N>(), v);
+          } else {
 #pragma unroll
-            for (int c = 0; c < 3; ++c) sm[(c * N + i2) * LD + i1] = v[c];
+            for (int c = 0; c < 3; ++c) v[c] = in[it][c < NB ? c : 0];
           }
-        }
-      } else {
 #pragma unroll
-        for (int it = 0; it < PF; ++it) {
-          const int i2 = grp + 3 * (base + it);
-          if (i2 < N) {
-            cx<R> v0, v1, v2;
-            if constexpr (PREP) {
-              PiBlock<R> P = pi_at<R, N>(d, inst, k3, i2 * N + i1, lam, i1, i2, lam[2 * N + k3]);
-              cx<R> a = in[it][0], b = in[it][1];
-              if constexpr (!WITH_S) {
-                a = cscale(a, scale3<R, N>());
-                b = cscale(b, scale3<R, N>());
-              }
-              if (side == 0) {
-                v0 = cfmac(P.p1[0], b, cneg(cmulc(P.p2[0], a)));
-                v1 = cfmac(P.p1[1], b, cneg(cmulc(P.p2[1], a)));
-                v2 = cfmac(P.p1[2], b, cneg(cmulc(P.p2[2], a)));
-              } else {
-                v0 = cfma(P.p2[0], b, cmul(P.p1[0], a));
-                v1 = cfma(P.p2[1], b, cmul(P.p1[1], a));
-                v2 = cfma(P.p2[2], b, cmul(P.p1[2], a));
-              }
-            } else {
-              v0 = in[it][0];
-              v1 = in[it][1];
-              v2 = in[it][NB - 1];
-            }
-            sm[(0 * N + i2) * LD + i1] = v0;
-            sm[(1 * N + i2) * LD + i1] = v1;
-            sm[(2 * N + i2) * LD + i1] = v2;
-          }
+          for (int c = 0; c < 3; ++c) sm[(c * N + i2) * LD + i1] = v[c];
         }
       }
     }
   });
   __syncthreads();
-  if (tid < 3 * N) {  // x rows
-    const int c = tid / N, i2 = tid - c * N;
-    cx<R>* row = sm + (c * N + i2) * LD;
-    cx<R> v[N];
+  if (act) {  // x rows
+    float2* row = sm + tid * LD;
+    float2 v[N];
 #pragma unroll
     for (int i = 0; i < N; ++i) v[i] = row[i];
-    fft<R, N, +1>(v);
+    fft<float, N, +1>(v);
 #pragma unroll
     for (int i = 0; i < N; ++i) row[i] = v[i];
   }
   __syncthreads();
-  if (tid < 3 * N) {  // y columns
-    const int c = tid / N, i1 = tid - c * N;
-    cx<R> v[N];
+  if (act) {  // y columns (field grp, column i1)
+    float2 v[N];
 #pragma unroll
-    for (int i = 0; i < N; ++i) v[i] = sm[(c * N + i) * LD + i1];
-    fft<R, N, +1>(v);
-    cx<R> sx = mk<R>(R(1), R(0));
-    const cx<R>* S = d.sxyz + (long long)inst * 3 * N;
-    if constexpr (WITH_S) sx = cscale(S[i1], R(1.0 / N));
-    cx<R>* o = out + vec * out_stride + (long long)(blockIdx.y * 3 + c) * Nq + (long long)k3 * N * N + i1;
+    for (int i = 0; i < N; ++i) v[i] = sm[(grp * N + i) * LD + i1];
+    fft<float, N, +1>(v);
+    float2* o = out + vec * out_stride + (long long)(blockIdx.y * 3 + grp) * Nq + (long long)k3 * N * N + i1;
 #pragma unroll
-    for (int i2 = 0; i2 < N; ++i2) {
-      cx<R> r = v[i2];
-      if constexpr (WITH_S) r = cmul(r, cmul(sx, S[N + i2]));
-      o[(long long)i2 * N] = r;
-    }
+    for (int i2 = 0; i2 < N; ++i2) o[(long long)i2 * N] = v[i2];
   }
 }
 
-// ---------------------------------------------------------------------------
-// plane_fwd: one CTA per (k3 plane, side, vector); 3N threads.
-// Forward DFT along y (columns, straight from global) and x (rows, shared
-// memory); WITH_S multiplies conj(S_x S_y) / n first.  POST applies
-// the Pi^H blocks of one side (SVD_Matrix_curl.m:63-64, handles Prs/Qrs):
+// k_plane_fwd: forward DFT along y (columns, straight from global) and x
+// (rows, shared memory).  POST applies the Pi^H blocks of one side
+// (SVD_Matrix_curl.m:63-64, handles Prs/Qrs):
 //   side 0 (Prs): a = -sum_c Pi2_c u_c,  b = sum_c Pi1_c u_c
 //   side 1 (Qrs): a = sum_c conj(Pi1_c) v_c, b = sum_c conj(Pi2_c) v_c
 // else copies the 3 components out.
-// ---------------------------------------------------------------------------
-template <class R, int N, bool POST, bool WITH_S>
-__global__ void __launch_bounds__(((3 * N + 31) / 32) * 32, sizeof(R) == 4 ? 2 : 1)
-k_plane_fwd(const cx<R>* __restrict__ w, cx<R>* __restrict__ y, PlanData<R> d, VecCtx ctx,
+template <int N, bool POST>
+__global__ void __launch_bounds__(((3 * N + 31) / 32) * 32, 2)
+k_plane_fwd(const float2* __restrict__ w, float2* __restrict__ y, PlanData<float> d, VecCtx ctx,
             long long w_stride, long long out_stride, long long out_side_stride, int side0) {
   constexpr int LD = N + 1;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  cx<R>* sm = reinterpret_cast<cx<R>*>(smem_raw);  // [3][N][LD]
+  float2* sm = reinterpret_cast<float2*>(smem_raw);  // [3][N][LD]
   const int k3 = blockIdx.x;
   const int vec = blockIdx.z;
   if (ctx.active && !ctx.active[vec]) return;
@@ -437,602 +398,537 @@ k_plane_fwd(const cx<R>* __restrict__ w, cx<R>* __restrict__ y, PlanData<R> d, V
   const int side = side0 + blockIdx.y;
   const long long Nq = (long long)N * N * N;
   const int tid = threadIdx.x;
-  const cx<R>* S = d.sxyz + (long long)inst * 3 * N;
-  const cx<R>* lam = d.lam + (long long)inst * 3 * N;
-  if constexpr (POST && sizeof(R) == 4) {
-    if (tid < N) pi_row_fill<N>(pi_rows<R, N>(sm), lam, k3, side, tid);
+  const int grp = tid / N, i1 = tid - grp * N;
+  const bool act = tid < 3 * N;
+  const float2* lam = d.lam + (long long)inst * 3 * N;
+  if constexpr (POST) {
+    if (tid < N) pi_row_fill<N>(pi_rows<N>(sm), lam, k3, side, tid);
   }
-  if (tid < 3 * N) {  // y columns
-    const int c = tid / N, i1 = tid - c * N;
-    const cx<R>* src = w + vec * w_stride + (long long)(blockIdx.y * 3 + c) * Nq + (long long)k3 * N * N + i1;
-    cx<R> v[N];
-    cx<R> sx = mk<R>(R(1), R(0));
-    if constexpr (WITH_S) sx = cscale(S[i1], R(1.0 / N));
+  if (act) {  // y columns (field grp, column i1)
+    const float2* src = w + vec * w_stride + (long long)(blockIdx.y * 3 + grp) * Nq + (long long)k3 * N * N + i1;
+    float2 v[N];
 #pragma unroll
-    for (int i2 = 0; i2 < N; ++i2) {
-      v[i2] = src[(long long)i2 * N];
-      if constexpr (WITH_S) v[i2] = cmulc(cmul(sx, S[N + i2]), v[i2]);
-    }
-    fft<R, N, -1>(v);
+    for (int i2 = 0; i2 < N; ++i2) v[i2] = src[(long long)i2 * N];
+    fft<float, N, -1>(v);
 #pragma unroll
-    for (int i2 = 0; i2 < N; ++i2) sm[(c * N + i2) * LD + i1] = v[i2];
+    for (int i2 = 0; i2 < N; ++i2) sm[(grp * N + i2) * LD + i1] = v[i2];
   }
   __syncthreads();
-  if (tid < 3 * N) {  // x rows
-    const int c = tid / N, i2 = tid - c * N;
-    cx<R>* row = sm + (c * N + i2) * LD;
-    cx<R> v[N];
+  if (act) {  // x rows
+    float2* row = sm + tid * LD;
+    float2 v[N];
 #pragma unroll
     for (int i = 0; i < N; ++i) v[i] = row[i];
-    fft<R, N, -1>(v);
+    fft<float, N, -1>(v);
 #pragma unroll
     for (int i = 0; i < N; ++i) row[i] = v[i];
   }
   __syncthreads();
-  cx<R>* o = y + vec * out_stride + blockIdx.y * out_side_stride + (long long)k3 * N * N;
-  if (tid < 3 * N) {
-    const int grp = tid / N, i1 = tid - grp * N;
-    if constexpr (POST && sizeof(R) == 4) {
-      const PiCol pc = pi_col<N>(lam, k3, side, i1);
+  if (!act) return;
+  float2* o = y + vec * out_stride + blockIdx.y * out_side_stride + (long long)k3 * N * N;
+  PiCol pc;
+  if constexpr (POST) pc = pi_col<N>(lam, k3, side, i1);
 #pragma unroll 4
-      for (int i2 = grp; i2 < N; i2 += 3) {
-        const cx<R> u[3] = {sm[(0 * N + i2) * LD + i1], sm[(1 * N + i2) * LD + i1], sm[(2 * N + i2) * LD + i1]};
-        cx<R> a, b;
-        pi_post(pi_vox(pi_rows<R, N>(sm) + i2, pc), side, u, WITH_S ? R(1) : scale3<R, N>(), a, b);
-        o[i2 * N + i1] = a;
-        o[Nq + i2 * N + i1] = b;
-      }
+  for (int i2 = grp; i2 < N; i2 += 3) {
+    const float2 u[3] = {sm[(0 * N + i2) * LD + i1], sm[(1 * N + i2) * LD + i1], sm[(2 * N + i2) * LD + i1]};
+    const int e = i2 * N + i1;
+    if constexpr (POST) {
+      float2 a, b;
+      pi_post(pi_vox(pi_rows<N>(sm) + i2, pc), side, u, scale3<float, N>(), a, b);
+      o[e] = a;
+      o[Nq + e] = b;
     } else {
-#pragma unroll 4
-      for (int i2 = grp; i2 < N; i2 += 3) {
-        const int e = i2 * N + i1;
-        cx<R> u0 = sm[(0 * N + i2) * LD + i1];
-        cx<R> u1 = sm[(1 * N + i2) * LD + i1];
-        cx<R> u2 = sm[(2 * N + i2) * LD + i1];
-        if constexpr (POST) {
-          PiBlock<R> P = pi_at<R, N>(d, inst, k3, e, lam, i1, i2, lam[2 * N + k3]);
-          cx<R> a, b;
-          if (side == 0) {
-            a = cneg(cfma(P.p2[2], u2, cfma(P.p2[1], u1, cmul(P.p2[0], u0))));
-            b = cfma(P.p1[2], u2, cfma(P.p1[1], u1, cmul(P.p1[0], u0)));
-          } else {
-            a = cfmac(P.p1[2], u2, cfmac(P.p1[1], u1, cmulc(P.p1[0], u0)));
-            b = cfmac(P.p2[2], u2, cfmac(P.p2[1], u1, cmulc(P.p2[0], u0)));
-          }
-          if constexpr (!WITH_S) {
-            a = cscale(a, scale3<R, N>());
-            b = cscale(b, scale3<R, N>());
-          }
-          o[e] = a;
-          o[Nq + e] = b;
-        } else {
-          o[e] = u0;
-          o[Nq + e] = u1;
-          o[2 * Nq + e] = u2;
-        }
-      }
+#pragma unroll
+      for (int c = 0; c < 3; ++c) o[c * Nq + e] = u[c];
     }
   }
 }
 
 // ---------------------------------------------------------------------------
-// Split-pencil plane kernels of fncB (k_plane_inv2 / k_plane_fwd2): the same
-// work as k_plane_inv<PREP> / k_plane_fwd<POST>, with G threads per pencil
-// instead of one.  A length N = G*M with gcd(G, M) = 1 is split by the
-// prime-factor index map (no twiddle factors):
+// complex128 and double-single field kernels: the same work, one CTA per
+// (k3 plane, field, vector), so that the arithmetic of a launch spreads over
+// the SMs in thirds of a plane.  (With the three fields in one CTA, 4 vectors
+// at n = 40 are 320 CTAs on 152 SMs, three rounds where 2.1 would do; and a
+// double-single plane of three fields fills an SM's shared memory, which left
+// one CTA per SM, waiting at its own barriers.)
+//
+// Every pencil is split over G threads, N = G*M (field_split): a whole pencil
+// is too much for one thread's registers beyond N ~ 32, and on small grids the
+// serial FP64 chain of one thread is what a kernel waits for.  Coprime G, M
+// use the prime-factor index map (no twiddle factors):
 //   n = (M*n1 + G*n2) mod N,  k = (M*A*k1 + G*B*k2) mod N,
 //   A = M^{-1} mod G, B = G^{-1} mod M,
-//   X[k] = sum_{n2} W_M^{n2 k2} sum_{n1} x[n] W_G^{n1 k1}.
-// Pass A: M length-G DFTs over n1 per pencil, in place in shared memory
-// (thread g of the pencil takes n2 = g, g+G, ...).  Pass B: thread k1 takes
-// the length-M DFT over n2 in registers.  A thread then holds M complex
-// values instead of N, so 3*N*G threads of a CTA fit two CTAs per SM
-// (N = 60: G = 3, 540 threads, 34 warps per SM against 12 for one thread per
-// 60-point pencil).
+//   X[k] = sum_{n2} W_M^{n2 k2} sum_{n1} x[n] W_G^{n1 k1};
+// powers of two the Cooley-Tukey one, n = M*n1 + n2, k = k1 + G*k2, with W_N^{n2 k1}
+// between the passes.
+// Pass A: the M length-G DFTs over n1 of every pencil, in place in shared
+// memory, dealt to the threads in one sequence.  Pass B: thread (k1, pencil)
+// takes the length-M DFT over n2 in registers.  The slots are computed at run
+// time: the kernels are bound by arithmetic, and branches that make them
+// immediate operands diverge in every warp that holds two values of k1 (a
+// third more FP64 instructions in pass A at n = 60).
 // ---------------------------------------------------------------------------
-
-// CTAs per SM the split kernels are compiled for: two for the default lane
-// count in complex64, one otherwise (the register allocation then decides).
-template <class R, int N, int G> constexpr int plane_min_blocks() {
-  return sizeof(R) == 4 && G == plane_split(N) ? 2 : 1;
+template <int N> struct Twiddles {
+  double c[N], s[N];
+};
+template <int N> constexpr Twiddles<N> make_twiddles() {
+  Twiddles<N> t{};
+  for (int i = 0; i < N; ++i) {
+    t.c[i] = cs2pi(i, N, 0);
+    t.s[i] = cs2pi(i, N, 1);
+  }
+  return t;
 }
+// exp(2 pi i m / N), m < N
+template <int N> static __constant__ Twiddles<N> kTwiddles = make_twiddles<N>();
+
+FAME_HD constexpr int gcd_of(int a, int b) { return b == 0 ? a : gcd_of(b, a % b); }
 
 template <int N, int G> struct Split {
   static constexpr int M = N / G;
-  static constexpr int A = fft_inv_mod(M % G, G);
-  static constexpr int B = fft_inv_mod(G % M, M);
-  static constexpr int T = 3 * N * G;                 // threads: (field, pencil, g)
-  static constexpr int TB = ((T + 31) / 32) * 32;
-  static constexpr int NA = (M + G - 1) / G;          // pass-A DFTs per thread (upper bound)
-  static_assert(G * M == N && A >= 0 && B >= 0, "coprime split");
-  FAME_HD static constexpr int in_slot(int n1, int n2) { return (M * n1 + G * n2) % N; }
-  FAME_HD static constexpr int out_slot(int k1, int k2) { return (M * A * k1 + G * B * k2) % N; }
+  static constexpr bool PFA = gcd_of(G, M) == 1;
+  static constexpr int A = PFA ? fft_inv_mod(M % G, G) : 0;
+  static constexpr int B = PFA ? fft_inv_mod(G % M, M) : 0;
+  static constexpr int NA = (M + G - 1) / G;          // rounds of pass A
+  static_assert(G * M == N, "a split of N");
+  FAME_HD static int wrap(int a) { return a >= N ? a - N : a; }
+  // element n1 of the DFT n2 of pass A; element n2 of row n1 of pass B
+  FAME_HD static int in_slot(int n1, int n2) { return PFA ? wrap(M * n1 + G * n2) : M * n1 + n2; }
+  // output k2 of row k1
+  FAME_HD static int out_slot(int k1, int k2) {
+    return PFA ? wrap((M * A * k1) % N + (G * B * k2) % N) : k1 + G * k2;
+  }
 };
 
-// Pass A on one pencil in shared memory (element i at p[i * STRIDE]) for the
-// thread with sub-pencil index GC (compile time, so that every slot index is
-// an immediate offset).
-template <class R, int N, int G, int S, int STRIDE, int GC>
-__device__ __forceinline__ void split_pass_a(cx<R>* p) {
+// One DFT of pass A (S: direction) with the twiddle of the Cooley-Tukey map.
+template <class R, int N, int G, int S> __device__ __forceinline__ void pass_a_dft(cx<R> (&a)[G], int n2) {
+  fft<R, G, S>(a);
+  if constexpr (!Split<N, G>::PFA) {
+#pragma unroll
+    for (int k1 = 1; k1 < G; ++k1) {
+      const double c = kTwiddles<N>.c[n2 * k1], s = kTwiddles<N>.s[n2 * k1];
+      a[k1] = cmul(mk<R>(R(c), R(S * s)), a[k1]);
+    }
+  }
+}
+
+// Pass A with T threads on NP pencils; base(p) points at element 0 of pencil
+// p, elements STRIDE apart.
+template <class R, int N, int G, int S, int STRIDE, int NP, int T, class F>
+__device__ __forceinline__ void split_pass_a(int tid, F&& base) {
   using SP = Split<N, G>;
-  static_for<0, SP::NA>([&](auto jc) {
-    constexpr int n2 = GC + decltype(jc)::value * G;
-    if constexpr (n2 < SP::M) {
+#pragma unroll
+  for (int j = 0; j < SP::NA; ++j) {
+    const int idx = tid + j * T;
+    if (tid < T && idx < NP * SP::M) {
+      const int n2 = idx / NP, p = idx - n2 * NP;
+      cx<R>* q = base(p);
       cx<R> a[G];
-      static_for<0, G>([&](auto n1c) { a[decltype(n1c)::value] = p[SP::in_slot(decltype(n1c)::value, n2) * STRIDE]; });
-      fft<R, G, S>(a);
-      static_for<0, G>([&](auto n1c) { p[SP::in_slot(decltype(n1c)::value, n2) * STRIDE] = a[decltype(n1c)::value]; });
+#pragma unroll
+      for (int n1 = 0; n1 < G; ++n1) a[n1] = q[SP::in_slot(n1, n2) * STRIDE];
+      pass_a_dft<R, N, G, S>(a, n2);
+#pragma unroll
+      for (int n1 = 0; n1 < G; ++n1) q[SP::in_slot(n1, n2) * STRIDE] = a[n1];
     }
-  });
+  }
 }
 
-// Pass B read: the M values of row K1 of one pencil.
-template <class R, int N, int G, int STRIDE, int K1>
-__device__ __forceinline__ void split_pass_b_load(const cx<R>* p, cx<R> (&z)[N / G]) {
+// Pass B read: the M values of row k1 of one pencil.
+template <class R, int N, int G, int STRIDE>
+__device__ __forceinline__ void split_pass_b_load(const cx<R>* p, int k1, cx<R> (&z)[N / G]) {
   using SP = Split<N, G>;
-  static_for<0, SP::M>([&](auto n2c) { z[decltype(n2c)::value] = p[SP::in_slot(K1, decltype(n2c)::value) * STRIDE]; });
+#pragma unroll
+  for (int n2 = 0; n2 < SP::M; ++n2) z[n2] = p[SP::in_slot(k1, n2) * STRIDE];
 }
 
-// Pass B write: X[out_slot(K1, k2)] = z[k2].
-template <class R, int N, int G, int STRIDE, int K1, class P>
-__device__ __forceinline__ void split_pass_b_store(P p, const cx<R> (&z)[N / G]) {
+// Pass B write: X[out_slot(k1, k2)] = z[k2].
+template <class R, int N, int G, int STRIDE>
+__device__ __forceinline__ void split_pass_b_store(cx<R>* p, int k1, const cx<R> (&z)[N / G]) {
   using SP = Split<N, G>;
-  static_for<0, SP::M>([&](auto k2c) { p[(long long)SP::out_slot(K1, decltype(k2c)::value) * STRIDE] = z[decltype(k2c)::value]; });
+#pragma unroll
+  for (int k2 = 0; k2 < SP::M; ++k2) p[SP::out_slot(k1, k2) * STRIDE] = z[k2];
 }
 
-// f(integral_constant<GC>) for the runtime g of this thread (warps are
-// uniform in g except the ones that straddle two sub-pencil groups).
-template <int G, class F> __device__ __forceinline__ void with_g(int g, F&& f) {
-  static_for<0, G>([&](auto gc) {
-    if (g == decltype(gc)::value) f(gc);
-  });
+template <class R, int N> struct FieldShape {
+  static constexpr int G = field_split(N);
+  static constexpr int KP = N <= 16 ? 2 : 1;       // planes per CTA: small planes share one, to fill its warps
+  static constexpr int NP = KP * N;                // pencils per axis
+  static constexpr int T = NP * G;                 // threads of the DFT passes
+  static constexpr int TB = ((T + 31) / 32) * 32 < 64 ? 64 : ((T + 31) / 32) * 32;
+  static constexpr int LD = N + 1;
+  static constexpr size_t SMEM = sizeof(cx<R>) * KP * N * LD;
+  static_assert(N % KP == 0, "whole CTAs of planes");
+};
+
+// Rows of the staged planes (pencil p at sm + p * LD): the length-N DFT along x
+// in place; thread (g, p).
+template <class R, int N, int S> __device__ __forceinline__ void field_rows(cx<R>* sm, int tid, int g, int p, bool act) {
+  using FS = FieldShape<R, N>;
+  constexpr int G = FS::G, M = N / G;
+  if constexpr (G > 1) {
+    split_pass_a<R, N, G, S, 1, FS::NP, FS::T>(tid, [&](int q) { return sm + q * FS::LD; });
+    __syncthreads();
+  }
+  cx<R>* row = sm + p * FS::LD;
+  cx<R> z[M];
+  if (act) {
+    split_pass_b_load<R, N, G, 1>(row, g, z);
+    fft<R, M, S>(z);
+  }
+  if constexpr (G > 1) __syncthreads();
+  if (act) split_pass_b_store<R, N, G, 1>(row, g, z);
+  __syncthreads();
 }
 
-template <class R, int N, int G, bool UPD>
-__global__ void __launch_bounds__(Split<N, G>::TB, plane_min_blocks<R, N, G>())
-k_plane_inv2(const cx<R>* __restrict__ x, cx<R>* __restrict__ out, PlanData<R> d, VecCtx ctx,
-             long long in_stride, long long in_side_stride, long long out_stride, int side0, DirUpd<R> upd) {
-  using SP = Split<N, G>;
-  constexpr int M = SP::M, T = SP::T, LD = N + 1;
+// grid: (n / KP, 3 * sides, vectors); blockIdx.y = 3 * (side - side0) + field
+template <class R, int N, bool PREP>
+__global__ void __launch_bounds__(FieldShape<R, N>::TB)
+k_field_inv(const cx<R>* __restrict__ x, cx<R>* __restrict__ out, PlanData<R> d, VecCtx ctx, long long in_stride,
+            long long in_side_stride, long long out_stride, int side0) {
+  using FS = FieldShape<R, N>;
+  constexpr int G = FS::G, M = N / G, LD = FS::LD, KP = FS::KP, TB = FS::TB;
+  constexpr int NN = N * N, Nq = NN * N;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  cx<R>* sm = reinterpret_cast<cx<R>*>(smem_raw);  // [3][N][LD]
-  const int k3 = blockIdx.x;
+  cx<R>* sm = reinterpret_cast<cx<R>*>(smem_raw);  // [KP][N][LD]
+  const int k3 = blockIdx.x * KP;
   const int vec = blockIdx.z;
   if (ctx.active && !ctx.active[vec]) return;
   const int inst = vec_inst(ctx, vec);
-  const int side = side0 + blockIdx.y;
-  const long long Nq = (long long)N * N * N;
-  const cx<R>* lam = d.lam + (long long)inst * 3 * N;
-  const cx<R>* xin = x + vec * in_stride + blockIdx.y * in_side_stride + (long long)k3 * N * N;
+  const int c = blockIdx.y % 3, side = side0 + blockIdx.y / 3;
   const int tid = threadIdx.x;
-  // Pi blocks (frequency voxel -> 3 components of this side), scaled for the
-  // three inverse DFTs: thread (column i1, row group) takes every NG-th row;
-  // all loads of a thread issued together.
-  {
-    constexpr int NG = 3 * G;
-    constexpr int ITEMS = (N + NG - 1) / NG;
-    const int grp = tid / N, i1 = tid - grp * N;
-    if constexpr (sizeof(R) == 4) {
-      if (tid < N) pi_row_fill<N>(pi_rows<R, N>(sm), lam, k3, side, tid);
-    }
-    cx<R> in[ITEMS][2];
+  const cx<R>* lam = d.lam + (long long)inst * 3 * N;
+  const cx<R>* xin = x + vec * in_stride + (blockIdx.y / 3) * in_side_stride + k3 * NN;
+  // the loads of U elements issued together
+  constexpr int ITEMS = (KP * NN + TB - 1) / TB;
+  constexpr int U = ITEMS < 4 ? ITEMS : 4;
+  for (int b = 0; b < ITEMS; b += U) {
+    cx<R> in[U][2];
+    PiComp<R> P[U];
 #pragma unroll
-    for (int it = 0; it < ITEMS; ++it) {
-      const int i2 = grp + it * NG;
-      if (tid < T && i2 < N) {
-        in[it][0] = load_io<R>(xin + i2 * N + i1);
-        in[it][1] = load_io<R>(xin + Nq + i2 * N + i1);
-      }
-    }
-    if constexpr (UPD) {  // p = z + beta p, written back (UPD: upd.z set)
-      const long long off = vec * in_stride + blockIdx.y * in_side_stride + (long long)k3 * N * N;
-      const cx<R>* zin = upd.z + off;
-      cx<R>* xw = const_cast<cx<R>*>(x) + off;
-      const R bt = R(upd.beta[vec]);
-#pragma unroll
-      for (int it = 0; it < ITEMS; ++it) {
-        const int i2 = grp + it * NG;
-        if (tid < T && i2 < N) {
-#pragma unroll
-          for (int c = 0; c < 2; ++c) {
-            in[it][c] = caxpy(bt, in[it][c], zin[c * Nq + i2 * N + i1]);
-            xw[c * Nq + i2 * N + i1] = in[it][c];
-          }
+    for (int u = 0; u < U; ++u) {
+      const int e = tid + (b + u) * TB;
+      if (e < KP * NN) {
+        if constexpr (PREP) {
+          in[u][0] = load_io<R>(xin + e);
+          in[u][1] = load_io<R>(xin + Nq + e);
+          P[u] = pi_comp<R, N>(d, inst, c, k3 * NN + e, lam);
+        } else {
+          in[u][0] = xin[(long long)c * Nq + e];
         }
       }
     }
-    const R sc = scale3<R, N>();
-    if constexpr (sizeof(R) == 4) {
-      __syncthreads();  // the row table
-      if (tid < T) {
-        const PiCol pc = pi_col<N>(lam, k3, side, i1);
 #pragma unroll
-        for (int it = 0; it < ITEMS; ++it) {
-          const int i2 = grp + it * NG;
-          if (i2 < N) {
-            cx<R> v[3];
-            pi_prep(pi_vox(pi_rows<R, N>(sm) + i2, pc), side, in[it][0], in[it][1], sc, v);
-#pragma unroll
-            for (int c = 0; c < 3; ++c) sm[(c * N + i2) * LD + i1] = v[c];
-          }
+    for (int u = 0; u < U; ++u) {
+      const int e = tid + (b + u) * TB;
+      if (e < KP * NN) {
+        const int r = e / N, i1 = e - r * N;
+        cx<R> v = in[u][0];
+        if constexpr (PREP) {
+          if (side == 0) v = cfmac(P[u].p1, in[u][1], cneg(cmulc(P[u].p2, in[u][0])));
+          else v = cfma(P[u].p2, in[u][1], cmul(P[u].p1, in[u][0]));
         }
-      }
-    } else {
-      const cx<R> lz = lam[2 * N + k3];
-#pragma unroll
-      for (int it = 0; it < ITEMS; ++it) {
-        const int i2 = grp + it * NG;
-        if (tid < T && i2 < N) {
-          PiBlock<R> P = pi_at<R, N>(d, inst, k3, i2 * N + i1, lam, i1, i2, lz);
-          const cx<R> a = cscale(in[it][0], sc), b = cscale(in[it][1], sc);
-          cx<R> v0, v1, v2;
-          if (side == 0) {
-            v0 = cfmac(P.p1[0], b, cneg(cmulc(P.p2[0], a)));
-            v1 = cfmac(P.p1[1], b, cneg(cmulc(P.p2[1], a)));
-            v2 = cfmac(P.p1[2], b, cneg(cmulc(P.p2[2], a)));
-          } else {
-            v0 = cfma(P.p2[0], b, cmul(P.p1[0], a));
-            v1 = cfma(P.p2[1], b, cmul(P.p1[1], a));
-            v2 = cfma(P.p2[2], b, cmul(P.p1[2], a));
-          }
-          sm[(0 * N + i2) * LD + i1] = v0;
-          sm[(1 * N + i2) * LD + i1] = v1;
-          sm[(2 * N + i2) * LD + i1] = v2;
-        }
+        sm[r * LD + i1] = v;
       }
     }
   }
   __syncthreads();
-  const int g = tid / (3 * N);
-  const int cp = tid - g * (3 * N);
-  const int c = cp / N, p = cp - c * N;
-  const bool act = tid < T;
-  // x rows (pencil p = row i2 of field c)
-  if (act) with_g<G>(g, [&](auto gc) { split_pass_a<R, N, G, +1, 1, decltype(gc)::value>(sm + (c * N + p) * LD); });
-  __syncthreads();
-  {
-    cx<R> z[M];
-    if (act)
-      with_g<G>(g, [&](auto gc) { split_pass_b_load<R, N, G, 1, decltype(gc)::value>(sm + (c * N + p) * LD, z); });
-    if (act) fft<R, M, +1>(z);
+  const int g = tid / FS::NP, p = tid - g * FS::NP;
+  const bool act = tid < FS::T;
+  field_rows<R, N, +1>(sm, tid, g, p, act);
+  // y columns, written straight to global
+  auto column = [&](int q) { return sm + (q / N) * N * LD + q % N; };
+  if constexpr (G > 1) {
+    split_pass_a<R, N, G, +1, LD, FS::NP, FS::T>(tid, column);
     __syncthreads();
-    if (act)
-      with_g<G>(g, [&](auto gc) { split_pass_b_store<R, N, G, 1, decltype(gc)::value>(sm + (c * N + p) * LD, z); });
   }
-  __syncthreads();
-  // y columns (pencil p = column i1 of field c), written straight to global
-  if (act) with_g<G>(g, [&](auto gc) { split_pass_a<R, N, G, +1, LD, decltype(gc)::value>(sm + c * N * LD + p); });
-  __syncthreads();
   if (act) {
     cx<R> z[M];
-    with_g<G>(g, [&](auto gc) { split_pass_b_load<R, N, G, LD, decltype(gc)::value>(sm + c * N * LD + p, z); });
+    split_pass_b_load<R, N, G, LD>(column(p), g, z);
     fft<R, M, +1>(z);
-    cx<R>* o = out + vec * out_stride + (long long)(blockIdx.y * 3 + c) * Nq + (long long)k3 * N * N + p;
-    with_g<G>(g, [&](auto gc) { split_pass_b_store<R, N, G, N, decltype(gc)::value>(o, z); });
+    cx<R>* o = out + vec * out_stride + (long long)blockIdx.y * Nq + (k3 + p / N) * NN + p % N;
+    split_pass_b_store<R, N, G, N>(o, g, z);
   }
 }
 
-template <class R, int N, int G>
-__global__ void __launch_bounds__(Split<N, G>::TB, plane_min_blocks<R, N, G>())
-k_plane_fwd2(const cx<R>* __restrict__ w, cx<R>* __restrict__ y, PlanData<R> d, VecCtx ctx,
-             long long w_stride, long long out_stride, long long out_side_stride, int side0) {
-  using SP = Split<N, G>;
-  constexpr int M = SP::M, T = SP::T, LD = N + 1;
+// POST: the three field CTAs of one (plane, side, vector) form a cluster; each
+// applies Pi^H on a third of the voxels, reading the other two fields from
+// its neighbours' shared memory.
+template <class R, int N, bool POST>
+__global__ void __launch_bounds__(FieldShape<R, N>::TB)
+k_field_fwd(const cx<R>* __restrict__ w, cx<R>* __restrict__ y, PlanData<R> d, VecCtx ctx, long long w_stride,
+            long long out_stride, long long out_side_stride, int side0) {
+  using FS = FieldShape<R, N>;
+  constexpr int G = FS::G, M = N / G, LD = FS::LD, KP = FS::KP, TB = FS::TB;
+  constexpr int NN = N * N, Nq = NN * N;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  cx<R>* sm = reinterpret_cast<cx<R>*>(smem_raw);  // [3][N][LD]
-  const int k3 = blockIdx.x;
+  cx<R>* sm = reinterpret_cast<cx<R>*>(smem_raw);  // [KP][N][LD]
+  const int k3 = blockIdx.x * KP;
   const int vec = blockIdx.z;
-  if (ctx.active && !ctx.active[vec]) return;
+  if (ctx.active && !ctx.active[vec]) return;  // the same for a whole cluster
   const int inst = vec_inst(ctx, vec);
-  const int side = side0 + blockIdx.y;
-  const long long Nq = (long long)N * N * N;
+  const int c = blockIdx.y % 3, side = side0 + blockIdx.y / 3;
   const int tid = threadIdx.x;
-  const int g = tid / (3 * N);
-  const int cp = tid - g * (3 * N);
-  const int c = cp / N, p = cp - c * N;
-  const bool act = tid < T;
-  const cx<R>* lam = d.lam + (long long)inst * 3 * N;
-  if constexpr (sizeof(R) == 4) {
-    if (tid < N) pi_row_fill<N>(pi_rows<R, N>(sm), lam, k3, side, tid);
-  }
-  // y columns, pass A straight from global (pencil p = column i1 of field c)
-  if (act) {
-    const cx<R>* src = w + vec * w_stride + (long long)(blockIdx.y * 3 + c) * Nq + (long long)k3 * N * N + p;
-    cx<R>* col = sm + c * N * LD + p;
-    with_g<G>(g, [&](auto gc) {
-      constexpr int GC = decltype(gc)::value;
-      cx<R> a[SP::NA][G];
-      static_for<0, SP::NA>([&](auto jc) {
-        constexpr int n2 = GC + decltype(jc)::value * G;
-        if constexpr (n2 < M)
-          static_for<0, G>([&](auto n1c) {
-            a[decltype(jc)::value][decltype(n1c)::value] = src[(long long)SP::in_slot(decltype(n1c)::value, n2) * N];
-          });
-      });
-      static_for<0, SP::NA>([&](auto jc) {
-        constexpr int j = decltype(jc)::value;
-        constexpr int n2 = GC + j * G;
-        if constexpr (n2 < M) {
-          fft<R, G, -1>(a[j]);
-          static_for<0, G>([&](auto n1c) { col[SP::in_slot(decltype(n1c)::value, n2) * LD] = a[j][decltype(n1c)::value]; });
-        }
-      });
-    });
-  }
-  __syncthreads();
-  {
-    cx<R> z[M];
-    if (act)
-      with_g<G>(g, [&](auto gc) { split_pass_b_load<R, N, G, LD, decltype(gc)::value>(sm + c * N * LD + p, z); });
-    if (act) fft<R, M, -1>(z);
-    __syncthreads();
-    if (act)
-      with_g<G>(g, [&](auto gc) { split_pass_b_store<R, N, G, LD, decltype(gc)::value>(sm + c * N * LD + p, z); });
-  }
-  __syncthreads();
-  // x rows (pencil p = row i2 of field c)
-  if (act) with_g<G>(g, [&](auto gc) { split_pass_a<R, N, G, -1, 1, decltype(gc)::value>(sm + (c * N + p) * LD); });
-  __syncthreads();
-  {
-    cx<R> z[M];
-    if (act)
-      with_g<G>(g, [&](auto gc) { split_pass_b_load<R, N, G, 1, decltype(gc)::value>(sm + (c * N + p) * LD, z); });
-    if (act) fft<R, M, -1>(z);
-    __syncthreads();
-    if (act)
-      with_g<G>(g, [&](auto gc) { split_pass_b_store<R, N, G, 1, decltype(gc)::value>(sm + (c * N + p) * LD, z); });
-  }
-  __syncthreads();
-  // Pi^H blocks of this side, scaled for the three forward DFTs
-  cx<R>* o = y + vec * out_stride + blockIdx.y * out_side_stride + (long long)k3 * N * N;
-  const R sc = scale3<R, N>();
-  if (!act) return;
-  const int grp = tid / N, i1 = tid - grp * N;
-  if constexpr (sizeof(R) == 4) {
-    const PiCol pc = pi_col<N>(lam, k3, side, i1);
-#pragma unroll 2
-    for (int i2 = grp; i2 < N; i2 += 3 * G) {
-      const cx<R> u[3] = {sm[(0 * N + i2) * LD + i1], sm[(1 * N + i2) * LD + i1], sm[(2 * N + i2) * LD + i1]};
-      cx<R> a, b;
-      pi_post(pi_vox(pi_rows<R, N>(sm) + i2, pc), side, u, sc, a, b);
-      o[i2 * N + i1] = a;
-      o[Nq + i2 * N + i1] = b;
-    }
-  } else {
-    const cx<R> lz = lam[2 * N + k3];
-    for (int i2 = grp; i2 < N; i2 += 3 * G) {
-      const int e = i2 * N + i1;
-      const cx<R> u0 = sm[(0 * N + i2) * LD + i1];
-      const cx<R> u1 = sm[(1 * N + i2) * LD + i1];
-      const cx<R> u2 = sm[(2 * N + i2) * LD + i1];
-      PiBlock<R> P = pi_at<R, N>(d, inst, k3, e, lam, i1, i2, lz);
-      cx<R> a, b;
-      if (side == 0) {
-        a = cneg(cfma(P.p2[2], u2, cfma(P.p2[1], u1, cmul(P.p2[0], u0))));
-        b = cfma(P.p1[2], u2, cfma(P.p1[1], u1, cmul(P.p1[0], u0)));
-      } else {
-        a = cfmac(P.p1[2], u2, cfmac(P.p1[1], u1, cmulc(P.p1[0], u0)));
-        b = cfmac(P.p2[2], u2, cfmac(P.p2[1], u1, cmulc(P.p2[0], u0)));
+  const int g = tid / FS::NP, p = tid - g * FS::NP;
+  const bool act = tid < FS::T;
+  // y columns, pass A (G = 1: the whole DFT) straight from global, every load
+  // of a thread issued before the first is used
+  const cx<R>* src = w + vec * w_stride + (long long)blockIdx.y * Nq + k3 * NN;
+  auto column = [&](int q) { return sm + (q / N) * N * LD + q % N; };
+  if constexpr (G > 1) {
+    using SP = Split<N, G>;
+    cx<R> a[SP::NA][G];
+#pragma unroll
+    for (int j = 0; j < SP::NA; ++j) {
+      const int idx = tid + j * FS::T;
+      if (act && idx < FS::NP * M) {
+        const int n2 = idx / FS::NP, q = idx - n2 * FS::NP;
+#pragma unroll
+        for (int n1 = 0; n1 < G; ++n1) a[j][n1] = src[(q / N) * NN + SP::in_slot(n1, n2) * N + q % N];
       }
-      store_io<R>(o + e, cscale(a, sc));
-      store_io<R>(o + Nq + e, cscale(b, sc));
+    }
+#pragma unroll
+    for (int j = 0; j < SP::NA; ++j) {
+      const int idx = tid + j * FS::T;
+      if (act && idx < FS::NP * M) {
+        const int n2 = idx / FS::NP;
+        cx<R>* col = column(idx - n2 * FS::NP);
+        pass_a_dft<R, N, G, -1>(a[j], n2);
+#pragma unroll
+        for (int n1 = 0; n1 < G; ++n1) col[SP::in_slot(n1, n2) * LD] = a[j][n1];
+      }
+    }
+    __syncthreads();
+    cx<R> z[M];
+    if (act) {
+      split_pass_b_load<R, N, G, LD>(column(p), g, z);
+      fft<R, M, -1>(z);
+    }
+    __syncthreads();
+    if (act) split_pass_b_store<R, N, G, LD>(column(p), g, z);
+  } else if (act) {
+    cx<R> v[N];
+#pragma unroll
+    for (int i2 = 0; i2 < N; ++i2) v[i2] = src[(p / N) * NN + i2 * N + p % N];
+    fft<R, N, -1>(v);
+    cx<R>* col = column(p);
+#pragma unroll
+    for (int i2 = 0; i2 < N; ++i2) col[i2 * LD] = v[i2];
+  }
+  __syncthreads();
+  field_rows<R, N, -1>(sm, tid, g, p, act);
+  cx<R>* o = y + vec * out_stride + (blockIdx.y / 3) * out_side_stride + k3 * NN;
+  if constexpr (POST) {
+    auto cluster = cooperative_groups::this_cluster();
+    cluster.sync();
+    const cx<R>* u0 = cluster.map_shared_rank(sm, 0);
+    const cx<R>* u1 = cluster.map_shared_rank(sm, 1);
+    const cx<R>* u2 = cluster.map_shared_rank(sm, 2);
+    const cx<R>* lam = d.lam + (long long)inst * 3 * N;
+    for (int e = c * TB + tid; e < KP * NN; e += 3 * TB) {
+      const int r = e / N, i1 = e - r * N;
+      const int q = r * LD + i1;
+      const cx<R> f[3] = {u0[q], u1[q], u2[q]};
+      // side 1: a = X, b = Y with X = sum conj(Pi1) v, Y = sum conj(Pi2) v;
+      // side 0: a = -Y, b = X with conj(Pi) for Pi (one instruction stream:
+      // two branches are computed both and selected)
+      cx<R> X, Y;
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        const PiComp<R> P = pi_comp<R, N>(d, inst, k, k3 * NN + e, lam);
+        const cx<R> p1 = conj_unless(P.p1, side), p2 = conj_unless(P.p2, side);
+        X = k == 0 ? cmulc(p1, f[k]) : cfmac(p1, f[k], X);
+        Y = k == 0 ? cmulc(p2, f[k]) : cfmac(p2, f[k], Y);
+      }
+      const cx<R> a = side ? X : cneg(Y), b = side ? Y : X;
+      store_io<R>(o + e, a);
+      store_io<R>(o + Nq + e, b);
+    }
+    cluster.sync();  // no CTA leaves while its shared memory is read
+  } else {
+    for (int e = tid; e < KP * NN; e += TB) {
+      const int r = e / N, i1 = e - r * N;
+      o[(long long)c * Nq + e] = sm[r * LD + i1];
     }
   }
 }
 
 // ---------------------------------------------------------------------------
-// col: DFT along z of every (i1, i2) column, in place; one thread per column.
-// SMODE 1: multiply S_z(i3) after (inverse); 2: multiply conj(S_z(i3)) before
-// (forward), both scaled by 1/sqrt(n); 0: neither (scale3).
+// col: DFT along z of every (i1, i2) column, src -> dst (which may be the
+// same).  SMODE 1: multiply the Bloch phase S = S_x S_y S_z and scale after
+// (inverse); 2: conj(S) and scale before (forward); 0: neither.
+//
+// complex64: k_col, one thread per column (N complex values in registers,
+// loads and stores coalesced along x).
 // ---------------------------------------------------------------------------
-template <class R, int N, int DIR, int SMODE>
-__global__ void __launch_bounds__(128, sizeof(R) == 4 ? 3 : 1)
-k_col(cx<R>* __restrict__ w, PlanData<R> d, VecCtx ctx, long long stride) {
+template <int N, int DIR, int SMODE>
+__global__ void __launch_bounds__(128, 3)
+k_col(const float2* src, float2* dst, PlanData<float> d, VecCtx ctx, long long stride, float scale) {
   const int col = blockIdx.x * blockDim.x + threadIdx.x;
   const int f = blockIdx.y;
   const int vec = blockIdx.z;
   if (col >= N * N) return;
   if (ctx.active && !ctx.active[vec]) return;
   const long long Nq = (long long)N * N * N;
-  cx<R>* p = w + vec * stride + (long long)f * Nq + col;
-  const cx<R>* Sz = d.sxyz + (long long)vec_inst(ctx, vec) * 3 * N + 2 * N;
-  cx<R> v[N];
+  const long long off = vec * stride + (long long)f * Nq + col;
+  const float2* p = src + off;
+  float2* o = dst + off;
+  const float2* S = d.sxyz + (long long)vec_inst(ctx, vec) * 3 * N;
+  float2 sxy = zero<float>();
+  if constexpr (SMODE != 0) sxy = cscale(cmul(S[col % N], S[N + col / N]), scale);
+  float2 v[N];
 #pragma unroll
   for (int i = 0; i < N; ++i) {
     v[i] = p[(long long)i * N * N];
-    if constexpr (SMODE == 2) v[i] = cmulc(Sz[i], v[i]);
+    if constexpr (SMODE == 2) v[i] = cmulc(cmul(S[2 * N + i], sxy), v[i]);
   }
-  fft<R, N, DIR>(v);
-  constexpr double scale = 1.0 / csqrt_int(N);
+  fft<float, N, DIR>(v);
 #pragma unroll
   for (int i = 0; i < N; ++i) {
-    cx<R> r = v[i];
-    if constexpr (SMODE != 0) r = cscale(r, R(scale));
-    if constexpr (SMODE == 1) r = cmul(Sz[i], r);
-    p[(long long)i * N * N] = r;
+    float2 r = v[i];
+    if constexpr (SMODE == 1) r = cmul(cmul(S[2 * N + i], sxy), r);
+    o[(long long)i * N * N] = r;
   }
 }
 
-inline dim3 grid_pts(long long Nq, int nvec, int tpb) {
-  return dim3((unsigned)((Nq + tpb - 1) / tpb), (unsigned)nvec, 1);
-}
+// complex128 and double-single: k_col2, with the split of the field kernels.
+// One CTA per (W columns, field, vector), W*G threads: pass A straight from
+// global, pass B straight to global.  With W = 32 a warp holds one k1 of 32
+// columns (no idle lanes: whole rows of 40 columns took 52 us where this takes
+// 44, 4 vectors at n = 40).  (One thread per 60-point column needs 255
+// registers and spills; at n = 16 it is a serial chain of 170 FP64 operations.)
+template <int N> FAME_HD constexpr int col_width() { return N <= 16 ? 16 : 32; }
 
-// Lanes per pencil of the split plane kernels for a tuned value (< 0: the
-// default of size N; 0: one thread per pencil) under the plan's option;
-// a count not compiled for N falls back to the default.
-template <class R, int N> inline int plane_lanes(const Plan& P, int tuned) {
-  if (std::is_same<R, ff>::value && (tuned == 0 || !P.opt_plane_split)) tuned = -1;  // double-single: split only
-  else if (!P.opt_plane_split || plane_split(N) == 0 || tuned == 0) return 0;
-  for (int i = 0; i < kPlaneLanesMax; ++i)
-    if (tuned > 0 && plane_lanes_alt(N, i) == tuned) return tuned;
-  return plane_split(N);
-}
-
-// The split an untuned fncB of nvec vectors takes (as a tuned value).  In
-// complex64: one thread per pencil once the 2 N nvec CTAs give every SM its
-// two resident ones (it needs a quarter fewer instructions and half the
-// shared-memory traffic: fncB of 4 vectors at n = 40 60 -> 50 us, 8 at n = 48
-// 116 -> 106, 10 at n = 60 260 -> 246), the size's split below that, where
-// the extra warps hide latency (one vector at n = 48 41.5 -> 37.5 us, n = 60
-// 52 -> 49).  nvec is the whole batch, so sub-batches do not change a result.
-template <class R, int N> inline int default_lanes(const Plan& P, int nvec) {
-  return std::is_same<R, float>::value && N * nvec >= P.sms ? 0 : -1;
-}
-
-// f(integral_constant<G>) for the compiled lane count G == lanes of size N.
-template <class R, int N, class F> inline void with_lanes(int lanes, F&& f) {
-  static_assert(kPlaneLanesMax == 3, "one branch per compiled lane count");
-  constexpr int g0 = plane_lanes_alt(N, 0), g1 = plane_lanes_alt(N, 1), g2 = plane_lanes_alt(N, 2);
-  if constexpr (g0 > 0)
-    if (lanes == g0) return f(std::integral_constant<int, g0>{});
-  if constexpr (g1 > 0)
-    if (lanes == g1) return f(std::integral_constant<int, g1>{});
-  if constexpr (g2 > 0)
-    if (lanes == g2) return f(std::integral_constant<int, g2>{});
-}
-
-template <class R, int N, bool PREP, bool WITH_S>
-cudaError_t plane_inv(const Plan& P, const PlanData<R>& d, const cx<R>* x, cx<R>* out, int nvec,
-                      int nside, int side0, long long in_stride, long long in_side_stride,
-                      long long out_stride, const VecCtx& ctx, cudaStream_t st, DirUpd<R> upd = DirUpd<R>(),
-                      int tuned_lanes = -1) {
-  constexpr size_t sm = plane_smem<R, N>();
-  if constexpr (PREP && !WITH_S && plane_split(N) > 0) {
-    const int lanes = plane_lanes<R, N>(P, tuned_lanes);
-    if (lanes > 0) {
-      cudaError_t e = cudaErrorInvalidValue;
-      // the CG direction update is compiled into its own variant, so the
-      // plain operator carries none of its code (the double-single operator
-      // never takes it)
-      auto launch = [&](auto kfn, int tb) {
-        e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        if (e != cudaSuccess) return;
-        FAME_LAUNCHED(1);
-        kfn<<<dim3(N, nside, nvec), tb, sm, st>>>(x, out, d, ctx, in_stride, in_side_stride, out_stride, side0, upd);
-        e = cudaGetLastError();
-      };
-      with_lanes<R, N>(lanes, [&](auto gc) {
-        constexpr int G = decltype(gc)::value;
-        if constexpr (!std::is_same<R, ff>::value) {
-          if (upd.z) return launch(k_plane_inv2<R, N, G, true>, Split<N, G>::TB);
-        }
-        launch(k_plane_inv2<R, N, G, false>, Split<N, G>::TB);
-      });
-      return e;
-    }
-  }
-  if constexpr (std::is_same<R, ff>::value && PREP && !WITH_S && plane_split(N) > 0) {
-    return cudaErrorInvalidValue;  // double-single: split kernels only (above)
-  } else {
-    const int threads = ((3 * N + 31) / 32) * 32;
-    auto kfn = k_plane_inv<R, N, PREP, WITH_S>;
-    cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    if (e != cudaSuccess) return e;
-    FAME_LAUNCHED(1);
-    kfn<<<dim3(N, nside, nvec), threads, sm, st>>>(x, out, d, ctx, in_stride, in_side_stride, out_stride,
-                                                   side0, upd);
-    return cudaGetLastError();
-  }
-}
-
-template <class R, int N, bool POST, bool WITH_S>
-cudaError_t plane_fwd(const Plan& P, const PlanData<R>& d, const cx<R>* w, cx<R>* y, int nvec, int nside,
-                      int side0, long long w_stride, long long out_stride, long long out_side_stride,
-                      const VecCtx& ctx, cudaStream_t st, int tuned_lanes = -1) {
-  constexpr size_t sm = plane_smem<R, N>();
-  if constexpr (POST && !WITH_S && plane_split(N) > 0) {
-    const int lanes = plane_lanes<R, N>(P, tuned_lanes);
-    if (lanes > 0) {
-      cudaError_t e = cudaErrorInvalidValue;
-      with_lanes<R, N>(lanes, [&](auto gc) {
-        constexpr int G = decltype(gc)::value;
-        auto kfn = k_plane_fwd2<R, N, G>;
-        e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        if (e != cudaSuccess) return;
-        FAME_LAUNCHED(1);
-        kfn<<<dim3(N, nside, nvec), Split<N, G>::TB, sm, st>>>(w, y, d, ctx, w_stride, out_stride,
-                                                               out_side_stride, side0);
-        e = cudaGetLastError();
-      });
-      return e;
-    }
-  }
-  if constexpr (std::is_same<R, ff>::value && POST && !WITH_S && plane_split(N) > 0) {
-    return cudaErrorInvalidValue;  // double-single: split kernels only (above)
-  } else {
-    const int threads = ((3 * N + 31) / 32) * 32;
-    auto kfn = k_plane_fwd<R, N, POST, WITH_S>;
-    cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    if (e != cudaSuccess) return e;
-    FAME_LAUNCHED(1);
-    kfn<<<dim3(N, nside, nvec), threads, sm, st>>>(w, y, d, ctx, w_stride, out_stride, out_side_stride,
-                                                   side0);
-    return cudaGetLastError();
-  }
-}
-
-// ---------------------------------------------------------------------------
-// col2: the z-DFT with the same prime-factor split as the plane kernels, for
-// the double-single type (one thread holding a whole 60-point column of
-// float-float pairs needs 240 registers of data alone).  One CTA per
-// (y row, field, vector): the row's N columns (all z) are staged in shared
-// memory with coalesced row loads, G threads per column do the length-G
-// passes in place, then each the length-M DFT of its sub-pencil in
-// registers, written straight back to global (consecutive threads hold
-// consecutive x).  No scale (scale3), no S multiply.
-// ---------------------------------------------------------------------------
-template <class R, int N, int DIR>
-__global__ void __launch_bounds__(((N * plane_split(N) + 31) / 32) * 32)
-k_col2(cx<R>* __restrict__ w, VecCtx ctx, long long stride) {
-  constexpr int G = plane_split(N);
+template <class R, int N, int DIR, int SMODE>
+__global__ void __launch_bounds__(((col_width<N>() * field_split(N) + 31) / 32) * 32)
+k_col2(const cx<R>* src, cx<R>* dst, PlanData<R> d, VecCtx ctx, long long stride, R scale) {
+  constexpr int G = field_split(N);
   using SP = Split<N, G>;
-  constexpr int M = SP::M, LD = N + 1, T = N * G;
+  constexpr int M = SP::M, W = col_width<N>(), LD = W + 1, T = W * G, NN = N * N;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cx<R>* sm = reinterpret_cast<cx<R>*>(smem_raw);  // [z][LD]
-  const int y = blockIdx.x;
   const int vec = blockIdx.z;
   if (ctx.active && !ctx.active[vec]) return;
-  const long long NN = (long long)N * N;
-  cx<R>* base = w + vec * stride + (long long)blockIdx.y * N * NN + (long long)y * N;
   const int tid = threadIdx.x;
-  for (int e = tid; e < N * N; e += blockDim.x) {
-    const int z = e / N, x = e - z * N;
-    sm[z * LD + x] = base[(long long)z * NN + x];
+  const int g = tid / W, x = tid - g * W;  // T threads: row k1 = g of column col
+  const int col = blockIdx.x * W + x;
+  const bool act = tid < T && col < NN;
+  const long long off = vec * stride + (long long)blockIdx.y * N * NN + blockIdx.x * W;
+  const cx<R>* p = src + off;
+  cx<R>* o = dst + off;
+  const cx<R>* S = d.sxyz + (long long)vec_inst(ctx, vec) * 3 * N;
+  cx<R> sxy = zero<R>();
+  if constexpr (SMODE != 0) sxy = cscale(cmul(S[col % N], S[N + (col / N) % N]), scale);
+  if constexpr (G > 1) {
+    cx<R> a[SP::NA][G];
+#pragma unroll
+    for (int j = 0; j < SP::NA; ++j) {
+      const int n2 = g + j * G;  // the round's DFTs n2 of this column
+      if (act && n2 < M) {
+#pragma unroll
+        for (int n1 = 0; n1 < G; ++n1) {
+          const int z = SP::in_slot(n1, n2);
+          a[j][n1] = p[z * NN + x];
+          if constexpr (SMODE == 2) a[j][n1] = cmulc(cmul(S[2 * N + z], sxy), a[j][n1]);
+        }
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < SP::NA; ++j) {
+      const int n2 = g + j * G;
+      if (act && n2 < M) {
+        pass_a_dft<R, N, G, DIR>(a[j], n2);
+#pragma unroll
+        for (int n1 = 0; n1 < G; ++n1) sm[SP::in_slot(n1, n2) * LD + x] = a[j][n1];
+      }
+    }
+    __syncthreads();
   }
-  __syncthreads();
-  const int g = tid / N, p = tid - g * N;
-  const bool act = tid < T;
-  if (act) with_g<G>(g, [&](auto gc) { split_pass_a<R, N, G, DIR, LD, decltype(gc)::value>(sm + p); });
-  __syncthreads();
   if (act) {
     cx<R> z[M];
-    with_g<G>(g, [&](auto gc) { split_pass_b_load<R, N, G, LD, decltype(gc)::value>(sm + p, z); });
+    if constexpr (G > 1) {
+      split_pass_b_load<R, N, G, LD>(sm + x, g, z);
+    } else {
+#pragma unroll
+      for (int i = 0; i < M; ++i) {
+        z[i] = p[i * NN + x];
+        if constexpr (SMODE == 2) z[i] = cmulc(cmul(S[2 * N + i], sxy), z[i]);
+      }
+    }
     fft<R, M, DIR>(z);
-    with_g<G>(g, [&](auto gc) { split_pass_b_store<R, N, G, (int)(N * N), decltype(gc)::value>(base + p, z); });
+#pragma unroll
+    for (int k2 = 0; k2 < M; ++k2) {
+      const int k = SP::out_slot(g, k2);
+      cx<R> r = z[k2];
+      if constexpr (SMODE == 1) r = cmul(cmul(S[2 * N + k], sxy), r);
+      o[k * NN + x] = r;
+    }
+  }
+}
+
+// Launch of kernel K as clusters of (1, cluster, 1) CTAs (cluster 1: plain).
+template <class K, class... A>
+inline cudaError_t launch_clustered(K kfn, dim3 grid, int tb, size_t sm, int cluster, cudaStream_t st, A... args) {
+  cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  if (e != cudaSuccess) return e;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(tb);
+  cfg.dynamicSmemBytes = sm;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = 1;
+  at[0].val.clusterDim.y = cluster;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = cluster > 1 ? 1 : 0;
+  FAME_LAUNCHED(1);
+  return cudaLaunchKernelEx(&cfg, kfn, args...);
+}
+
+template <class R, int N, bool PREP>
+cudaError_t plane_inv(const PlanData<R>& d, const cx<R>* x, cx<R>* out, int nvec, int nside, int side0,
+                      long long in_stride, long long in_side_stride, long long out_stride, const VecCtx& ctx,
+                      cudaStream_t st, DirUpd<R> upd = DirUpd<R>()) {
+  if constexpr (sizeof(cx<R>) == 8) {
+    return launch_clustered(k_plane_inv<N, PREP>, dim3(N, nside, nvec), ((3 * N + 31) / 32) * 32, plane_smem<N>(), 1,
+                            st, x, out, d, ctx, in_stride, in_side_stride, out_stride, side0, upd);
+  } else {
+    using FS = FieldShape<R, N>;
+    return launch_clustered(k_field_inv<R, N, PREP>, dim3(N / FS::KP, 3 * nside, nvec), FS::TB, FS::SMEM, 1, st, x, out,
+                            d, ctx, in_stride, in_side_stride, out_stride, side0);
+  }
+}
+
+template <class R, int N, bool POST>
+cudaError_t plane_fwd(const PlanData<R>& d, const cx<R>* w, cx<R>* y, int nvec, int nside, int side0,
+                      long long w_stride, long long out_stride, long long out_side_stride, const VecCtx& ctx,
+                      cudaStream_t st) {
+  if constexpr (sizeof(cx<R>) == 8) {
+    return launch_clustered(k_plane_fwd<N, POST>, dim3(N, nside, nvec), ((3 * N + 31) / 32) * 32, plane_smem<N>(), 1,
+                            st, w, y, d, ctx, w_stride, out_stride, out_side_stride, side0);
+  } else {
+    using FS = FieldShape<R, N>;
+    return launch_clustered(k_field_fwd<R, N, POST>, dim3(N / FS::KP, 3 * nside, nvec), FS::TB, FS::SMEM, POST ? 3 : 1,
+                            st, w, y, d, ctx, w_stride, out_stride, out_side_stride, side0);
   }
 }
 
 template <class R, int N, int DIR, int SMODE>
-cudaError_t col(const Plan& P, const PlanData<R>& d, cx<R>* w, int nfield, int nvec, long long stride, const VecCtx& ctx,
-                cudaStream_t st) {
-  if constexpr (std::is_same<R, ff>::value && SMODE == 0 && plane_split(N) > 0) {
-    constexpr int G = plane_split(N);
-    const size_t sm = sizeof(cx<R>) * N * (N + 1);
-    auto kfn = k_col2<R, N, DIR>;
-    cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    if (e != cudaSuccess) return e;
-    FAME_LAUNCHED(1);
-    kfn<<<dim3(N, nfield, nvec), ((N * G + 31) / 32) * 32, sm, st>>>(w, ctx, stride);
-    return cudaGetLastError();
+cudaError_t col(const Plan& P, const PlanData<R>& d, const cx<R>* src, cx<R>* dst, int nfield, int nvec,
+                long long stride, const VecCtx& ctx, cudaStream_t st, R scale = R(1)) {
+  if constexpr (sizeof(cx<R>) == 16) {
+    constexpr int G = field_split(N), W = col_width<N>();
+    return launch_clustered(k_col2<R, N, DIR, SMODE>, dim3((N * N + W - 1) / W, nfield, nvec),
+                            ((W * G + 31) / 32) * 32, G > 1 ? sizeof(cx<R>) * N * (W + 1) : 0, 1, st, src, dst, d, ctx,
+                            stride, scale);
   } else {
-    // One warp per CTA in complex128 and for small complex64 batches: the work
-    // of a launch is then spread over the SMs warp by warp (two vectors at
-    // n = 30 are 96 CTAs of four warps, up to four warps on an SM where the
-    // even share is 2.2: 23 -> 16 us), 128 threads where there are plenty.
-    const int tpb = sizeof(R) == 8 || (long long)N * N * nfield * nvec < 128LL * 6 * P.sms ? 32 : 128;
+    // one warp per CTA for small batches, so that the work spreads over the
+    // SMs, 128 threads where there are plenty
+    const int tpb = (long long)N * N * nfield * nvec < 128LL * 6 * P.sms ? 32 : 128;
     dim3 g((N * N + tpb - 1) / tpb, nfield, nvec);
     FAME_LAUNCHED(1);
-    k_col<R, N, DIR, SMODE><<<g, tpb, 0, st>>>(w, d, ctx, stride);
+    k_col<N, DIR, SMODE><<<g, tpb, 0, st>>>(src, dst, d, ctx, stride, scale);
     return cudaGetLastError();
   }
 }
@@ -1048,20 +944,17 @@ cudaError_t col(const Plan& P, const PlanData<R>& d, cx<R>* w, int nfield, int n
 // w^H [M J^H; J N] w for the spatial fields w the stencil reads; the stencil
 // pass accumulates it while it writes its output.
 //
-// pupd_z / pupd_beta (may be null): x is a CG direction p, updated first as
-// p = z + beta p (in place) by the plane kernel that reads it.
+// pupd_z / pupd_beta (may be null, complex64 only): x is a CG direction p,
+// updated first as p = z + beta p (in place) by the plane kernel that reads it.
 template <class R, int N>
 cudaError_t fncB_n(const Plan& P, const cx<R>* x, cx<R>* y, int nvec, const VecCtx& ctx, cx<R>* w0, cx<R>* w1,
                    cudaStream_t st, double2* pq, const cx<R>* pupd_z, const double* pupd_beta) {
-  static_assert(!std::is_same<R, ff>::value || plane_split(N) > 0,
-                "the double-single fncB reads and writes complex128 through the split plane kernels");
   PlanData<R> d = pdata<R>(P);
   if (!P.opt_pi_table) d.pi = nullptr;  // evaluate Pi in the plane kernels instead
   const long long Nq = P.Nq;
   const TuneEntry tn = tune_for(P, tune_prec<R>(), nvec);
   const int chunk = sub_batch(tn, nvec);
   const int tz = sweep_planes<R, N>(P, chunk);
-  const int lanes = tn.lanes >= 0 ? tn.lanes : default_lanes<R, N>(P, nvec);
   for (int v0 = 0; v0 < nvec; v0 += chunk) {
     const int nv = std::min(chunk, nvec - v0);
     const VecCtx c = sub_ctx(ctx, v0);
@@ -1073,9 +966,9 @@ cudaError_t fncB_n(const Plan& P, const cx<R>* x, cx<R>* y, int nvec, const VecC
       upd.z = pupd_z + (size_t)v0 * 4 * Nq;
       upd.beta = pupd_beta + v0;
     }
-    e = plane_inv<R, N, true, false>(P, d, xs, w0, nv, 2, 0, 4 * Nq, 2 * Nq, 6 * Nq, c, st, upd, lanes);
+    e = plane_inv<R, N, true>(d, xs, w0, nv, 2, 0, 4 * Nq, 2 * Nq, 6 * Nq, c, st, upd);
     if (e != cudaSuccess) return e;
-    e = col<R, N, +1, 0>(P, d, w0, 6, nv, 6 * Nq, c, st);
+    e = col<R, N, +1, 0>(P, d, w0, w0, 6, nv, 6 * Nq, c, st);
     if (e != cudaSuccess) return e;
     // material stencil: single pass w0 -> w1, or the two-kernel form in place on w0
     cx<R>* wm = w0;
@@ -1086,9 +979,9 @@ cudaError_t fncB_n(const Plan& P, const cx<R>* x, cx<R>* y, int nvec, const VecC
       e = stencil_n<R, N>(P, w0, w0, w1, nv, c, st, tn.stencil_tpb, false);
     }
     if (e != cudaSuccess) return e;
-    e = col<R, N, -1, 0>(P, d, wm, 6, nv, 6 * Nq, c, st);
+    e = col<R, N, -1, 0>(P, d, wm, wm, 6, nv, 6 * Nq, c, st);
     if (e != cudaSuccess) return e;
-    e = plane_fwd<R, N, true, false>(P, d, wm, ys, nv, 2, 0, 6 * Nq, 4 * Nq, 2 * Nq, c, st, lanes);
+    e = plane_fwd<R, N, true>(d, wm, ys, nv, 2, 0, 6 * Nq, 4 * Nq, 2 * Nq, c, st);
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
@@ -1098,9 +991,9 @@ template <class R, int N>
 cudaError_t fields_inv_n(const Plan& P, const cx<R>* x, cx<R>* w, int nvec, const VecCtx& ctx, cudaStream_t st) {
   const PlanData<R>& d = pdata<R>(P);
   const long long Nq = P.Nq;
-  cudaError_t e = plane_inv<R, N, true, false>(P, d, x, w, nvec, 2, 0, 4 * Nq, 2 * Nq, 6 * Nq, ctx, st);
+  cudaError_t e = plane_inv<R, N, true>(d, x, w, nvec, 2, 0, 4 * Nq, 2 * Nq, 6 * Nq, ctx, st);
   if (e != cudaSuccess) return e;
-  return col<R, N, +1, 0>(P, d, w, 6, nvec, 6 * Nq, ctx, st);
+  return col<R, N, +1, 0>(P, d, w, w, 6, nvec, 6 * Nq, ctx, st);
 }
 
 template <class R, int N>
@@ -1108,20 +1001,17 @@ cudaError_t transform_n(const Plan& P, int trans, const cx<R>* x, cx<R>* y, int 
                         cudaStream_t st) {
   const PlanData<R>& d = pdata<R>(P);
   const long long Nq = P.Nq;
+  const R scale = R(1.0 / (double(N) * csqrt_int(N)));
   cudaError_t e;
   if (trans == 0) {
-    e = plane_inv<R, N, false, true>(P, d, x, y, nvec, 1, 0, 3 * Nq, 0, 3 * Nq, ctx, st);
+    e = plane_inv<R, N, false>(d, x, y, nvec, 1, 0, 3 * Nq, 0, 3 * Nq, ctx, st);
     if (e != cudaSuccess) return e;
-    return col<R, N, +1, 1>(P, d, y, 3, nvec, 3 * Nq, ctx, st);
+    return col<R, N, +1, 1>(P, d, y, y, 3, nvec, 3 * Nq, ctx, st, scale);
   }
-  // transpose: z first (conj(S_z) before), then y, x with conj(S_x S_y) before.
-  if (x != y) {
-    e = cudaMemcpyAsync(y, x, sizeof(cx<R>) * 3 * Nq * nvec, cudaMemcpyDeviceToDevice, st);
-    if (e != cudaSuccess) return e;
-  }
-  e = col<R, N, -1, 2>(P, d, y, 3, nvec, 3 * Nq, ctx, st);
+  // transpose: z first (with conj(S) before), then y, x
+  e = col<R, N, -1, 2>(P, d, x, y, 3, nvec, 3 * Nq, ctx, st, scale);
   if (e != cudaSuccess) return e;
-  return plane_fwd<R, N, false, true>(P, d, y, y, nvec, 1, 0, 3 * Nq, 3 * Nq, 0, ctx, st);
+  return plane_fwd<R, N, false>(d, y, y, nvec, 1, 0, 3 * Nq, 3 * Nq, 0, ctx, st);
 }
 
 template <class R, int N>
@@ -1131,16 +1021,14 @@ cudaError_t handle_n(const Plan& P, int which, const cx<R>* x, cx<R>* y, int nve
   const long long Nq = P.Nq;
   cudaError_t e;
   if (which == 0 || which == 1) {  // Pr / Qr : 2Nq -> 3Nq
-    e = plane_inv<R, N, true, true>(P, d, x, y, nvec, 1, which, 2 * Nq, 0, 3 * Nq, ctx, st);
+    e = plane_inv<R, N, true>(d, x, y, nvec, 1, which, 2 * Nq, 0, 3 * Nq, ctx, st);
     if (e != cudaSuccess) return e;
-    return col<R, N, +1, 1>(P, d, y, 3, nvec, 3 * Nq, ctx, st);
+    return col<R, N, +1, 1>(P, d, y, y, 3, nvec, 3 * Nq, ctx, st);
   }
   // Prs / Qrs : 3Nq -> 2Nq through the 3Nq scratch w0
-  e = cudaMemcpyAsync(w0, x, sizeof(cx<R>) * 3 * Nq * nvec, cudaMemcpyDeviceToDevice, st);
+  e = col<R, N, -1, 2>(P, d, x, w0, 3, nvec, 3 * Nq, ctx, st);
   if (e != cudaSuccess) return e;
-  e = col<R, N, -1, 2>(P, d, w0, 3, nvec, 3 * Nq, ctx, st);
-  if (e != cudaSuccess) return e;
-  return plane_fwd<R, N, true, true>(P, d, w0, y, nvec, 1, which - 2, 3 * Nq, 2 * Nq, 0, ctx, st);
+  return plane_fwd<R, N, true>(d, w0, y, nvec, 1, which - 2, 3 * Nq, 2 * Nq, 0, ctx, st);
 }
 
 

@@ -2,6 +2,7 @@
 // size-templated transforms and material stencil instantiated in
 // fncb_inst_*.cu.
 #include "fncb_impl.cuh"
+#include "krylov.h"
 
 namespace fame {
 namespace detail {
@@ -30,8 +31,8 @@ __global__ void k_fncA(const cx<R>* __restrict__ x, cx<R>* __restrict__ y, PlanD
   yv[3 * Nq] = cscale(cmul_i<-1>(b1), inv);
 }
 
-// Pi1 | Pi2 per frequency voxel of each instance (SVD_Matrix_curl.m:45-57),
-// the same pi_block the transform kernels would evaluate.
+// n^{-3/2} (Pi1 | Pi2) per frequency voxel of each instance
+// (SVD_Matrix_curl.m:45-57), [6][n^3]: what pi_comp would evaluate.
 template <class R>
 __global__ void k_pi_table(const cx<R>* __restrict__ lam_all, int n, long long Nq, cx<R>* __restrict__ out) {
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -40,11 +41,12 @@ __global__ void k_pi_table(const cx<R>* __restrict__ lam_all, int n, long long N
   const int i1 = int(idx % n), i2 = int((idx / n) % n), i3 = int(idx / ((long long)n * n));
   const cx<R>* lam = lam_all + (long long)inst * 3 * n;
   const PiBlock<R> P = pi_block<R>(lam[i1], lam[n + i2], lam[2 * n + i3]);
-  cx<R>* o = out + ((long long)inst * Nq + idx) * 6;
+  const R sc = R(1) / (R(n) * sqrt(R(n)));
+  cx<R>* o = out + (long long)inst * 6 * Nq + idx;
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
-    o[i] = P.p1[i];
-    o[3 + i] = P.p2[i];
+    o[i * Nq] = cscale(P.p1[i], sc);
+    o[(3 + i) * Nq] = cscale(P.p2[i], sc);
   }
 }
 
@@ -225,6 +227,17 @@ template <class R>
 cudaError_t launch_fncB(const Plan& P, const cx<R>* x, cx<R>* y, int nvec, const VecCtx& ctx, cx<R>* w0,
                         cx<R>* w1, cudaStream_t st, double2* pq, const cx<R>* pupd_z, const double* pupd_beta) {
   if (nvec <= 0) return cudaSuccess;
+  if constexpr (sizeof(R) == 8) {
+    // complex128: the CG direction in its own pass (three field CTAs read each
+    // element of x, so none of them may rewrite it; the pass is small beside
+    // the FP64 arithmetic)
+    if (pupd_z) {
+      const long long L = 4 * P.Nq;
+      cudaError_t e = cg_p<R>(const_cast<cx<R>*>(x), pupd_z, L, L, nvec, pupd_beta, ctx.active, st);
+      if (e != cudaSuccess) return e;
+      pupd_z = nullptr;
+    }
+  }
   switch (P.n) {
 #define FAME_CASE(NN) case NN: return fncB_n<R, NN>(P, x, y, nvec, ctx, w0, w1, st, pq, pupd_z, pupd_beta);
     FAME_FOR_EACH_N(FAME_CASE)

@@ -197,8 +197,7 @@ int pcg_batched(Plan& P, const cx<R>* b, cx<R>* x, int nvec, const int* d_inst, 
                                        sizeof(R) == 4 ? (uintptr_t)P.d32.pc : (uintptr_t)P.d64.pc,
                                        (uintptr_t)tune_for(P, tune_prec<R>(), nvec).chunk,
                                        (uintptr_t)tune_for(P, tune_prec<R>(), nvec).stencil_tpb,
-                                       (uintptr_t)nblk_pq, (uintptr_t)P.opt_plane_split,
-                                       (uintptr_t)P.opt_pi_table};
+                                       (uintptr_t)nblk_pq, (uintptr_t)P.opt_pi_table};
   bool use_graph = P.opt_graph != 0;
   bool any = std::any_of(act.begin(), act.end(), [](int a) { return a != 0; });
   int it = 1;

@@ -235,8 +235,8 @@ class Plan:
         count).  With `cache` (a JSON file path) a setting measured before on
         the same device, grid, precision and width is installed without
         re-timing, and new measurements are added to the file.
-        Returns dict(chunk, stencil_tpb, lanes, us, cached) (lanes: threads
-        per FFT pencil of the plane kernels, -1 the size's default)."""
+        Returns dict(chunk, stencil_tpb, lanes, us, cached) (lanes: always -1,
+        one split of the FFT pencils is compiled per size and precision)."""
         import json
         import os
         nvec = self.nk if nvec is None else int(nvec)

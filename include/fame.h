@@ -99,9 +99,8 @@ int fame_set_stream(fame_plan_t plan, void* stream);
  *                     tolerance, which is tightened by the spread of the
  *                     wanted Ritz values and starts there at near-zero wave
  *                     vectors [1e-13].
- *   FAME_OPT_PLANE_SPLIT  fncB plane kernels with several threads per FFT
- *                     pencil on the grid sizes that have them [1]; 0 keeps
- *                     one thread per pencil (same results to rounding).
+ *   FAME_OPT_PLANE_SPLIT  accepted, without effect: the transform kernels
+ *                     take one split of the FFT pencils per size and precision.
  *   FAME_OPT_SIRA_NEAREST  fame_jdsira's Ritz choice: 0 the reference's 'CL'
  *                     (real Ritz values above the target, closest first;
  *                     Choose_Ritz_Pair_Unsymm4.m:176-186) [0]; 1 the closest
@@ -159,15 +158,13 @@ int fame_refine_residuals(fame_plan_t plan, double* before, int n);
  * fncB sequence for precision `prec` and batch width `nvec` on this plan
  * (vectors per launch sequence: the whole batch, 1/2, 1/4, 1/8 of it or any
  * width up to 16; the material stencil: 0 = single pass, or 128, 256, 512
- * threads per block of the two-kernel form; the plane kernels' split of each
- * FFT pencil: threads per pencil, every count compiled for the grid size, or
- * one) and keep the fastest for later calls with that width.  Outputs (may be
- * NULL): the chosen chunk (0 = whole batch), stencil setting and the measured
- * microseconds of one fncB.  fame_set_tune installs a chunk and stencil
- * setting directly (e.g. from a cache), keeping the width's split;
- * fame_set_tune_lanes installs the split (-1 = the size's default, 0 = one
- * thread per pencil, else a compiled count; others fall back to the
- * default); fame_get_tune reads the installed setting (lanes -1 = default).
+ * threads per block of the two-kernel form) and keep the fastest for later
+ * calls with that width.  Outputs (may be NULL): the chosen chunk (0 = whole
+ * batch), stencil setting and the measured microseconds of one fncB.
+ * fame_set_tune installs a chunk and stencil setting directly (e.g. from a
+ * cache).  fame_set_tune_lanes records a count of threads per FFT pencil
+ * (-1 = default) that fame_get_tune returns; every size and precision has one
+ * compiled split, so it has no other effect.
  */
 int fame_autotune(fame_plan_t plan, int prec, int nvec, int* chunk, int* stencil_tpb, double* us);
 int fame_set_tune(fame_plan_t plan, int prec, int nvec, int chunk, int stencil_tpb);
