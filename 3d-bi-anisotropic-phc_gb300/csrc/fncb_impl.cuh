@@ -45,6 +45,7 @@
 
 #include "fame_internal.h"
 #include "fft_reg.cuh"
+#include "launch.h"
 #include "fncb_material.cuh"
 
 namespace fame {
@@ -278,7 +279,6 @@ k_plane_inv(const float2* __restrict__ x, float2* __restrict__ out, PlanData<flo
   float2* sm = reinterpret_cast<float2*>(smem_raw);  // [3][N][LD]
   const int k3 = blockIdx.x;
   const int vec = blockIdx.z;
-  if (ctx.active && !ctx.active[vec]) return;
   const int inst = vec_inst(ctx, vec);
   const int side = side0 + blockIdx.y;
   const long long Nq = (long long)N * N * N;
@@ -292,9 +292,11 @@ k_plane_inv(const float2* __restrict__ x, float2* __restrict__ out, PlanData<flo
   // any is used, so a CTA waits for one memory round trip per batch.
   const int grp = tid / N, i1 = tid - grp * N;
   const bool act = tid < 3 * N;
-  if constexpr (PREP) {
+  if constexpr (PREP) {  // plan tables only: before the wait
     if (tid < N) pi_row_fill<N>(pi_rows<N>(sm), lam, k3, side, tid);
   }
+  pdl_wait();
+  if (ctx.active && !ctx.active[vec]) return;
   constexpr int ITEMS = (N + 2) / 3;
   constexpr int NB = PREP ? 2 : 3;                        // input blocks
   constexpr int NBATCH = (ITEMS * NB + 23) / 24;
@@ -393,7 +395,6 @@ k_plane_fwd(const float2* __restrict__ w, float2* __restrict__ y, PlanData<float
   float2* sm = reinterpret_cast<float2*>(smem_raw);  // [3][N][LD]
   const int k3 = blockIdx.x;
   const int vec = blockIdx.z;
-  if (ctx.active && !ctx.active[vec]) return;
   const int inst = vec_inst(ctx, vec);
   const int side = side0 + blockIdx.y;
   const long long Nq = (long long)N * N * N;
@@ -404,6 +405,8 @@ k_plane_fwd(const float2* __restrict__ w, float2* __restrict__ y, PlanData<float
   if constexpr (POST) {
     if (tid < N) pi_row_fill<N>(pi_rows<N>(sm), lam, k3, side, tid);
   }
+  pdl_wait();
+  if (ctx.active && !ctx.active[vec]) return;
   if (act) {  // y columns (field grp, column i1)
     const float2* src = w + vec * w_stride + (long long)(blockIdx.y * 3 + grp) * Nq + (long long)k3 * N * N + i1;
     float2 v[N];
@@ -592,6 +595,7 @@ k_field_inv(const cx<R>* __restrict__ x, cx<R>* __restrict__ out, PlanData<R> d,
   cx<R>* sm = reinterpret_cast<cx<R>*>(smem_raw);  // [KP][N][LD]
   const int k3 = blockIdx.x * KP;
   const int vec = blockIdx.z;
+  pdl_wait();
   if (ctx.active && !ctx.active[vec]) return;
   const int inst = vec_inst(ctx, vec);
   const int c = blockIdx.y % 3, side = side0 + blockIdx.y / 3;
@@ -664,6 +668,7 @@ k_field_fwd(const cx<R>* __restrict__ w, cx<R>* __restrict__ y, PlanData<R> d, V
   cx<R>* sm = reinterpret_cast<cx<R>*>(smem_raw);  // [KP][N][LD]
   const int k3 = blockIdx.x * KP;
   const int vec = blockIdx.z;
+  pdl_wait();
   if (ctx.active && !ctx.active[vec]) return;  // the same for a whole cluster
   const int inst = vec_inst(ctx, vec);
   const int c = blockIdx.y % 3, side = side0 + blockIdx.y / 3;
@@ -766,6 +771,7 @@ k_col(const float2* src, float2* dst, PlanData<float> d, VecCtx ctx, long long s
   const int col = blockIdx.x * blockDim.x + threadIdx.x;
   const int f = blockIdx.y;
   const int vec = blockIdx.z;
+  pdl_wait();
   if (col >= N * N) return;
   if (ctx.active && !ctx.active[vec]) return;
   const long long Nq = (long long)N * N * N;
@@ -807,6 +813,7 @@ k_col2(const cx<R>* src, cx<R>* dst, PlanData<R> d, VecCtx ctx, long long stride
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cx<R>* sm = reinterpret_cast<cx<R>*>(smem_raw);  // [z][LD]
   const int vec = blockIdx.z;
+  pdl_wait();
   if (ctx.active && !ctx.active[vec]) return;
   const int tid = threadIdx.x;
   const int g = tid / W, x = tid - g * W;  // T threads: row k1 = g of column col
@@ -865,38 +872,17 @@ k_col2(const cx<R>* src, cx<R>* dst, PlanData<R> d, VecCtx ctx, long long stride
   }
 }
 
-// Launch of kernel K as clusters of (1, cluster, 1) CTAs (cluster 1: plain).
-template <class K, class... A>
-inline cudaError_t launch_clustered(K kfn, dim3 grid, int tb, size_t sm, int cluster, cudaStream_t st, A... args) {
-  cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  if (e != cudaSuccess) return e;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3(tb);
-  cfg.dynamicSmemBytes = sm;
-  cfg.stream = st;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = 1;
-  at[0].val.clusterDim.y = cluster;
-  at[0].val.clusterDim.z = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = cluster > 1 ? 1 : 0;
-  FAME_LAUNCHED(1);
-  return cudaLaunchKernelEx(&cfg, kfn, args...);
-}
-
 template <class R, int N, bool PREP>
 cudaError_t plane_inv(const PlanData<R>& d, const cx<R>* x, cx<R>* out, int nvec, int nside, int side0,
                       long long in_stride, long long in_side_stride, long long out_stride, const VecCtx& ctx,
                       cudaStream_t st, DirUpd<R> upd = DirUpd<R>()) {
   if constexpr (sizeof(cx<R>) == 8) {
-    return launch_clustered(k_plane_inv<N, PREP>, dim3(N, nside, nvec), ((3 * N + 31) / 32) * 32, plane_smem<N>(), 1,
-                            st, x, out, d, ctx, in_stride, in_side_stride, out_stride, side0, upd);
+    return launch<k_plane_inv<N, PREP>>(dim3(N, nside, nvec), ((3 * N + 31) / 32) * 32, plane_smem<N>(), st, x, out,
+                                            d, ctx, in_stride, in_side_stride, out_stride, side0, upd);
   } else {
     using FS = FieldShape<R, N>;
-    return launch_clustered(k_field_inv<R, N, PREP>, dim3(N / FS::KP, 3 * nside, nvec), FS::TB, FS::SMEM, 1, st, x, out,
-                            d, ctx, in_stride, in_side_stride, out_stride, side0);
+    return launch<k_field_inv<R, N, PREP>>(dim3(N / FS::KP, 3 * nside, nvec), FS::TB, FS::SMEM, st, x, out, d, ctx,
+                                               in_stride, in_side_stride, out_stride, side0);
   }
 }
 
@@ -905,12 +891,12 @@ cudaError_t plane_fwd(const PlanData<R>& d, const cx<R>* w, cx<R>* y, int nvec, 
                       long long w_stride, long long out_stride, long long out_side_stride, const VecCtx& ctx,
                       cudaStream_t st) {
   if constexpr (sizeof(cx<R>) == 8) {
-    return launch_clustered(k_plane_fwd<N, POST>, dim3(N, nside, nvec), ((3 * N + 31) / 32) * 32, plane_smem<N>(), 1,
-                            st, w, y, d, ctx, w_stride, out_stride, out_side_stride, side0);
+    return launch<k_plane_fwd<N, POST>>(dim3(N, nside, nvec), ((3 * N + 31) / 32) * 32, plane_smem<N>(), st, w, y, d,
+                                            ctx, w_stride, out_stride, out_side_stride, side0);
   } else {
     using FS = FieldShape<R, N>;
-    return launch_clustered(k_field_fwd<R, N, POST>, dim3(N / FS::KP, 3 * nside, nvec), FS::TB, FS::SMEM, POST ? 3 : 1,
-                            st, w, y, d, ctx, w_stride, out_stride, out_side_stride, side0);
+    return launch<k_field_fwd<R, N, POST>, POST ? 3 : 1>(dim3(N / FS::KP, 3 * nside, nvec), FS::TB, FS::SMEM, st, w,
+                                                             y, d, ctx, w_stride, out_stride, out_side_stride, side0);
   }
 }
 
@@ -919,17 +905,15 @@ cudaError_t col(const Plan& P, const PlanData<R>& d, const cx<R>* src, cx<R>* ds
                 long long stride, const VecCtx& ctx, cudaStream_t st, R scale = R(1)) {
   if constexpr (sizeof(cx<R>) == 16) {
     constexpr int G = field_split(N), W = col_width<N>();
-    return launch_clustered(k_col2<R, N, DIR, SMODE>, dim3((N * N + W - 1) / W, nfield, nvec),
-                            ((W * G + 31) / 32) * 32, G > 1 ? sizeof(cx<R>) * N * (W + 1) : 0, 1, st, src, dst, d, ctx,
-                            stride, scale);
+    return launch<k_col2<R, N, DIR, SMODE>>(dim3((N * N + W - 1) / W, nfield, nvec), ((W * G + 31) / 32) * 32,
+                                                G > 1 ? sizeof(cx<R>) * N * (W + 1) : 0, st, src, dst, d, ctx, stride,
+                                                scale);
   } else {
     // one warp per CTA for small batches, so that the work spreads over the
     // SMs, 128 threads where there are plenty
     const int tpb = (long long)N * N * nfield * nvec < 128LL * 6 * P.sms ? 32 : 128;
-    dim3 g((N * N + tpb - 1) / tpb, nfield, nvec);
-    FAME_LAUNCHED(1);
-    k_col<N, DIR, SMODE><<<g, tpb, 0, st>>>(src, dst, d, ctx, stride, scale);
-    return cudaGetLastError();
+    return launch<k_col<N, DIR, SMODE>>(dim3((N * N + tpb - 1) / tpb, nfield, nvec), tpb, 0, st, src, dst, d, ctx,
+                                            stride, scale);
   }
 }
 

@@ -22,6 +22,7 @@
 #pragma once
 
 #include "fame_internal.h"
+#include "launch.h"
 
 namespace fame {
 namespace detail {
@@ -142,6 +143,7 @@ k_vertex(const cx<R>* __restrict__ uv, cx<R>* __restrict__ h, PlanData<R> d,
   constexpr int NN = N * N, Nq = NN * N;
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
   const int vec = blockIdx.y;
+  pdl_wait();
   if (idx >= Nq) return;
   if (ctx.active && !ctx.active[vec]) return;
   const int inst = vec_inst(ctx, vec);
@@ -184,6 +186,7 @@ k_faceedge(const cx<R>* uv, const cx<R>* __restrict__ h, cx<R>* out, PlanData<R>
   constexpr int NN = N * N, Nq = NN * N;
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
   const int vec = blockIdx.y;
+  pdl_wait();
   if (idx >= Nq) return;
   if (ctx.active && !ctx.active[vec]) return;
   const int inst = vec_inst(ctx, vec);
@@ -307,6 +310,7 @@ k_sweep(const cx<R>* __restrict__ uv, cx<R>* __restrict__ out, PlanData<R> d, co
   const int z0 = blockIdx.y * tz;
   const int nz = min(tz, N - z0);                            // planes of this chunk
   const int vec = blockIdx.z;
+  pdl_wait();
   if (ctx.active && !ctx.active[vec]) return;
   const int inst = vec_inst(ctx, vec);
   const int tid = threadIdx.x;
@@ -506,13 +510,9 @@ cudaError_t sweep_n(const Plan& P, const cx<R>* w, cx<R>* out, int nvec, const V
   using SH = SweepShape<R, N>;
   const PlanData<R>& d = pdata<R>(P);
   return with_kind<R>(d, [&](auto kc) -> cudaError_t {
-    auto kfn = k_sweep<R, N, decltype(kc)::value>;
-    cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SH::SMEM);
-    if (e != cudaSuccess) return e;
-    const dim3 g(N / SH::TY, (N + tz - 1) / tz, nvec);
-    FAME_LAUNCHED(1);
-    kfn<<<g, SH::TPB, SH::SMEM, st>>>(w, out, d, P.d_phase, P.nphase, ctx, 6LL * N * N * N, tz, wdot);
-    return cudaGetLastError();
+    return launch<k_sweep<R, N, decltype(kc)::value>>(dim3(N / SH::TY, (N + tz - 1) / tz, nvec), SH::TPB, SH::SMEM,
+                                                          st, w, out, d, P.d_phase, P.nphase, ctx, 6LL * N * N * N, tz,
+                                                          wdot);
   });
 }
 
@@ -531,13 +531,9 @@ cudaError_t stencil_n(const Plan& P, const cx<R>* w, cx<R>* out, cx<R>* h, int n
   const PlanData<R>& d = pdata<R>(P);
   return with_kind<R>(d, [&](auto kc) -> cudaError_t {
     constexpr int K = decltype(kc)::value;
-    FAME_LAUNCHED(1);
-    k_vertex<R, N, K><<<g, tpb, 0, st>>>(w, h, d, P.d_phase, P.nphase, ctx, 6LL * Nq, bloch);
-    cudaError_t e = cudaGetLastError();
+    cudaError_t e = launch<k_vertex<R, N, K>>(g, tpb, 0, st, w, h, d, P.d_phase, P.nphase, ctx, 6LL * Nq, bloch);
     if (e != cudaSuccess) return e;
-    FAME_LAUNCHED(1);
-    k_faceedge<R, N, K><<<g, tpb, 0, st>>>(w, h, out, d, P.d_phase, P.nphase, ctx, 6LL * Nq, bloch);
-    return cudaGetLastError();
+    return launch<k_faceedge<R, N, K>>(g, tpb, 0, st, w, h, out, d, P.d_phase, P.nphase, ctx, 6LL * Nq, bloch);
   });
 }
 

@@ -15,6 +15,7 @@ __global__ void k_fncA(const cx<R>* __restrict__ x, cx<R>* __restrict__ y, PlanD
   const long long Nq = (long long)n * n * n;
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int vec = blockIdx.y;
+  pdl_wait();
   if (idx >= Nq) return;
   if (ctx.active && !ctx.active[vec]) return;
   const int i1 = int(idx % n), i2 = int((idx / n) % n), i3 = int(idx / ((long long)n * n));
@@ -249,9 +250,7 @@ cudaError_t launch_fncB(const Plan& P, const cx<R>* x, cx<R>* y, int nvec, const
 template <class R>
 cudaError_t launch_fncA(const Plan& P, const cx<R>* x, cx<R>* y, int nvec, const VecCtx& ctx, cudaStream_t st) {
   if (nvec <= 0) return cudaSuccess;
-  FAME_LAUNCHED(1);
-  k_fncA<R><<<grid_pts1(P.Nq, nvec, 256), 256, 0, st>>>(x, y, pdata<R>(P), ctx, P.n);
-  return cudaGetLastError();
+  return launch<k_fncA<R>>(grid_pts1(P.Nq, nvec, 256), 256, 0, st, x, y, pdata<R>(P), ctx, P.n);
 }
 
 template <class R>

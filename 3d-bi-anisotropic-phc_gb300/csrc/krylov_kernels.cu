@@ -4,6 +4,7 @@
 // Every kernel works on a batch of vectors, one vector per k-point instance,
 // and skips vectors whose `active` flag is 0.
 #include "krylov.h"
+#include "launch.h"
 
 namespace fame {
 namespace {
@@ -43,6 +44,7 @@ k_dot_partial(const cx<R>* __restrict__ a, long long a_vstride, long long a_cstr
   const int m = blockIdx.z;
   const int nblk = gridDim.x;
   double2* out = partial + ((long long)vec * ma + m) * nblk + blockIdx.x;
+  pdl_wait();
   if (active && !active[vec]) {
     if (threadIdx.x == 0) *out = make_double2(0.0, 0.0);
     return;
@@ -81,6 +83,7 @@ k_cg_xr_dot(cx<R>* __restrict__ x, cx<R>* __restrict__ r, const cx<R>* __restric
   const int vec = blockIdx.y;
   const int nblk = gridDim.x;
   double2* out = partial + (long long)vec * nblk + blockIdx.x;
+  pdl_wait();
   if (active && !active[vec]) {
     if (threadIdx.x == 0) *out = make_double2(0.0, 0.0);
     return;
@@ -105,6 +108,7 @@ k_cg_xr_dot(cx<R>* __restrict__ x, cx<R>* __restrict__ r, const cx<R>* __restric
 __global__ void __launch_bounds__(kRedThreads)
 k_dot_final(const double2* __restrict__ partial, int nblk, double2* __restrict__ out) {
   const long long row = blockIdx.x;  // vec * ma + m
+  pdl_wait();
   double2 s = make_double2(0.0, 0.0);
   for (int i = threadIdx.x; i < nblk; i += blockDim.x) {
     double2 p = partial[row * nblk + i];
@@ -156,6 +160,7 @@ template <class R>
 __global__ void k_cg_p(cx<R>* __restrict__ p, const cx<R>* __restrict__ r, long long len, long long stride,
                        const double* __restrict__ beta, const int* __restrict__ active) {
   const int vec = blockIdx.y;
+  pdl_wait();
   if (active && !active[vec]) return;
   const R b = R(beta[vec]);
   const long long o = vec * stride;
@@ -220,6 +225,7 @@ k_cg_scalars_red(int stage, const double2* __restrict__ partial, int nblk, doubl
                  const double* __restrict__ tol2b2, int* __restrict__ active, int* __restrict__ iters,
                  double* __restrict__ res2) {
   const int v = blockIdx.x;
+  pdl_wait();
   if (!active[v]) return;
   double2 s = make_double2(0.0, 0.0);
   for (int i = threadIdx.x; i < nblk; i += blockDim.x) {
@@ -490,12 +496,10 @@ cudaError_t dot_batched(const cx<R>* a, long long a_vstride, long long a_cstride
                         long long b_vstride, long long len, int nvec, double2* out, double2* partial,
                         int nblk, const int* active, cudaStream_t st) {
   if (nvec <= 0 || ma <= 0) return cudaSuccess;
-  dim3 g(nblk, nvec, ma);
-  FAME_LAUNCHED(1);
-  k_dot_partial<R><<<g, kRedThreads, 0, st>>>(a, a_vstride, a_cstride, ma, b, b_vstride, len, partial, active);
-  FAME_LAUNCHED(1);
-  k_dot_final<<<nvec * ma, kRedThreads, 0, st>>>(partial, nblk, out);
-  return cudaGetLastError();
+  cudaError_t e = launch<k_dot_partial<R>>(dim3(nblk, nvec, ma), kRedThreads, 0, st, a, a_vstride, a_cstride, ma, b,
+                                               b_vstride, len, partial, active);
+  if (e != cudaSuccess) return e;
+  return launch<k_dot_final>(dim3(nvec * ma), kRedThreads, 0, st, (const double2*)partial, nblk, out);
 }
 
 template <class R>
@@ -520,38 +524,32 @@ cudaError_t cg_xr(cx<R>* x, cx<R>* r, const cx<R>* p, const cx<R>* q, long long 
 }
 
 cudaError_t dot_final(const double2* partial, int nblk, int nrows, double2* out, cudaStream_t st) {
-  FAME_LAUNCHED(1);
-  k_dot_final<<<nrows, kRedThreads, 0, st>>>(partial, nblk, out);
-  return cudaGetLastError();
+  return launch<k_dot_final>(dim3(nrows), kRedThreads, 0, st, partial, nblk, out);
 }
 
 template <class R>
 cudaError_t cg_xr_dot(cx<R>* x, cx<R>* r, const cx<R>* p, const cx<R>* q, long long len, long long stride, int nvec,
                       const double* alpha, const int* active, double2* out, double2* partial, int nblk,
                       cudaStream_t st) {
-  FAME_LAUNCHED(1);
-  k_cg_xr_dot<R><<<dim3(nblk, nvec), kRedThreads, 0, st>>>(x, r, p, q, len, stride, alpha, active, partial);
-  FAME_LAUNCHED(1);
-  k_dot_final<<<nvec, kRedThreads, 0, st>>>(partial, nblk, out);
-  return cudaGetLastError();
+  cudaError_t e = launch<k_cg_xr_dot<R>>(dim3(nblk, nvec), kRedThreads, 0, st, x, r, p, q, len, stride, alpha, active,
+                                             partial);
+  if (e != cudaSuccess) return e;
+  return launch<k_dot_final>(dim3(nvec), kRedThreads, 0, st, (const double2*)partial, nblk, out);
 }
 
 template <class R>
 cudaError_t dot_partial(const cx<R>* a, const cx<R>* b, long long len, long long stride, int nvec, double2* partial,
                         int nblk, const int* active, cudaStream_t st) {
   if (nvec <= 0) return cudaSuccess;
-  FAME_LAUNCHED(1);
-  k_dot_partial<R><<<dim3(nblk, nvec, 1), kRedThreads, 0, st>>>(a, stride, 0, 1, b, stride, len, partial, active);
-  return cudaGetLastError();
+  return launch<k_dot_partial<R>>(dim3(nblk, nvec, 1), kRedThreads, 0, st, a, stride, 0LL, 1, b, stride, len, partial,
+                                      active);
 }
 
 template <class R>
 cudaError_t cg_xr_partial(cx<R>* x, cx<R>* r, const cx<R>* p, const cx<R>* q, long long len, long long stride,
                           int nvec, const double* alpha, const int* active, double2* partial, int nblk,
                           cudaStream_t st) {
-  FAME_LAUNCHED(1);
-  k_cg_xr_dot<R><<<dim3(nblk, nvec), kRedThreads, 0, st>>>(x, r, p, q, len, stride, alpha, active, partial);
-  return cudaGetLastError();
+  return launch<k_cg_xr_dot<R>>(dim3(nblk, nvec), kRedThreads, 0, st, x, r, p, q, len, stride, alpha, active, partial);
 }
 
 // Q_v[:, col_v] = V_v, BQ_v[:, col_v] = BV_v (and their complex64 copies when
@@ -640,10 +638,8 @@ cudaError_t while_active(const int* active, int nvec, int* passes, int max_passe
 cudaError_t cg_scalars_red(int stage, int nvec, const double2* partial, int nblk, double2* dot, double* rho,
                            double* alpha, double* beta, const double* tol2b2, int* active, int* iters, double* res2,
                            cudaStream_t st) {
-  FAME_LAUNCHED(1);
-  k_cg_scalars_red<<<nvec, kRedThreads, 0, st>>>(stage, partial, nblk, dot, rho, alpha, beta, tol2b2, active, iters,
-                                                 res2);
-  return cudaGetLastError();
+  return launch<k_cg_scalars_red>(dim3(nvec), kRedThreads, 0, st, stage, partial, nblk, dot, rho, alpha, beta, tol2b2,
+                                      active, iters, res2);
 }
 
 template <class R>
@@ -651,9 +647,7 @@ cudaError_t cg_p(cx<R>* p, const cx<R>* r, long long len, long long stride, int 
                  const int* active, cudaStream_t st) {
   int gx = grid_for(len);
   if (gx > 1024) gx = 1024;
-  FAME_LAUNCHED(1);
-  k_cg_p<R><<<dim3(gx, nvec), 256, 0, st>>>(p, r, len, stride, beta, active);
-  return cudaGetLastError();
+  return launch<k_cg_p<R>>(dim3(gx, nvec), 256, 0, st, p, r, len, stride, beta, active);
 }
 
 cudaError_t cg_scalars(int stage, int nvec, const double2* dot, double* rho, double* alpha, double* beta,

@@ -14,6 +14,7 @@
 // depend on it.
 #include "fncb_impl.cuh"
 #include "krylov.h"
+#include "launch.h"
 
 namespace fame {
 namespace {
@@ -176,6 +177,7 @@ k_precond_apply(const cx<R>* __restrict__ r, cx<R>* __restrict__ z, const cx<R>*
   const int vec = blockIdx.y;
   const int nblk = gridDim.x;
   double2* out = partial + (long long)vec * nblk + blockIdx.x;
+  pdl_wait();
   if (ctx.active && !ctx.active[vec]) {
     if (threadIdx.x == 0) *out = make_double2(0.0, 0.0);
     return;
@@ -207,6 +209,7 @@ k_pcg_update(cx<R>* __restrict__ x, cx<R>* __restrict__ r, cx<R>* __restrict__ z
   const int vec = blockIdx.y;
   const int nblk = gridDim.x;
   double2* out = partial + (long long)vec * nblk + blockIdx.x;
+  pdl_wait();
   if (ctx.active && !ctx.active[vec]) {
     if (threadIdx.x == 0) *out = make_double2(0.0, 0.0);
     return;
@@ -326,9 +329,7 @@ template <class R>
 cudaError_t precond_apply(const Plan& P, const cx<R>* r, cx<R>* z, int nvec, const VecCtx& ctx, double2* partial,
                           int nblk, cudaStream_t st) {
   const PlanData<R>& d = detail::pdata<R>(P);
-  FAME_LAUNCHED(1);
-  k_precond_apply<R><<<dim3(nblk, nvec), kThreads, 0, st>>>(r, z, d.pc, ctx, P.Nq, partial);
-  return cudaGetLastError();
+  return launch<k_precond_apply<R>>(dim3(nblk, nvec), kThreads, 0, st, r, z, d.pc, ctx, P.Nq, partial);
 }
 
 template <class R>
@@ -336,9 +337,8 @@ cudaError_t pcg_update(const Plan& P, cx<R>* x, cx<R>* r, cx<R>* z, const cx<R>*
                        const VecCtx& ctx, const double* alpha, double2* partial, int nblk, cudaStream_t st,
                        const CgAlpha& ca) {
   const PlanData<R>& d = detail::pdata<R>(P);
-  FAME_LAUNCHED(1);
-  k_pcg_update<R><<<dim3(nblk, nvec), kThreads, 0, st>>>(x, r, z, p, q, d.pc, ctx, P.Nq, alpha, partial, ca);
-  return cudaGetLastError();
+  return launch<k_pcg_update<R>>(dim3(nblk, nvec), kThreads, 0, st, x, r, z, p, q, d.pc, ctx, P.Nq, alpha, partial,
+                                     ca);
 }
 
 template cudaError_t build_precond<float>(Plan&, cudaStream_t);
