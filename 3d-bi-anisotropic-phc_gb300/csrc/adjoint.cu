@@ -278,15 +278,14 @@ int fame_eig_gradient(fame_plan_t h, int nvec, const int* inst, const void* x, c
   cudaError_t e = ensure_work(P, (size_t)nvec);
   if (e != cudaSuccess) return cuda_fail(&P, e, "fame_eig_gradient work");
   double2* w = (double2*)P.d_work;
-  int* d_inst = nullptr;
-  if (inst) {
-    d_inst = (int*)workspace(P, 40, sizeof(int) * nvec, &e);
+  VecCtx ctx;
+  ctx.nk = P.nk;
+  if (inst && !small_inst(ctx, inst, nvec)) {
+    int* d_inst = (int*)workspace(P, 40, sizeof(int) * nvec, &e);
     if (e == cudaSuccess) e = h2d_async(P, d_inst, inst, sizeof(int) * nvec);
     if (e != cudaSuccess) return cuda_fail(&P, e, "fame_eig_gradient inst");
+    ctx.inst = d_inst;
   }
-  VecCtx ctx;
-  ctx.inst = d_inst;
-  ctx.nk = P.nk;
   e = launch_fields_inv<double>(P, (const double2*)x, w, nvec, ctx, st);
   if (e != cudaSuccess) return cuda_fail(&P, e, "fame_eig_gradient fields");
   GradParams gp;

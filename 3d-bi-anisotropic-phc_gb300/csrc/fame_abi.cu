@@ -105,9 +105,8 @@ cudaError_t upload_inst(Plan& P, const int* inst_host, int nvec, const int** d_i
     if (e != cudaSuccess) return e;
     P.inst_cap = nvec;
   }
-  cudaError_t e = cudaMemcpyAsync(P.d_inst, inst_host, sizeof(int) * nvec, cudaMemcpyHostToDevice, P.stream);
   *d_inst_out = P.d_inst;
-  return e;
+  return h2d_async(P, P.d_inst, inst_host, sizeof(int) * nvec);
 }
 
 cudaError_t ensure_stage(Plan& P, size_t bytes) {
@@ -465,10 +464,10 @@ namespace fame {
 // in_len / out_len: complex elements per vector.  body(x_dev, y_dev, ctx).
 template <class F>
 int run_op(fame_plan_t h, int prec, const void* x, void* y, int nvec, const int* inst, int flags, long long in_len,
-           long long out_len, const char* name, F&& body) {
+           long long out_len, const char* name, F&& body, bool inst_on_device = false) {
   if (!h) return FAME_ERR_BAD_ARG;
   Plan& P = h->P;
-  if (prec != FAME_C128 && prec != FAME_C64 && !(prec == FAME_C128_DS && std::string(name) == "fame_apply_B"))
+  if (prec != FAME_C128 && prec != FAME_C64 && !(prec == FAME_C128_DS && std::strcmp(name, "fame_apply_B") == 0))
     return fail(&P, FAME_ERR_BAD_ARG, std::string(name) + ": bad precision");
   if (prec == FAME_C128_DS && !ds_supported(P.n))
     return fail(&P, FAME_ERR_UNSUPPORTED, std::string(name) + ": no double-single fncB for this grid size");
@@ -493,8 +492,11 @@ int run_op(fame_plan_t h, int prec, const void* x, void* y, int nvec, const int*
   }
   VecCtx ctx;
   ctx.nk = P.nk;
-  e = upload_inst(P, inst, nvec, &ctx.inst);
-  if (e != cudaSuccess) return cuda_fail(&P, e, name);
+  // (the solver keeps the device copy's address in its captured graphs)
+  if (inst && (inst_on_device || !small_inst(ctx, inst, nvec))) {
+    e = upload_inst(P, inst, nvec, &ctx.inst);
+    if (e != cudaSuccess) return cuda_fail(&P, e, name);
+  }
   int rc = body(xd, yd, ctx);
   if (rc != FAME_OK) return rc;
   if (flags & FAME_HOST_PTR) {
@@ -605,7 +607,7 @@ int fame_apply_Binv(fame_plan_t h, int prec, const void* x, void* y, int nvec, c
                                                   relres)
                              : pcg_batched<double>(P, (const double2*)xd, (double2*)yd, nvec, ctx.inst, tol, maxit,
                                                    iters, relres);
-                });
+                }, true);
 }
 
 int fame_material_blocks(const double* c6, const double* lattice, double* out) {

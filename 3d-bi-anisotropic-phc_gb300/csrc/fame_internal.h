@@ -34,15 +34,24 @@ extern unsigned long long g_host_launches;
    __atomic_fetch_sub(&::fame::g_host_launches, (unsigned long long)(n), __ATOMIC_RELAXED))
 
 // Which vectors of a batch belong to which k-point instance, and which are
-// still active (converged vectors of a batched solve are skipped).
+// still active (converged vectors of a batched solve are skipped).  Up to
+// kSmallInst instance indices travel in the kernel arguments: a device copy
+// costs a call more than its own launches on small grids.
+constexpr int kSmallInst = 32;
 struct VecCtx {
-  const int* inst = nullptr;    // device [nvec] instance index, or null: (v + vofs) % nk
+  const int* inst = nullptr;    // device [nvec] instance index, or null: small, or (v + vofs) % nk
   const int* active = nullptr;  // device [nvec] 0/1, or null: all active
   int nk = 1;
   int vofs = 0;                 // index of vector 0 in the caller's batch (sub-batches)
+  int nsmall = 0;               // entries of small in use
+  uint8_t small[kSmallInst] = {};
 };
 
-FAME_HD int vec_inst(const VecCtx& c, int v) { return c.inst ? c.inst[v] : ((v + c.vofs) % c.nk); }
+FAME_HD int vec_inst(const VecCtx& c, int v) {
+  if (c.inst) return c.inst[v];
+  const int w = v + c.vofs;
+  return c.nsmall > 0 ? c.small[w] : w % c.nk;
+}
 
 // The same context for the sub-batch of vectors [v0, ...).
 inline VecCtx sub_ctx(const VecCtx& c, int v0) {
@@ -51,6 +60,14 @@ inline VecCtx sub_ctx(const VecCtx& c, int v0) {
   if (s.active) s.active += v0;
   s.vofs += v0;
   return s;
+}
+
+// Puts host instance indices into ctx if they fit (else the caller uploads them).
+inline bool small_inst(VecCtx& ctx, const int* inst, int nvec) {
+  if (nvec > kSmallInst || ctx.nk > 256) return false;
+  ctx.nsmall = nvec;
+  for (int v = 0; v < nvec; ++v) ctx.small[v] = (uint8_t)inst[v];
+  return true;
 }
 
 // Threads per FFT pencil of the complex128 / double-single kernels for size n.

@@ -162,15 +162,14 @@ extern "C" int fame_restore(fame_plan_t h, int nvec, const int* inst, const void
   const size_t six = sizeof(double2) * 6 * (size_t)Nq * nvec;
   double2* eh = (double2*)workspace(P, 45, six, &e);
   if (e != cudaSuccess) return cuda_fail(&P, e, "fame_restore scratch");
-  int* d_inst = nullptr;
-  if (inst) {
-    d_inst = (int*)workspace(P, 46, sizeof(int) * nvec, &e);
+  VecCtx ctx;
+  ctx.nk = P.nk;
+  if (inst && !small_inst(ctx, inst, nvec)) {
+    int* d_inst = (int*)workspace(P, 46, sizeof(int) * nvec, &e);
     if (e == cudaSuccess) e = h2d_async(P, d_inst, inst, sizeof(int) * nvec);
     if (e != cudaSuccess) return cuda_fail(&P, e, "fame_restore inst");
+    ctx.inst = d_inst;
   }
-  VecCtx ctx;
-  ctx.inst = d_inst;
-  ctx.nk = P.nk;
   const dim3 g((unsigned)((Nq + kT - 1) / kT), (unsigned)nvec);
 #define RS_CK(expr, what)                              \
   do {                                                 \

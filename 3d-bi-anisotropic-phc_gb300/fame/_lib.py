@@ -66,21 +66,21 @@ SIGNATURES = {
     "fame_last_error": (C.c_char_p, [_vp]),
     "fame_refine_residuals": (C.c_int, [_vp, C.POINTER(C.c_double), C.c_int]),
     "fame_plan_info": (_i, [_vp, _pi, _pi, _pll]),
-    "fame_apply_A": (_i, [_vp, _i, _vp, _vp, _i, _pi, _i]),
-    "fame_apply_B": (_i, [_vp, _i, _vp, _vp, _i, _pi, _i]),
+    "fame_apply_A": (_i, [_vp, _i, _vp, _vp, _i, _vp, _i]),
+    "fame_apply_B": (_i, [_vp, _i, _vp, _vp, _i, _vp, _i]),
     "fame_apply_B_noalloc": (_i, [_vp, _i, _vp, _vp, _i]),
-    "fame_apply_Binv": (_i, [_vp, _i, _vp, _vp, _i, _pi, _d, _i, _pi, _pd, _i]),
-    "fame_curl_transform": (_i, [_vp, _i, _i, _vp, _vp, _i, _pi, _i]),
-    "fame_apply_handle": (_i, [_vp, _i, _i, _vp, _vp, _i, _pi, _i]),
-    "fame_apply_material": (_i, [_vp, _i, _vp, _vp, _i, _pi, _i]),
+    "fame_apply_Binv": (_i, [_vp, _i, _vp, _vp, _i, _vp, _d, _i, _pi, _pd, _i]),
+    "fame_curl_transform": (_i, [_vp, _i, _i, _vp, _vp, _i, _vp, _i]),
+    "fame_apply_handle": (_i, [_vp, _i, _i, _vp, _vp, _i, _vp, _i]),
+    "fame_apply_material": (_i, [_vp, _i, _vp, _vp, _i, _vp, _i]),
     "fame_lanczos": (_i, [_vp, _i, _i, _i, _d, _i, _i, _pd, _d, _pd, _vp, _pd, _pll]),
     "fame_band_solve": (_i, [_vp, _i, _i, _d, _i, _i, _d, _pd, _vp, _pd, _pll]),
     "fame_material_blocks": (_i, [_pd, _pd, _pd]),
     "fame_jdsira": (_i, [_vp, _i, _i, _i, _d, _d, _d, _i, _i, _d, _i, _pd, _vp, _pd, _pll]),
     "fame_plan_create_field": (_i, [C.POINTER(_vp), _i, _i, _pd, _pd, _pd, _pd]),
     "fame_set_field": (_i, [_vp, _pd, _pd]),
-    "fame_eig_gradient": (_i, [_vp, _i, _pi, _vp, _pd, _pd, _vp, _vp, _i, _pd]),
-    "fame_restore": (_i, [_vp, _i, _pi, _vp, _pd, _vp, _vp, _pd, _pd, _pd, _i]),
+    "fame_eig_gradient": (_i, [_vp, _i, _vp, _vp, _pd, _pd, _vp, _vp, _i, _pd]),
+    "fame_restore": (_i, [_vp, _i, _vp, _vp, _pd, _vp, _vp, _pd, _pd, _pd, _i]),
     "fame_autotune": (_i, [_vp, _i, _i, _pi, _pi, _pd]),
     "fame_set_tune": (_i, [_vp, _i, _i, _i, _i]),
     "fame_set_tune_lanes": (_i, [_vp, _i, _i, _i]),

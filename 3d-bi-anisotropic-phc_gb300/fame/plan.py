@@ -36,6 +36,25 @@ def _prec_of(x):
     raise TypeError(f"unsupported dtype {x.dtype}")
 
 
+def _instances(inst, nvec):
+    """Instance indices of a call as a contiguous int32 array of nvec entries
+    (broadcast where shorter) and its address, or (None, None)."""
+    if inst is None:
+        return None, None
+    if not (isinstance(inst, np.ndarray) and inst.dtype == np.int32 and inst.shape == (nvec,) and
+            inst.flags.c_contiguous):
+        inst = np.ascontiguousarray(np.broadcast_to(np.asarray(inst, dtype=np.int32), (nvec,)))
+    return inst, inst.ctypes.data
+
+
+def _current_stream():
+    """Torch's current CUDA stream of the current device as an integer handle.
+    (The Stream object that torch.cuda.current_stream() builds costs more than
+    a kernel launch.)"""
+    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+    return raw(torch.cuda.current_device()) if raw is not None else torch.cuda.current_stream().cuda_stream
+
+
 def _tune_prec(prec):
     """Tuning key of 'c64', 'c128' or 'c128ds' (complex128 vectors, double-single
     arithmetic: the mixed inner solves' residuals), or the FAME_* code itself."""
@@ -144,10 +163,7 @@ class Plan:
             g_g = torch.zeros(self.Nq, dtype=torch.float64, device=ev.device)
         else:
             g_e, g_g = out
-        ip = None
-        if inst is not None:
-            ia = np.ascontiguousarray(np.broadcast_to(np.asarray(inst, dtype=np.int32), (nvec,)))
-            ip = ia.ctypes.data_as(C.POINTER(C.c_int))
+        ia, ip = _instances(inst, nvec)
         xbx = np.zeros(nvec)
         pd = C.POINTER(C.c_double)
         self._stream()
@@ -173,10 +189,7 @@ class Plan:
         res = np.zeros(nvec)
         me = np.zeros(nvec)
         mh = np.zeros(nvec)
-        ip = None
-        if inst is not None:
-            ia = np.ascontiguousarray(np.broadcast_to(np.asarray(inst, dtype=np.int32), (nvec,)))
-            ip = ia.ctypes.data_as(C.POINTER(C.c_int))
+        ia, ip = _instances(inst, nvec)
         pd = C.POINTER(C.c_double)
         self._stream()
         rc = self._lib.fame_restore(self._h, nvec, ip, C.c_void_p(ev.data_ptr()), om.ctypes.data_as(pd),
@@ -210,8 +223,8 @@ class Plan:
         return self._h
 
     def _stream(self):
-        if torch is not None and torch.cuda.is_available():
-            self._lib.fame_set_stream(self._h, C.c_void_p(torch.cuda.current_stream().cuda_stream))
+        if torch is not None and (torch.cuda.is_initialized() or torch.cuda.is_available()):
+            self._lib.fame_set_stream(self._h, _current_stream())
 
     def sync(self):
         check(self._lib.fame_sync(self._h), self._h, "fame_sync")
@@ -311,17 +324,14 @@ class Plan:
             xx = xx.contiguous()
             nvec = xx.shape[0]
             y = torch.empty((nvec, out_len), dtype=xx.dtype, device=xx.device)
-            xp, yp, flags = C.c_void_p(xx.data_ptr()), C.c_void_p(y.data_ptr()), 0
+            xp, yp, flags = xx.data_ptr(), y.data_ptr(), 0
             self._stream()
         else:
             xx = np.ascontiguousarray(np.asarray(x).reshape(1, -1) if single else np.asarray(x))
             nvec = xx.shape[0]
             y = np.empty((nvec, out_len), dtype=xx.dtype)
-            xp, yp, flags = C.c_void_p(xx.ctypes.data), C.c_void_p(y.ctypes.data), L.FAME_HOST_PTR
-        ip = None
-        if inst is not None:
-            ia = np.ascontiguousarray(np.broadcast_to(np.asarray(inst, dtype=np.int32), (nvec,)))
-            ip = ia.ctypes.data_as(C.POINTER(C.c_int))
+            xp, yp, flags = xx.ctypes.data, y.ctypes.data, L.FAME_HOST_PTR
+        ia, ip = _instances(inst, nvec)
         rc = fn(self._h, prec, *extra[:1], xp, yp, nvec, ip, *extra[1:], flags) if extra else \
             fn(self._h, prec, xp, yp, nvec, ip, flags)
         check(rc, self._h, name)
@@ -358,19 +368,16 @@ class Plan:
             xx = (x.reshape(1, -1) if single else x).contiguous()
             nvec = xx.shape[0]
             y = torch.empty_like(xx)
-            xp, yp, flags = C.c_void_p(xx.data_ptr()), C.c_void_p(y.data_ptr()), 0
+            xp, yp, flags = xx.data_ptr(), y.data_ptr(), 0
             self._stream()
         else:
             xx = np.ascontiguousarray(np.asarray(x).reshape(1, -1) if single else np.asarray(x))
             nvec = xx.shape[0]
             y = np.empty_like(xx)
-            xp, yp, flags = C.c_void_p(xx.ctypes.data), C.c_void_p(y.ctypes.data), L.FAME_HOST_PTR
+            xp, yp, flags = xx.ctypes.data, y.ctypes.data, L.FAME_HOST_PTR
         its = np.zeros(nvec, dtype=np.int32)
         rr = np.zeros(nvec, dtype=np.float64)
-        ip = None
-        if inst is not None:
-            ia = np.ascontiguousarray(np.broadcast_to(np.asarray(inst, dtype=np.int32), (nvec,)))
-            ip = ia.ctypes.data_as(C.POINTER(C.c_int))
+        ia, ip = _instances(inst, nvec)
         rc = self._lib.fame_apply_Binv(self._h, prec, xp, yp, nvec, ip, float(tol), int(maxit),
                                        its.ctypes.data_as(C.POINTER(C.c_int)),
                                        rr.ctypes.data_as(C.POINTER(C.c_double)), flags)
