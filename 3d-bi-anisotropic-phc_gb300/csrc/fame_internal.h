@@ -211,12 +211,10 @@ template <class R> cudaError_t build_pi_table(Plan& P);
 
 // ---- kernel launchers (fncb_kernels.cu) ----
 // pq (may be null): partial sums of Re(x^H B x), fncB_pq_partials(P, nvec)
-// per vector, written when that count is non-zero.  pupd_z (may be null): x
-// is a CG direction that is first updated in place, x = pupd_z + pupd_beta[v] x.
+// per vector, written when that count is non-zero.
 template <class R>
 cudaError_t launch_fncB(const Plan& P, const cx<R>* x, cx<R>* y, int nvec, const VecCtx& ctx,
-                        cx<R>* w0, cx<R>* w1, cudaStream_t st, double2* pq = nullptr,
-                        const cx<R>* pupd_z = nullptr, const double* pupd_beta = nullptr);
+                        cx<R>* w0, cx<R>* w1, cudaStream_t st, double2* pq = nullptr);
 template <class R> int fncB_pq_partials(const Plan& P, int nvec);
 // Grid sizes with a compiled double-single fncB (FAME_FOR_EACH_DS_N).
 bool ds_supported(int n);
@@ -259,10 +257,12 @@ cudaError_t launch_material(const Plan& P, const cx<R>* uv, cx<R>* out, int nvec
 // volume-averaged vertex tensors, block diagonal in the frequency basis
 // (one 4x4 Hermitian block per voxel).  Built once per plan and precision.
 template <class R> cudaError_t build_precond(Plan& P, cudaStream_t st);
-// z = M r per vector; partial sums (Re r'z, |r|^2) per block into partial.
+// Start of a CG solve on the active vectors: x = 0, r = b, z = M b, p = z
+// (precond) or p = b; partial sums (Re b'p, |b|^2) per block into partial (0
+// for inactive vectors, whose x stays as it is).
 template <class R>
-cudaError_t precond_apply(const Plan& P, const cx<R>* r, cx<R>* z, int nvec, const VecCtx& ctx, double2* partial,
-                          int nblk, cudaStream_t st);
+cudaError_t pcg_start(const Plan& P, bool precond, const cx<R>* b, cx<R>* x, cx<R>* r, cx<R>* z, cx<R>* p, int nvec,
+                      const VecCtx& ctx, double2* partial, int nblk, cudaStream_t st);
 // The CG step length computed inside the update instead of by a separate
 // scalar kernel: every CTA of vector v reduces v's `nblk` partial sums of
 // p^H q in one fixed order, so all of them use the same alpha = rho / p^H q;

@@ -247,14 +247,6 @@ template <class R> __device__ __forceinline__ void store_io(cx<R>* p, cx<R> v) {
   }
 }
 
-// The conjugate-gradient direction update p = z + beta p, done by the first
-// kernel of fncB on the p it reads (z == null: no update).  Each CTA rewrites
-// the plane of p it loads, so the separate update pass over p disappears.
-template <class R> struct DirUpd {
-  const cx<R>* z = nullptr;     // same layout and strides as p
-  const double* beta = nullptr; // [nvec] of this launch
-};
-
 // ---------------------------------------------------------------------------
 // complex64 plane kernels: one CTA per (k3 plane, side, vector), 3N threads,
 // one thread per pencil (N <= 64 complex values in registers).
@@ -273,7 +265,7 @@ template <class R> struct DirUpd {
 template <int N, bool PREP>
 __global__ void __launch_bounds__(((3 * N + 31) / 32) * 32, 2)
 k_plane_inv(const float2* __restrict__ x, float2* __restrict__ out, PlanData<float> d, VecCtx ctx,
-            long long in_stride, long long in_side_stride, long long out_stride, int side0, DirUpd<float> upd) {
+            long long in_stride, long long in_side_stride, long long out_stride, int side0) {
   constexpr int LD = N + 1;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   float2* sm = reinterpret_cast<float2*>(smem_raw);  // [3][N][LD]
@@ -310,31 +302,6 @@ k_plane_inv(const float2* __restrict__ x, float2* __restrict__ out, PlanData<flo
       if (act && i2 < N) {
 #pragma unroll
         for (int c = 0; c < NB; ++c) in[it][c] = xin[c * Nq + i2 * N + i1];
-      }
-    }
-    if (PREP && upd.z) {  // p = z + beta p, written back
-      const float2* zin = upd.z + off;
-      float2* xw = const_cast<float2*>(x) + off;
-      const float bt = float(upd.beta[vec]);
-      float2 zz[PF][NB];
-#pragma unroll
-      for (int it = 0; it < PF; ++it) {
-        const int i2 = grp + 3 * (base + it);
-        if (act && i2 < N) {
-#pragma unroll
-          for (int c = 0; c < NB; ++c) zz[it][c] = zin[c * Nq + i2 * N + i1];
-        }
-      }
-#pragma unroll
-      for (int it = 0; it < PF; ++it) {
-        const int i2 = grp + 3 * (base + it);
-        if (act && i2 < N) {
-#pragma unroll
-          for (int c = 0; c < NB; ++c) {
-            in[it][c] = caxpy(bt, in[it][c], zz[it][c]);
-            xw[c * Nq + i2 * N + i1] = in[it][c];
-          }
-        }
       }
     }
     if constexpr (PREP && decltype(bc)::value == 0) __syncthreads();  // the row table
@@ -875,10 +842,10 @@ k_col2(const cx<R>* src, cx<R>* dst, PlanData<R> d, VecCtx ctx, long long stride
 template <class R, int N, bool PREP>
 cudaError_t plane_inv(const PlanData<R>& d, const cx<R>* x, cx<R>* out, int nvec, int nside, int side0,
                       long long in_stride, long long in_side_stride, long long out_stride, const VecCtx& ctx,
-                      cudaStream_t st, DirUpd<R> upd = DirUpd<R>()) {
+                      cudaStream_t st) {
   if constexpr (sizeof(cx<R>) == 8) {
     return launch<k_plane_inv<N, PREP>>(dim3(N, nside, nvec), ((3 * N + 31) / 32) * 32, plane_smem<N>(), st, x, out,
-                                            d, ctx, in_stride, in_side_stride, out_stride, side0, upd);
+                                            d, ctx, in_stride, in_side_stride, out_stride, side0);
   } else {
     using FS = FieldShape<R, N>;
     return launch<k_field_inv<R, N, PREP>>(dim3(N / FS::KP, 3 * nside, nvec), FS::TB, FS::SMEM, st, x, out, d, ctx,
@@ -927,12 +894,9 @@ cudaError_t col(const Plan& P, const PlanData<R>& d, const cx<R>* src, cx<R>* ds
 // transforms are unitary and Pi has orthonormal columns, so x^H B x equals
 // w^H [M J^H; J N] w for the spatial fields w the stencil reads; the stencil
 // pass accumulates it while it writes its output.
-//
-// pupd_z / pupd_beta (may be null, complex64 only): x is a CG direction p,
-// updated first as p = z + beta p (in place) by the plane kernel that reads it.
 template <class R, int N>
 cudaError_t fncB_n(const Plan& P, const cx<R>* x, cx<R>* y, int nvec, const VecCtx& ctx, cx<R>* w0, cx<R>* w1,
-                   cudaStream_t st, double2* pq, const cx<R>* pupd_z, const double* pupd_beta) {
+                   cudaStream_t st, double2* pq) {
   PlanData<R> d = pdata<R>(P);
   if (!P.opt_pi_table) d.pi = nullptr;  // evaluate Pi in the plane kernels instead
   const long long Nq = P.Nq;
@@ -945,12 +909,7 @@ cudaError_t fncB_n(const Plan& P, const cx<R>* x, cx<R>* y, int nvec, const VecC
     const cx<R>* xs = x + (size_t)v0 * 4 * Nq;
     cx<R>* ys = y + (size_t)v0 * 4 * Nq;
     cudaError_t e;
-    DirUpd<R> upd;
-    if (pupd_z) {
-      upd.z = pupd_z + (size_t)v0 * 4 * Nq;
-      upd.beta = pupd_beta + v0;
-    }
-    e = plane_inv<R, N, true>(d, xs, w0, nv, 2, 0, 4 * Nq, 2 * Nq, 6 * Nq, c, st, upd);
+    e = plane_inv<R, N, true>(d, xs, w0, nv, 2, 0, 4 * Nq, 2 * Nq, 6 * Nq, c, st);
     if (e != cudaSuccess) return e;
     e = col<R, N, +1, 0>(P, d, w0, w0, 6, nv, 6 * Nq, c, st);
     if (e != cudaSuccess) return e;
@@ -1024,7 +983,7 @@ cudaError_t handle_n(const Plan& P, int which, const cx<R>* x, cx<R>* y, int nve
 // suppress instantiation in other translation units).
 #define FAME_SIZE_SIGS(PFX, R, NN)                                                                                 \
   PFX cudaError_t fame::detail::fncB_n<R, NN>(const Plan&, const cx<R>*, cx<R>*, int, const VecCtx&, cx<R>*,       \
-                                              cx<R>*, cudaStream_t, double2*, const cx<R>*, const double*);       \
+                                              cx<R>*, cudaStream_t, double2*);                                    \
   PFX cudaError_t fame::detail::stencil_n<R, NN>(const Plan&, const cx<R>*, cx<R>*, cx<R>*, int, const VecCtx&,    \
                                                  cudaStream_t, int, bool);                                         \
   PFX cudaError_t fame::detail::fields_inv_n<R, NN>(const Plan&, const cx<R>*, cx<R>*, int, const VecCtx&,         \
@@ -1045,5 +1004,5 @@ cudaError_t handle_n(const Plan& P, int which, const cx<R>* x, cx<R>* y, int nve
 #define FAME_DS_SIGS(PFX, NN)                                                                                      \
   PFX cudaError_t fame::detail::fncB_n<fame::ff, NN>(const Plan&, const cx<fame::ff>*, cx<fame::ff>*, int,         \
                                                      const VecCtx&, cx<fame::ff>*, cx<fame::ff>*, cudaStream_t,    \
-                                                     double2*, const cx<fame::ff>*, const double*);
+                                                     double2*);
 #define FAME_INST_DS(NN) FAME_DS_SIGS(template, NN)

@@ -2,7 +2,6 @@
 // size-templated transforms and material stencil instantiated in
 // fncb_inst_*.cu.
 #include "fncb_impl.cuh"
-#include "krylov.h"
 
 namespace fame {
 namespace detail {
@@ -194,7 +193,7 @@ cudaError_t launch_fncB_ds(const Plan& P, const double2* x, double2* y, int nvec
   cff* w1 = w0 + (size_t)nvec * 6 * P.Nq;
   switch (P.n) {
 #define FAME_CASE(NN) \
-  case NN: return fncB_n<ff, NN>(P, xd, yd, nvec, ctx, w0, w1, st, nullptr, nullptr, nullptr);
+  case NN: return fncB_n<ff, NN>(P, xd, yd, nvec, ctx, w0, w1, st, nullptr);
     FAME_FOR_EACH_DS_N(FAME_CASE)
 #undef FAME_CASE
     default: return cudaErrorInvalidValue;
@@ -226,21 +225,10 @@ bool n_supported(int n) {
 
 template <class R>
 cudaError_t launch_fncB(const Plan& P, const cx<R>* x, cx<R>* y, int nvec, const VecCtx& ctx, cx<R>* w0,
-                        cx<R>* w1, cudaStream_t st, double2* pq, const cx<R>* pupd_z, const double* pupd_beta) {
+                        cx<R>* w1, cudaStream_t st, double2* pq) {
   if (nvec <= 0) return cudaSuccess;
-  if constexpr (sizeof(R) == 8) {
-    // complex128: the CG direction in its own pass (three field CTAs read each
-    // element of x, so none of them may rewrite it; the pass is small beside
-    // the FP64 arithmetic)
-    if (pupd_z) {
-      const long long L = 4 * P.Nq;
-      cudaError_t e = cg_p<R>(const_cast<cx<R>*>(x), pupd_z, L, L, nvec, pupd_beta, ctx.active, st);
-      if (e != cudaSuccess) return e;
-      pupd_z = nullptr;
-    }
-  }
   switch (P.n) {
-#define FAME_CASE(NN) case NN: return fncB_n<R, NN>(P, x, y, nvec, ctx, w0, w1, st, pq, pupd_z, pupd_beta);
+#define FAME_CASE(NN) case NN: return fncB_n<R, NN>(P, x, y, nvec, ctx, w0, w1, st, pq);
     FAME_FOR_EACH_N(FAME_CASE)
 #undef FAME_CASE
     default: return cudaErrorInvalidValue;
@@ -308,7 +296,7 @@ cudaError_t launch_material(const Plan& P, const cx<R>* uv, cx<R>* out, int nvec
 
 #define FAME_INST(R)                                                                                      \
   template cudaError_t launch_fncB<R>(const Plan&, const cx<R>*, cx<R>*, int, const VecCtx&, cx<R>*,     \
-                                      cx<R>*, cudaStream_t, double2*, const cx<R>*, const double*);       \
+                                      cx<R>*, cudaStream_t, double2*);                                    \
   template int fncB_pq_partials<R>(const Plan&, int);                                                     \
   template cudaError_t launch_fncA<R>(const Plan&, const cx<R>*, cx<R>*, int, const VecCtx&,             \
                                       cudaStream_t);                                                      \

@@ -13,30 +13,30 @@ cudaError_t dot_batched(const cx<R>* a, long long a_vstride, long long a_cstride
 template <class R>
 cudaError_t axpby_batched(const cx<R>* x, cx<R>* y, long long len, long long stride, int nvec,
                           const double2* alpha, const double2* beta, const int* active, cudaStream_t st);
-template <class R>
-cudaError_t cg_xr(cx<R>* x, cx<R>* r, const cx<R>* p, const cx<R>* q, long long len, long long stride, int nvec,
-                  const double* alpha, const int* active, cudaStream_t st);
 // out[row] = sum of partial[row][0..nblk)
 cudaError_t dot_final(const double2* partial, int nblk, int nrows, double2* out, cudaStream_t st);
-// x += alpha p ; r -= alpha q ; out[v] = (|r_v|^2, |r_v|^2) (fused)
-template <class R>
-cudaError_t cg_xr_dot(cx<R>* x, cx<R>* r, const cx<R>* p, const cx<R>* q, long long len, long long stride, int nvec,
-                      const double* alpha, const int* active, double2* out, double2* partial, int nblk,
-                      cudaStream_t st);
-template <class R>
-cudaError_t cg_p(cx<R>* p, const cx<R>* r, long long len, long long stride, int nvec, const double* beta,
-                 const int* active, cudaStream_t st);
-cudaError_t cg_scalars(int stage, int nvec, const double2* dot, double* rho, double* alpha, double* beta,
-                       const double* tol2b2, int* active, int* iters, double* res2, cudaStream_t st);
-// cg_scalars on the sums of nblk partials per vector (partial[v * nblk + i]),
-// the sums also stored in dot[v]; one launch.
 // Condition kernel of a graph-resident loop (graph_replay_while): *passes
 // += 1, and the loop goes on while any active[v] and *passes < max_passes.
 cudaError_t while_active(const int* active, int nvec, int* passes, int max_passes, cudaGraphConditionalHandle h,
                          cudaStream_t st);
-cudaError_t cg_scalars_red(int stage, int nvec, const double2* partial, int nblk, double2* dot, double* rho,
-                           double* alpha, double* beta, const double* tol2b2, int* active, int* iters, double* res2,
-                           cudaStream_t st);
+// Start of a CG solve from the partials (Re b^H z, |b|^2) of pcg_start: rho, bb
+// = res2 = |b|^2, tol2b2 = (tolv |b|)^2, iters = 0; clears active[v] where b_v is
+// zero or not finite.
+cudaError_t cg_init(int nvec, const double2* partial, int nblk, const double* tolv, double* rho, double* tol2b2,
+                    double* bb, double* res2, int* active, int* iters, cudaStream_t st);
+// alpha_v = rho_v / Re(p^H q)_v from the nblk partials per vector
+// (partial[v * nblk + i], the sum also stored in dot[v]); a vector whose
+// p^H q is not positive is stopped with a negative iteration count.
+cudaError_t cg_alpha(int nvec, const double2* partial, int nblk, double2* dot, const double* rho, double* alpha,
+                     int* active, int* iters, cudaStream_t st);
+// The end of a CG iteration in one launch: (rz, rn) = (Re r^H z, |r|^2) from
+// the partials, rho_next = rz, res2 = rn, the iteration count and the
+// convergence test, and for the vectors still active p = z + (rz / rho) p.
+// rho and rho_next are two arrays (every CTA of a vector reads rho).
+template <class R>
+cudaError_t cg_dir(cx<R>* p, const cx<R>* z, long long len, int nvec, const double2* partial, int nblk,
+                   const double* rho, double* rho_next, double2* dot, const double* tol2b2, int* active, int* iters,
+                   double* res2, int ncta, cudaStream_t st);
 // Gram-Schmidt over a batch of instances, one launch each for all of them:
 // vector v of r (stride rs) works against columns span[v].x ..
 // span[v].x + span[v].y - 1 of its block X + v*xs (columns len apart);

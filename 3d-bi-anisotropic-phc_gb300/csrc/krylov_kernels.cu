@@ -137,93 +137,9 @@ __global__ void k_axpby(const cx<R>* __restrict__ x, cx<R>* __restrict__ y, long
   }
 }
 
-// CG update: x += a p ; r -= a q  with a = rho / Re(p'q) per vector.
-template <class R>
-__global__ void k_cg_xr(cx<R>* __restrict__ x, cx<R>* __restrict__ r, const cx<R>* __restrict__ p,
-                        const cx<R>* __restrict__ q, long long len, long long stride,
-                        const double* __restrict__ alpha, const int* __restrict__ active) {
-  const int vec = blockIdx.y;
-  if (active && !active[vec]) return;
-  const R a = R(alpha[vec]);
-  const long long o = vec * stride;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < len; i += (long long)gridDim.x * blockDim.x) {
-    cx<R> pi = p[o + i], qi = q[o + i], xi = x[o + i], ri = r[o + i];
-    xi.x += a * pi.x; xi.y += a * pi.y;
-    ri.x -= a * qi.x; ri.y -= a * qi.y;
-    x[o + i] = xi;
-    r[o + i] = ri;
-  }
-}
-
-// p = r + beta p
-template <class R>
-__global__ void k_cg_p(cx<R>* __restrict__ p, const cx<R>* __restrict__ r, long long len, long long stride,
-                       const double* __restrict__ beta, const int* __restrict__ active) {
-  const int vec = blockIdx.y;
-  pdl_wait();
-  if (active && !active[vec]) return;
-  const R b = R(beta[vec]);
-  const long long o = vec * stride;
-  const long long step = (long long)gridDim.x * blockDim.x;
-  long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  for (; i + step < len; i += 2 * step) {  // both elements' loads before the stores
-    const cx<R> pi = p[o + i], ri = r[o + i], pj = p[o + i + step], rj = r[o + i + step];
-    p[o + i] = mk<R>(ri.x + b * pi.x, ri.y + b * pi.y);
-    p[o + i + step] = mk<R>(rj.x + b * pj.x, rj.y + b * pj.y);
-  }
-  if (i < len) {
-    const cx<R> pi = p[o + i], ri = r[o + i];
-    p[o + i] = mk<R>(ri.x + b * pi.x, ri.y + b * pi.y);
-  }
-}
-
-// Per-vector CG scalars.  stage 0: alpha = rho/Re(pq); stage 1: convergence
-// test on rho_new and beta = rho_new/rho.
-// iters[v] counts the completed iterations of vector v on the device (so an
-// iteration needs no host-side argument and can be replayed from a graph);
-// a negative count flags breakdown at that iteration.
-__global__ void k_cg_scalars(int stage, int nvec, const double2* __restrict__ dot, double* __restrict__ rho,
-                             double* __restrict__ alpha, double* __restrict__ beta,
-                             const double* __restrict__ tol2b2, int* __restrict__ active,
-                             int* __restrict__ iters, double* __restrict__ res2) {
-  const int v = blockIdx.x * blockDim.x + threadIdx.x;
-  if (v >= nvec || !active[v]) return;
-  const int it = iters[v] + 1;
-  if (stage == 0) {
-    const double pq = dot[v].x;
-    alpha[v] = (pq != 0.0 && isfinite(pq)) ? rho[v] / pq : 0.0;
-    if (!(pq > 0.0) || !isfinite(pq)) {  // breakdown: B must be HPD
-      active[v] = 0;
-      iters[v] = -it;
-    }
-  } else {
-    // dot = (Re r'z, |r|^2) with z = M r (z = r without preconditioner)
-    const double rz = dot[v].x;
-    const double rn = dot[v].y;
-    res2[v] = rn;
-    beta[v] = rho[v] != 0.0 ? rz / rho[v] : 0.0;
-    rho[v] = rz;
-    iters[v] = it;
-    if (!isfinite(rn) || !isfinite(rz)) {  // NaN / Inf: stop and flag
-      active[v] = 0;
-      iters[v] = -it;
-    } else if (rn <= tol2b2[v]) {
-      active[v] = 0;  // converged: ||r|| <= tol ||b||
-    } else if (!(rz > 0.0)) {  // indefinite preconditioned system
-      active[v] = 0;
-      iters[v] = -it;
-    }
-  }
-}
-
-// k_cg_scalars preceded by the reduction of the vector's nblk partials (one
-// CTA per vector; the block sum has a fixed order, so the iterates repeat
-// run to run).
 __global__ void __launch_bounds__(kRedThreads)
-k_cg_scalars_red(int stage, const double2* __restrict__ partial, int nblk, double2* __restrict__ dot,
-                 double* __restrict__ rho, double* __restrict__ alpha, double* __restrict__ beta,
-                 const double* __restrict__ tol2b2, int* __restrict__ active, int* __restrict__ iters,
-                 double* __restrict__ res2) {
+k_cg_alpha(const double2* __restrict__ partial, int nblk, double2* __restrict__ dot, const double* __restrict__ rho,
+           double* __restrict__ alpha, int* __restrict__ active, int* __restrict__ iters) {
   const int v = blockIdx.x;
   pdl_wait();
   if (!active[v]) return;
@@ -236,30 +152,112 @@ k_cg_scalars_red(int stage, const double2* __restrict__ partial, int nblk, doubl
   s = block_sum2(s);
   if (threadIdx.x != 0) return;
   dot[v] = s;
-  const int it = iters[v] + 1;
-  if (stage == 0) {
-    const double pq = s.x;
-    alpha[v] = (pq != 0.0 && isfinite(pq)) ? rho[v] / pq : 0.0;
-    if (!(pq > 0.0) || !isfinite(pq)) {  // breakdown: B must be HPD
-      active[v] = 0;
-      iters[v] = -it;
-    }
-  } else {
+  const bool ok = s.x > 0.0 && isfinite(s.x);
+  alpha[v] = ok ? rho[v] / s.x : 0.0;
+  if (!ok) {  // breakdown: B must be HPD
+    active[v] = 0;
+    iters[v] = -(iters[v] + 1);
+  }
+}
+
+// Scalars of a CG solve from the partials (Re b^H z, |b|^2) of its start: rho,
+// |b|^2, the stopping threshold (tol_v |b|)^2, the counts; vectors with a zero
+// or non-finite right-hand side are not active.
+__global__ void __launch_bounds__(kRedThreads)
+k_cg_init(const double2* __restrict__ partial, int nblk, const double* __restrict__ tolv, double* __restrict__ rho,
+          double* __restrict__ tol2b2, double* __restrict__ bb, double* __restrict__ res2, int* __restrict__ active,
+          int* __restrict__ iters) {
+  const int v = blockIdx.x;
+  pdl_wait();
+  double2 s = make_double2(0.0, 0.0);
+  for (int i = threadIdx.x; i < nblk; i += blockDim.x) {
+    const double2 p = partial[(long long)v * nblk + i];
+    s.x += p.x;
+    s.y += p.y;
+  }
+  s = block_sum2(s);
+  if (threadIdx.x != 0) return;
+  rho[v] = s.x;
+  bb[v] = s.y;
+  res2[v] = s.y;
+  tol2b2[v] = tolv[v] * tolv[v] * s.y;
+  iters[v] = 0;
+  if (!(s.y > 0.0) || !isfinite(s.y)) active[v] = 0;
+}
+
+// End of a CG iteration (cg_dir).  Every CTA of a vector reduces the partials
+// in the same order, so all use the same beta; CTA 0 records the scalars.
+// iters[v] counts the completed iterations of vector v on the device (so an
+// iteration needs no host-side argument and can be replayed from a graph);
+// a negative count flags breakdown at that iteration.
+// HBM-bound (reads p and z, writes p).  One launch replaces a scalar kernel (6
+// us of latency on one CTA per vector) and the update of p inside fncB's first
+// plane kernel, which ran it at half the bandwidth (8 vectors at n = 48: 52 us
+// for the two and the transform, 38 now).
+template <class R>
+__global__ void __launch_bounds__(kRedThreads)
+k_cg_dir(cx<R>* __restrict__ p, const cx<R>* __restrict__ z, long long len, const double2* __restrict__ partial,
+         int nblk, const double* __restrict__ rho, double* __restrict__ rho_next, double2* __restrict__ dot,
+         const double* __restrict__ tol2b2, int* active, int* iters, double* __restrict__ res2) {
+  const int v = blockIdx.y;
+  __shared__ int s_act;
+  __shared__ double s_beta;
+  pdl_wait();
+  // one read per CTA: CTA 0 may clear the flag while others start
+  if (threadIdx.x == 0) s_act = active[v];
+  __syncthreads();
+  if (!s_act) return;
+  double2 s = make_double2(0.0, 0.0);
+  for (int i = threadIdx.x; i < nblk; i += blockDim.x) {
+    const double2 q = partial[(long long)v * nblk + i];
+    s.x += q.x;
+    s.y += q.y;
+  }
+  s = block_sum2(s);
+  if (threadIdx.x == 0) {
     const double rz = s.x, rn = s.y;  // (Re r'z, |r|^2), z = M r (z = r without preconditioner)
-    res2[v] = rn;
-    beta[v] = rho[v] != 0.0 ? rz / rho[v] : 0.0;
-    rho[v] = rz;
-    iters[v] = it;
-    if (!isfinite(rn) || !isfinite(rz)) {
-      active[v] = 0;
-      iters[v] = -it;
-    } else if (rn <= tol2b2[v]) {
-      active[v] = 0;
-    } else if (!(rz > 0.0)) {
-      active[v] = 0;
-      iters[v] = -it;
+    const double r0 = rho[v];
+    s_beta = r0 != 0.0 ? rz / r0 : 0.0;
+    const bool bad = !isfinite(rn) || !isfinite(rz);
+    const bool conv = !bad && rn <= tol2b2[v];        // ||r|| <= tol ||b||
+    const bool indef = !bad && !conv && !(rz > 0.0);  // indefinite preconditioned system
+    s_act = !(bad || conv || indef);
+    if (blockIdx.x == 0) {
+      const int it = iters[v] + 1;
+      dot[v] = s;
+      res2[v] = rn;
+      rho_next[v] = rz;
+      iters[v] = bad || indef ? -it : it;
+      if (!s_act) active[v] = 0;
     }
   }
+  __syncthreads();
+  if (!s_act) return;
+  const R b = R(s_beta);
+  const long long o = (long long)v * len;
+  const long long step = (long long)gridDim.x * blockDim.x;
+  constexpr int U = 16 / sizeof(cx<R>);  // elements per 16-byte access (len is a multiple of 4)
+  struct alignas(16) Pack { cx<R> e[U]; };
+  Pack* pp = reinterpret_cast<Pack*>(p + o);
+  const Pack* zp = reinterpret_cast<const Pack*>(z + o);
+  const long long n = len / U;
+  long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  auto one = [&](const Pack& a, Pack c) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) c.e[u] = caxpy(b, c.e[u], a.e[u]);
+    return c;
+  };
+  for (; i + 3 * step < n; i += 4 * step) {  // four packs in flight
+    Pack a[4], c[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      a[u] = zp[i + u * step];
+      c[u] = pp[i + u * step];
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) pp[i + u * step] = one(a[u], c[u]);
+  }
+  for (; i < n; i += step) pp[i] = one(zp[i], pp[i]);
 }
 
 // out[:, j] = sum_i in[:, i] * U[i, j]  (U real, p x k, column-major), all columns of one vector block
@@ -513,28 +511,8 @@ cudaError_t axpby_batched(const cx<R>* x, cx<R>* y, long long len, long long str
   return cudaGetLastError();
 }
 
-template <class R>
-cudaError_t cg_xr(cx<R>* x, cx<R>* r, const cx<R>* p, const cx<R>* q, long long len, long long stride, int nvec,
-                  const double* alpha, const int* active, cudaStream_t st) {
-  int gx = grid_for(len);
-  if (gx > 1024) gx = 1024;
-  FAME_LAUNCHED(1);
-  k_cg_xr<R><<<dim3(gx, nvec), 256, 0, st>>>(x, r, p, q, len, stride, alpha, active);
-  return cudaGetLastError();
-}
-
 cudaError_t dot_final(const double2* partial, int nblk, int nrows, double2* out, cudaStream_t st) {
   return launch<k_dot_final>(dim3(nrows), kRedThreads, 0, st, partial, nblk, out);
-}
-
-template <class R>
-cudaError_t cg_xr_dot(cx<R>* x, cx<R>* r, const cx<R>* p, const cx<R>* q, long long len, long long stride, int nvec,
-                      const double* alpha, const int* active, double2* out, double2* partial, int nblk,
-                      cudaStream_t st) {
-  cudaError_t e = launch<k_cg_xr_dot<R>>(dim3(nblk, nvec), kRedThreads, 0, st, x, r, p, q, len, stride, alpha, active,
-                                             partial);
-  if (e != cudaSuccess) return e;
-  return launch<k_dot_final>(dim3(nvec), kRedThreads, 0, st, (const double2*)partial, nblk, out);
 }
 
 template <class R>
@@ -635,27 +613,22 @@ cudaError_t while_active(const int* active, int nvec, int* passes, int max_passe
   return cudaGetLastError();
 }
 
-cudaError_t cg_scalars_red(int stage, int nvec, const double2* partial, int nblk, double2* dot, double* rho,
-                           double* alpha, double* beta, const double* tol2b2, int* active, int* iters, double* res2,
-                           cudaStream_t st) {
-  return launch<k_cg_scalars_red>(dim3(nvec), kRedThreads, 0, st, stage, partial, nblk, dot, rho, alpha, beta, tol2b2,
-                                      active, iters, res2);
+cudaError_t cg_alpha(int nvec, const double2* partial, int nblk, double2* dot, const double* rho, double* alpha,
+                     int* active, int* iters, cudaStream_t st) {
+  return launch<k_cg_alpha>(dim3(nvec), kRedThreads, 0, st, partial, nblk, dot, rho, alpha, active, iters);
+}
+
+cudaError_t cg_init(int nvec, const double2* partial, int nblk, const double* tolv, double* rho, double* tol2b2,
+                    double* bb, double* res2, int* active, int* iters, cudaStream_t st) {
+  return launch<k_cg_init>(dim3(nvec), kRedThreads, 0, st, partial, nblk, tolv, rho, tol2b2, bb, res2, active, iters);
 }
 
 template <class R>
-cudaError_t cg_p(cx<R>* p, const cx<R>* r, long long len, long long stride, int nvec, const double* beta,
-                 const int* active, cudaStream_t st) {
-  int gx = grid_for(len);
-  if (gx > 1024) gx = 1024;
-  return launch<k_cg_p<R>>(dim3(gx, nvec), 256, 0, st, p, r, len, stride, beta, active);
-}
-
-cudaError_t cg_scalars(int stage, int nvec, const double2* dot, double* rho, double* alpha, double* beta,
-                       const double* tol2b2, int* active, int* iters, double* res2, cudaStream_t st) {
-  FAME_LAUNCHED(1);
-  k_cg_scalars<<<(nvec + 127) / 128, 128, 0, st>>>(stage, nvec, dot, rho, alpha, beta, tol2b2, active, iters,
-                                                    res2);
-  return cudaGetLastError();
+cudaError_t cg_dir(cx<R>* p, const cx<R>* z, long long len, int nvec, const double2* partial, int nblk,
+                   const double* rho, double* rho_next, double2* dot, const double* tol2b2, int* active, int* iters,
+                   double* res2, int ncta, cudaStream_t st) {
+  return launch<k_cg_dir<R>>(dim3(ncta, nvec), kRedThreads, 0, st, p, z, len, partial, nblk, rho, rho_next, dot, tol2b2,
+                             active, iters, res2);
 }
 
 template <class R>
@@ -756,12 +729,8 @@ template cudaError_t scale_batched<float>(const cx<float>*, cx<float>*, long lon
                                       long long, int, double2*, double2*, int, const int*, cudaStream_t); \
   template cudaError_t axpby_batched<R>(const cx<R>*, cx<R>*, long long, long long, int, const double2*, \
                                         const double2*, const int*, cudaStream_t);                       \
-  template cudaError_t cg_xr<R>(cx<R>*, cx<R>*, const cx<R>*, const cx<R>*, long long, long long, int,   \
-                                const double*, const int*, cudaStream_t);                                 \
-  template cudaError_t cg_p<R>(cx<R>*, const cx<R>*, long long, long long, int, const double*,           \
-                               const int*, cudaStream_t);                                                 \
-  template cudaError_t cg_xr_dot<R>(cx<R>*, cx<R>*, const cx<R>*, const cx<R>*, long long, long long, int, \
-                                    const double*, const int*, double2*, double2*, int, cudaStream_t);    \
+  template cudaError_t cg_dir<R>(cx<R>*, const cx<R>*, long long, int, const double2*, int, const double*, \
+                                 double*, double2*, const double*, int*, int*, double*, int, cudaStream_t); \
   template cudaError_t block_rot<R>(const cx<R>*, cx<R>*, long long, long long, int, int, const double*, \
                                     cudaStream_t);                                                        \
   template cudaError_t sub_combo<R>(cx<R>*, const cx<R>*, long long, long long, int, const double2*,     \

@@ -170,10 +170,13 @@ __device__ __forceinline__ double2 block_sum2b(double2 v) {
   return v;
 }
 
+// The start of a CG solve in one pass (pcg_start): reads b and the block,
+// writes x, r, p (and z).
 template <class R>
 __global__ void __launch_bounds__(kThreads)
-k_precond_apply(const cx<R>* __restrict__ r, cx<R>* __restrict__ z, const cx<R>* __restrict__ pc_all, VecCtx ctx,
-                long long Nq, double2* __restrict__ partial) {
+k_pcg_start(const cx<R>* __restrict__ b, cx<R>* __restrict__ x, cx<R>* __restrict__ r, cx<R>* __restrict__ z,
+            cx<R>* __restrict__ p, const cx<R>* __restrict__ pc_all, VecCtx ctx, long long Nq,
+            double2* __restrict__ partial) {
   const int vec = blockIdx.y;
   const int nblk = gridDim.x;
   double2* out = partial + (long long)vec * nblk + blockIdx.x;
@@ -182,17 +185,21 @@ k_precond_apply(const cx<R>* __restrict__ r, cx<R>* __restrict__ z, const cx<R>*
     if (threadIdx.x == 0) *out = make_double2(0.0, 0.0);
     return;
   }
-  const cx<R>* pc = pc_all + (long long)vec_inst(ctx, vec) * kPcSlots * Nq;
+  const cx<R>* pc = pc_all ? pc_all + (long long)vec_inst(ctx, vec) * kPcSlots * Nq : nullptr;
   const long long o = vec * 4 * Nq;
   R srz = 0, srr = 0;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < Nq; i += (long long)nblk * blockDim.x) {
     cx<R> rv[4], zv[4];
 #pragma unroll
-    for (int c = 0; c < 4; ++c) rv[c] = r[o + c * Nq + i];
-    mvec4<R>(load_block<R>(pc, Nq, i), rv, zv);
+    for (int c = 0; c < 4; ++c) zv[c] = rv[c] = b[o + c * Nq + i];
+    if (pc) mvec4<R>(load_block<R>(pc, Nq, i), rv, zv);
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
-      z[o + c * Nq + i] = zv[c];
+      const long long k = o + c * Nq + i;
+      x[k] = zero<R>();
+      r[k] = rv[c];
+      p[k] = zv[c];
+      if (pc) z[k] = zv[c];
       srz += rv[c].x * zv[c].x + rv[c].y * zv[c].y;
       srr += rv[c].x * rv[c].x + rv[c].y * rv[c].y;
     }
@@ -326,10 +333,10 @@ template <class R> cudaError_t build_precond(Plan& P, cudaStream_t st) {
 }
 
 template <class R>
-cudaError_t precond_apply(const Plan& P, const cx<R>* r, cx<R>* z, int nvec, const VecCtx& ctx, double2* partial,
-                          int nblk, cudaStream_t st) {
-  const PlanData<R>& d = detail::pdata<R>(P);
-  return launch<k_precond_apply<R>>(dim3(nblk, nvec), kThreads, 0, st, r, z, d.pc, ctx, P.Nq, partial);
+cudaError_t pcg_start(const Plan& P, bool precond, const cx<R>* b, cx<R>* x, cx<R>* r, cx<R>* z, cx<R>* p, int nvec,
+                      const VecCtx& ctx, double2* partial, int nblk, cudaStream_t st) {
+  const cx<R>* pc = precond ? detail::pdata<R>(P).pc : nullptr;
+  return launch<k_pcg_start<R>>(dim3(nblk, nvec), kThreads, 0, st, b, x, r, z, p, pc, ctx, P.Nq, partial);
 }
 
 template <class R>
@@ -343,10 +350,10 @@ cudaError_t pcg_update(const Plan& P, cx<R>* x, cx<R>* r, cx<R>* z, const cx<R>*
 
 template cudaError_t build_precond<float>(Plan&, cudaStream_t);
 template cudaError_t build_precond<double>(Plan&, cudaStream_t);
-template cudaError_t precond_apply<float>(const Plan&, const float2*, float2*, int, const VecCtx&, double2*, int,
-                                          cudaStream_t);
-template cudaError_t precond_apply<double>(const Plan&, const double2*, double2*, int, const VecCtx&, double2*, int,
-                                           cudaStream_t);
+template cudaError_t pcg_start<float>(const Plan&, bool, const cx<float>*, cx<float>*, cx<float>*, cx<float>*, cx<float>*, int,
+                                         const VecCtx&, double2*, int, cudaStream_t);
+template cudaError_t pcg_start<double>(const Plan&, bool, const cx<double>*, cx<double>*, cx<double>*, cx<double>*, cx<double>*, int,
+                                         const VecCtx&, double2*, int, cudaStream_t);
 template cudaError_t pcg_update<float>(const Plan&, float2*, float2*, float2*, const float2*, const float2*, int,
                                        const VecCtx&, const double*, double2*, int, cudaStream_t, const CgAlpha&);
 template cudaError_t pcg_update<double>(const Plan&, double2*, double2*, double2*, const double2*, const double2*, int,

@@ -45,12 +45,30 @@ static int dot_blocks(const Plan& P, long long len, int nvec) {
   return (int)std::max(1LL, std::min(512LL, b));
 }
 
-// Device scalars of the batched CG, carved from one workspace.
+// Device scalars of the batched CG, carved from one workspace.  tolv and
+// active are uploaded together, active to res2 downloaded together.
 struct CgScalars {
-  double *rho, *alpha, *beta, *tol2b2, *res2;
+  double2* dot;
+  double *rho, *rho2, *alpha, *tol2b2;  // rho, rho2: of even and odd iterations
+  double* tolv;
   int *active, *iters;
   int* passes;  // passes of the graph-resident iteration loop
-  double2* dot;
+  double *bb, *res2;
+  static size_t bytes(int nvec) { return (sizeof(double2) + 7 * sizeof(double) + 2 * sizeof(int)) * nvec + 64; }
+  static size_t down_bytes(int nvec) { return (2 * sizeof(int) + 2 * sizeof(double)) * nvec + 2 * sizeof(int); }
+  void carve(char* s, int nvec) {
+    dot = (double2*)s;
+    rho = (double*)(dot + nvec);
+    rho2 = rho + nvec;
+    alpha = rho2 + nvec;
+    tol2b2 = alpha + nvec;
+    tolv = tol2b2 + nvec;
+    active = (int*)(tolv + nvec);
+    iters = active + nvec;
+    passes = iters + nvec;  // one, and one unused for alignment
+    bb = (double*)(passes + 2);
+    res2 = bb + nvec;
+  }
 };
 
 template <class R>
@@ -67,19 +85,10 @@ int pcg_batched(Plan& P, const cx<R>* b, cx<R>* x, int nvec, const int* d_inst, 
   FAME_CK(e, "pcg workspace");
   cx<R>* q = (cx<R>*)workspace(P, WS_PCG_Q + (sizeof(R) == 4 ? 100 : 0), vb, &e);
   FAME_CK(e, "pcg workspace");
-  const size_t sb = (5 * sizeof(double) + 2 * sizeof(int) + sizeof(double2)) * nvec + 4 * sizeof(int) + 64;
-  char* s = (char*)workspace(P, WS_PCG_SCAL, sb, &e);
+  char* s = (char*)workspace(P, WS_PCG_SCAL, CgScalars::bytes(nvec), &e);
   FAME_CK(e, "pcg workspace");
   CgScalars S;
-  S.dot = (double2*)s;
-  S.rho = (double*)(S.dot + nvec);
-  S.alpha = S.rho + nvec;
-  S.beta = S.alpha + nvec;
-  S.tol2b2 = S.beta + nvec;
-  S.res2 = S.tol2b2 + nvec;
-  S.active = (int*)(S.res2 + nvec);
-  S.iters = S.active + nvec;
-  S.passes = S.iters + nvec;
+  S.carve(s, nvec);
   const int nblk = dot_blocks(P, L, nvec);
   // p^H B p from the stencil pass of fncB where its tuned form provides it
   const int nblk_pq = fncB_pq_partials<R>(P, nvec);
@@ -93,39 +102,21 @@ int pcg_batched(Plan& P, const cx<R>* b, cx<R>* x, int nvec, const int* d_inst, 
   cx<R>* w0 = (cx<R>*)P.d_work;
   cx<R>* w1 = w0 + (size_t)nvec * 6 * P.Nq;
 
-  std::vector<int> act(nvec, 1);
-  if (h_mask)
-    for (int v = 0; v < nvec; ++v) act[v] = h_mask[v] ? 1 : 0;
-  FAME_CK(h2d_async(P, S.active, act.data(), sizeof(int) * nvec), "pcg init");
-  // ||b||^2 per vector
-  FAME_CK(dot_batched<R>(b, L, 0, 1, b, L, L, nvec, S.dot, part, nblk, S.active, st), "pcg dot");
-  std::vector<double2> bb(nvec);
-  FAME_CK(cudaMemcpyAsync(bb.data(), S.dot, sizeof(double2) * nvec, cudaMemcpyDeviceToHost, st), "pcg init");
-  FAME_CK(cudaStreamSynchronize(st), "pcg init");
-  std::vector<double> rho(nvec), t2(nvec);
+  // The start runs on the device without a host wait: the tolerances and the
+  // mask go up in one copy, one pass sets x, r, z, p and the partial sums, one
+  // small kernel the scalars.  (Three waits and ten small copies and memsets
+  // before took 0.15 ms of host time per solve.)
+  auto selected = [&](int v) { return h_mask ? h_mask[v] != 0 : true; };
+  std::vector<char> up((sizeof(double) + sizeof(int)) * (size_t)nvec);
+  bool any = false;
   for (int v = 0; v < nvec; ++v) {
-    rho[v] = bb[v].x;
     const double tv = tolv ? tolv[v] : tol;
-    t2[v] = tv * tv * bb[v].x;
-    if (act[v] && !std::isfinite(bb[v].x)) return fail(&P, FAME_ERR_NAN, "pcg: non-finite right-hand side");
-    if (act[v] && !(bb[v].x > 0.0)) {  // zero right-hand side: x = 0
-      act[v] = 0;
-    }
+    const int a = selected(v) ? 1 : 0;
+    any |= a != 0;
+    std::memcpy(up.data() + sizeof(double) * v, &tv, sizeof(double));
+    std::memcpy(up.data() + sizeof(double) * nvec + sizeof(int) * v, &a, sizeof(int));
   }
-  std::vector<int> it0(nvec, 0);
-  const std::vector<double> zero_beta(nvec, 0.0);  // the first direction is z itself
-  FAME_CK(h2d_async(P, S.beta, zero_beta.data(), sizeof(double) * nvec), "pcg init");
-  FAME_CK(h2d_async(P, S.rho, rho.data(), sizeof(double) * nvec), "pcg init");
-  FAME_CK(h2d_async(P, S.tol2b2, t2.data(), sizeof(double) * nvec), "pcg init");
-  FAME_CK(h2d_async(P, S.res2, rho.data(), sizeof(double) * nvec), "pcg init");
-  FAME_CK(h2d_async(P, S.iters, it0.data(), sizeof(int) * nvec), "pcg init");
-  for (int v = 0; v < nvec; ++v) {
-    const bool sel = h_mask ? h_mask[v] != 0 : true;
-    if (!sel) continue;
-    FAME_CK(cudaMemsetAsync(x + (size_t)v * L, 0, sizeof(cx<R>) * L, st), "pcg init");
-  }
-  FAME_CK(h2d_async(P, S.active, act.data(), sizeof(int) * nvec), "pcg init");
-  FAME_CK(cudaMemcpyAsync(r, b, vb, cudaMemcpyDeviceToDevice, st), "pcg init");
+  FAME_CK(h2d_async(P, S.tolv, up.data(), up.size()), "pcg init");
   VecCtx ctx;
   ctx.inst = d_inst;
   ctx.active = S.active;
@@ -138,55 +129,44 @@ int pcg_batched(Plan& P, const cx<R>* b, cx<R>* x, int nvec, const int* d_inst, 
     z = (cx<R>*)workspace(P, WS_PCG_Z + (sizeof(R) == 4 ? 100 : 0), vb, &e);
     FAME_CK(e, "pcg workspace");
     FAME_CK(build_precond<R>(P, st), "pcg preconditioner");
-    FAME_CK(precond_apply<R>(P, b, z, nvec, ctx, part, nblkv, st), "pcg precond");
-    FAME_CK(cudaMemcpyAsync(p, z, vb, cudaMemcpyDeviceToDevice, st), "pcg init");
-    FAME_CK(dot_final(part, nblkv, nvec, S.dot, st), "pcg precond");
-    std::vector<double2> rz(nvec);
-    FAME_CK(cudaMemcpyAsync(rz.data(), S.dot, sizeof(double2) * nvec, cudaMemcpyDeviceToHost, st), "pcg init");
-    FAME_CK(cudaStreamSynchronize(st), "pcg init");
-    for (int v = 0; v < nvec; ++v) rho[v] = act[v] ? rz[v].x : 0.0;
-    FAME_CK(h2d_async(P, S.rho, rho.data(), sizeof(double) * nvec), "pcg init");
-    FAME_CK(cudaStreamSynchronize(st), "pcg init");
-  } else {
-    FAME_CK(cudaMemcpyAsync(p, b, vb, cudaMemcpyDeviceToDevice, st), "pcg init");
   }
+  FAME_CK(pcg_start<R>(P, pre, b, x, r, z, p, nvec, ctx, part, nblkv, st), "pcg start");
+  FAME_CK(cg_init(nvec, part, nblkv, S.tolv, S.rho, S.tol2b2, S.bb, S.res2, S.active, S.iters, st), "pcg init");
   // One CG iteration: every kernel reads its scalars and active flags from
   // the device, so a block of iterations is a fixed launch sequence that is
   // captured once per (sizes, pointers) and replayed from a CUDA graph.
-  //   p = z + beta p, q = B p         (the update done by fncB's first kernel;
-  //                                     beta = 0 before the first iteration;
-  //                                     with the partials of p^H q when the
+  //   q = B p                         (with the partials of p^H q when the
   //                                     stencil pass provides them)
   //   alpha = rho / p^H q             (preconditioned: reduced by the update
   //                                     kernel itself; else one scalar launch)
   //   x += alpha p, r -= alpha q, z = M r, partials of (r^H z, |r|^2)
-  //   beta, rho, convergence          (partials reduced in the same launch)
-  // Preconditioned, that is two glue launches per iteration.
-  CgAlpha ca;
-  if (pre) {
-    ca.pq = part;
-    ca.nblk = nblk_pq ? nblk_pq : nblk;
-    ca.rho = S.rho;
-    ca.alpha = S.alpha;
-    ca.dot = S.dot;
-    ca.active = S.active;
-    ca.iters = S.iters;
-  }
-  auto iteration = [&](cudaStream_t cs) -> cudaError_t {
-    cudaError_t e2 = launch_fncB<R>(P, p, q, nvec, ctx, w0, w1, cs, nblk_pq ? part : nullptr, pre ? z : r, S.beta);
+  //   beta, rho, convergence, p = z + beta p   (partials reduced in the same launch)
+  // Preconditioned, that is two glue launches per iteration.  Iteration i reads
+  // rho from one of two arrays and writes the other (i odd / even; the blocks
+  // of chk iterations are even).
+  auto iteration = [&](cudaStream_t cs, int i) -> cudaError_t {
+    double* rho_in = i & 1 ? S.rho2 : S.rho;
+    double* rho_out = i & 1 ? S.rho : S.rho2;
+    cudaError_t e2 = launch_fncB<R>(P, p, q, nvec, ctx, w0, w1, cs, nblk_pq ? part : nullptr);
     if (e2 == cudaSuccess && !nblk_pq) e2 = dot_partial<R>(p, q, L, L, nvec, part, nblk, S.active, cs);
     if (pre) {
       // the update's own partial sums go to part2 (part still holds p^H q)
+      CgAlpha ca;
+      ca.pq = part;
+      ca.nblk = nblk_pq ? nblk_pq : nblk;
+      ca.rho = rho_in;
+      ca.alpha = S.alpha;
+      ca.dot = S.dot;
+      ca.active = S.active;
+      ca.iters = S.iters;
       if (e2 == cudaSuccess) e2 = pcg_update<R>(P, x, r, z, p, q, nvec, ctx, S.alpha, part2, nblkv, cs, ca);
     } else {
-      if (e2 == cudaSuccess)
-        e2 = cg_scalars_red(0, nvec, part, nblk, S.dot, S.rho, S.alpha, S.beta, S.tol2b2, S.active, S.iters,
-                            S.res2, cs);
+      if (e2 == cudaSuccess) e2 = cg_alpha(nvec, part, nblk_pq ? nblk_pq : nblk, S.dot, rho_in, S.alpha, S.active, S.iters, cs);
       if (e2 == cudaSuccess) e2 = cg_xr_partial<R>(x, r, p, q, L, L, nvec, S.alpha, S.active, part, nblk, cs);
     }
     if (e2 == cudaSuccess)
-      e2 = cg_scalars_red(1, nvec, pre ? part2 : part, pre ? nblkv : nblk, S.dot, S.rho, S.alpha, S.beta, S.tol2b2,
-                          S.active, S.iters, S.res2, cs);
+      e2 = cg_dir<R>(p, pre ? z : r, L, nvec, pre ? part2 : part, pre ? nblkv : nblk, rho_in, rho_out, S.dot, S.tol2b2,
+                     S.active, S.iters, S.res2, nblk, cs);
     return e2;
   };
   const int chk = 4;
@@ -198,8 +178,20 @@ int pcg_batched(Plan& P, const cx<R>* b, cx<R>* x, int nvec, const int* d_inst, 
                                        (uintptr_t)tune_for(P, tune_prec<R>(), nvec).chunk,
                                        (uintptr_t)tune_for(P, tune_prec<R>(), nvec).stencil_tpb,
                                        (uintptr_t)nblk_pq, (uintptr_t)P.opt_pi_table};
+  // active flags, counts and norms of every vector, after the work issued so far
+  std::vector<char> down(CgScalars::down_bytes(nvec));
+  const int* act = (const int*)down.data();
+  const int* its = act + nvec;
+  const int* passes = its + nvec;
+  const double* bb = (const double*)(passes + 2);
+  const double* r2 = bb + nvec;
+  auto download = [&]() -> cudaError_t {
+    cudaError_t e2 = cudaMemcpyAsync(down.data(), S.active, down.size(), cudaMemcpyDeviceToHost, st);
+    if (e2 == cudaSuccess) e2 = cudaStreamSynchronize(st);
+    any = std::any_of(act, act + nvec, [](int a) { return a != 0; });
+    return e2;
+  };
   bool use_graph = P.opt_graph != 0;
-  bool any = std::any_of(act.begin(), act.end(), [](int a) { return a != 0; });
   int it = 1;
   if (P.opt_graph >= 2 && any && maxit >= chk) {
     // the whole loop of chk-iteration blocks in one graph launch, the
@@ -210,30 +202,27 @@ int pcg_batched(Plan& P, const cx<R>* b, cx<R>* x, int nvec, const int* d_inst, 
     unsigned long long body_nodes = 0;
     cudaError_t ge = graph_replay_while(P, wkey, [&](cudaStream_t cs) -> cudaError_t {
       for (int i = 0; i < chk; ++i) {
-        cudaError_t e2 = iteration(cs);
+        cudaError_t e2 = iteration(cs, i);
         if (e2 != cudaSuccess) return e2;
       }
       return cudaSuccess;
     }, S.active, nvec, S.passes, maxit / chk, &body_nodes);
     if (ge == cudaSuccess) {
-      int passes = 0;
-      FAME_CK(cudaMemcpyAsync(act.data(), S.active, sizeof(int) * nvec, cudaMemcpyDeviceToHost, st), "pcg check");
-      FAME_CK(cudaMemcpyAsync(&passes, S.passes, sizeof(int), cudaMemcpyDeviceToHost, st), "pcg check");
-      FAME_CK(cudaStreamSynchronize(st), "pcg check");
-      FAME_KERNELS_RAN(body_nodes * (unsigned long long)passes);
-      it = 1 + passes * chk;
-      any = std::any_of(act.begin(), act.end(), [](int a) { return a != 0; });
+      FAME_CK(download(), "pcg check");
+      FAME_KERNELS_RAN(body_nodes * (unsigned long long)*passes);
+      it = 1 + *passes * chk;
     } else {
       cudaGetLastError();  // no graph loop (nothing of it ran): the blocks below take over
     }
   }
+  bool fresh = it > 1;  // `down` holds the state after the last iteration issued
   for (; it <= maxit && any; it += chk) {
     const int nit = std::min(chk, maxit - it + 1);
     bool done = false;
     if (use_graph && nit == chk) {
       cudaError_t ge = graph_replay(P, gkey, [&](cudaStream_t cs) -> cudaError_t {
         for (int i = 0; i < chk; ++i) {
-          cudaError_t e2 = iteration(cs);
+          cudaError_t e2 = iteration(cs, i);
           if (e2 != cudaSuccess) return e2;
         }
         return cudaSuccess;
@@ -242,23 +231,18 @@ int pcg_batched(Plan& P, const cx<R>* b, cx<R>* x, int nvec, const int* d_inst, 
       else use_graph = false;  // capture unavailable: issue directly from now on
     }
     if (!done)
-      for (int i = 0; i < nit; ++i) FAME_CK(iteration(st), "pcg iteration");
-    FAME_CK(cudaMemcpyAsync(act.data(), S.active, sizeof(int) * nvec, cudaMemcpyDeviceToHost, st), "pcg check");
-    FAME_CK(cudaStreamSynchronize(st), "pcg check");
-    any = std::any_of(act.begin(), act.end(), [](int a) { return a != 0; });
+      for (int i = 0; i < nit; ++i) FAME_CK(iteration(st, i), "pcg iteration");
+    FAME_CK(download(), "pcg check");
+    fresh = true;
   }
-  std::vector<int> its(nvec);
-  std::vector<double> r2(nvec);
-  FAME_CK(cudaMemcpyAsync(its.data(), S.iters, sizeof(int) * nvec, cudaMemcpyDeviceToHost, st), "pcg out");
-  FAME_CK(cudaMemcpyAsync(r2.data(), S.res2, sizeof(double) * nvec, cudaMemcpyDeviceToHost, st), "pcg out");
-  FAME_CK(cudaMemcpyAsync(act.data(), S.active, sizeof(int) * nvec, cudaMemcpyDeviceToHost, st), "pcg out");
-  FAME_CK(cudaStreamSynchronize(st), "pcg out");
+  if (!fresh) FAME_CK(download(), "pcg out");
+  for (int v = 0; v < nvec; ++v)
+    if (selected(v) && !std::isfinite(bb[v])) return fail(&P, FAME_ERR_NAN, "pcg: non-finite right-hand side");
   int rc = FAME_OK;
   for (int v = 0; v < nvec; ++v) {
-    const bool sel = h_mask ? h_mask[v] != 0 : true;
-    if (!sel) continue;
+    if (!selected(v)) continue;
     if (iters_out) iters_out[v] = its[v];
-    if (relres_out) relres_out[v] = bb[v].x > 0.0 ? std::sqrt(std::max(r2[v], 0.0) / bb[v].x) : 0.0;
+    if (relres_out) relres_out[v] = bb[v] > 0.0 ? std::sqrt(std::max(r2[v], 0.0) / bb[v]) : 0.0;
     if (its[v] < 0) rc = std::isfinite(r2[v]) ? FAME_ERR_BREAKDOWN : FAME_ERR_NAN;
     else if (act[v] && rc == FAME_OK) rc = FAME_ERR_NOT_CONVERGED;
   }
