@@ -263,13 +263,13 @@ template <class R> cudaError_t build_precond(Plan& P, cudaStream_t st);
 template <class R>
 cudaError_t pcg_start(const Plan& P, bool precond, const cx<R>* b, cx<R>* x, cx<R>* r, cx<R>* z, cx<R>* p, int nvec,
                       const VecCtx& ctx, double2* partial, int nblk, cudaStream_t st);
-// The CG step length computed inside the update instead of by a separate
-// scalar kernel: every CTA of vector v reduces v's `nblk` partial sums of
-// p^H q in one fixed order, so all of them use the same alpha = rho / p^H q;
-// CTA 0 records alpha and the dot, and on breakdown (p^H q <= 0 or not
-// finite) clears active[v] and negates the iteration count (alpha 0).
+// The CG step length, computed inside the update: every CTA of vector v reduces
+// v's `nblk` partial sums of p^H q in one fixed order, so all of them use the
+// same alpha = rho / p^H q; CTA 0 records alpha and the dot, and on breakdown
+// (p^H q <= 0 or not finite) clears active[v] and negates the iteration count
+// (alpha 0).
 struct CgAlpha {
-  const double2* pq = nullptr;  // [nvec][nblk] partial sums, or null: alpha given
+  const double2* pq = nullptr;  // [nvec][nblk] partial sums
   int nblk = 0;
   const double* rho = nullptr;
   double* alpha = nullptr;
@@ -280,8 +280,7 @@ struct CgAlpha {
 // x += a p ; r -= a q ; z = M r ; partial (Re r'z, |r|^2)
 template <class R>
 cudaError_t pcg_update(const Plan& P, cx<R>* x, cx<R>* r, cx<R>* z, const cx<R>* p, const cx<R>* q, int nvec,
-                       const VecCtx& ctx, const double* alpha, double2* partial, int nblk, cudaStream_t st,
-                       const CgAlpha& ca = CgAlpha());
+                       const VecCtx& ctx, double2* partial, int nblk, cudaStream_t st, const CgAlpha& ca);
 
 bool n_supported(int n);
 

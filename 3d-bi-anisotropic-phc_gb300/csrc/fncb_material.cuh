@@ -248,7 +248,8 @@ k_faceedge(const cx<R>* uv, const cx<R>* __restrict__ h, cx<R>* out, PlanData<R>
 // sweeps through the chunk plane by plane, thread (r, x) on vertex row y0 + r
 // (r = TY is the +y neighbour the scatter needs, evaluated but not written):
 //   * the fields of a plane (rows y0-1 .. y0+TY) are staged in shared memory
-//     by cp.async, one plane ahead of the plane being computed;
+//     by cp.async, the next plane in flight while this one is computed, the one
+//     after it issued as soon as stage 1 has read its buffer;
 //   * stage 1 gathers U, V and evaluates the vertex product.  Whatever the
 //     next plane needs of this one is kept in registers, already summed over
 //     its in-plane neighbours: s0 = u_0 + T_y^H u_0, s1 = u_1 + T_x^H u_1, u_5;
@@ -317,14 +318,6 @@ k_sweep(const cx<R>* __restrict__ uv, cx<R>* __restrict__ out, PlanData<R> d, co
   const cx<R>* src = uv + vec * stride;
   cx<R>* dst = out + vec * stride;
   const cx<R> Tx = d.tau[inst * 3], Ty = d.tau[inst * 3 + 1], Tz = d.tau[inst * 3 + 2];
-  const R* tab = nullptr;
-  if constexpr (KIND != kMatField) {
-    tab = d.stn + (size_t)inst * nphase * TS;
-    if (nphase <= SH::TAB_MAX) {
-      for (int i = tid; i < nphase * TS; i += TPB) Tb[i] = tab[i];
-      tab = Tb;
-    }
-  }
   // This thread's 16-byte chunks of a staged plane: shared-memory offset and
   // global offset within the plane, the same for every plane of the sweep.
   int soff[SH::NCH], goff[SH::NCH];
@@ -348,6 +341,16 @@ k_sweep(const cx<R>* __restrict__ uv, cx<R>* __restrict__ out, PlanData<R> d, co
       if (tid + i * TPB < SH::CH) cp_async16(F + soff[i], sp + goff[i]);
     cp_async_commit();
   };
+  stage(0);
+  stage(1);
+  const R* tab = nullptr;
+  if constexpr (KIND != kMatField) {
+    tab = d.stn + (size_t)inst * nphase * TS;
+    if (nphase <= SH::TAB_MAX) {
+      for (int i = tid; i < nphase * TS; i += TPB) Tb[i] = tab[i];
+      tab = Tb;
+    }
+  }
 
   const int r = tid / N, x = tid - r * N;
   const bool act = tid < HR * N;   // stage 1
@@ -362,11 +365,10 @@ k_sweep(const cx<R>* __restrict__ uv, cx<R>* __restrict__ out, PlanData<R> d, co
   // partial outputs q0, q1, q5 with the fields f0, f1, f5 they still need
   cx<R> s0 = zero<R>(), s1 = zero<R>(), f0 = zero<R>(), f1 = zero<R>(), f5 = zero<R>();
   cx<R> q0 = zero<R>(), q1 = zero<R>(), q5 = zero<R>();
-  stage(0);
   for (int s = 0; s <= nz + 1; ++s) {
-    cp_async_wait<0>();
-    __syncthreads();  // plane s visible; H, D and the other field buffer free again
-    if (s <= nz) stage(s + 1);
+    if (s <= nz) cp_async_wait<1>();
+    else cp_async_wait<0>();
+    __syncthreads();  // plane s visible; H, D free again
     const cx<R>* F = Fb + (s & 1) * SH::F_ELEMS;
     auto at = [&](int f, int rr, int xx) { return F[(f * FR + rr) * N + xx]; };
     const int zc = (z0 - 1 + s + N) % N;
@@ -402,7 +404,8 @@ k_sweep(const cx<R>* __restrict__ uv, cx<R>* __restrict__ out, PlanData<R> d, co
       s0 = p0;
       s1 = p1;
     }
-    __syncthreads();
+    __syncthreads();  // H, D visible; the buffer of plane s free again
+    if (s < nz) stage(s + 2);
     if (s >= 1 && outp) {
       auto h = [&](int f, int rr, int xx) { return H[(f * HR + rr) * N + xx]; };
       auto dd = [&](int f, int rr, int xx) { return D[(f * HR + rr) * N + xx]; };

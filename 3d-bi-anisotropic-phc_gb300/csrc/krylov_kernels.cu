@@ -12,18 +12,19 @@ namespace {
 constexpr int kRedThreads = 256;
 
 // Block-wide sum of a (double re, double im) pair; result valid in thread 0.
+// Through shared memory by one warp: 24 FP64 warp instructions instead of the
+// 90 of a shuffle tree in every warp (each takes the SM's FP64 pipe for 16
+// cycles, and small launches are mostly their reductions).
 __device__ __forceinline__ double2 block_sum2(double2 v) {
-  __shared__ double2 sh[kRedThreads / 32];
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    v.x += __shfl_down_sync(0xffffffffu, v.x, o);
-    v.y += __shfl_down_sync(0xffffffffu, v.y, o);
-  }
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  if (lane == 0) sh[wid] = v;
+  __shared__ double2 sh[kRedThreads];
+  sh[threadIdx.x] = v;
   __syncthreads();
-  if (wid == 0) {
-    v = lane < (blockDim.x >> 5) ? sh[lane] : make_double2(0.0, 0.0);
+  if (threadIdx.x < 32) {
+#pragma unroll
+    for (int k = 1; k < kRedThreads / 32; ++k) {
+      v.x += sh[threadIdx.x + 32 * k].x;
+      v.y += sh[threadIdx.x + 32 * k].y;
+    }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
       v.x += __shfl_down_sync(0xffffffffu, v.x, o);
@@ -31,6 +32,23 @@ __device__ __forceinline__ double2 block_sum2(double2 v) {
     }
   }
   return v;
+}
+
+// Sum of n partials, by the first warp of the block; valid in thread 0.
+__device__ __forceinline__ double2 warp_sum2(const double2* __restrict__ q, int n) {
+  double2 s = make_double2(0.0, 0.0);
+  if (threadIdx.x < 32) {
+    for (int j = threadIdx.x; j < n; j += 32) {
+      s.x += q[j].x;
+      s.y += q[j].y;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      s.x += __shfl_down_sync(0xffffffffu, s.x, o);
+      s.y += __shfl_down_sync(0xffffffffu, s.y, o);
+    }
+  }
+  return s;
 }
 
 // partial[v][m][blk] = sum over the block's slice of conj(a_m) * b
@@ -55,19 +73,19 @@ k_dot_partial(const cx<R>* __restrict__ a, long long a_vstride, long long a_cstr
   // sums a few dozen products; FP64 is rate-limited on this part), then FP64
   // across threads and blocks.
   R sx0 = 0, sy0 = 0, sx1 = 0, sy1 = 0;
-  const long long step = (long long)nblk * blockDim.x;
-  long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  for (; i + step < len; i += 2 * step) {
-    cx<R> x = av[i], y = bv[i], x2 = av[i + step], y2 = bv[i + step];
-    sx0 += x.x * y.x + x.y * y.y;
-    sy0 += x.x * y.y - x.y * y.x;
-    sx1 += x2.x * y2.x + x2.y * y2.y;
-    sy1 += x2.x * y2.y - x2.y * y2.x;
+  const long long chunk = (len + nblk - 1) / nblk, end = min(len, (blockIdx.x + 1) * chunk);
+  long long i = blockIdx.x * chunk + threadIdx.x;
+  for (; i + kRedThreads < end; i += 2 * kRedThreads) {
+    cx<R> x = av[i], y = bv[i], x2 = av[i + kRedThreads], y2 = bv[i + kRedThreads];
+    sx0 = rfma(x.x, y.x, rfma(x.y, y.y, sx0));
+    sy0 = rfma(x.x, y.y, rfma(-x.y, y.x, sy0));
+    sx1 = rfma(x2.x, y2.x, rfma(x2.y, y2.y, sx1));
+    sy1 = rfma(x2.x, y2.y, rfma(-x2.y, y2.x, sy1));
   }
-  if (i < len) {
+  if (i < end) {
     cx<R> x = av[i], y = bv[i];
-    sx0 += x.x * y.x + x.y * y.y;
-    sy0 += x.x * y.y - x.y * y.x;
+    sx0 = rfma(x.x, y.x, rfma(x.y, y.y, sx0));
+    sy0 = rfma(x.x, y.y, rfma(-x.y, y.x, sy0));
   }
   double2 s = make_double2(double(sx0) + double(sx1), double(sy0) + double(sy1));
   s = block_sum2(s);
@@ -91,7 +109,8 @@ k_cg_xr_dot(cx<R>* __restrict__ x, cx<R>* __restrict__ r, const cx<R>* __restric
   const R a = R(alpha[vec]);
   const long long o = vec * stride;
   R s0 = 0;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < len; i += (long long)nblk * blockDim.x) {
+  const long long chunk = (len + nblk - 1) / nblk, end = min(len, (blockIdx.x + 1) * chunk);
+  for (long long i = blockIdx.x * chunk + threadIdx.x; i < end; i += kRedThreads) {
     cx<R> pi = p[o + i], qi = q[o + i], xi = x[o + i], ri = r[o + i];
     xi.x += a * pi.x;
     xi.y += a * pi.y;
@@ -105,17 +124,11 @@ k_cg_xr_dot(cx<R>* __restrict__ x, cx<R>* __restrict__ r, const cx<R>* __restric
   if (threadIdx.x == 0) *out = s;
 }
 
-__global__ void __launch_bounds__(kRedThreads)
+__global__ void __launch_bounds__(32)
 k_dot_final(const double2* __restrict__ partial, int nblk, double2* __restrict__ out) {
   const long long row = blockIdx.x;  // vec * ma + m
   pdl_wait();
-  double2 s = make_double2(0.0, 0.0);
-  for (int i = threadIdx.x; i < nblk; i += blockDim.x) {
-    double2 p = partial[row * nblk + i];
-    s.x += p.x;
-    s.y += p.y;
-  }
-  s = block_sum2(s);
+  const double2 s = warp_sum2(partial + row * nblk, nblk);
   if (threadIdx.x == 0) out[row] = s;
 }
 
@@ -137,19 +150,13 @@ __global__ void k_axpby(const cx<R>* __restrict__ x, cx<R>* __restrict__ y, long
   }
 }
 
-__global__ void __launch_bounds__(kRedThreads)
+__global__ void __launch_bounds__(32)
 k_cg_alpha(const double2* __restrict__ partial, int nblk, double2* __restrict__ dot, const double* __restrict__ rho,
            double* __restrict__ alpha, int* __restrict__ active, int* __restrict__ iters) {
   const int v = blockIdx.x;
   pdl_wait();
   if (!active[v]) return;
-  double2 s = make_double2(0.0, 0.0);
-  for (int i = threadIdx.x; i < nblk; i += blockDim.x) {
-    const double2 p = partial[(long long)v * nblk + i];
-    s.x += p.x;
-    s.y += p.y;
-  }
-  s = block_sum2(s);
+  const double2 s = warp_sum2(partial + (long long)v * nblk, nblk);
   if (threadIdx.x != 0) return;
   dot[v] = s;
   const bool ok = s.x > 0.0 && isfinite(s.x);
@@ -163,19 +170,13 @@ k_cg_alpha(const double2* __restrict__ partial, int nblk, double2* __restrict__ 
 // Scalars of a CG solve from the partials (Re b^H z, |b|^2) of its start: rho,
 // |b|^2, the stopping threshold (tol_v |b|)^2, the counts; vectors with a zero
 // or non-finite right-hand side are not active.
-__global__ void __launch_bounds__(kRedThreads)
+__global__ void __launch_bounds__(32)
 k_cg_init(const double2* __restrict__ partial, int nblk, const double* __restrict__ tolv, double* __restrict__ rho,
           double* __restrict__ tol2b2, double* __restrict__ bb, double* __restrict__ res2, int* __restrict__ active,
           int* __restrict__ iters) {
   const int v = blockIdx.x;
   pdl_wait();
-  double2 s = make_double2(0.0, 0.0);
-  for (int i = threadIdx.x; i < nblk; i += blockDim.x) {
-    const double2 p = partial[(long long)v * nblk + i];
-    s.x += p.x;
-    s.y += p.y;
-  }
-  s = block_sum2(s);
+  const double2 s = warp_sum2(partial + (long long)v * nblk, nblk);
   if (threadIdx.x != 0) return;
   rho[v] = s.x;
   bb[v] = s.y;
@@ -190,10 +191,11 @@ k_cg_init(const double2* __restrict__ partial, int nblk, const double* __restric
 // iters[v] counts the completed iterations of vector v on the device (so an
 // iteration needs no host-side argument and can be replayed from a graph);
 // a negative count flags breakdown at that iteration.
-// HBM-bound (reads p and z, writes p).  One launch replaces a scalar kernel (6
-// us of latency on one CTA per vector) and the update of p inside fncB's first
-// plane kernel, which ran it at half the bandwidth (8 vectors at n = 48: 52 us
-// for the two and the transform, 38 now).
+// HBM-bound (reads p and z, writes p), the first elements loaded while the
+// partials are reduced.  One launch replaces a scalar kernel (6 us of latency
+// on one CTA per vector) and the update of p inside fncB's first plane kernel,
+// which ran it at half the bandwidth (8 vectors at n = 48: 55 us for the two
+// and the transform, 39 now).
 template <class R>
 __global__ void __launch_bounds__(kRedThreads)
 k_cg_dir(cx<R>* __restrict__ p, const cx<R>* __restrict__ z, long long len, const double2* __restrict__ partial,
@@ -207,13 +209,27 @@ k_cg_dir(cx<R>* __restrict__ p, const cx<R>* __restrict__ z, long long len, cons
   if (threadIdx.x == 0) s_act = active[v];
   __syncthreads();
   if (!s_act) return;
-  double2 s = make_double2(0.0, 0.0);
-  for (int i = threadIdx.x; i < nblk; i += blockDim.x) {
-    const double2 q = partial[(long long)v * nblk + i];
-    s.x += q.x;
-    s.y += q.y;
-  }
-  s = block_sum2(s);
+  constexpr int U = 16 / sizeof(cx<R>);  // elements per 16-byte access (len is a multiple of 4)
+  struct alignas(16) Pack {
+    cx<R> e[U];
+  };
+  Pack* pp = reinterpret_cast<Pack*>(p + (long long)v * len);
+  const Pack* zp = reinterpret_cast<const Pack*>(z + (long long)v * len);
+  const int np = int(len / U), chunk = (np + gridDim.x - 1) / gridDim.x;
+  const int end = min(np, (int(blockIdx.x) + 1) * chunk);
+  int i = blockIdx.x * chunk + threadIdx.x;
+  constexpr int B = 4;  // packs in flight; the first ones during the reduction
+  Pack a[B], c[B];
+  auto load = [&]() {
+#pragma unroll
+    for (int u = 0; u < B; ++u)
+      if (i + u * kRedThreads < end) {
+        a[u] = zp[i + u * kRedThreads];
+        c[u] = pp[i + u * kRedThreads];
+      }
+  };
+  load();
+  const double2 s = warp_sum2(partial + (long long)v * nblk, nblk);
   if (threadIdx.x == 0) {
     const double rz = s.x, rn = s.y;  // (Re r'z, |r|^2), z = M r (z = r without preconditioner)
     const double r0 = rho[v];
@@ -234,30 +250,17 @@ k_cg_dir(cx<R>* __restrict__ p, const cx<R>* __restrict__ z, long long len, cons
   __syncthreads();
   if (!s_act) return;
   const R b = R(s_beta);
-  const long long o = (long long)v * len;
-  const long long step = (long long)gridDim.x * blockDim.x;
-  constexpr int U = 16 / sizeof(cx<R>);  // elements per 16-byte access (len is a multiple of 4)
-  struct alignas(16) Pack { cx<R> e[U]; };
-  Pack* pp = reinterpret_cast<Pack*>(p + o);
-  const Pack* zp = reinterpret_cast<const Pack*>(z + o);
-  const long long n = len / U;
-  long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  auto one = [&](const Pack& a, Pack c) {
+  while (i < end) {
 #pragma unroll
-    for (int u = 0; u < U; ++u) c.e[u] = caxpy(b, c.e[u], a.e[u]);
-    return c;
-  };
-  for (; i + 3 * step < n; i += 4 * step) {  // four packs in flight
-    Pack a[4], c[4];
+    for (int u = 0; u < B; ++u)
+      if (i + u * kRedThreads < end) {
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      a[u] = zp[i + u * step];
-      c[u] = pp[i + u * step];
-    }
-#pragma unroll
-    for (int u = 0; u < 4; ++u) pp[i + u * step] = one(a[u], c[u]);
+        for (int w = 0; w < U; ++w) c[u].e[w] = caxpy(b, c[u].e[w], a[u].e[w]);
+        pp[i + u * kRedThreads] = c[u];
+      }
+    i += B * kRedThreads;
+    load();
   }
-  for (; i < n; i += step) pp[i] = one(zp[i], pp[i]);
 }
 
 // out[:, j] = sum_i in[:, i] * U[i, j]  (U real, p x k, column-major), all columns of one vector block
@@ -497,7 +500,7 @@ cudaError_t dot_batched(const cx<R>* a, long long a_vstride, long long a_cstride
   cudaError_t e = launch<k_dot_partial<R>>(dim3(nblk, nvec, ma), kRedThreads, 0, st, a, a_vstride, a_cstride, ma, b,
                                                b_vstride, len, partial, active);
   if (e != cudaSuccess) return e;
-  return launch<k_dot_final>(dim3(nvec * ma), kRedThreads, 0, st, (const double2*)partial, nblk, out);
+  return launch<k_dot_final>(dim3(nvec * ma), 32, 0, st, (const double2*)partial, nblk, out);
 }
 
 template <class R>
@@ -512,7 +515,7 @@ cudaError_t axpby_batched(const cx<R>* x, cx<R>* y, long long len, long long str
 }
 
 cudaError_t dot_final(const double2* partial, int nblk, int nrows, double2* out, cudaStream_t st) {
-  return launch<k_dot_final>(dim3(nrows), kRedThreads, 0, st, partial, nblk, out);
+  return launch<k_dot_final>(dim3(nrows), 32, 0, st, partial, nblk, out);
 }
 
 template <class R>
@@ -615,12 +618,12 @@ cudaError_t while_active(const int* active, int nvec, int* passes, int max_passe
 
 cudaError_t cg_alpha(int nvec, const double2* partial, int nblk, double2* dot, const double* rho, double* alpha,
                      int* active, int* iters, cudaStream_t st) {
-  return launch<k_cg_alpha>(dim3(nvec), kRedThreads, 0, st, partial, nblk, dot, rho, alpha, active, iters);
+  return launch<k_cg_alpha>(dim3(nvec), 32, 0, st, partial, nblk, dot, rho, alpha, active, iters);
 }
 
 cudaError_t cg_init(int nvec, const double2* partial, int nblk, const double* tolv, double* rho, double* tol2b2,
                     double* bb, double* res2, int* active, int* iters, cudaStream_t st) {
-  return launch<k_cg_init>(dim3(nvec), kRedThreads, 0, st, partial, nblk, tolv, rho, tol2b2, bb, res2, active, iters);
+  return launch<k_cg_init>(dim3(nvec), 32, 0, st, partial, nblk, tolv, rho, tol2b2, bb, res2, active, iters);
 }
 
 template <class R>

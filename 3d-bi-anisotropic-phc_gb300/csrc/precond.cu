@@ -149,18 +149,17 @@ __device__ __forceinline__ void mvec4(const Block4<R>& b, const cx<R> r[4], cx<R
 
 constexpr int kThreads = 256;
 
+// Block-wide sum, valid in thread 0 (block_sum2 of krylov_kernels.cu).
 __device__ __forceinline__ double2 block_sum2b(double2 v) {
-  __shared__ double2 sh[kThreads / 32];
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    v.x += __shfl_down_sync(0xffffffffu, v.x, o);
-    v.y += __shfl_down_sync(0xffffffffu, v.y, o);
-  }
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  if (lane == 0) sh[wid] = v;
+  __shared__ double2 sh[kThreads];
+  sh[threadIdx.x] = v;
   __syncthreads();
-  if (wid == 0) {
-    v = lane < (blockDim.x >> 5) ? sh[lane] : make_double2(0.0, 0.0);
+  if (threadIdx.x < 32) {
+#pragma unroll
+    for (int k = 1; k < kThreads / 32; ++k) {
+      v.x += sh[threadIdx.x + 32 * k].x;
+      v.y += sh[threadIdx.x + 32 * k].y;
+    }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
       v.x += __shfl_down_sync(0xffffffffu, v.x, o);
@@ -188,7 +187,8 @@ k_pcg_start(const cx<R>* __restrict__ b, cx<R>* __restrict__ x, cx<R>* __restric
   const cx<R>* pc = pc_all ? pc_all + (long long)vec_inst(ctx, vec) * kPcSlots * Nq : nullptr;
   const long long o = vec * 4 * Nq;
   R srz = 0, srr = 0;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < Nq; i += (long long)nblk * blockDim.x) {
+  const long long chunk = (Nq + nblk - 1) / nblk, end = min(Nq, (blockIdx.x + 1) * chunk);
+  for (long long i = blockIdx.x * chunk + threadIdx.x; i < end; i += kThreads) {
     cx<R> rv[4], zv[4];
 #pragma unroll
     for (int c = 0; c < 4; ++c) zv[c] = rv[c] = b[o + c * Nq + i];
@@ -208,100 +208,116 @@ k_pcg_start(const cx<R>* __restrict__ b, cx<R>* __restrict__ x, cx<R>* __restric
   if (threadIdx.x == 0) *out = s;
 }
 
+// CG update of one vector's chunk of voxels per CTA: x += a p, r -= a q, z = M r
+// and the partial sums.  HBM-bound on large batches (8 vectors at n = 48: 255 MB
+// in 41 us), latency-bound on small ones, so that
+//   * a CTA takes one contiguous chunk, and the CTAs of a launch are whole
+//     multiples of what fits the SMs (update_blocks);
+//   * the loads of the first elements are issued before the step length, which
+//     every CTA reduces from the stencil pass's partials, is waited for;
+//   * complex64 moves two voxels per 16-byte access.
+// 4 vectors at n = 40 (complex64) 20 -> 14 us, 2 at n = 30 (complex128) 26 -> 13.
 template <class R>
 __global__ void __launch_bounds__(kThreads, sizeof(R) == 4 ? 2 : 1)
 k_pcg_update(cx<R>* __restrict__ x, cx<R>* __restrict__ r, cx<R>* __restrict__ z, const cx<R>* __restrict__ p,
              const cx<R>* __restrict__ q, const cx<R>* __restrict__ pc_all, VecCtx ctx, long long Nq,
-             const double* __restrict__ alpha, double2* __restrict__ partial, CgAlpha ca) {
+             double2* __restrict__ partial, CgAlpha ca) {
+  constexpr int U = 16 / sizeof(cx<R>);  // voxels per 16-byte access (n^3 is even)
+  struct alignas(16) Pack {
+    cx<R> e[U];
+  };
   const int vec = blockIdx.y;
   const int nblk = gridDim.x;
   double2* out = partial + (long long)vec * nblk + blockIdx.x;
+  __shared__ int s_act;
+  __shared__ double s_alpha;
   pdl_wait();
-  if (ctx.active && !ctx.active[vec]) {
+  // one read per CTA: CTA 0 may clear the flag while others start
+  if (threadIdx.x == 0) s_act = ctx.active ? ctx.active[vec] : 1;
+  __syncthreads();
+  if (!s_act) {
     if (threadIdx.x == 0) *out = make_double2(0.0, 0.0);
     return;
   }
-  R a;
-  if (ca.pq) {
-    __shared__ double s_alpha;
-    if (threadIdx.x < 32) {
-      double sx = 0.0, sy = 0.0;
-      for (int i = threadIdx.x; i < ca.nblk; i += 32) {
-        const double2 t = ca.pq[(long long)vec * ca.nblk + i];
-        sx += t.x;
-        sy += t.y;
-      }
+  const cx<R>* pc = pc_all + (long long)vec_inst(ctx, vec) * kPcSlots * Nq;
+  const long long o = vec * 4 * Nq;
+  const int np = int(Nq / U), chunk = (np + nblk - 1) / nblk;  // packs, packs per CTA
+  const int end = min(np, (int(blockIdx.x) + 1) * chunk);
+  int i = blockIdx.x * chunk + threadIdx.x;
+  Pack pk[4], qk[4], xk[4], rk[4], bk[kPcSlots];
+  auto load = [&](int j) {
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        sx += __shfl_down_sync(0xffffffffu, sx, o);
-        sy += __shfl_down_sync(0xffffffffu, sy, o);
-      }
-      if (threadIdx.x == 0) {
-        const bool ok = sx > 0.0 && isfinite(sx);
-        const double av = ok ? ca.rho[vec] / sx : 0.0;
-        s_alpha = av;
-        if (blockIdx.x == 0) {
-          ca.alpha[vec] = av;
-          ca.dot[vec] = make_double2(sx, sy);
-          if (!ok) {  // breakdown: B must be HPD
-            ca.active[vec] = 0;
-            ca.iters[vec] = -(ca.iters[vec] + 1);
-          }
+    for (int c = 0; c < 4; ++c) {
+      const long long k = o + c * Nq + (long long)j * U;
+      pk[c] = *reinterpret_cast<const Pack*>(p + k);
+      qk[c] = *reinterpret_cast<const Pack*>(q + k);
+      xk[c] = *reinterpret_cast<const Pack*>(x + k);
+      rk[c] = *reinterpret_cast<const Pack*>(r + k);
+    }
+#pragma unroll
+    for (int c = 0; c < kPcSlots; ++c) bk[c] = *reinterpret_cast<const Pack*>(pc + c * Nq + (long long)j * U);
+  };
+  if (i < end) load(i);
+  if (threadIdx.x < 32) {
+    double sx = 0.0, sy = 0.0;
+    for (int j = threadIdx.x; j < ca.nblk; j += 32) {
+      const double2 t = ca.pq[(long long)vec * ca.nblk + j];
+      sx += t.x;
+      sy += t.y;
+    }
+#pragma unroll
+    for (int w = 16; w > 0; w >>= 1) {
+      sx += __shfl_down_sync(0xffffffffu, sx, w);
+      sy += __shfl_down_sync(0xffffffffu, sy, w);
+    }
+    if (threadIdx.x == 0) {
+      const bool ok = sx > 0.0 && isfinite(sx);
+      const double av = ok ? ca.rho[vec] / sx : 0.0;
+      s_alpha = av;
+      if (blockIdx.x == 0) {
+        ca.alpha[vec] = av;
+        ca.dot[vec] = make_double2(sx, sy);
+        if (!ok) {  // breakdown: B must be HPD
+          ca.active[vec] = 0;
+          ca.iters[vec] = -(ca.iters[vec] + 1);
         }
       }
     }
-    __syncthreads();
-    a = R(s_alpha);
-  } else {
-    a = R(alpha[vec]);
   }
-  const cx<R>* pc = pc_all + (long long)vec_inst(ctx, vec) * kPcSlots * Nq;
-  const long long o = vec * 4 * Nq;
+  __syncthreads();
+  const R a = R(s_alpha);
   R srz = 0, srr = 0;
-  const long long stride = (long long)nblk * blockDim.x;
-  // two voxels per pass, every load of both issued before any store
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < Nq; i += 2 * stride) {
-    const long long i2 = i + stride;
-    const bool two = i2 < Nq;
-    cx<R> pk[2][4], qk[2][4], xk[2][4], rk[2][4];
-    Block4<R> bk[2];
+  while (i < end) {
+    Pack zk[4];
 #pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      if (u == 1 && !two) break;
-      const long long iv = u ? i2 : i;
+    for (int u = 0; u < U; ++u) {
+      cx<R> rv[4], zv[4];
+      Block4<R> bl;
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
-        const long long k = o + c * Nq + iv;
-        pk[u][c] = p[k];
-        qk[u][c] = q[k];
-        xk[u][c] = x[k];
-        rk[u][c] = r[k];
+        xk[c].e[u] = caxpy(a, pk[c].e[u], xk[c].e[u]);
+        rk[c].e[u] = caxpy(-a, qk[c].e[u], rk[c].e[u]);
+        rv[c] = rk[c].e[u];
       }
-      bk[u] = load_block<R>(pc, Nq, iv);
-    }
 #pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      if (u == 1 && !two) break;
-      const long long iv = u ? i2 : i;
-      cx<R> zv[4];
+      for (int c = 0; c < kPcSlots; ++c) bl.s[c] = bk[c].e[u];
+      mvec4<R>(bl, rv, zv);
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
-        xk[u][c].x += a * pk[u][c].x;
-        xk[u][c].y += a * pk[u][c].y;
-        rk[u][c].x -= a * qk[u][c].x;
-        rk[u][c].y -= a * qk[u][c].y;
-      }
-      mvec4<R>(bk[u], rk[u], zv);
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const long long k = o + c * Nq + iv;
-        x[k] = xk[u][c];
-        r[k] = rk[u][c];
-        z[k] = zv[c];
-        srz += rk[u][c].x * zv[c].x + rk[u][c].y * zv[c].y;
-        srr += rk[u][c].x * rk[u][c].x + rk[u][c].y * rk[u][c].y;
+        zk[c].e[u] = zv[c];
+        srz += rv[c].x * zv[c].x + rv[c].y * zv[c].y;
+        srr += rv[c].x * rv[c].x + rv[c].y * rv[c].y;
       }
     }
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const long long k = o + c * Nq + (long long)i * U;
+      *reinterpret_cast<Pack*>(x + k) = xk[c];
+      *reinterpret_cast<Pack*>(r + k) = rk[c];
+      *reinterpret_cast<Pack*>(z + k) = zk[c];
+    }
+    i += kThreads;
+    if (i < end) load(i);
   }
   double2 s = block_sum2b(make_double2(double(srz), double(srr)));
   if (threadIdx.x == 0) *out = s;
@@ -341,11 +357,9 @@ cudaError_t pcg_start(const Plan& P, bool precond, const cx<R>* b, cx<R>* x, cx<
 
 template <class R>
 cudaError_t pcg_update(const Plan& P, cx<R>* x, cx<R>* r, cx<R>* z, const cx<R>* p, const cx<R>* q, int nvec,
-                       const VecCtx& ctx, const double* alpha, double2* partial, int nblk, cudaStream_t st,
-                       const CgAlpha& ca) {
+                       const VecCtx& ctx, double2* partial, int nblk, cudaStream_t st, const CgAlpha& ca) {
   const PlanData<R>& d = detail::pdata<R>(P);
-  return launch<k_pcg_update<R>>(dim3(nblk, nvec), kThreads, 0, st, x, r, z, p, q, d.pc, ctx, P.Nq, alpha, partial,
-                                     ca);
+  return launch<k_pcg_update<R>>(dim3(nblk, nvec), kThreads, 0, st, x, r, z, p, q, d.pc, ctx, P.Nq, partial, ca);
 }
 
 template cudaError_t build_precond<float>(Plan&, cudaStream_t);
@@ -355,8 +369,8 @@ template cudaError_t pcg_start<float>(const Plan&, bool, const cx<float>*, cx<fl
 template cudaError_t pcg_start<double>(const Plan&, bool, const cx<double>*, cx<double>*, cx<double>*, cx<double>*, cx<double>*, int,
                                          const VecCtx&, double2*, int, cudaStream_t);
 template cudaError_t pcg_update<float>(const Plan&, float2*, float2*, float2*, const float2*, const float2*, int,
-                                       const VecCtx&, const double*, double2*, int, cudaStream_t, const CgAlpha&);
+                                       const VecCtx&, double2*, int, cudaStream_t, const CgAlpha&);
 template cudaError_t pcg_update<double>(const Plan&, double2*, double2*, double2*, const double2*, const double2*, int,
-                                        const VecCtx&, const double*, double2*, int, cudaStream_t, const CgAlpha&);
+                                        const VecCtx&, double2*, int, cudaStream_t, const CgAlpha&);
 
 }  // namespace fame

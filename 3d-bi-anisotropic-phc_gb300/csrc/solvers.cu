@@ -33,16 +33,17 @@ enum WsId {
     if (e_ != cudaSuccess) return cuda_fail(&P, e_, where); \
   } while (0)
 
-// CTAs per vector of the grid-stride reduction and update kernels: together
-// at most four per SM (one wave at four resident CTAs, two at two), so that
-// no CTA of a batch waits for a partial last wave, and no more than one
-// element per thread.  (A floor of eight elements per thread left 28 CTAs for
-// two vectors at n = 30, and the complex128 update at 71 us of a 290 us CG
-// iteration; one element per thread: 25 us.)
-static int dot_blocks(const Plan& P, long long len, int nvec) {
-  const long long target = std::max(1, 4 * P.sms / std::max(1, nvec));
-  const long long b = std::min(target, (len + 255) / 256);
-  return (int)std::max(1LL, std::min(512LL, b));
+// CTAs per vector of the reduction and update kernels of 256 threads: the
+// launch's total is a whole number of CTAs per SM (up to per_sm), as many as
+// give each `each` elements, so that every SM ends with the same work.  (Eight
+// elements per thread at least left 28 CTAs for two vectors at n = 30; one
+// element per thread, 212 CTAs on 152 SMs, each with its reduction in FP64: the
+// complex128 update took 71 and 26 us of a CG iteration, 13 with one CTA per SM.)
+static int dot_blocks(const Plan& P, long long len, int nvec, int per_sm = 4, int each = 1024) {
+  nvec = std::max(1, nvec);
+  const long long k = std::max(1LL, std::min<long long>(per_sm, len * nvec / ((long long)each * P.sms)));
+  const long long b = std::max(1LL, k * P.sms / nvec);
+  return (int)std::min(512LL, std::min(b, (len + 31) / 32));
 }
 
 // Device scalars of the batched CG, carved from one workspace.  tolv and
@@ -92,7 +93,7 @@ int pcg_batched(Plan& P, const cx<R>* b, cx<R>* x, int nvec, const int* d_inst, 
   const int nblk = dot_blocks(P, L, nvec);
   // p^H B p from the stencil pass of fncB where its tuned form provides it
   const int nblk_pq = fncB_pq_partials<R>(P, nvec);
-  const int nblkv0 = dot_blocks(P, P.Nq, nvec);
+  const int nblkv0 = dot_blocks(P, P.Nq, nvec, sizeof(R) == 4 ? 2 : 1, 512);
   const int npart = std::max(std::max(nblk, nblk_pq), nblkv0);
   double2* part = (double2*)workspace(P, WS_PCG_PART, sizeof(double2) * npart * nvec + 64, &e);
   FAME_CK(e, "pcg workspace");
@@ -124,7 +125,7 @@ int pcg_batched(Plan& P, const cx<R>* b, cx<R>* x, int nvec, const int* d_inst, 
   // Preconditioned CG (M = B0^{-1}, precond.cu) or plain CG as in fncinvB.m.
   const bool pre = P.opt_precond != 0;
   cx<R>* z = nullptr;
-  const int nblkv = dot_blocks(P, P.Nq, nvec);  // per-voxel fused kernels
+  const int nblkv = nblkv0;  // per-voxel fused kernels: the CTAs that fit at once
   if (pre) {
     z = (cx<R>*)workspace(P, WS_PCG_Z + (sizeof(R) == 4 ? 100 : 0), vb, &e);
     FAME_CK(e, "pcg workspace");
@@ -159,7 +160,7 @@ int pcg_batched(Plan& P, const cx<R>* b, cx<R>* x, int nvec, const int* d_inst, 
       ca.dot = S.dot;
       ca.active = S.active;
       ca.iters = S.iters;
-      if (e2 == cudaSuccess) e2 = pcg_update<R>(P, x, r, z, p, q, nvec, ctx, S.alpha, part2, nblkv, cs, ca);
+      if (e2 == cudaSuccess) e2 = pcg_update<R>(P, x, r, z, p, q, nvec, ctx, part2, nblkv, cs, ca);
     } else {
       if (e2 == cudaSuccess) e2 = cg_alpha(nvec, part, nblk_pq ? nblk_pq : nblk, S.dot, rho_in, S.alpha, S.active, S.iters, cs);
       if (e2 == cudaSuccess) e2 = cg_xr_partial<R>(x, r, p, q, L, L, nvec, S.alpha, S.active, part, nblk, cs);
