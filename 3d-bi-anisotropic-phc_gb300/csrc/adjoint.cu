@@ -31,122 +31,142 @@
 #include <vector>
 
 #include "fame_internal.h"
+#include "launch.h"
 
 namespace fame {
 namespace {
 
 struct VertexQuads {
-  double qu, qv;
-  double2 quv;
+  double qu, qv, qi;  // Qu, Qv, Im Quv
 };
 
-__device__ __forceinline__ VertexQuads vertex_quads(const double2* __restrict__ f, long long Nq, int n,
-                                                    long long idx, double2 tx, double2 ty, double2 tz,
-                                                    const double* __restrict__ G) {
-  const int i1 = int(idx % n), i2 = int((idx / n) % n), i3 = int(idx / ((long long)n * n));
-  const long long dxm = i1 == 0 ? n - 1 : -1;
-  const long long dym = i2 == 0 ? (long long)(n - 1) * n : -(long long)n;
-  const long long dzm = i3 == 0 ? (long long)(n - 1) * n * n : -(long long)n * n;
-  auto a2 = [](double2 z) { return z.x * z.x + z.y * z.y; };
-  auto face = [&](const double2* g, long long da, long long db, double2 ta, double2 tb, double& au) {
-    double2 s = g[0];
-    s = cfma(ta, g[da], s);
-    s = cfma(tb, g[db], s);
-    s = cfma(cmul(ta, tb), g[da + db], s);
-    au = 0.25 * (a2(g[0]) + a2(g[da]) + a2(g[db]) + a2(g[da + db]));
-    return cscale(s, 0.25);
+// The gathers are kept unscaled (4 U, 2 V) and the factors applied to the sums;
+// off-diagonal sums run over su_i = sum_{j!=i} G_ij U_j (142 FP64 operations per
+// vertex and vector).
+__device__ __forceinline__ VertexQuads vertex_quads(const double2* __restrict__ f, long long Nq, int n, int idx,
+                                                    double2 tx, double2 ty, double2 tz, const double* __restrict__ G) {
+  const int i1 = idx % n, i2 = (idx / n) % n, i3 = idx / (n * n);
+  const int dxm = i1 == 0 ? n - 1 : -1;
+  const int dym = i2 == 0 ? (n - 1) * n : -n;
+  const int dzm = i3 == 0 ? (n - 1) * n * n : -n * n;
+  auto a2 = [](double2 z, double acc) { return fma(z.x, z.x, fma(z.y, z.y, acc)); };
+  auto face = [&](const double2* g, int da, int db, double2 ta, double2 tb, double& au) {
+    const double2 g00 = g[0], ga = g[da], gb = g[db], gab = g[da + db];
+    au = a2(g00, a2(ga, a2(gb, a2(gab, 0.0))));
+    return cfma(ta, cfma(tb, gab, ga), cfma(tb, gb, g00));
   };
   double2 U[3], V[3];
   double Au[3], Av[3];
   U[0] = face(f, dym, dzm, ty, tz, Au[0]);
   U[1] = face(f + Nq, dxm, dzm, tx, tz, Au[1]);
   U[2] = face(f + 2 * Nq, dxm, dym, tx, ty, Au[2]);
-  const double2* v0 = f + 3 * Nq;
-  const double2* v1 = f + 4 * Nq;
-  const double2* v2 = f + 5 * Nq;
-  V[0] = cscale(cfma(tx, v0[dxm], v0[0]), 0.5);
-  V[1] = cscale(cfma(ty, v1[dym], v1[0]), 0.5);
-  V[2] = cscale(cfma(tz, v2[dzm], v2[0]), 0.5);
-  Av[0] = 0.5 * (a2(v0[0]) + a2(v0[dxm]));
-  Av[1] = 0.5 * (a2(v1[0]) + a2(v1[dym]));
-  Av[2] = 0.5 * (a2(v2[0]) + a2(v2[dzm]));
-  VertexQuads r{0.0, 0.0, make_double2(0.0, 0.0)};
+  auto edge = [&](const double2* g, int da, double2 ta, double& av) {
+    const double2 g0 = g[0], ga = g[da];
+    av = a2(g0, a2(ga, 0.0));
+    return cfma(ta, ga, g0);
+  };
+  V[0] = edge(f + 3 * Nq, dxm, tx, Av[0]);
+  V[1] = edge(f + 4 * Nq, dym, ty, Av[1]);
+  V[2] = edge(f + 5 * Nq, dzm, tz, Av[2]);
+  double du = 0.0, dv = 0.0, qi = 0.0, lu = 0.0, lv = 0.0;
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
-    r.qu += G[i * 4] * Au[i];
-    r.qv += G[i * 4] * Av[i];
-#pragma unroll
-    for (int j = 0; j < 3; ++j) {
-      const double gij = G[i * 3 + j];
-      if (j != i) {
-        r.qu += gij * (U[i].x * U[j].x + U[i].y * U[j].y);
-        r.qv += gij * (V[i].x * V[j].x + V[i].y * V[j].y);
-      }
-      r.quv = cadd(r.quv, cscale(cmulc(V[i], U[j]), gij));
-    }
+    const int j = (i + 1) % 3, k = (i + 2) % 3;
+    const double gj = G[i * 3 + j], gk = G[i * 3 + k], gi = G[i * 4];
+    const double2 su = caxpy(gj, U[j], cscale(U[k], gk)), sv = caxpy(gj, V[j], cscale(V[k], gk));
+    du = fma(U[i].x, su.x, fma(U[i].y, su.y, du));
+    dv = fma(V[i].x, sv.x, fma(V[i].y, sv.y, dv));
+    const double2 tu = caxpy(gi, U[i], su);
+    qi = fma(V[i].x, tu.y, fma(-V[i].y, tu.x, qi));
+    lu = fma(gi, Au[i], lu);
+    lv = fma(gi, Av[i], lv);
   }
-  return r;
+  return VertexQuads{fma(0.0625, du, 0.25 * lu), fma(0.25, dv, 0.5 * lv), 0.125 * qi};
 }
 
 struct GradParams {
   double G[9];
 };
 
-constexpr int kGradThreads = 256;
+constexpr int kGradThreads = 128;
 
-// q summed per vector (x^H B x), one partial per block.
+// Qu, Qv, Im Quv of every vertex and vector into quads [nvec][3][Nq], and q
+// summed per vector (x^H B x), one partial per block.  FP64-rate-bound; the
+// quadratic forms are evaluated once here and only read by k_grad (evaluating
+// them in both took 171 of 300 us per call, 3 vectors at n = 40).
 __global__ void __launch_bounds__(kGradThreads)
-k_quad_sum(const double2* __restrict__ w, const double* __restrict__ fld, PlanData<double> d, VecCtx ctx, int n,
-           GradParams gp, double* __restrict__ partial) {
+k_quads(const double2* __restrict__ w, const double* __restrict__ fld, PlanData<double> d, VecCtx ctx, int n,
+        GradParams gp, double* __restrict__ quads, double* __restrict__ partial) {
   const long long Nq = (long long)n * n * n;
   const int vec = blockIdx.y;
+  pdl_wait();
   const int inst = vec_inst(ctx, vec);
   const double2 tx = cconj(d.tau[inst * 3]), ty = cconj(d.tau[inst * 3 + 1]), tz = cconj(d.tau[inst * 3 + 2]);
+  const int idx = blockIdx.x * kGradThreads + threadIdx.x;
   double acc = 0.0;
-  for (long long idx = (long long)blockIdx.x * kGradThreads + threadIdx.x; idx < Nq;
-       idx += (long long)gridDim.x * kGradThreads) {
-    VertexQuads q = vertex_quads(w + vec * 6 * Nq + idx, Nq, n, idx, tx, ty, tz, gp.G);
-    acc += fld[Nq + idx] * q.qu + fld[idx] * q.qv + 2.0 * fld[2 * Nq + idx] * q.quv.y;
+  if (idx < Nq) {
+    const VertexQuads q = vertex_quads(w + vec * 6 * Nq + idx, Nq, n, idx, tx, ty, tz, gp.G);
+    double* o = quads + vec * 3 * Nq + idx;
+    o[0] = q.qu;
+    o[Nq] = q.qv;
+    o[2 * Nq] = q.qi;
+    acc = fma(fld[Nq + idx], q.qu, fma(fld[idx], q.qv, 2.0 * fld[2 * Nq + idx] * q.qi));
   }
   __shared__ double red[kGradThreads];
   red[threadIdx.x] = acc;
   __syncthreads();
-  for (int s = kGradThreads / 2; s > 0; s >>= 1) {
-    if (threadIdx.x < s) red[threadIdx.x] += red[threadIdx.x + s];
-    __syncthreads();
+  if (threadIdx.x < 32) {
+#pragma unroll
+    for (int k = 1; k < kGradThreads / 32; ++k) acc += red[threadIdx.x + 32 * k];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
+    if (threadIdx.x == 0) partial[(long long)vec * gridDim.x + blockIdx.x] = acc;
   }
-  if (threadIdx.x == 0) partial[(long long)vec * gridDim.x + blockIdx.x] = red[0];
 }
 
-// g_eps, g_gamma (+)= sum_v scale_v dq_v/dp at every vertex.
+// xbx[v] = x^H B x, scale[v] = weight omega / xbx (one warp per vector).
+__global__ void __launch_bounds__(32)
+k_grad_scale(const double* __restrict__ partial, int nblk, const double* __restrict__ wom, double* __restrict__ xbx,
+             double* __restrict__ scale) {
+  const int v = blockIdx.x;
+  pdl_wait();
+  double s = 0.0;
+  for (int j = threadIdx.x; j < nblk; j += 32) s += partial[(long long)v * nblk + j];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+  if (threadIdx.x == 0) {
+    xbx[v] = s;
+    scale[v] = wom[v] / s;
+  }
+}
+
+// g_eps, g_gamma (+)= sum_v scale_v dq_v/dp at every vertex; untouched when any
+// x^H B x is not positive (the call reports it).
 __global__ void __launch_bounds__(kGradThreads)
-k_grad(const double2* __restrict__ w, const double* __restrict__ fld, const double* __restrict__ eg,
-       PlanData<double> d, VecCtx ctx, int n, int nvec, GradParams gp, const double* __restrict__ scale,
-       double* __restrict__ g_eps, double* __restrict__ g_gam, int accumulate) {
-  const long long Nq = (long long)n * n * n;
+k_grad(const double* __restrict__ quads, const double* __restrict__ fld, const double* __restrict__ eg, int nvec,
+       long long Nq, const double* __restrict__ xbx, const double* __restrict__ scale, double* __restrict__ g_eps,
+       double* __restrict__ g_gam, int accumulate) {
   const long long idx = (long long)blockIdx.x * kGradThreads + threadIdx.x;
+  pdl_wait();
   if (idx >= Nq) return;
+  for (int vec = 0; vec < nvec; ++vec)
+    if (!(xbx[vec] > 0.0) || !isfinite(xbx[vec])) return;
+  double su = 0.0, sv = 0.0, si = 0.0;
+  for (int vec = 0; vec < nvec; ++vec) {
+    const double s = scale[vec];
+    const double* q = quads + vec * 3 * Nq + idx;
+    su = fma(s, q[0], su);
+    sv = fma(s, q[Nq], sv);
+    si = fma(s, q[2 * Nq], si);
+  }
   const double a = fld[idx], eps = eg[idx], gam = eg[Nq + idx];
   const double a2 = a * a;
   const double db_de = -gam * gam * a2, da_de = -a2, dg_de = -gam * a2;
   const double db_dg = 2.0 * eps * gam * a2, da_dg = 2.0 * gam * a2, dg_dg = a * (1.0 + 2.0 * gam * gam * a);
-  double se = 0.0, sg = 0.0;
-  for (int vec = 0; vec < nvec; ++vec) {
-    const double s = scale[vec];
-    if (s == 0.0) continue;
-    const int inst = vec_inst(ctx, vec);
-    const double2 tx = cconj(d.tau[inst * 3]), ty = cconj(d.tau[inst * 3 + 1]), tz = cconj(d.tau[inst * 3 + 2]);
-    VertexQuads q = vertex_quads(w + vec * 6 * Nq + idx, Nq, n, idx, tx, ty, tz, gp.G);
-    se += s * (db_de * q.qu + da_de * q.qv + 2.0 * dg_de * q.quv.y);
-    sg += s * (db_dg * q.qu + da_dg * q.qv + 2.0 * dg_dg * q.quv.y);
-  }
-  if (accumulate) {
-    g_eps[idx] += se;
-    g_gam[idx] += sg;
-  } else {
-    g_eps[idx] = se;
-    g_gam[idx] = sg;
-  }
+  const double se = db_de * su + da_de * sv + 2.0 * dg_de * si;
+  const double sg = db_dg * su + da_dg * sv + 2.0 * dg_dg * si;
+  g_eps[idx] = accumulate ? g_eps[idx] + se : se;
+  g_gam[idx] = accumulate ? g_gam[idx] + sg : sg;
 }
 
 template <class R>
@@ -290,33 +310,34 @@ int fame_eig_gradient(fame_plan_t h, int nvec, const int* inst, const void* x, c
   if (e != cudaSuccess) return cuda_fail(&P, e, "fame_eig_gradient fields");
   GradParams gp;
   for (int i = 0; i < 9; ++i) gp.G[i] = P.d64.gram[i];
-  const int nblk = 152;
-  double* partial = (double*)workspace(P, 41, sizeof(double) * nblk * nvec, &e);
+  const int nblk = int((P.Nq + kGradThreads - 1) / kGradThreads);
+  double* partial = (double*)workspace(P, 41, sizeof(double) * ((size_t)nblk + 3) * nvec, &e);
   if (e != cudaSuccess) return cuda_fail(&P, e, "fame_eig_gradient scratch");
-  FAME_LAUNCHED(1);
-  k_quad_sum<<<dim3(nblk, nvec), kGradThreads, 0, st>>>(w, P.d64.fld, P.d64, ctx, P.n, gp, partial);
-  e = cudaGetLastError();
-  if (e != cudaSuccess) return cuda_fail(&P, e, "k_quad_sum");
-  std::vector<double> hp((size_t)nblk * nvec);
-  e = cudaMemcpyAsync(hp.data(), partial, sizeof(double) * hp.size(), cudaMemcpyDeviceToHost, st);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-  if (e != cudaSuccess) return cuda_fail(&P, e, "fame_eig_gradient norm");
-  std::vector<double> scale(nvec);
+  double* d_wom = partial + (size_t)nblk * nvec;
+  double* d_xbx = d_wom + nvec;
+  double* d_scale = d_xbx + nvec;
+  std::vector<double> wom(nvec);
+  for (int v = 0; v < nvec; ++v) wom[v] = weight[v] * omega[v];
+  e = h2d_async(P, d_wom, wom.data(), sizeof(double) * nvec);
+  if (e != cudaSuccess) return cuda_fail(&P, e, "fame_eig_gradient scale");
+  double* quads = (double*)(w + (size_t)nvec * 6 * P.Nq);  // the second half of the work arrays
+  e = launch<k_quads>(dim3(nblk, nvec), kGradThreads, 0, st, w, P.d64.fld, P.d64, ctx, P.n, gp, quads, partial);
+  if (e == cudaSuccess) e = launch<k_grad_scale>(dim3(nvec), 32, 0, st, partial, nblk, d_wom, d_xbx, d_scale);
+  if (e != cudaSuccess) return cuda_fail(&P, e, "fame_eig_gradient forms");
+  // the host waits for x^H B x only, with the gradient kernel behind it in the
+  // stream, so the next call's work follows without a gap
+  double* h_xbx = nullptr;
+  e = d2h_begin(P, (void**)&h_xbx, d_xbx, sizeof(double) * nvec);
+  if (e == cudaSuccess)
+    e = launch<k_grad>(dim3(nblk), kGradThreads, 0, st, quads, P.d64.fld, P.d_eps_gam, nvec, P.Nq, d_xbx, d_scale, g_eps,
+                       g_gamma, accumulate);
+  if (e == cudaSuccess) e = d2h_wait(P);
+  if (e != cudaSuccess) return cuda_fail(&P, e, "k_grad");
   for (int v = 0; v < nvec; ++v) {
-    double s = 0.0;
-    for (int b = 0; b < nblk; ++b) s += hp[(size_t)v * nblk + b];
+    const double s = h_xbx[v];
     if (xbx) xbx[v] = s;
     if (!(s > 0.0) || !std::isfinite(s)) return fail(&P, FAME_ERR_NAN, "fame_eig_gradient: x^H B x is not positive");
-    scale[v] = weight[v] * omega[v] / s;
   }
-  double* d_scale = (double*)workspace(P, 42, sizeof(double) * nvec, &e);
-  if (e == cudaSuccess) e = h2d_async(P, d_scale, scale.data(), sizeof(double) * nvec);
-  if (e != cudaSuccess) return cuda_fail(&P, e, "fame_eig_gradient scale");
-  FAME_LAUNCHED(1);
-  k_grad<<<(unsigned)((P.Nq + kGradThreads - 1) / kGradThreads), kGradThreads, 0, st>>>(
-      w, P.d64.fld, P.d_eps_gam, P.d64, ctx, P.n, nvec, gp, d_scale, g_eps, g_gamma, accumulate);
-  e = cudaGetLastError();
-  if (e != cudaSuccess) return cuda_fail(&P, e, "k_grad");
   return FAME_OK;
 }
 

@@ -57,13 +57,36 @@ void* workspace(Plan& P, int id, size_t bytes, cudaError_t* err) {
 
 constexpr size_t kRingBytes = 1 << 20;
 
+static cudaError_t ensure_ring(Plan& P) {
+  if (P.h_ring) return cudaSuccess;
+  cudaError_t e = cudaMallocHost((void**)&P.h_ring, kRingBytes + kDownBytes);
+  if (e != cudaSuccess) P.h_ring = nullptr;
+  P.ring_pos = 0;
+  return e;
+}
+
+cudaError_t d2h_begin(Plan& P, void** host, const void* src, size_t bytes) {
+  if (cudaError_t e = ensure_ring(P)) return e;
+  if (!P.down_event) {
+    cudaError_t e = cudaEventCreateWithFlags(&P.down_event, cudaEventDisableTiming);
+    if (e != cudaSuccess) return e;
+  }
+  if (bytes > kDownBytes) {
+    P.h_down.resize(bytes);
+    *host = P.h_down.data();
+    cudaError_t e = cudaMemcpyAsync(*host, src, bytes, cudaMemcpyDeviceToHost, P.stream);
+    return e == cudaSuccess ? cudaEventRecord(P.down_event, P.stream) : e;
+  }
+  *host = P.h_ring + kRingBytes;
+  cudaError_t e = cudaMemcpyAsync(*host, src, bytes, cudaMemcpyDeviceToHost, P.stream);
+  return e == cudaSuccess ? cudaEventRecord(P.down_event, P.stream) : e;
+}
+
+cudaError_t d2h_wait(Plan& P) { return cudaEventSynchronize(P.down_event); }
+
 cudaError_t h2d_async(Plan& P, void* dst, const void* src, size_t bytes) {
   if (bytes == 0) return cudaSuccess;
-  if (!P.h_ring) {
-    cudaError_t e = cudaMallocHost((void**)&P.h_ring, kRingBytes);
-    if (e != cudaSuccess) return e;
-    P.ring_pos = 0;
-  }
+  if (cudaError_t e = ensure_ring(P)) return e;
   if (bytes > kRingBytes) return cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice);
   if (P.ring_pos + bytes > kRingBytes) {  // wrap only once earlier copies have been consumed
     cudaError_t e = cudaStreamSynchronize(P.stream);
@@ -368,6 +391,7 @@ int fame_plan_destroy(fame_plan_t h) {
   cudaFree(P.d_eps_gam);
   free_graphs(P);
   if (P.h_ring) cudaFreeHost(P.h_ring);
+  if (P.down_event) cudaEventDestroy(P.down_event);
   free_workspaces(P);
   delete h;
   return FAME_OK;

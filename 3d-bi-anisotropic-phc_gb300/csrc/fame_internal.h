@@ -171,6 +171,9 @@ struct Plan {
   // would synchronise the stream)
   char* h_ring = nullptr;
   size_t ring_pos = 0;
+  // downloads (d2h_begin): the last kDownBytes of the ring's allocation
+  cudaEvent_t down_event = nullptr;
+  std::vector<char> h_down;
   // captured launch sequences (graph.cu)
   cudaStream_t cap_stream = nullptr;
   std::vector<GraphEntry> graphs;
@@ -197,6 +200,14 @@ void free_graphs(Plan& P);
 
 // Asynchronous small upload through the plan's pinned ring (stream-ordered).
 cudaError_t h2d_async(Plan& P, void* dst, const void* src, size_t bytes);
+
+// Small download of up to kDownBytes through the plan's pinned memory: enqueues
+// the copy and marks the point; d2h_wait waits for that point only, not for
+// work enqueued after it.  *host stays valid until the next d2h_begin.  (A
+// larger download goes to a host vector of the plan and completes at once.)
+constexpr size_t kDownBytes = 64 << 10;
+cudaError_t d2h_begin(Plan& P, void** host, const void* src, size_t bytes);
+cudaError_t d2h_wait(Plan& P);
 
 // Workspace slot `id` of at least `bytes` bytes (contents not preserved on growth).
 void* workspace(Plan& P, int id, size_t bytes, cudaError_t* err);

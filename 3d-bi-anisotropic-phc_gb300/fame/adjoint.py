@@ -51,15 +51,34 @@ def solve_bands(plan, nbands, tol=1e-10, prec="c128", inner_tol=1e-12, p=None):
     return np.stack(oms), evs
 
 
+# eigenvectors per backward call: one call evaluates the k-points of a group
+# together (four calls of three vectors at n = 40 left the GPU idle for a third
+# of the time), bounded so that the joined copy and the call's scratch stay small
+GROUP_VECTORS = 32
+
+
 def gradient(plan, evs, omega, weights, cluster_tol=1e-8):
     """sum_{k,b} weights[k,b] d omega[k,b] / d(eps, gamma): FP64 CUDA tensors (Nq,)."""
     g_e = torch.zeros(plan.Nq, dtype=torch.float64, device="cuda")
     g_g = torch.zeros_like(g_e)
+    group = []
+
+    def flush():
+        if group:
+            ev = torch.cat([e.reshape(-1, 4 * plan.Nq) for _, e, _, _ in group]) if len(group) > 1 else group[0][1]
+            inst = np.concatenate([np.full(len(w), k, dtype=np.int32) for k, _, _, w in group])
+            plan.eig_gradient(ev, np.concatenate([o for _, _, o, _ in group]),
+                              np.concatenate([w for _, _, _, w in group]), inst=inst, out=(g_e, g_g), accumulate=True)
+            group.clear()
+
     for k, ev in enumerate(evs):
         w = cluster_weights(omega[k], weights[k], cluster_tol)
         if not np.any(w):
             continue
-        plan.eig_gradient(ev, omega[k], w, inst=k, out=(g_e, g_g), accumulate=True)
+        if group and sum(len(q[3]) for q in group) + len(w) > GROUP_VECTORS:
+            flush()
+        group.append((k, ev, np.asarray(omega[k], dtype=np.float64), w))
+    flush()
     return g_e, g_g
 
 
