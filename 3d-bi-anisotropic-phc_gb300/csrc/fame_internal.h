@@ -287,11 +287,12 @@ struct CgAlpha {
   double2* dot = nullptr;
   int* active = nullptr;
   int* iters = nullptr;
+  int* go = nullptr;  // set where the iteration takes its step, else cleared
 };
-// x += a p ; r -= a q ; z = M r ; partial (Re r'z, |r|^2)
+// r -= a q ; z = M r ; partial (Re r'z, |r|^2)
 template <class R>
-cudaError_t pcg_update(const Plan& P, cx<R>* x, cx<R>* r, cx<R>* z, const cx<R>* p, const cx<R>* q, int nvec,
-                       const VecCtx& ctx, double2* partial, int nblk, cudaStream_t st, const CgAlpha& ca);
+cudaError_t pcg_update(const Plan& P, cx<R>* r, cx<R>* z, const cx<R>* q, int nvec, const VecCtx& ctx, double2* partial,
+                       int nblk, cudaStream_t st, const CgAlpha& ca);
 
 bool n_supported(int n);
 

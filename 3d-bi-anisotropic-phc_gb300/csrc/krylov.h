@@ -28,15 +28,15 @@ cudaError_t cg_init(int nvec, const double2* partial, int nblk, const double* to
 // (partial[v * nblk + i], the sum also stored in dot[v]); a vector whose
 // p^H q is not positive is stopped with a negative iteration count.
 cudaError_t cg_alpha(int nvec, const double2* partial, int nblk, double2* dot, const double* rho, double* alpha,
-                     int* active, int* iters, cudaStream_t st);
+                     int* active, int* iters, int* go, cudaStream_t st);
 // The end of a CG iteration in one launch: (rz, rn) = (Re r^H z, |r|^2) from
 // the partials, rho_next = rz, res2 = rn, the iteration count and the
-// convergence test, and for the vectors still active p = z + (rz / rho) p.
-// rho and rho_next are two arrays (every CTA of a vector reads rho).
+// convergence test, x += alpha p, and for the vectors still active p = z + (rz /
+// rho) p.  rho and rho_next are two arrays (every CTA of a vector reads rho).
 template <class R>
-cudaError_t cg_dir(cx<R>* p, const cx<R>* z, long long len, int nvec, const double2* partial, int nblk,
-                   const double* rho, double* rho_next, double2* dot, const double* tol2b2, int* active, int* iters,
-                   double* res2, int ncta, cudaStream_t st);
+cudaError_t cg_dir(cx<R>* x, cx<R>* p, const cx<R>* z, long long len, int nvec, const double2* partial, int nblk,
+                   const double* alpha, const double* rho, double* rho_next, double2* dot, const double* tol2b2,
+                   const int* go, int* active, int* iters, double* res2, int ncta, cudaStream_t st);
 // Gram-Schmidt over a batch of instances, one launch each for all of them:
 // vector v of r (stride rs) works against columns span[v].x ..
 // span[v].x + span[v].y - 1 of its block X + v*xs (columns len apart);
@@ -58,11 +58,10 @@ cudaError_t gs_combo_lo(double2* r, long long rs, const float2* X, long long xs,
 template <class R>
 cudaError_t dot_partial(const cx<R>* a, const cx<R>* b, long long len, long long stride, int nvec, double2* partial,
                         int nblk, const int* active, cudaStream_t st);
-// x += alpha p ; r -= alpha q ; partial (|r|^2, |r|^2) per block (no final reduction)
+// r -= alpha q ; partial (|r|^2, |r|^2) per block (no final reduction)
 template <class R>
-cudaError_t cg_xr_partial(cx<R>* x, cx<R>* r, const cx<R>* p, const cx<R>* q, long long len, long long stride,
-                          int nvec, const double* alpha, const int* active, double2* partial, int nblk,
-                          cudaStream_t st);
+cudaError_t cg_r_partial(cx<R>* r, const cx<R>* q, long long len, int nvec, const double* alpha, const int* active,
+                         double2* partial, int nblk, cudaStream_t st);
 template <class R>
 cudaError_t block_rot(const cx<R>* in, cx<R>* out, long long len, long long ld, int p, int k, const double* U,
                       cudaStream_t st);

@@ -92,12 +92,11 @@ k_dot_partial(const cx<R>* __restrict__ a, long long a_vstride, long long a_cstr
   if (threadIdx.x == 0) *out = s;
 }
 
-// Fused CG update and residual norm: x += a p ; r -= a q ; partial |r|^2.
+// Residual update of the unpreconditioned CG: r -= a q ; partial (|r|^2, |r|^2).
 template <class R>
 __global__ void __launch_bounds__(kRedThreads)
-k_cg_xr_dot(cx<R>* __restrict__ x, cx<R>* __restrict__ r, const cx<R>* __restrict__ p, const cx<R>* __restrict__ q,
-            long long len, long long stride, const double* __restrict__ alpha, const int* __restrict__ active,
-            double2* __restrict__ partial) {
+k_cg_r_dot(cx<R>* __restrict__ r, const cx<R>* __restrict__ q, long long len, const double* __restrict__ alpha,
+           const int* __restrict__ active, double2* __restrict__ partial) {
   const int vec = blockIdx.y;
   const int nblk = gridDim.x;
   double2* out = partial + (long long)vec * nblk + blockIdx.x;
@@ -107,20 +106,15 @@ k_cg_xr_dot(cx<R>* __restrict__ x, cx<R>* __restrict__ r, const cx<R>* __restric
     return;
   }
   const R a = R(alpha[vec]);
-  const long long o = vec * stride;
+  const long long o = vec * len;
   R s0 = 0;
   const long long chunk = (len + nblk - 1) / nblk, end = min(len, (blockIdx.x + 1) * chunk);
   for (long long i = blockIdx.x * chunk + threadIdx.x; i < end; i += kRedThreads) {
-    cx<R> pi = p[o + i], qi = q[o + i], xi = x[o + i], ri = r[o + i];
-    xi.x += a * pi.x;
-    xi.y += a * pi.y;
-    ri.x -= a * qi.x;
-    ri.y -= a * qi.y;
-    x[o + i] = xi;
+    const cx<R> ri = caxpy(-a, q[o + i], r[o + i]);
     r[o + i] = ri;
     s0 += ri.x * ri.x + ri.y * ri.y;
   }
-  double2 s = block_sum2(make_double2(double(s0), double(s0)));
+  const double2 s = block_sum2(make_double2(double(s0), double(s0)));
   if (threadIdx.x == 0) *out = s;
 }
 
@@ -152,15 +146,19 @@ __global__ void k_axpby(const cx<R>* __restrict__ x, cx<R>* __restrict__ y, long
 
 __global__ void __launch_bounds__(32)
 k_cg_alpha(const double2* __restrict__ partial, int nblk, double2* __restrict__ dot, const double* __restrict__ rho,
-           double* __restrict__ alpha, int* __restrict__ active, int* __restrict__ iters) {
+           double* __restrict__ alpha, int* __restrict__ active, int* __restrict__ iters, int* __restrict__ go) {
   const int v = blockIdx.x;
   pdl_wait();
-  if (!active[v]) return;
+  if (!active[v]) {
+    if (threadIdx.x == 0) go[v] = 0;
+    return;
+  }
   const double2 s = warp_sum2(partial + (long long)v * nblk, nblk);
   if (threadIdx.x != 0) return;
   dot[v] = s;
   const bool ok = s.x > 0.0 && isfinite(s.x);
   alpha[v] = ok ? rho[v] / s.x : 0.0;
+  go[v] = ok;
   if (!ok) {  // breakdown: B must be HPD
     active[v] = 0;
     iters[v] = -(iters[v] + 1);
@@ -186,46 +184,51 @@ k_cg_init(const double2* __restrict__ partial, int nblk, const double* __restric
   if (!(s.y > 0.0) || !isfinite(s.y)) active[v] = 0;
 }
 
-// End of a CG iteration (cg_dir).  Every CTA of a vector reduces the partials
+// End of a CG iteration (cg_dir): x += alpha p, the convergence test, and p = z +
+// beta p for the vectors that go on.  Every CTA of a vector reduces the partials
 // in the same order, so all use the same beta; CTA 0 records the scalars.
 // iters[v] counts the completed iterations of vector v on the device (so an
 // iteration needs no host-side argument and can be replayed from a graph);
 // a negative count flags breakdown at that iteration.
-// HBM-bound (reads p and z, writes p), the first elements loaded while the
-// partials are reduced.  One launch replaces a scalar kernel (6 us of latency
-// on one CTA per vector) and the update of p inside fncB's first plane kernel,
-// which ran it at half the bandwidth (8 vectors at n = 48: 55 us for the two
-// and the transform, 39 now).
+// HBM-bound (reads p, z, x, writes p and x: 141 MB in 24 us for 8 vectors at
+// n = 48), the first elements loaded while the partials are reduced.  One launch
+// replaces a scalar kernel (6 us of latency on one CTA per vector), the update
+// of x in k_pcg_update (p is read once less: the two kernels 60 -> 53 us) and
+// the one of p inside fncB's first plane kernel, which ran it at half the
+// bandwidth.
 template <class R>
 __global__ void __launch_bounds__(kRedThreads)
-k_cg_dir(cx<R>* __restrict__ p, const cx<R>* __restrict__ z, long long len, const double2* __restrict__ partial,
-         int nblk, const double* __restrict__ rho, double* __restrict__ rho_next, double2* __restrict__ dot,
-         const double* __restrict__ tol2b2, int* active, int* iters, double* __restrict__ res2) {
+k_cg_dir(cx<R>* __restrict__ x, cx<R>* __restrict__ p, const cx<R>* __restrict__ z, long long len,
+         const double2* __restrict__ partial, int nblk, const double* __restrict__ alpha,
+         const double* __restrict__ rho, double* __restrict__ rho_next, double2* __restrict__ dot,
+         const double* __restrict__ tol2b2, const int* __restrict__ go, int* __restrict__ active,
+         int* __restrict__ iters, double* __restrict__ res2) {
   const int v = blockIdx.y;
   __shared__ int s_act;
   __shared__ double s_beta;
   pdl_wait();
-  // one read per CTA: CTA 0 may clear the flag while others start
-  if (threadIdx.x == 0) s_act = active[v];
-  __syncthreads();
-  if (!s_act) return;
+  // not active[v]: CTA 0 clears that one on convergence, and a CTA that starts
+  // after it still owes its part of x
+  if (!go[v]) return;
   constexpr int U = 16 / sizeof(cx<R>);  // elements per 16-byte access (len is a multiple of 4)
   struct alignas(16) Pack {
     cx<R> e[U];
   };
+  Pack* xp = reinterpret_cast<Pack*>(x + (long long)v * len);
   Pack* pp = reinterpret_cast<Pack*>(p + (long long)v * len);
   const Pack* zp = reinterpret_cast<const Pack*>(z + (long long)v * len);
   const int np = int(len / U), chunk = (np + gridDim.x - 1) / gridDim.x;
   const int end = min(np, (int(blockIdx.x) + 1) * chunk);
   int i = blockIdx.x * chunk + threadIdx.x;
-  constexpr int B = 4;  // packs in flight; the first ones during the reduction
-  Pack a[B], c[B];
+  constexpr int B = 3;  // packs of each in flight; the first ones during the reduction
+  Pack a[B], c[B], e[B];
   auto load = [&]() {
 #pragma unroll
     for (int u = 0; u < B; ++u)
       if (i + u * kRedThreads < end) {
         a[u] = zp[i + u * kRedThreads];
         c[u] = pp[i + u * kRedThreads];
+        e[u] = xp[i + u * kRedThreads];
       }
   };
   load();
@@ -248,15 +251,19 @@ k_cg_dir(cx<R>* __restrict__ p, const cx<R>* __restrict__ z, long long len, cons
     }
   }
   __syncthreads();
-  if (!s_act) return;
-  const R b = R(s_beta);
+  const bool more = s_act != 0;  // a vector that stops here needs no further direction
+  const R al = R(alpha[v]), b = R(s_beta);
   while (i < end) {
 #pragma unroll
     for (int u = 0; u < B; ++u)
       if (i + u * kRedThreads < end) {
 #pragma unroll
-        for (int w = 0; w < U; ++w) c[u].e[w] = caxpy(b, c[u].e[w], a[u].e[w]);
-        pp[i + u * kRedThreads] = c[u];
+        for (int w = 0; w < U; ++w) {
+          e[u].e[w] = caxpy(al, c[u].e[w], e[u].e[w]);
+          c[u].e[w] = caxpy(b, c[u].e[w], a[u].e[w]);
+        }
+        xp[i + u * kRedThreads] = e[u];
+        if (more) pp[i + u * kRedThreads] = c[u];
       }
     i += B * kRedThreads;
     load();
@@ -527,10 +534,9 @@ cudaError_t dot_partial(const cx<R>* a, const cx<R>* b, long long len, long long
 }
 
 template <class R>
-cudaError_t cg_xr_partial(cx<R>* x, cx<R>* r, const cx<R>* p, const cx<R>* q, long long len, long long stride,
-                          int nvec, const double* alpha, const int* active, double2* partial, int nblk,
-                          cudaStream_t st) {
-  return launch<k_cg_xr_dot<R>>(dim3(nblk, nvec), kRedThreads, 0, st, x, r, p, q, len, stride, alpha, active, partial);
+cudaError_t cg_r_partial(cx<R>* r, const cx<R>* q, long long len, int nvec, const double* alpha, const int* active,
+                         double2* partial, int nblk, cudaStream_t st) {
+  return launch<k_cg_r_dot<R>>(dim3(nblk, nvec), kRedThreads, 0, st, r, q, len, alpha, active, partial);
 }
 
 // Q_v[:, col_v] = V_v, BQ_v[:, col_v] = BV_v (and their complex64 copies when
@@ -617,8 +623,8 @@ cudaError_t while_active(const int* active, int nvec, int* passes, int max_passe
 }
 
 cudaError_t cg_alpha(int nvec, const double2* partial, int nblk, double2* dot, const double* rho, double* alpha,
-                     int* active, int* iters, cudaStream_t st) {
-  return launch<k_cg_alpha>(dim3(nvec), 32, 0, st, partial, nblk, dot, rho, alpha, active, iters);
+                     int* active, int* iters, int* go, cudaStream_t st) {
+  return launch<k_cg_alpha>(dim3(nvec), 32, 0, st, partial, nblk, dot, rho, alpha, active, iters, go);
 }
 
 cudaError_t cg_init(int nvec, const double2* partial, int nblk, const double* tolv, double* rho, double* tol2b2,
@@ -627,11 +633,11 @@ cudaError_t cg_init(int nvec, const double2* partial, int nblk, const double* to
 }
 
 template <class R>
-cudaError_t cg_dir(cx<R>* p, const cx<R>* z, long long len, int nvec, const double2* partial, int nblk,
-                   const double* rho, double* rho_next, double2* dot, const double* tol2b2, int* active, int* iters,
-                   double* res2, int ncta, cudaStream_t st) {
-  return launch<k_cg_dir<R>>(dim3(ncta, nvec), kRedThreads, 0, st, p, z, len, partial, nblk, rho, rho_next, dot, tol2b2,
-                             active, iters, res2);
+cudaError_t cg_dir(cx<R>* x, cx<R>* p, const cx<R>* z, long long len, int nvec, const double2* partial, int nblk,
+                   const double* alpha, const double* rho, double* rho_next, double2* dot, const double* tol2b2,
+                   const int* go, int* active, int* iters, double* res2, int ncta, cudaStream_t st) {
+  return launch<k_cg_dir<R>>(dim3(ncta, nvec), kRedThreads, 0, st, x, p, z, len, partial, nblk, alpha, rho, rho_next, dot,
+                             tol2b2, go, active, iters, res2);
 }
 
 template <class R>
@@ -732,16 +738,17 @@ template cudaError_t scale_batched<float>(const cx<float>*, cx<float>*, long lon
                                       long long, int, double2*, double2*, int, const int*, cudaStream_t); \
   template cudaError_t axpby_batched<R>(const cx<R>*, cx<R>*, long long, long long, int, const double2*, \
                                         const double2*, const int*, cudaStream_t);                       \
-  template cudaError_t cg_dir<R>(cx<R>*, const cx<R>*, long long, int, const double2*, int, const double*, \
-                                 double*, double2*, const double*, int*, int*, double*, int, cudaStream_t); \
+  template cudaError_t cg_dir<R>(cx<R>*, cx<R>*, const cx<R>*, long long, int, const double2*, int,        \
+                                 const double*, const double*, double*, double2*, const double*,          \
+                                 const int*, int*, int*, double*, int, cudaStream_t);                     \
   template cudaError_t block_rot<R>(const cx<R>*, cx<R>*, long long, long long, int, int, const double*, \
                                     cudaStream_t);                                                        \
   template cudaError_t sub_combo<R>(cx<R>*, const cx<R>*, long long, long long, int, const double2*,     \
                                     cudaStream_t);                                                        \
   template cudaError_t dot_partial<R>(const cx<R>*, const cx<R>*, long long, long long, int, double2*,   \
                                       int, const int*, cudaStream_t);                                     \
-  template cudaError_t cg_xr_partial<R>(cx<R>*, cx<R>*, const cx<R>*, const cx<R>*, long long, long long, \
-                                        int, const double*, const int*, double2*, int, cudaStream_t);
+  template cudaError_t cg_r_partial<R>(cx<R>*, const cx<R>*, long long, int, const double*, const int*,     \
+                                       double2*, int, cudaStream_t);
 FAME_KINST(float)
 FAME_KINST(double)
 template cudaError_t convert<float, double>(const cx<double>*, cx<float>*, long long, cudaStream_t);

@@ -208,20 +208,20 @@ k_pcg_start(const cx<R>* __restrict__ b, cx<R>* __restrict__ x, cx<R>* __restric
   if (threadIdx.x == 0) *out = s;
 }
 
-// CG update of one vector's chunk of voxels per CTA: x += a p, r -= a q, z = M r
-// and the partial sums.  HBM-bound on large batches (8 vectors at n = 48: 255 MB
-// in 41 us), latency-bound on small ones, so that
+// CG update of one vector's chunk of voxels per CTA: r -= a q, z = M r and the
+// partial sums (x += a p is left to k_cg_dir, which reads p anyway).  HBM-bound
+// on large batches, latency-bound on small ones, so that
 //   * a CTA takes one contiguous chunk, and the CTAs of a launch are whole
 //     multiples of what fits the SMs (update_blocks);
 //   * the loads of the first elements are issued before the step length, which
 //     every CTA reduces from the stencil pass's partials, is waited for;
 //   * complex64 moves two voxels per 16-byte access.
-// 4 vectors at n = 40 (complex64) 20 -> 14 us, 2 at n = 30 (complex128) 26 -> 13.
+// 4 vectors at n = 40 (complex64) 20 -> 11 us, 2 at n = 30 (complex128) 26 -> 12,
+// 8 at n = 48 (complex64) 44 -> 30 (184 MB, 6.2 TB/s).
 template <class R>
 __global__ void __launch_bounds__(kThreads, sizeof(R) == 4 ? 2 : 1)
-k_pcg_update(cx<R>* __restrict__ x, cx<R>* __restrict__ r, cx<R>* __restrict__ z, const cx<R>* __restrict__ p,
-             const cx<R>* __restrict__ q, const cx<R>* __restrict__ pc_all, VecCtx ctx, long long Nq,
-             double2* __restrict__ partial, CgAlpha ca) {
+k_pcg_update(cx<R>* __restrict__ r, cx<R>* __restrict__ z, const cx<R>* __restrict__ q,
+             const cx<R>* __restrict__ pc_all, VecCtx ctx, long long Nq, double2* __restrict__ partial, CgAlpha ca) {
   constexpr int U = 16 / sizeof(cx<R>);  // voxels per 16-byte access (n^3 is even)
   struct alignas(16) Pack {
     cx<R> e[U];
@@ -236,7 +236,10 @@ k_pcg_update(cx<R>* __restrict__ x, cx<R>* __restrict__ r, cx<R>* __restrict__ z
   if (threadIdx.x == 0) s_act = ctx.active ? ctx.active[vec] : 1;
   __syncthreads();
   if (!s_act) {
-    if (threadIdx.x == 0) *out = make_double2(0.0, 0.0);
+    if (threadIdx.x == 0) {
+      *out = make_double2(0.0, 0.0);
+      if (blockIdx.x == 0) ca.go[vec] = 0;
+    }
     return;
   }
   const cx<R>* pc = pc_all + (long long)vec_inst(ctx, vec) * kPcSlots * Nq;
@@ -244,14 +247,12 @@ k_pcg_update(cx<R>* __restrict__ x, cx<R>* __restrict__ r, cx<R>* __restrict__ z
   const int np = int(Nq / U), chunk = (np + nblk - 1) / nblk;  // packs, packs per CTA
   const int end = min(np, (int(blockIdx.x) + 1) * chunk);
   int i = blockIdx.x * chunk + threadIdx.x;
-  Pack pk[4], qk[4], xk[4], rk[4], bk[kPcSlots];
+  Pack qk[4], rk[4], bk[kPcSlots];
   auto load = [&](int j) {
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
       const long long k = o + c * Nq + (long long)j * U;
-      pk[c] = *reinterpret_cast<const Pack*>(p + k);
       qk[c] = *reinterpret_cast<const Pack*>(q + k);
-      xk[c] = *reinterpret_cast<const Pack*>(x + k);
       rk[c] = *reinterpret_cast<const Pack*>(r + k);
     }
 #pragma unroll
@@ -276,6 +277,7 @@ k_pcg_update(cx<R>* __restrict__ x, cx<R>* __restrict__ r, cx<R>* __restrict__ z
       s_alpha = av;
       if (blockIdx.x == 0) {
         ca.alpha[vec] = av;
+        ca.go[vec] = ok;
         ca.dot[vec] = make_double2(sx, sy);
         if (!ok) {  // breakdown: B must be HPD
           ca.active[vec] = 0;
@@ -295,7 +297,6 @@ k_pcg_update(cx<R>* __restrict__ x, cx<R>* __restrict__ r, cx<R>* __restrict__ z
       Block4<R> bl;
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
-        xk[c].e[u] = caxpy(a, pk[c].e[u], xk[c].e[u]);
         rk[c].e[u] = caxpy(-a, qk[c].e[u], rk[c].e[u]);
         rv[c] = rk[c].e[u];
       }
@@ -312,7 +313,6 @@ k_pcg_update(cx<R>* __restrict__ x, cx<R>* __restrict__ r, cx<R>* __restrict__ z
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
       const long long k = o + c * Nq + (long long)i * U;
-      *reinterpret_cast<Pack*>(x + k) = xk[c];
       *reinterpret_cast<Pack*>(r + k) = rk[c];
       *reinterpret_cast<Pack*>(z + k) = zk[c];
     }
@@ -356,10 +356,10 @@ cudaError_t pcg_start(const Plan& P, bool precond, const cx<R>* b, cx<R>* x, cx<
 }
 
 template <class R>
-cudaError_t pcg_update(const Plan& P, cx<R>* x, cx<R>* r, cx<R>* z, const cx<R>* p, const cx<R>* q, int nvec,
-                       const VecCtx& ctx, double2* partial, int nblk, cudaStream_t st, const CgAlpha& ca) {
+cudaError_t pcg_update(const Plan& P, cx<R>* r, cx<R>* z, const cx<R>* q, int nvec, const VecCtx& ctx,
+                       double2* partial, int nblk, cudaStream_t st, const CgAlpha& ca) {
   const PlanData<R>& d = detail::pdata<R>(P);
-  return launch<k_pcg_update<R>>(dim3(nblk, nvec), kThreads, 0, st, x, r, z, p, q, d.pc, ctx, P.Nq, partial, ca);
+  return launch<k_pcg_update<R>>(dim3(nblk, nvec), kThreads, 0, st, r, z, q, d.pc, ctx, P.Nq, partial, ca);
 }
 
 template cudaError_t build_precond<float>(Plan&, cudaStream_t);
@@ -368,9 +368,9 @@ template cudaError_t pcg_start<float>(const Plan&, bool, const cx<float>*, cx<fl
                                          const VecCtx&, double2*, int, cudaStream_t);
 template cudaError_t pcg_start<double>(const Plan&, bool, const cx<double>*, cx<double>*, cx<double>*, cx<double>*, cx<double>*, int,
                                          const VecCtx&, double2*, int, cudaStream_t);
-template cudaError_t pcg_update<float>(const Plan&, float2*, float2*, float2*, const float2*, const float2*, int,
-                                       const VecCtx&, double2*, int, cudaStream_t, const CgAlpha&);
-template cudaError_t pcg_update<double>(const Plan&, double2*, double2*, double2*, const double2*, const double2*, int,
-                                        const VecCtx&, double2*, int, cudaStream_t, const CgAlpha&);
+template cudaError_t pcg_update<float>(const Plan&, cx<float>*, cx<float>*, const cx<float>*, int, const VecCtx&,
+                                       double2*, int, cudaStream_t, const CgAlpha&);
+template cudaError_t pcg_update<double>(const Plan&, cx<double>*, cx<double>*, const cx<double>*, int, const VecCtx&,
+                                        double2*, int, cudaStream_t, const CgAlpha&);
 
 }  // namespace fame

@@ -55,7 +55,8 @@ struct CgScalars {
   int *active, *iters;
   int* passes;  // passes of the graph-resident iteration loop
   double *bb, *res2;
-  static size_t bytes(int nvec) { return (sizeof(double2) + 7 * sizeof(double) + 2 * sizeof(int)) * nvec + 64; }
+  int* go;  // the vectors that take this iteration's step
+  static size_t bytes(int nvec) { return (sizeof(double2) + 7 * sizeof(double) + 3 * sizeof(int)) * nvec + 64; }
   static size_t down_bytes(int nvec) { return (2 * sizeof(int) + 2 * sizeof(double)) * nvec + 2 * sizeof(int); }
   void carve(char* s, int nvec) {
     dot = (double2*)s;
@@ -69,6 +70,7 @@ struct CgScalars {
     passes = iters + nvec;  // one, and one unused for alignment
     bb = (double*)(passes + 2);
     res2 = bb + nvec;
+    go = (int*)(res2 + nvec);
   }
 };
 
@@ -140,8 +142,9 @@ int pcg_batched(Plan& P, const cx<R>* b, cx<R>* x, int nvec, const int* d_inst, 
   //                                     stencil pass provides them)
   //   alpha = rho / p^H q             (preconditioned: reduced by the update
   //                                     kernel itself; else one scalar launch)
-  //   x += alpha p, r -= alpha q, z = M r, partials of (r^H z, |r|^2)
-  //   beta, rho, convergence, p = z + beta p   (partials reduced in the same launch)
+  //   r -= alpha q, z = M r, partials of (r^H z, |r|^2)
+  //   beta, rho, convergence, x += alpha p, p = z + beta p   (partials reduced in
+  //                                     the same launch)
   // Preconditioned, that is two glue launches per iteration.  Iteration i reads
   // rho from one of two arrays and writes the other (i odd / even; the blocks
   // of chk iterations are even).
@@ -160,14 +163,16 @@ int pcg_batched(Plan& P, const cx<R>* b, cx<R>* x, int nvec, const int* d_inst, 
       ca.dot = S.dot;
       ca.active = S.active;
       ca.iters = S.iters;
-      if (e2 == cudaSuccess) e2 = pcg_update<R>(P, x, r, z, p, q, nvec, ctx, part2, nblkv, cs, ca);
+      ca.go = S.go;
+      if (e2 == cudaSuccess) e2 = pcg_update<R>(P, r, z, q, nvec, ctx, part2, nblkv, cs, ca);
     } else {
-      if (e2 == cudaSuccess) e2 = cg_alpha(nvec, part, nblk_pq ? nblk_pq : nblk, S.dot, rho_in, S.alpha, S.active, S.iters, cs);
-      if (e2 == cudaSuccess) e2 = cg_xr_partial<R>(x, r, p, q, L, L, nvec, S.alpha, S.active, part, nblk, cs);
+      if (e2 == cudaSuccess) e2 = cg_alpha(nvec, part, nblk_pq ? nblk_pq : nblk, S.dot, rho_in, S.alpha, S.active, S.iters,
+                                              S.go, cs);
+      if (e2 == cudaSuccess) e2 = cg_r_partial<R>(r, q, L, nvec, S.alpha, S.active, part, nblk, cs);
     }
     if (e2 == cudaSuccess)
-      e2 = cg_dir<R>(p, pre ? z : r, L, nvec, pre ? part2 : part, pre ? nblkv : nblk, rho_in, rho_out, S.dot, S.tol2b2,
-                     S.active, S.iters, S.res2, nblk, cs);
+      e2 = cg_dir<R>(x, p, pre ? z : r, L, nvec, pre ? part2 : part, pre ? nblkv : nblk, S.alpha, rho_in, rho_out, S.dot,
+                     S.tol2b2, S.go, S.active, S.iters, S.res2, dot_blocks(P, L, nvec, 2, 2048), cs);
     return e2;
   };
   const int chk = 4;
