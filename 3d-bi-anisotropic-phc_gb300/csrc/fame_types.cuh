@@ -147,7 +147,7 @@ template <int S, class V> FAME_HD V cmul_i(V a) {
   if (S > 0) { z.x = -a.y; z.y = a.x; } else { z.x = a.y; z.y = -a.x; }
   return z;
 }
-#if defined(__CUDA_ARCH__)
+#if defined(__CUDA_ARCH__) && __CUDA_ARCH__ >= 1000  // host checks compile these headers for other targets
 // complex64 on the device: both components in one packed FP32 instruction
 // (the FP32 pipe takes the same time for it as for two scalar ones, but it
 // costs one issue slot, and the complex64 kernels are bound by issue).
