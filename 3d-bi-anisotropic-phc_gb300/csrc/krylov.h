@@ -49,11 +49,11 @@ cudaError_t gs_dots(const double2* X, long long xs, const double2* r, long long 
 // is given) for every v with col[v] >= 0; blocks xs apart, vectors len apart.
 cudaError_t gs_store(double2* Q, double2* BQ, float2* Q32, float2* BQ32, long long xs, const double2* V,
                      const double2* BV, long long len, int nv, const int* col, cudaStream_t st);
-// r_v -= sum_i coef[v*cstride + i] X_v[col0_v + i], FP64 or from complex64 copies
-cudaError_t gs_combo(double2* r, long long rs, const double2* X, long long xs, long long len, int nv,
-                     const int2* span, const double2* coef, int cstride, cudaStream_t st);
-cudaError_t gs_combo_lo(double2* r, long long rs, const float2* X, long long xs, long long len, int nv,
-                        const int2* span, const double2* coef, int cstride, cudaStream_t st);
+// r_v -= sum_i coef[v*cstride + i] X_v[col0_v + i], FP64 or from complex64 copies;
+// with r2, r2 and X2 likewise in the same launch
+template <class XT>
+cudaError_t gs_combo(double2* r, double2* r2, long long rs, const XT* X, const XT* X2, long long xs, long long len,
+                     int nv, const int2* span, const double2* coef, int cstride, cudaStream_t st);
 // partial[v * nblk + i] = block i's share of a_v^H b_v (no final reduction)
 template <class R>
 cudaError_t dot_partial(const cx<R>* a, const cx<R>* b, long long len, long long stride, int nvec, double2* partial,

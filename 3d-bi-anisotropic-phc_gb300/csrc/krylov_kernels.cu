@@ -338,78 +338,102 @@ __global__ void k_block_comb(const cx<R>* __restrict__ in, cx<R>* __restrict__ o
 // m = 0 skips it) of its block X + v * xs (columns len apart).
 // ---------------------------------------------------------------------------
 // partial[(v * maxm + i) * nblk + blk] = block's share of X_v[col0_v + i]^H r_v
+// FP64-rate-bound (4 fused operations per element; 12 -> 7 us a column of 4 x
+// 256000 with them, where the plain expressions take 6).
 __global__ void __launch_bounds__(kRedThreads)
 k_gs_dot_partial(const double2* __restrict__ X, long long xs, const double2* __restrict__ r, long long rs,
                  long long len, const int2* __restrict__ span, int maxm, double2* __restrict__ partial) {
   const int v = blockIdx.y, i = blockIdx.z, nblk = gridDim.x;
+  pdl_wait();
   const int2 sp = span[v];
   if (i >= sp.y) return;
   const double2* a = X + v * xs + (long long)(sp.x + i) * len;
   const double2* b = r + v * rs;
-  double sx = 0.0, sy = 0.0;
-  for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < len; k += (long long)nblk * blockDim.x) {
-    const double2 x = a[k], y = b[k];
-    sx += x.x * y.x + x.y * y.y;
-    sy += x.x * y.y - x.y * y.x;
+  double sx0 = 0.0, sy0 = 0.0, sx1 = 0.0, sy1 = 0.0;
+  const long long chunk = (len + nblk - 1) / nblk, end = min(len, (blockIdx.x + 1) * chunk);
+  long long k = blockIdx.x * chunk + threadIdx.x;
+  for (; k + kRedThreads < end; k += 2 * kRedThreads) {
+    const double2 x = a[k], y = b[k], x2 = a[k + kRedThreads], y2 = b[k + kRedThreads];
+    sx0 = rfma(x.x, y.x, rfma(x.y, y.y, sx0));
+    sy0 = rfma(x.x, y.y, rfma(-x.y, y.x, sy0));
+    sx1 = rfma(x2.x, y2.x, rfma(x2.y, y2.y, sx1));
+    sy1 = rfma(x2.x, y2.y, rfma(-x2.y, y2.x, sy1));
   }
-  const double2 s = block_sum2(make_double2(sx, sy));
+  if (k < end) {
+    const double2 x = a[k], y = b[k];
+    sx0 = rfma(x.x, y.x, rfma(x.y, y.y, sx0));
+    sy0 = rfma(x.x, y.y, rfma(-x.y, y.x, sy0));
+  }
+  const double2 s = block_sum2(make_double2(sx0 + sx1, sy0 + sy1));
   if (threadIdx.x == 0) partial[((long long)v * maxm + i) * nblk + blockIdx.x] = s;
 }
 
 // coef[v * cstride + i] = sum over blocks (i < m_v)
-__global__ void __launch_bounds__(kRedThreads)
+__global__ void __launch_bounds__(32)
 k_gs_dot_final(const double2* __restrict__ partial, int nblk, int maxm, const int2* __restrict__ span,
                double2* __restrict__ coef, int cstride) {
   const int v = blockIdx.x / maxm, i = blockIdx.x - v * maxm;
+  pdl_wait();
   if (i >= span[v].y) return;
-  double2 s = make_double2(0.0, 0.0);
-  for (int t = threadIdx.x; t < nblk; t += blockDim.x) {
-    const double2 q = partial[((long long)v * maxm + i) * nblk + t];
-    s.x += q.x;
-    s.y += q.y;
-  }
-  s = block_sum2(s);
+  const double2 s = warp_sum2(partial + ((long long)v * maxm + i) * nblk, nblk);
   if (threadIdx.x == 0) coef[(long long)v * cstride + i] = s;
 }
 
-// r_v -= sum_i coef[v * cstride + i] X_v[col0_v + i]  (FP64, or from a complex64 copy when XL)
+// r_v -= sum_i coef[v * cstride + i] X_v[col0_v + i], and with r2 the same with X2
+// (blockIdx.z), FP64 or from complex64 copies (the correction in FP32).  FP64:
+// rate-bound, 4 fused operations per column and row.  complex64: HBM-bound; the
+// coefficients are rounded once per CTA (converting them at every use kept the
+// FP64 pipe busy for 31 of 44 us at 9 columns of 4 x 256000), 16-byte loads.
 template <class XT>
-__global__ void k_gs_combo(double2* __restrict__ r, long long rs, const XT* __restrict__ X, long long xs,
-                           long long len, const int2* __restrict__ span, const double2* __restrict__ coef,
-                           int cstride) {
-  __shared__ double2 cs[128];
+__global__ void __launch_bounds__(kRedThreads)
+k_gs_combo(double2* __restrict__ r, double2* __restrict__ r2, long long rs, const XT* __restrict__ X,
+           const XT* __restrict__ X2, long long xs, long long len, const int2* __restrict__ span,
+           const double2* __restrict__ coef, int cstride) {
+  using S = decltype(XT::x);
+  constexpr int U = 16 / sizeof(XT);  // rows per access (len is a multiple of 4)
+  struct alignas(16) Pack {
+    XT e[U];
+  };
+  __shared__ XT cs[128];
   const int v = blockIdx.y;
+  pdl_wait();
   const int2 sp = span[v];
   if (sp.y <= 0) return;
-  for (int i = threadIdx.x; i < sp.y; i += blockDim.x) cs[i] = coef[(long long)v * cstride + i];
+  for (int i = threadIdx.x; i < sp.y; i += kRedThreads) {
+    const double2 c = coef[(long long)v * cstride + i];
+    cs[i] = mk<S>(S(c.x), S(c.y));
+  }
+  const int np = int(len / U);
+  const Pack* x = reinterpret_cast<const Pack*>((blockIdx.z ? X2 : X) + v * xs + (long long)sp.x * len);
+  double2* rv = (blockIdx.z ? r2 : r) + v * rs;
   __syncthreads();
-  const XT* x = X + v * xs + (long long)sp.x * len;
-  double2* rv = r + v * rs;
-  for (long long row = (long long)blockIdx.x * blockDim.x + threadIdx.x; row < len;
-       row += (long long)gridDim.x * blockDim.x) {
-    if constexpr (sizeof(XT) == 8) {  // complex64 copy: the correction in FP32
-      float ax = 0.f, ay = 0.f;
-      for (int i = 0; i < sp.y; ++i) {
-        const XT q = x[(long long)i * len + row];
-        const float cx_ = float(cs[i].x), cy_ = float(cs[i].y);
-        ax += cx_ * q.x - cy_ * q.y;
-        ay += cx_ * q.y + cy_ * q.x;
-      }
-      double2 o = rv[row];
-      o.x -= double(ax);
-      o.y -= double(ay);
-      rv[row] = o;
-    } else {
-      double ax = 0.0, ay = 0.0;
-      for (int i = 0; i < sp.y; ++i) {
-        const XT q = x[(long long)i * len + row];
-        ax += cs[i].x * q.x - cs[i].y * q.y;
-        ay += cs[i].x * q.y + cs[i].y * q.x;
-      }
-      double2 o = rv[row];
-      o.x -= ax;
-      o.y -= ay;
-      rv[row] = o;
+  for (int k = blockIdx.x * kRedThreads + threadIdx.x; k < np; k += gridDim.x * kRedThreads) {
+    XT acc[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) acc[u] = mk<S>(S(0), S(0));
+    double2 o[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) o[u] = rv[(long long)k * U + u];
+    int i = 0;
+    for (; i + 4 <= sp.y; i += 4) {  // four columns' loads in flight
+      Pack q[4];
+#pragma unroll
+      for (int w = 0; w < 4; ++w) q[w] = x[(long long)(i + w) * np + k];
+#pragma unroll
+      for (int w = 0; w < 4; ++w)
+#pragma unroll
+        for (int u = 0; u < U; ++u) acc[u] = cfma(cs[i + w], q[w].e[u], acc[u]);
+    }
+    for (; i < sp.y; ++i) {
+      const Pack q = x[(long long)i * np + k];
+#pragma unroll
+      for (int u = 0; u < U; ++u) acc[u] = cfma(cs[i], q.e[u], acc[u]);
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      o[u].x -= double(acc[u].x);
+      o[u].y -= double(acc[u].y);
+      rv[(long long)k * U + u] = o[u];
     }
   }
 }
@@ -573,32 +597,24 @@ cudaError_t gs_dots(const double2* X, long long xs, const double2* r, long long 
                     const int2* span, int maxm, double2* coef, int cstride, double2* partial, int nblk,
                     cudaStream_t st) {
   if (nv <= 0 || maxm <= 0) return cudaSuccess;
-  FAME_LAUNCHED(1);
-  k_gs_dot_partial<<<dim3(nblk, nv, maxm), kRedThreads, 0, st>>>(X, xs, r, rs, len, span, maxm, partial);
-  FAME_LAUNCHED(1);
-  k_gs_dot_final<<<nv * maxm, kRedThreads, 0, st>>>(partial, nblk, maxm, span, coef, cstride);
-  return cudaGetLastError();
+  cudaError_t e = launch<k_gs_dot_partial>(dim3(nblk, nv, maxm), kRedThreads, 0, st, X, xs, r, rs, len, span, maxm,
+                                           partial);
+  if (e != cudaSuccess) return e;
+  return launch<k_gs_dot_final>(dim3(nv * maxm), 32, 0, st, (const double2*)partial, nblk, maxm, span, coef, cstride);
 }
 
-cudaError_t gs_combo(double2* r, long long rs, const double2* X, long long xs, long long len, int nv,
-                     const int2* span, const double2* coef, int cstride, cudaStream_t st) {
+template <class XT>
+cudaError_t gs_combo(double2* r, double2* r2, long long rs, const XT* X, const XT* X2, long long xs, long long len,
+                     int nv, const int2* span, const double2* coef, int cstride, cudaStream_t st) {
   if (nv <= 0) return cudaSuccess;
-  int gx = grid_for(len);
-  if (gx > 1024) gx = 1024;
-  FAME_LAUNCHED(1);
-  k_gs_combo<double2><<<dim3(gx, nv), 256, 0, st>>>(r, rs, X, xs, len, span, coef, cstride);
-  return cudaGetLastError();
+  const int gx = (int)std::min(1024LL, (len * (long long)sizeof(XT) / 16 + kRedThreads - 1) / kRedThreads);
+  return launch<k_gs_combo<XT>>(dim3(gx, nv, r2 ? 2 : 1), kRedThreads, 0, st, r, r2, rs, X, X2, xs, len, span, coef,
+                                cstride);
 }
-
-cudaError_t gs_combo_lo(double2* r, long long rs, const float2* X, long long xs, long long len, int nv,
-                        const int2* span, const double2* coef, int cstride, cudaStream_t st) {
-  if (nv <= 0) return cudaSuccess;
-  int gx = grid_for(len);
-  if (gx > 1024) gx = 1024;
-  FAME_LAUNCHED(1);
-  k_gs_combo<float2><<<dim3(gx, nv), 256, 0, st>>>(r, rs, X, xs, len, span, coef, cstride);
-  return cudaGetLastError();
-}
+template cudaError_t gs_combo<double2>(double2*, double2*, long long, const double2*, const double2*, long long,
+                                       long long, int, const int2*, const double2*, int, cudaStream_t);
+template cudaError_t gs_combo<float2>(double2*, double2*, long long, const float2*, const float2*, long long,
+                                      long long, int, const int2*, const double2*, int, cudaStream_t);
 
 // The loop condition of a graph-resident iteration loop: one pass of the
 // body done (*passes + 1); continue while any vector is active and fewer

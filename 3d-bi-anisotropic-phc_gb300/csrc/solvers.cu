@@ -802,21 +802,24 @@ int lanczos_run(Plan& P, int prec, const std::vector<int>& insts, int k0, double
     return d;
   };
   const long long qs = (long long)p * L;  // instance stride of Q, BQ and their copies
-  // r_a -= sum (B q_i)^H r_a q_i over span (and B r likewise), FP64 or with complex64 corrections
+  // r_a -= sum coef_i q_i over the span (and B r likewise), FP64 or with complex64 corrections
+  double2* BPRm = mixed ? BPR : nullptr;
+  auto combo = [&](const int2* d, bool lo) -> int {
+    if (lo) FAME_CK(gs_combo<float2>(PR, BPRm, L, Q32, BQ32, qs, L, na, d, coef, 128, st), "lanczos gs");
+    else FAME_CK(gs_combo<double2>(PR, BPRm, L, Q, BQ, qs, L, na, d, coef, 128, st), "lanczos gs");
+    return FAME_OK;
+  };
+  // ... with coef_i = (B q_i)^H r_a
   auto project_b = [&](const std::vector<int2>& sp, bool lo) -> int {
     int maxm = 0;
     const int2* d = upload_span(sp, &maxm);
     if (!d) return cuda_fail(&P, cudaErrorUnknown, "lanczos span upload");
     if (maxm == 0) return FAME_OK;
-    FAME_CK(gs_dots(BQ, qs, PR, L, L, na, d, maxm, coef, 128, gspart, nblkg, st), "lanczos gs dot");
-    if (lo) {
-      FAME_CK(gs_combo_lo(PR, L, Q32, qs, L, na, d, coef, 128, st), "lanczos gs");
-      if (mixed) FAME_CK(gs_combo_lo(BPR, L, BQ32, qs, L, na, d, coef, 128, st), "lanczos gs");
-    } else {
-      FAME_CK(gs_combo(PR, L, Q, qs, L, na, d, coef, 128, st), "lanczos gs");
-      if (mixed) FAME_CK(gs_combo(BPR, L, BQ, qs, L, na, d, coef, 128, st), "lanczos gs");
-    }
-    return FAME_OK;
+    // many columns: fewer CTAs per column, 16 per SM in all (each ends with a
+    // reduction in FP64)
+    const int nb = std::min(nblkg, std::max(1, 16 * P.sms / (na * maxm)));
+    FAME_CK(gs_dots(BQ, qs, PR, L, L, na, d, maxm, coef, 128, gspart, nb, st), "lanczos gs dot");
+    return combo(d, lo);
   };
 
   // v0 (Lanczos.m:8; band_structure...:78-80): ones, or the caller's vector
@@ -949,10 +952,7 @@ int lanczos_run(Plan& P, int prec, const std::vector<int>& insts, int k0, double
       const int2* d = upload_span(sp, &maxm);
       if (!d) return cuda_fail(&P, cudaErrorUnknown, "lanczos span upload");
       FAME_CK(h2d_async(P, coef, hcf.data(), sizeof(double2) * hcf.size()), "lanczos gs");
-      if (maxm > 0) {
-        FAME_CK(gs_combo(PR, L, Q, qs, L, na, d, coef, 128, st), "lanczos gs");
-        if (mixed) FAME_CK(gs_combo(BPR, L, BQ, qs, L, na, d, coef, 128, st), "lanczos gs");
-      }
+      if (maxm > 0 && (rc = combo(d, false))) return rc;
       if ((rc = project_b(sp63, false))) return rc;
       if ((rc = project_b(sp66, false))) return rc;
       if (mixed)  // ||r||_B^2 before the full pass (DGKS test below)
