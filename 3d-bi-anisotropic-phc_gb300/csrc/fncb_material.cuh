@@ -270,6 +270,12 @@ template <class R, int N> struct SweepShape {
   static constexpr int FR = TY + 2;                       // staged field rows
   static constexpr int HR = TY + 1;                       // vertex rows
   static constexpr int TPB = ((HR * N + 31) / 32) * 32;
+  // CTAs per SM: the 16384 registers of an SM's quarter hold 5 warps of 96
+  // registers (complex64; complex128: 3 of 168).  Left to itself the compiler took
+  // 130 for the general tensors at n = 30, 36, 50, 60, 64, one CTA fewer per SM
+  // (fncB of ten vectors at n = 60 then 217 us, now 197; 16 at n = 30 50, now 44).
+  static constexpr int WARPS = sizeof(R) == 4 ? 20 : 12;
+  static constexpr int CTAS = WARPS >= TPB / 32 ? WARPS / (TPB / 32) : 1;
   static constexpr int F_ELEMS = 6 * FR * N;              // one staged plane (complex)
   static constexpr int H_ELEMS = 5 * HR * N;              // shared vertex values of one plane (complex)
   static constexpr int D_ELEMS = 5 * HR * N;              // shared diagonals of one plane (real)
@@ -294,7 +300,7 @@ template <int K> __device__ __forceinline__ void cp_async_wait() {
 }
 
 template <class R, int N, int KIND>
-__global__ void __launch_bounds__(SweepShape<R, N>::TPB)
+__global__ void __launch_bounds__(SweepShape<R, N>::TPB, sizeof(R) == 4 && KIND == kMatGeneral ? SweepShape<R, N>::CTAS : 0)
 k_sweep(const cx<R>* __restrict__ uv, cx<R>* __restrict__ out, PlanData<R> d, const uint8_t* __restrict__ phase,
         int nphase, VecCtx ctx, long long stride, int tz, double2* __restrict__ wdot) {
   using SH = SweepShape<R, N>;
@@ -484,11 +490,11 @@ template <class R, class F> inline cudaError_t with_kind(const PlanData<R>& d, F
 // with the least (waves of resident CTAs) x (planes a CTA steps through; its
 // halo planes cost about 1.5).  One vector of a small grid takes one or two
 // planes per CTA (n = 24: 12 planes in series took 19 us of a 35 us fncB),
-// full batches long chunks.
+// full batches long chunks.  The count of resident CTAs has to be the real one:
+// 4 vectors at n = 40 in 400 CTAs, where 304 are resident, took 15.6 us, 11.3 in 280.
 template <class R, int N> inline int sweep_planes(const Plan& P, int nv) {
   using SH = SweepShape<R, N>;
-  const int per_sm = std::max<int>(1, std::min<int>({2048 / SH::TPB, int((227u << 10) / (SH::SMEM + 1024)),
-                                                    65536 / (SH::TPB * (sizeof(R) == 4 ? 96 : 168))}));
+  const int per_sm = std::max<int>(1, std::min<int>(SH::CTAS, int((227u << 10) / (SH::SMEM + 1024))));
   const long long slots = (long long)per_sm * P.sms;
   int best = N;
   double cost = 1e300;
