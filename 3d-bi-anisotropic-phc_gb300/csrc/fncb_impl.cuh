@@ -623,11 +623,15 @@ k_field_inv(const cx<R>* __restrict__ x, cx<R>* __restrict__ out, PlanData<R> d,
 
 // POST: the three field CTAs of one (plane, side, vector) form a cluster; each
 // applies Pi^H on a third of the voxels, reading the other two fields from
-// its neighbours' shared memory.
-template <class R, int N, bool POST>
+// its neighbours' shared memory.  POST 2 also sums Re(xp^H y) over the CTA's
+// voxels for xp laid out as y (one partial per CTA): in a CG iteration one
+// pass over p and q less (c128, two vectors at n = 30: a launch of 5.3 us).
+enum { kCopy = 0, kPi = 1, kPiDot = 2 };
+template <class R, int N, int POST>
 __global__ void __launch_bounds__(FieldShape<R, N>::TB)
 k_field_fwd(const cx<R>* __restrict__ w, cx<R>* __restrict__ y, PlanData<R> d, VecCtx ctx, long long w_stride,
-            long long out_stride, long long out_side_stride, int side0) {
+            long long out_stride, long long out_side_stride, int side0, const cx<R>* __restrict__ xp,
+            double2* __restrict__ pq) {
   using FS = FieldShape<R, N>;
   constexpr int G = FS::G, M = N / G, LD = FS::LD, KP = FS::KP, TB = FS::TB;
   constexpr int NN = N * N, Nq = NN * N;
@@ -688,8 +692,10 @@ k_field_fwd(const cx<R>* __restrict__ w, cx<R>* __restrict__ y, PlanData<R> d, V
   }
   __syncthreads();
   field_rows<R, N, -1>(sm, tid, g, p, act);
-  cx<R>* o = y + vec * out_stride + (blockIdx.y / 3) * out_side_stride + k3 * NN;
-  if constexpr (POST) {
+  const long long oo = vec * out_stride + (blockIdx.y / 3) * out_side_stride + k3 * NN;
+  cx<R>* o = y + oo;
+  if constexpr (POST != kCopy) {
+    double dot = 0.0;
     auto cluster = cooperative_groups::this_cluster();
     cluster.sync();
     const cx<R>* u0 = cluster.map_shared_rank(sm, 0);
@@ -699,6 +705,11 @@ k_field_fwd(const cx<R>* __restrict__ w, cx<R>* __restrict__ y, PlanData<R> d, V
     for (int e = c * TB + tid; e < KP * NN; e += 3 * TB) {
       const int r = e / N, i1 = e - r * N;
       const int q = r * LD + i1;
+      cx<R> xa, xb;
+      if constexpr (POST == kPiDot) {
+        xa = xp[oo + e];
+        xb = xp[oo + Nq + e];
+      }
       const cx<R> f[3] = {u0[q], u1[q], u2[q]};
       // side 1: a = X, b = Y with X = sum conj(Pi1) v, Y = sum conj(Pi2) v;
       // side 0: a = -Y, b = X with conj(Pi) for Pi (one instruction stream:
@@ -714,8 +725,24 @@ k_field_fwd(const cx<R>* __restrict__ w, cx<R>* __restrict__ y, PlanData<R> d, V
       const cx<R> a = side ? X : cneg(Y), b = side ? Y : X;
       store_io<R>(o + e, a);
       store_io<R>(o + Nq + e, b);
+      if constexpr (POST == kPiDot)
+        dot = rfma(xa.x, a.x, rfma(xa.y, a.y, rfma(xb.x, b.x, rfma(xb.y, b.y, dot))));
     }
-    cluster.sync();  // no CTA leaves while its shared memory is read
+    if constexpr (POST == kPiDot) {
+      __shared__ double sh[TB];
+      sh[tid] = dot;
+      cluster.sync();
+      if (tid < 32) {
+#pragma unroll
+        for (int k = 1; k < TB / 32; ++k) dot += sh[tid + 32 * k];
+#pragma unroll
+        for (int k = 16; k > 0; k >>= 1) dot += __shfl_down_sync(0xffffffffu, dot, k);
+        if (tid == 0)
+          pq[(long long)vec * gridDim.x * gridDim.y + blockIdx.y * gridDim.x + blockIdx.x] = make_double2(dot, 0.0);
+      }
+    } else {
+      cluster.sync();  // no CTA leaves while its shared memory is read
+    }
   } else {
     for (int e = tid; e < KP * NN; e += TB) {
       const int r = e / N, i1 = e - r * N;
@@ -856,14 +883,19 @@ cudaError_t plane_inv(const PlanData<R>& d, const cx<R>* x, cx<R>* out, int nvec
 template <class R, int N, bool POST>
 cudaError_t plane_fwd(const PlanData<R>& d, const cx<R>* w, cx<R>* y, int nvec, int nside, int side0,
                       long long w_stride, long long out_stride, long long out_side_stride, const VecCtx& ctx,
-                      cudaStream_t st) {
+                      cudaStream_t st, const cx<R>* xp = nullptr, double2* pq = nullptr) {
   if constexpr (sizeof(cx<R>) == 8) {
     return launch<k_plane_fwd<N, POST>>(dim3(N, nside, nvec), ((3 * N + 31) / 32) * 32, plane_smem<N>(), st, w, y, d,
                                             ctx, w_stride, out_stride, out_side_stride, side0);
   } else {
     using FS = FieldShape<R, N>;
-    return launch<k_field_fwd<R, N, POST>, POST ? 3 : 1>(dim3(N / FS::KP, 3 * nside, nvec), FS::TB, FS::SMEM, st, w,
-                                                             y, d, ctx, w_stride, out_stride, out_side_stride, side0);
+    const dim3 g(N / FS::KP, 3 * nside, nvec);
+    if constexpr (POST && std::is_same_v<R, double>)
+      if (pq)
+        return launch<k_field_fwd<R, N, kPiDot>, 3>(g, FS::TB, FS::SMEM, st, w, y, d, ctx, w_stride, out_stride,
+                                                    out_side_stride, side0, xp, pq);
+    return launch<k_field_fwd<R, N, POST ? kPi : kCopy>, POST ? 3 : 1>(g, FS::TB, FS::SMEM, st, w, y, d, ctx, w_stride,
+                                                                       out_stride, out_side_stride, side0, xp, pq);
   }
 }
 
@@ -889,11 +921,16 @@ cudaError_t col(const Plan& P, const PlanData<R>& d, const cx<R>* src, cx<R>* ds
 // the six-field intermediates of a sub-batch can stay in L2; the stencil
 // kernels run with tpb threads per block.  Both come from fame_autotune.
 //
-// pq (may be null): with the single-pass stencil, per-CTA partial sums of
-// Re(x^H B x) (sweep_partials_n per vector, vector-major).  The curl-SVD
-// transforms are unitary and Pi has orthonormal columns, so x^H B x equals
-// w^H [M J^H; J N] w for the spatial fields w the stencil reads; the stencil
-// pass accumulates it while it writes its output.
+// pq (may be null): per-CTA partial sums of Re(x^H B x), pq_partials_n per vector,
+// vector-major.  With the single-pass stencil: the curl-SVD transforms are
+// unitary and Pi has orthonormal columns, so x^H B x equals w^H [M J^H; J N] w for
+// the spatial fields w the stencil reads; the stencil pass accumulates it while
+// it writes its output.  With the two-kernel form of complex128: the last kernel
+// does, from x and the y it writes.
+template <class R, int N> int pq_partials_n(const Plan& P, const TuneEntry& tn, int nvec) {
+  if (tn.stencil_tpb == 0) return sweep_partials_n<R, N>(sweep_planes<R, N>(P, sub_batch(tn, nvec)));
+  return std::is_same_v<R, double> ? 6 * N / FieldShape<R, N>::KP : 0;
+}
 template <class R, int N>
 cudaError_t fncB_n(const Plan& P, const cx<R>* x, cx<R>* y, int nvec, const VecCtx& ctx, cx<R>* w0, cx<R>* w1,
                    cudaStream_t st, double2* pq) {
@@ -902,7 +939,7 @@ cudaError_t fncB_n(const Plan& P, const cx<R>* x, cx<R>* y, int nvec, const VecC
   const long long Nq = P.Nq;
   const TuneEntry tn = tune_for(P, tune_prec<R>(), nvec);
   const int chunk = sub_batch(tn, nvec);
-  const int tz = sweep_planes<R, N>(P, chunk);
+  const int tz = sweep_planes<R, N>(P, chunk), npq = pq_partials_n<R, N>(P, tn, nvec);
   for (int v0 = 0; v0 < nvec; v0 += chunk) {
     const int nv = std::min(chunk, nvec - v0);
     const VecCtx c = sub_ctx(ctx, v0);
@@ -913,10 +950,11 @@ cudaError_t fncB_n(const Plan& P, const cx<R>* x, cx<R>* y, int nvec, const VecC
     if (e != cudaSuccess) return e;
     e = col<R, N, +1, 0>(P, d, w0, w0, 6, nv, 6 * Nq, c, st);
     if (e != cudaSuccess) return e;
+    double2* pqs = pq ? pq + (size_t)v0 * npq : nullptr;
     // material stencil: single pass w0 -> w1, or the two-kernel form in place on w0
     cx<R>* wm = w0;
     if (tn.stencil_tpb == 0) {
-      e = sweep_n<R, N>(P, w0, w1, nv, c, st, tz, pq ? pq + (size_t)v0 * sweep_partials_n<R, N>(tz) : nullptr);
+      e = sweep_n<R, N>(P, w0, w1, nv, c, st, tz, pqs);
       wm = w1;
     } else {
       e = stencil_n<R, N>(P, w0, w0, w1, nv, c, st, tn.stencil_tpb, false);
@@ -924,7 +962,8 @@ cudaError_t fncB_n(const Plan& P, const cx<R>* x, cx<R>* y, int nvec, const VecC
     if (e != cudaSuccess) return e;
     e = col<R, N, -1, 0>(P, d, wm, wm, 6, nv, 6 * Nq, c, st);
     if (e != cudaSuccess) return e;
-    e = plane_fwd<R, N, true>(d, wm, ys, nv, 2, 0, 6 * Nq, 4 * Nq, 2 * Nq, c, st);
+    e = plane_fwd<R, N, true>(d, wm, ys, nv, 2, 0, 6 * Nq, 4 * Nq, 2 * Nq, c, st, xs,
+                              tn.stencil_tpb == 0 ? nullptr : pqs);
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;

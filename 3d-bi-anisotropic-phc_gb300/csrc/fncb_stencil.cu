@@ -205,9 +205,8 @@ cudaError_t launch_fncB_ds(const Plan& P, const double2* x, double2* y, int nvec
 template <class R>
 int fncB_pq_partials(const Plan& P, int nvec) {
   const TuneEntry tn = tune_for(P, tune_prec<R>(), nvec);
-  if (tn.stencil_tpb != 0) return 0;
   switch (P.n) {
-#define FAME_CASE(NN) case NN: return sweep_partials_n<R, NN>(sweep_planes<R, NN>(P, sub_batch(tn, nvec)));
+#define FAME_CASE(NN) case NN: return pq_partials_n<R, NN>(P, tn, nvec);
     FAME_FOR_EACH_N(FAME_CASE)
 #undef FAME_CASE
     default: return 0;

@@ -93,7 +93,7 @@ int pcg_batched(Plan& P, const cx<R>* b, cx<R>* x, int nvec, const int* d_inst, 
   CgScalars S;
   S.carve(s, nvec);
   const int nblk = dot_blocks(P, L, nvec);
-  // p^H B p from the stencil pass of fncB where its tuned form provides it
+  // p^H B p from the passes of fncB where its form provides it
   const int nblk_pq = fncB_pq_partials<R>(P, nvec);
   const int nblkv0 = dot_blocks(P, P.Nq, nvec, sizeof(R) == 4 ? 2 : 1, 512);
   const int npart = std::max(std::max(nblk, nblk_pq), nblkv0);
