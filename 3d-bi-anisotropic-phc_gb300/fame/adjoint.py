@@ -65,19 +65,23 @@ def gradient(plan, evs, omega, weights, cluster_tol=1e-8):
 
     def flush():
         if group:
-            ev = torch.cat([e.reshape(-1, 4 * plan.Nq) for _, e, _, _ in group]) if len(group) > 1 else group[0][1]
-            inst = np.concatenate([np.full(len(w), k, dtype=np.int32) for k, _, _, w in group])
-            plan.eig_gradient(ev, np.concatenate([o for _, _, o, _ in group]),
-                              np.concatenate([w for _, _, _, w in group]), inst=inst, out=(g_e, g_g), accumulate=True)
+            ev = torch.cat([g[1] for g in group]) if len(group) > 1 else group[0][1]
+            inst, om, w = (np.concatenate([g[i] for g in group]) for i in (0, 2, 3))
+            plan.eig_gradient(ev, om, w, inst=inst, out=(g_e, g_g), accumulate=True)
             group.clear()
 
     for k, ev in enumerate(evs):
         w = cluster_weights(omega[k], weights[k], cluster_tol)
         if not np.any(w):
             continue
-        if group and sum(len(q[3]) for q in group) + len(w) > GROUP_VECTORS:
+        ev = ev.reshape(-1, 4 * plan.Nq)
+        if ev.dtype != torch.complex128:  # joining them would convert it
+            raise TypeError("eigenvectors must be complex128")
+        nvec = ev.shape[0]
+        om, w = (np.broadcast_to(np.asarray(q, dtype=np.float64), (nvec,)) for q in (omega[k], w))
+        if group and sum(len(g[0]) for g in group) + nvec > GROUP_VECTORS:
             flush()
-        group.append((k, ev, np.asarray(omega[k], dtype=np.float64), w))
+        group.append((np.full(nvec, k, dtype=np.int32), ev, om, w))
     flush()
     return g_e, g_g
 
