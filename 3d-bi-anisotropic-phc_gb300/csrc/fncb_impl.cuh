@@ -794,9 +794,12 @@ k_col(const float2* src, float2* dst, PlanData<float> d, VecCtx ctx, long long s
 // One CTA per (W columns, field, vector), W*G threads: pass A straight from
 // global, pass B straight to global.  With W = 32 a warp holds one k1 of 32
 // columns (no idle lanes: whole rows of 40 columns took 52 us where this takes
-// 44, 4 vectors at n = 40).  (One thread per 60-point column needs 255
+// 44, 4 vectors at n = 40); an even split takes 16, two k1 to a warp, as smaller
+// CTAs leave the SMs more evenly loaded (615 of 32 columns for five transforms at
+// n = 36 put 5 on some SMs and 4 on the others: 89 us, 83 with 16; fncB of one
+// vector at n = 32 81 -> 78, at n = 50 313 -> 305).  (One thread per 60-point column needs 255
 // registers and spills; at n = 16 it is a serial chain of 170 FP64 operations.)
-template <int N> FAME_HD constexpr int col_width() { return N <= 16 ? 16 : 32; }
+template <int N> FAME_HD constexpr int col_width() { return N <= 16 || field_split(N) % 2 == 0 ? 16 : 32; }
 
 template <class R, int N, int DIR, int SMODE>
 __global__ void __launch_bounds__(((col_width<N>() * field_split(N) + 31) / 32) * 32)
