@@ -25,6 +25,9 @@ __device__ __forceinline__ double2 dmk(double a, double b) { return make_double2
 // diagonal entries packed in two).
 constexpr int kPcSlots = 8;
 
+// FP64-rate-bound, once per plan: some 670 operations per voxel, with the
+// Hermitian halves computed once and L D L^H in place of a Gauss-Jordan of the
+// full block and its identity (8 instances at n = 48 2.3 -> 1.0 ms).
 __global__ void __launch_bounds__(128)
 k_precond_build64(const double2* __restrict__ lam_all, const double2* __restrict__ avg_all, int n, double2* pc64,
                   float2* pc32) {
@@ -35,93 +38,136 @@ k_precond_build64(const double2* __restrict__ lam_all, const double2* __restrict
   const int i1 = int(idx % n), i2 = int((idx / n) % n), i3 = int(idx / ((long long)n * n));
   const double2* lam = lam_all + (long long)inst * 3 * n;
   const double2 L[3] = {lam[i1], lam[n + i2], lam[2 * n + i3]};
-  double2 c[3];
-  for (int d = 0; d < 3; ++d) c[d] = dmk(2.0 + L[d].x / n, L[d].y / n);
+  // cv_i = c_i / 2, cu_i = c_a c_b / 4 of the two other axes
+  double2 cv[3], cu[3];
+  const double rn = 0.5 / n;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) cv[d] = dmk(rfma(L[d].x, rn, 1.0), L[d].y * rn);
+#pragma unroll
+  for (int d = 0; d < 3; ++d) cu[d] = cmul(cv[d == 0 ? 1 : 0], cv[d == 2 ? 1 : 2]);
   const double2* T = avg_all + (long long)inst * 27;
   const double2* Nh = T;
   const double2* Mh = T + 9;
   const double2* J = T + 18;
-  double2 Guu[3][3], Gvv[3][3], Gvu[3][3];
-  auto ax = [](int i, int s) { return i == 0 ? (s == 0 ? 1 : 2) : i == 1 ? (s == 0 ? 0 : 2) : (s == 0 ? 0 : 1); };
-  for (int i = 0; i < 3; ++i)
-    for (int j = 0; j < 3; ++j) {
-      const double2 ci = cmul(c[ax(i, 0)], c[ax(i, 1)]);
-      const double2 cj = cmul(c[ax(j, 0)], c[ax(j, 1)]);
-      if (i == j) {
-        Guu[i][j] = dmk(Mh[i * 3 + i].x, 0.0);
-        Gvv[i][j] = dmk(Nh[i * 3 + i].x, 0.0);
-      } else {
-        Guu[i][j] = cscale(cmul(cmul(ci, Mh[i * 3 + j]), cconj(cj)), 1.0 / 16.0);
-        Gvv[i][j] = cscale(cmul(cmul(c[i], Nh[i * 3 + j]), cconj(c[j])), 0.25);
-      }
-      Gvu[i][j] = cscale(cmul(cmul(c[i], J[i * 3 + j]), cconj(cj)), 0.125);
-    }
-  detail::PiBlock<double> P = detail::pi_block<double>(L[0], L[1], L[2]);
   // columns of Pi: u-side e0 = -conj(Pi2), e1 = conj(Pi1); v-side f0 = Pi1, f1 = Pi2
-  double2 col[4][3];
+  const detail::PiBlock<double> P = detail::pi_block<double>(L[0], L[1], L[2]);
+  double2 e[2][3];
+#pragma unroll
   for (int r = 0; r < 3; ++r) {
-    col[0][r] = cneg(cconj(P.p2[r]));
-    col[1][r] = cconj(P.p1[r]);
-    col[2][r] = P.p1[r];
-    col[3][r] = P.p2[r];
+    e[0][r] = cneg(cconj(P.p2[r]));
+    e[1][r] = cconj(P.p1[r]);
   }
-  // B0[a][b] = col_a^H G col_b
-  double2 B[4][4];
-  for (int a = 0; a < 4; ++a)
-    for (int b = 0; b < 4; ++b) {
-      double2 s = dmk(0.0, 0.0);
-      for (int r = 0; r < 3; ++r) {
-        double2 g = dmk(0.0, 0.0);
-        for (int q = 0; q < 3; ++q) {
-          double2 Gr;
-          if (a < 2 && b < 2) Gr = Guu[r][q];
-          else if (a >= 2 && b >= 2) Gr = Gvv[r][q];
-          else if (a >= 2) Gr = Gvu[r][q];   // v row, u column
-          else Gr = cconj(Gvu[q][r]);        // u row, v column: Guv = Gvu^H
-          g = cfma(Gr, col[b][q], g);
-        }
-        s = cfmac(col[a][r], g, s);
-      }
-      B[a][b] = s;
-    }
-  // Gauss-Jordan inverse of the Hermitian positive definite block
-  double2 Minv[4][4];
-  for (int a = 0; a < 4; ++a)
-    for (int b = 0; b < 4; ++b) Minv[a][b] = dmk(a == b ? 1.0 : 0.0, 0.0);
-  bool ok = true;
-  for (int p = 0; p < 4; ++p) {
-    const double piv = B[p][p].x;
-    if (!(piv > 0.0)) {
-      ok = false;
-      break;
-    }
-    const double2 inv = dmk(1.0 / piv, 0.0);
-    for (int b = 0; b < 4; ++b) {
-      B[p][b] = cmul(B[p][b], inv);
-      Minv[p][b] = cmul(Minv[p][b], inv);
-    }
-    for (int a = 0; a < 4; ++a) {
-      if (a == p) continue;
-      const double2 f = B[a][p];
-      for (int b = 0; b < 4; ++b) {
-        B[a][b] = csub(B[a][b], cmul(f, B[p][b]));
-        Minv[a][b] = csub(Minv[a][b], cmul(f, Minv[p][b]));
+  const double2* f[2] = {P.p1, P.p2};
+  // G[r][q] of a Hermitian symbol with scales s: s_r t_rq conj(s_q), real diagonal t_rr
+  auto symbol = [](const double2* t, const double2* s, double2 (&G)[3][3]) {
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+      G[r][r] = dmk(t[4 * r].x, 0.0);
+#pragma unroll
+      for (int q = r + 1; q < 3; ++q) {
+        G[r][q] = cmulc(s[q], cmul(s[r], t[3 * r + q]));
+        G[q][r] = cconj(G[r][q]);
       }
     }
+  };
+  auto row = [](const double2 (&g)[3], const double2* v, int real) {  // sum_q g_q v_q; g[real] is real
+    double2 w = dmk(0.0, 0.0);
+#pragma unroll
+    for (int q = 0; q < 3; ++q) w = q == real ? caxpy(g[q].x, v[q], w) : cfma(g[q], v[q], w);
+    return w;
+  };
+  auto dot = [](const double2* a, const double2 (&g)[3]) {
+    return cfmac(a[2], g[2], cfmac(a[1], g[1], cmulc(a[0], g[0])));
+  };
+  auto dotr = [](const double2* a, const double2 (&g)[3]) {
+    double w = 0.0;
+#pragma unroll
+    for (int r = 0; r < 3; ++r) w = rfma(a[r].x, g[r].x, rfma(a[r].y, g[r].y, w));
+    return w;
+  };
+  // lower triangle of B0 in the order e0, e1, f0, f1
+  double b00, b11, b22, b33;
+  double2 b10, b32, bvu[2][2];
+  double2 g0[3], g1[3], G[3][3];
+  symbol(Mh, cu, G);
+#pragma unroll
+  for (int r = 0; r < 3; ++r) {
+    g0[r] = row(G[r], e[0], r);
+    g1[r] = row(G[r], e[1], r);
   }
-  if (!ok)  // not positive definite (non-physical material): identity
-    for (int a = 0; a < 4; ++a)
-      for (int b = 0; b < 4; ++b) Minv[a][b] = dmk(a == b ? 1.0 : 0.0, 0.0);
+  b00 = dotr(e[0], g0);
+  b10 = dot(e[1], g0);
+  b11 = dotr(e[1], g1);
+  symbol(Nh, cv, G);
+#pragma unroll
+  for (int r = 0; r < 3; ++r) {
+    g0[r] = row(G[r], f[0], r);
+    g1[r] = row(G[r], f[1], r);
+  }
+  b22 = dotr(f[0], g0);
+  b32 = dot(f[1], g0);
+  b33 = dotr(f[1], g1);
+#pragma unroll
+  for (int r = 0; r < 3; ++r) {
+#pragma unroll
+    for (int q = 0; q < 3; ++q) G[r][q] = cmulc(cu[q], cmul(cv[r], J[3 * r + q]));
+    g0[r] = row(G[r], e[0], -1);
+    g1[r] = row(G[r], e[1], -1);
+  }
+#pragma unroll
+  for (int a = 0; a < 2; ++a) {
+    bvu[a][0] = dot(f[a], g0);
+    bvu[a][1] = dot(f[a], g1);
+  }
+  double2 b20 = bvu[0][0], b21 = bvu[0][1], b30 = bvu[1][0], b31 = bvu[1][1];
+  // B0 = L D L^H: a -= l conj(b) with l = b'/d
+  auto sub = [](double2 l, double2 b, double2 a) { return cfmac(b, cneg(l), a); };
+  auto subr = [](double2 l, double2 b, double a) { return rfma(-l.x, b.x, rfma(-l.y, b.y, a)); };
+  const double r0 = 1.0 / b00;
+  const double2 l10 = cscale(b10, r0), l20 = cscale(b20, r0), l30 = cscale(b30, r0);
+  b11 = subr(l10, b10, b11);
+  b21 = sub(l20, b10, b21);
+  b31 = sub(l30, b10, b31);
+  b22 = subr(l20, b20, b22);
+  b32 = sub(l30, b20, b32);
+  b33 = subr(l30, b30, b33);
+  const double r1 = 1.0 / b11;
+  const double2 l21 = cscale(b21, r1), l31 = cscale(b31, r1);
+  b22 = subr(l21, b21, b22);
+  b32 = sub(l31, b21, b32);
+  b33 = subr(l31, b31, b33);
+  const double r2 = 1.0 / b22;
+  const double2 l32 = cscale(b32, r2);
+  b33 = subr(l32, b32, b33);
+  const double r3 = 1.0 / b33;
+  // X = L^{-1}, M = X^H D^{-1} X
+  const double2 x10 = cneg(l10), x21 = cneg(l21), x32 = cneg(l32);
+  const double2 x20 = cneg(cfma(l21, x10, l20));
+  const double2 x31 = cneg(cfma(l32, x21, l31));
+  const double2 x30 = cneg(cfma(l32, x20, cfma(l31, x10, l30)));
+  const double2 w30 = cscale(x30, r3), w31 = cscale(x31, r3), w32 = cscale(x32, r3);
+  const double2 w20 = cscale(x20, r2), w21 = cscale(x21, r2), w10 = cscale(x10, r1);
+  auto add = [](double2 w, double2 x, double a) { return rfma(w.x, x.x, rfma(w.y, x.y, a)); };
+  double m00 = add(w30, x30, add(w20, x20, add(w10, x10, r0)));
+  double m11 = add(w31, x31, add(w21, x21, r1));
+  double m22 = add(w32, x32, r2);
+  double m33 = r3;
+  double2 m01 = cfmac(w30, x31, cfmac(w20, x21, cconj(w10)));
+  double2 m02 = cfmac(w30, x32, cconj(w20));
+  double2 m03 = cconj(w30);
+  double2 m12 = cfmac(w31, x32, cconj(w21));
+  double2 m13 = cconj(w31), m23 = cconj(w32);
+  if (!(b00 > 0.0 && b11 > 0.0 && b22 > 0.0 && b33 > 0.0)) {  // not positive definite (non-physical material): identity
+    m00 = m11 = m22 = m33 = 1.0;
+    m01 = m02 = m03 = m12 = m13 = m23 = dmk(0.0, 0.0);
+  }
   // packed: (m00, m11) | (m22, m33) | m01 | m02 | m03 | m12 | m13 | m23
-  double2 v[kPcSlots];
-  v[0] = dmk(Minv[0][0].x, Minv[1][1].x);
-  v[1] = dmk(Minv[2][2].x, Minv[3][3].x);
-  const int ent[6][2] = {{0, 1}, {0, 2}, {0, 3}, {1, 2}, {1, 3}, {2, 3}};
-  for (int e = 0; e < 6; ++e) v[2 + e] = Minv[ent[e][0]][ent[e][1]];
-  for (int e = 0; e < kPcSlots; ++e) {
-    const long long o = ((long long)inst * kPcSlots + e) * Nq + idx;
-    if (pc64) pc64[o] = v[e];
-    if (pc32) pc32[o] = make_float2(float(v[e].x), float(v[e].y));
+  const double2 v[kPcSlots] = {dmk(m00, m11), dmk(m22, m33), m01, m02, m03, m12, m13, m23};
+#pragma unroll
+  for (int k = 0; k < kPcSlots; ++k) {
+    const long long o = ((long long)inst * kPcSlots + k) * Nq + idx;
+    if (pc64) pc64[o] = v[k];
+    if (pc32) pc32[o] = make_float2(float(v[k].x), float(v[k].y));
   }
 }
 

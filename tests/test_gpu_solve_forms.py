@@ -79,3 +79,21 @@ def test_gradient_in_groups(cuda, fame_lib):
         assert float(torch.linalg.norm(a - b) / torch.linalg.norm(b)) < 1e-12
     with pytest.raises(TypeError):
         fame.adjoint.gradient(plan, [ev[0], ev[1].to(torch.complex64), ev[2]], om, w)
+
+
+@pytest.mark.parametrize("n", [4, 6, 24])
+def test_preconditioner_inverts_a_homogeneous_medium(cuda, fame_lib, n):
+    """One general Hermitian medium everywhere: fncB is then the 4x4 blocks that
+    the preconditioner inverts, and the first iteration solves the system but
+    for rounding (some hundred units of it, 1e-13; the bound is 1e-11)."""
+    rng = np.random.default_rng(2)
+    t = np.zeros((2, 1, 27), dtype=np.complex128)
+    for k in range(2):
+        for b in range(2):
+            m = rng.standard_normal((3, 3)) + 1j * rng.standard_normal((3, 3))
+            t[k, 0, 9 * b:9 * b + 9] = (0.1 * (m + m.conj().T) + (2.0 + b) * np.eye(3)).ravel()
+        t[k, 0, 18:] = 0.1 * (rng.standard_normal(9) + 1j * rng.standard_normal(9))
+    plan = fame.Plan(n, rng.uniform(0.3, 2.5, size=(2, 3)), np.zeros(n ** 3, np.uint8), t)
+    b = torch.randn(2, 4 * n ** 3, dtype=torch.complex128, device="cuda")
+    _, its, rr = plan.apply_Binv(b, tol=1e-11, maxit=50)
+    assert np.all(np.asarray(its) == 1) and np.all(np.asarray(rr) < 1e-11)
