@@ -78,7 +78,8 @@ def gradient(plan, evs, omega, weights, cluster_tol=1e-8):
         if ev.dtype != torch.complex128:  # joining them would convert it
             raise TypeError("eigenvectors must be complex128")
         nvec = ev.shape[0]
-        om, w = (np.broadcast_to(np.asarray(q, dtype=np.float64), (nvec,)) for q in (omega[k], w))
+        om, w = (q if q.shape == (nvec,) else np.broadcast_to(q, (nvec,))
+                 for q in (np.asarray(omega[k], dtype=np.float64), w))
         if group and sum(len(g[0]) for g in group) + nvec > GROUP_VECTORS:
             flush()
         group.append((np.full(nvec, k, dtype=np.int32), ev, om, w))
