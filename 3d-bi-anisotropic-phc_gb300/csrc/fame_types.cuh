@@ -83,6 +83,47 @@ struct ff {
   friend FAME_HD ff rsqrt(ff a) { return ff(1.0 / ::sqrt(static_cast<double>(a))); }
 };
 
+// ff(double) and double(ff) by bit operations: the same results, where the
+// plain forms take 4 and 3 operations of the FP64 pipe (64 times rarer than FP32
+// ones; loading and storing complex128 vectors kept it busy for a third of the
+// time of the double-single plane kernels).  Both return false, and leave the
+// plain form to the caller, outside the range of exponents that the bits cover.
+FAME_HD uint32_t f32_bits(float f) {
+  union { float f; uint32_t u; } c;
+  c.f = f;
+  return c.u;
+}
+FAME_HD float bits_f32(uint32_t u) {
+  union { float f; uint32_t u; } c;
+  c.u = u;
+  return c.f;
+}
+// d as its upper and lower 32 bits
+FAME_HD bool ff_split_bits(uint32_t dh, uint32_t dl, ff& v) {
+  const uint32_t sign = dh & 0x80000000u, mag = dh ^ sign, e = mag >> 20;  // biased exponent
+  // hi = d rounded to 24 bits, the remainder r units of 2^(e - 1023 - 52)
+  uint32_t h = ((mag - (896u << 20)) << 3) | (dl >> 29);
+  uint32_t r = dl & 0x1fffffffu;
+  const bool up = r + (h & 1u) > 0x10000000u;  // to nearest, ties to even
+  h += up ? 1u : 0u;
+  r = up ? 0x20000000u - r : r;
+  // r < 2^29 in two exact parts, rounded once
+  const float rf = fmaf(bits_f32(0x4b000000u | (r >> 6)) - 8388608.0f, 64.0f,
+                        bits_f32(0x4b000000u | (r & 63u)) - 8388608.0f);
+  const float unit = bits_f32((((e - (1023 + 52 - 127)) << 23) | sign) ^ (up ? 0x80000000u : 0u));
+  const bool zero = (mag | dl) == 0u;
+  v.hi = bits_f32(zero ? sign : h | sign);
+  v.lo = zero ? 0.0f : rf * unit;
+  return zero || (e >= 1023 - 74 && e < 1023 + 127);
+}
+// f as the upper and lower 32 bits of a double
+FAME_HD bool f32_widen_bits(float f, uint32_t& dh, uint32_t& dl) {
+  const uint32_t u = f32_bits(f), mag = u & 0x7fffffffu;
+  dh = (u & 0x80000000u) | (mag ? (mag >> 3) + (896u << 20) : 0u);
+  dl = u << 29;
+  return mag == 0u || (mag >= 0x00800000u && mag < 0x7f800000u);
+}
+
 struct cff {
   ff x, y;
 };

@@ -226,14 +226,18 @@ template <int N> __device__ __forceinline__ PiRow* pi_rows(float2* sm) {
 
 // Operator input / output of the field kernels.  The double-single
 // operator reads and writes complex128 vectors (the caller's), converting
-// on load and store, so it needs no conversion passes; the conversions run
-// on the FP64 pipe, which its float-float arithmetic leaves idle.
+// on load and store, so it needs no conversion passes; by bit operations, as
+// an FP64 or conversion instruction takes as long as 64 FP32 ones.
 template <class R> __device__ __forceinline__ cx<R> load_io(const cx<R>* p) {
   if constexpr (std::is_same<R, ff>::value) {
     const double2 v = *reinterpret_cast<const double2*>(p);
     cff c;
-    c.x = ff(v.x);
-    c.y = ff(v.y);
+    const bool ok = ff_split_bits(__double2hiint(v.x), __double2loint(v.x), c.x) &
+                    ff_split_bits(__double2hiint(v.y), __double2loint(v.y), c.y);
+    if (__any_sync(__activemask(), !ok)) {  // a branch of the whole warp, so that the FP64 form costs nothing elsewhere
+      c.x = ff(v.x);
+      c.y = ff(v.y);
+    }
     return c;
   } else {
     return *p;
@@ -241,7 +245,13 @@ template <class R> __device__ __forceinline__ cx<R> load_io(const cx<R>* p) {
 }
 template <class R> __device__ __forceinline__ void store_io(cx<R>* p, cx<R> v) {
   if constexpr (std::is_same<R, ff>::value) {
-    *reinterpret_cast<double2*>(p) = make_double2(double(v.x), double(v.y));
+    uint32_t h[4], l[4];
+    const bool ok = f32_widen_bits(v.x.hi, h[0], l[0]) & f32_widen_bits(v.x.lo, h[1], l[1]) &
+                    f32_widen_bits(v.y.hi, h[2], l[2]) & f32_widen_bits(v.y.lo, h[3], l[3]);
+    double2 o = make_double2(__hiloint2double(h[0], l[0]) + __hiloint2double(h[1], l[1]),
+                             __hiloint2double(h[2], l[2]) + __hiloint2double(h[3], l[3]));
+    if (__any_sync(__activemask(), !ok)) o = make_double2(double(v.x), double(v.y));
+    *reinterpret_cast<double2*>(p) = o;
   } else {
     *p = v;
   }
