@@ -535,6 +535,11 @@ template <class R, int N> struct FieldShape {
   static constexpr int NP = KP * N;                // pencils per axis
   static constexpr int T = NP * G;                 // threads of the DFT passes
   static constexpr int TB = ((T + 31) / 32) * 32 < 64 ? 64 : ((T + 31) / 32) * 32;
+  // Double-single waits on latencies at two CTAs per SM (n = 60: 128 registers, 36 %
+  // issue): up to 24 warps of 80 registers, without spills at the two elements
+  // in flight of k_field_inv (ten vectors at n = 60 844 -> 762 us there, one vector's
+  // fncB 372 -> 272 as its 360 CTAs then fit at once).  The FP64 rate bounds double.
+  static constexpr int CTAS = !std::is_same_v<R, ff> ? 0 : 24 / (TB / 32) > 0 ? 24 / (TB / 32) : 1;
   static constexpr int LD = N + 1;
   static constexpr size_t SMEM = sizeof(cx<R>) * KP * N * LD;
   static_assert(N % KP == 0, "whole CTAs of planes");
@@ -562,7 +567,7 @@ template <class R, int N, int S> __device__ __forceinline__ void field_rows(cx<R
 
 // grid: (n / KP, 3 * sides, vectors); blockIdx.y = 3 * (side - side0) + field
 template <class R, int N, bool PREP>
-__global__ void __launch_bounds__(FieldShape<R, N>::TB)
+__global__ void __launch_bounds__(FieldShape<R, N>::TB, FieldShape<R, N>::CTAS)
 k_field_inv(const cx<R>* __restrict__ x, cx<R>* __restrict__ out, PlanData<R> d, VecCtx ctx, long long in_stride,
             long long in_side_stride, long long out_stride, int side0) {
   using FS = FieldShape<R, N>;
@@ -581,7 +586,7 @@ k_field_inv(const cx<R>* __restrict__ x, cx<R>* __restrict__ out, PlanData<R> d,
   const cx<R>* xin = x + vec * in_stride + (blockIdx.y / 3) * in_side_stride + k3 * NN;
   // the loads of U elements issued together
   constexpr int ITEMS = (KP * NN + TB - 1) / TB;
-  constexpr int U = ITEMS < 4 ? ITEMS : 4;
+  constexpr int UMAX = std::is_same_v<R, ff> ? 2 : 4, U = ITEMS < UMAX ? ITEMS : UMAX;
   for (int b = 0; b < ITEMS; b += U) {
     cx<R> in[U][2];
     PiComp<R> P[U];
@@ -638,7 +643,7 @@ k_field_inv(const cx<R>* __restrict__ x, cx<R>* __restrict__ out, PlanData<R> d,
 // pass over p and q less (c128, two vectors at n = 30: a launch of 5.3 us).
 enum { kCopy = 0, kPi = 1, kPiDot = 2 };
 template <class R, int N, int POST>
-__global__ void __launch_bounds__(FieldShape<R, N>::TB)
+__global__ void __launch_bounds__(FieldShape<R, N>::TB, FieldShape<R, N>::CTAS)
 k_field_fwd(const cx<R>* __restrict__ w, cx<R>* __restrict__ y, PlanData<R> d, VecCtx ctx, long long w_stride,
             long long out_stride, long long out_side_stride, int side0, const cx<R>* __restrict__ xp,
             double2* __restrict__ pq) {
