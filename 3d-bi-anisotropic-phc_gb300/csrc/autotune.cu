@@ -27,6 +27,16 @@ TuneEntry tune_for(const Plan& P, int prec, int nvec) {
   // the SMs (two vectors at n = 30, complex128: 143 us with blocks of 256,
   // 136 with 128)
   d.stencil_tpb = prec == FAME_C64 ? 0 : 128;
+  // complex64 in two halves where the six-field buffers of the batch are beyond
+  // 1.5 times the L2 and those of a half fit in it: its launches stay wide, and the
+  // z passes and the stencil find their input in L2 (ten vectors at n = 60 192 -> 179 us,
+  // twelve 244 -> 225, 34 at n = 40 213 -> 198, 80 at n = 30 200 -> 186, 150 at n = 24 187 ->
+  // 170).  Between 1 and 1.5 times the L2 the halves lose as often as they win (15 at
+  // n = 50 180 -> 194, 18 at n = 48 177 -> 175), halves that hardly fit gain little or
+  // lose (nine at n = 64 223 -> 227), and thirds lose.
+  const long long bytes = 12LL * P.Nq * (long long)sizeof(float2);  // both buffers of a vector
+  const int half = (nvec + 1) / 2;
+  if (prec == FAME_C64 && 2 * bytes * nvec > 3LL * P.l2 && bytes * half <= P.l2) d.untuned = half;
   return d;
 }
 
@@ -35,7 +45,7 @@ TuneEntry tune_for(const Plan& P, int prec, int nvec) {
 static void put_tune(Plan& P, const TuneEntry& t) {
   for (TuneEntry& u : P.tune)
     if (u.prec == t.prec && u.nvec == t.nvec) {
-      if (u.chunk != t.chunk || u.stencil_tpb != t.stencil_tpb || u.lanes != t.lanes) free_graphs(P);
+      if (u.chunk != t.chunk || u.untuned != t.untuned || u.stencil_tpb != t.stencil_tpb || u.lanes != t.lanes) free_graphs(P);
       u = t;
       return;
     }
@@ -160,6 +170,7 @@ int fame_set_tune(fame_plan_t h, int prec, int nvec, int chunk, int stencil_tpb)
     return fail(&P, FAME_ERR_BAD_ARG, "fame_set_tune: bad argument");
   TuneEntry t = tune_for(P, prec, nvec);  // keeps the width's split
   t.chunk = chunk >= nvec ? 0 : chunk;
+  t.untuned = 0;
   t.stencil_tpb = stencil_tpb;
   put_tune(P, t);
   return FAME_OK;

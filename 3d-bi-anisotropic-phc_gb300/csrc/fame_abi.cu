@@ -355,6 +355,7 @@ int fame_plan_create(fame_plan_t* out, int n, int nk, const double* theta, const
   }
   cudaError_t e = cudaGetDevice(&P.device);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&P.sms, cudaDevAttrMultiProcessorCount, P.device);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&P.l2, cudaDevAttrL2CacheSize, P.device);
   if (e == cudaSuccess) e = cudaMalloc(&P.d_phase, P.Nq);
   if (e == cudaSuccess) e = cudaMemcpy(P.d_phase, phase, P.Nq, cudaMemcpyHostToDevice);
   if (e != cudaSuccess) {

@@ -81,7 +81,8 @@ FAME_HD constexpr int field_split(int n) {
 // stencil's form (single pass, or threads per block of the two-kernel form).
 struct TuneEntry {
   int prec = 0, nvec = 0;
-  int chunk = 0;         // 0: whole batch
+  int chunk = 0;         // 0: whole batch, but for untuned batches see untuned
+  int untuned = 0;       // vectors per sequence where nothing was installed (0: whole batch)
   int stencil_tpb = 0;   // 0: single-pass k_sweep; 128/256/512: two-kernel form
   int lanes = -1;        // kept for its callers (fame_set_tune_lanes); the kernels take one split per size
   double us = 0.0;       // measured time of one fncB on the batch
@@ -124,6 +125,7 @@ struct Plan {
   int nphase = 0;
   int device = 0;
   int sms = 152;     // SMs of that device
+  int l2 = 0;        // bytes of its L2
   cudaStream_t stream = nullptr;
   // options (fame_set_option)
   int opt_precond = 1;                // CG on B preconditioned by the averaged-medium B0^{-1}
@@ -182,7 +184,10 @@ struct Plan {
 };
 
 // Vectors per launch sequence of a batch of nvec.
-inline int sub_batch(const TuneEntry& t, int nvec) { return t.chunk > 0 && t.chunk < nvec ? t.chunk : nvec; }
+inline int sub_batch(const TuneEntry& t, int nvec) {
+  const int c = t.chunk > 0 ? t.chunk : t.untuned;
+  return c > 0 && c < nvec ? c : nvec;
+}
 // Tuned launch parameters for (prec, nvec), or the defaults.
 TuneEntry tune_for(const Plan& P, int prec, int nvec);
 // The tuning key of an arithmetic type (FAME_C64, FAME_C128, FAME_C128_DS).

@@ -258,7 +258,7 @@ k_pcg_start(const cx<R>* __restrict__ b, cx<R>* __restrict__ x, cx<R>* __restric
 // partial sums (x += a p is left to k_cg_dir, which reads p anyway).  HBM-bound
 // on large batches, latency-bound on small ones, so that
 //   * a CTA takes one contiguous chunk, and the CTAs of a launch are whole
-//     multiples of what fits the SMs (update_blocks);
+//     multiples of what fits the SMs (dot_blocks);
 //   * the loads of the first elements are issued before the step length, which
 //     every CTA reduces from the stencil pass's partials, is waited for;
 //   * complex64 moves two voxels per 16-byte access.

@@ -97,3 +97,15 @@ def test_preconditioner_inverts_a_homogeneous_medium(cuda, fame_lib, n):
     b = torch.randn(2, 4 * n ** 3, dtype=torch.complex128, device="cuda")
     _, its, rr = plan.apply_Binv(b, tol=1e-11, maxit=50)
     assert np.all(np.asarray(its) == 1) and np.all(np.asarray(rr) < 1e-11)
+
+
+@pytest.mark.parametrize("n,nvec", [(24, 161), (60, 10)])
+def test_halves_of_a_large_batch(cuda, fame_lib, n, nvec):
+    """A complex64 batch far beyond the L2 runs as two halves unless something is
+    installed for its width: the same result to the last bit."""
+    plan = plan_of(n, 1, seed=3)
+    x = torch.randn(nvec, 4 * n ** 3, dtype=torch.complex64, device="cuda")
+    inst = np.zeros(nvec, dtype=np.int32)
+    y = plan.apply_B(x, inst)
+    plan.set_tune("c64", nvec, 0, 0)
+    assert torch.equal(plan.apply_B(x, inst), y)
