@@ -162,7 +162,8 @@ int fame_refine_residuals(fame_plan_t plan, double* before, int n);
  * calls with that width.  Outputs (may be NULL): the chosen chunk (0 = whole
  * batch), stencil setting and the measured microseconds of one fncB.
  * fame_set_tune installs a chunk and stencil setting directly (e.g. from a
- * cache).  fame_set_tune_lanes records a count of threads per FFT pencil
+ * cache).  With nothing installed for a width, a complex64 batch whose
+ * intermediates exceed 1.5 times the L2 runs as two halves.  fame_set_tune_lanes records a count of threads per FFT pencil
  * (-1 = default) that fame_get_tune returns; every size and precision has one
  * compiled split, so it has no other effect.
  */
