@@ -13,8 +13,6 @@ cudaError_t dot_batched(const cx<R>* a, long long a_vstride, long long a_cstride
 template <class R>
 cudaError_t axpby_batched(const cx<R>* x, cx<R>* y, long long len, long long stride, int nvec,
                           const double2* alpha, const double2* beta, const int* active, cudaStream_t st);
-// out[row] = sum of partial[row][0..nblk)
-cudaError_t dot_final(const double2* partial, int nblk, int nrows, double2* out, cudaStream_t st);
 // Condition kernel of a graph-resident loop (graph_replay_while): *passes
 // += 1, and the loop goes on while any active[v] and *passes < max_passes.
 cudaError_t while_active(const int* active, int nvec, int* passes, int max_passes, cudaGraphConditionalHandle h,

@@ -545,10 +545,6 @@ cudaError_t axpby_batched(const cx<R>* x, cx<R>* y, long long len, long long str
   return cudaGetLastError();
 }
 
-cudaError_t dot_final(const double2* partial, int nblk, int nrows, double2* out, cudaStream_t st) {
-  return launch<k_dot_final>(dim3(nrows), 32, 0, st, partial, nblk, out);
-}
-
 template <class R>
 cudaError_t dot_partial(const cx<R>* a, const cx<R>* b, long long len, long long stride, int nvec, double2* partial,
                         int nblk, const int* active, cudaStream_t st) {
