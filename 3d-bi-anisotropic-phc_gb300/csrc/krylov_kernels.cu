@@ -196,7 +196,9 @@ k_cg_init(const double2* __restrict__ partial, int nblk, const double* __restric
 // of x in k_pcg_update (p is read once less: the two kernels 60 -> 53 us) and
 // the one of p inside fncB's first plane kernel, which ran it at half the
 // bandwidth.
-template <class R>
+// p and z are workspaces, x may be the caller's: with XALIGNED false (complex64
+// at an odd element of a larger array) its elements are accessed one by one.
+template <class R, bool XALIGNED>
 __global__ void __launch_bounds__(kRedThreads)
 k_cg_dir(cx<R>* __restrict__ x, cx<R>* __restrict__ p, const cx<R>* __restrict__ z, long long len,
          const double2* __restrict__ partial, int nblk, const double* __restrict__ alpha,
@@ -214,7 +216,7 @@ k_cg_dir(cx<R>* __restrict__ x, cx<R>* __restrict__ p, const cx<R>* __restrict__
   struct alignas(16) Pack {
     cx<R> e[U];
   };
-  Pack* xp = reinterpret_cast<Pack*>(x + (long long)v * len);
+  cx<R>* xv = x + (long long)v * len;
   Pack* pp = reinterpret_cast<Pack*>(p + (long long)v * len);
   const Pack* zp = reinterpret_cast<const Pack*>(z + (long long)v * len);
   const int np = int(len / U), chunk = (np + gridDim.x - 1) / gridDim.x;
@@ -228,7 +230,13 @@ k_cg_dir(cx<R>* __restrict__ x, cx<R>* __restrict__ p, const cx<R>* __restrict__
       if (i + u * kRedThreads < end) {
         a[u] = zp[i + u * kRedThreads];
         c[u] = pp[i + u * kRedThreads];
-        e[u] = xp[i + u * kRedThreads];
+        cx<R>* xe = xv + (long long)(i + u * kRedThreads) * U;
+        if constexpr (XALIGNED) {
+          e[u] = *reinterpret_cast<const Pack*>(xe);
+        } else {
+#pragma unroll
+          for (int w = 0; w < U; ++w) e[u].e[w] = xe[w];
+        }
       }
   };
   load();
@@ -262,7 +270,13 @@ k_cg_dir(cx<R>* __restrict__ x, cx<R>* __restrict__ p, const cx<R>* __restrict__
           e[u].e[w] = caxpy(al, c[u].e[w], e[u].e[w]);
           c[u].e[w] = caxpy(b, c[u].e[w], a[u].e[w]);
         }
-        xp[i + u * kRedThreads] = e[u];
+        cx<R>* xe = xv + (long long)(i + u * kRedThreads) * U;
+        if constexpr (XALIGNED) {
+          *reinterpret_cast<Pack*>(xe) = e[u];
+        } else {
+#pragma unroll
+          for (int w = 0; w < U; ++w) xe[w] = e[u].e[w];
+        }
         if (more) pp[i + u * kRedThreads] = c[u];
       }
     i += B * kRedThreads;
@@ -648,8 +662,12 @@ template <class R>
 cudaError_t cg_dir(cx<R>* x, cx<R>* p, const cx<R>* z, long long len, int nvec, const double2* partial, int nblk,
                    const double* alpha, const double* rho, double* rho_next, double2* dot, const double* tol2b2,
                    const int* go, int* active, int* iters, double* res2, int ncta, cudaStream_t st) {
-  return launch<k_cg_dir<R>>(dim3(ncta, nvec), kRedThreads, 0, st, x, p, z, len, partial, nblk, alpha, rho, rho_next, dot,
-                             tol2b2, go, active, iters, res2);
+  if constexpr (sizeof(cx<R>) < 16)
+    if ((uintptr_t)x % 16 != 0)  // every vector then, as len is even
+      return launch<k_cg_dir<R, false>>(dim3(ncta, nvec), kRedThreads, 0, st, x, p, z, len, partial, nblk, alpha, rho,
+                                        rho_next, dot, tol2b2, go, active, iters, res2);
+  return launch<k_cg_dir<R, true>>(dim3(ncta, nvec), kRedThreads, 0, st, x, p, z, len, partial, nblk, alpha, rho, rho_next,
+                                   dot, tol2b2, go, active, iters, res2);
 }
 
 template <class R>
