@@ -141,6 +141,24 @@ FAME_HD float rfma(float a, float b, float c) { return fmaf(a, b, c); }
 FAME_HD double rfma(double a, double b, double c) { return fma(a, b, c); }
 FAME_HD ff rfma(ff a, ff b, ff c) { return a * b + c; }
 
+// A thread's running sum.  FP32: with the rounding error of every addition kept
+// beside it (exactly, Knuth's two-sum), so that a sum of any length carries the
+// rounding of its terms and of one final addition; FP64: plain.  The terms are sums over
+// a voxel or an element, so a wide batch, whose threads go through many voxels,
+// rounds no more than a narrow one.
+template <class R> struct RunSum {
+  R hi = R(0), lo = R(0);
+  FAME_HD void add(R t) {
+    const R s = hi + t;
+    if constexpr (std::is_same<R, float>::value) {
+      const R u = s - hi;
+      lo += (hi - (s - u)) + (t - u);
+    }
+    hi = s;
+  }
+  FAME_HD double value() const { return double(hi) + double(lo); }
+};
+
 template <class V> FAME_HD V cadd(V a, V b) { a.x += b.x; a.y += b.y; return a; }
 template <class V> FAME_HD V csub(V a, V b) { a.x -= b.x; a.y -= b.y; return a; }
 template <class V> FAME_HD V cneg(V a) { a.x = -a.x; a.y = -a.y; return a; }

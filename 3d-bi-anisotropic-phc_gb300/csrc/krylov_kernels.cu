@@ -107,14 +107,14 @@ k_cg_r_dot(cx<R>* __restrict__ r, const cx<R>* __restrict__ q, long long len, co
   }
   const R a = R(alpha[vec]);
   const long long o = vec * len;
-  R s0 = 0;
+  RunSum<R> s0;
   const long long chunk = (len + nblk - 1) / nblk, end = min(len, (blockIdx.x + 1) * chunk);
   for (long long i = blockIdx.x * chunk + threadIdx.x; i < end; i += kRedThreads) {
     const cx<R> ri = caxpy(-a, q[o + i], r[o + i]);
     r[o + i] = ri;
-    s0 += ri.x * ri.x + ri.y * ri.y;
+    s0.add(rfma(ri.x, ri.x, ri.y * ri.y));
   }
-  const double2 s = block_sum2(make_double2(double(s0), double(s0)));
+  const double2 s = block_sum2(make_double2(s0.value(), s0.value()));
   if (threadIdx.x == 0) *out = s;
 }
 

@@ -232,13 +232,14 @@ k_pcg_start(const cx<R>* __restrict__ b, cx<R>* __restrict__ x, cx<R>* __restric
   }
   const cx<R>* pc = pc_all ? pc_all + (long long)vec_inst(ctx, vec) * kPcSlots * Nq : nullptr;
   const long long o = vec * 4 * Nq;
-  R srz = 0, srr = 0;
+  RunSum<R> srz, srr;
   const long long chunk = (Nq + nblk - 1) / nblk, end = min(Nq, (blockIdx.x + 1) * chunk);
   for (long long i = blockIdx.x * chunk + threadIdx.x; i < end; i += kThreads) {
     cx<R> rv[4], zv[4];
 #pragma unroll
     for (int c = 0; c < 4; ++c) zv[c] = rv[c] = b[o + c * Nq + i];
     if (pc) mvec4<R>(load_block<R>(pc, Nq, i), rv, zv);
+    R trz = 0, trr = 0;
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
       const long long k = o + c * Nq + i;
@@ -246,11 +247,13 @@ k_pcg_start(const cx<R>* __restrict__ b, cx<R>* __restrict__ x, cx<R>* __restric
       r[k] = rv[c];
       p[k] = zv[c];
       if (pc) z[k] = zv[c];
-      srz += rv[c].x * zv[c].x + rv[c].y * zv[c].y;
-      srr += rv[c].x * rv[c].x + rv[c].y * rv[c].y;
+      trz = rfma(rv[c].x, zv[c].x, rfma(rv[c].y, zv[c].y, trz));
+      trr = rfma(rv[c].x, rv[c].x, rfma(rv[c].y, rv[c].y, trr));
     }
+    srz.add(trz);
+    srr.add(trr);
   }
-  double2 s = block_sum2b(make_double2(double(srz), double(srr)));
+  double2 s = block_sum2b(make_double2(srz.value(), srr.value()));
   if (threadIdx.x == 0) *out = s;
 }
 
@@ -334,7 +337,7 @@ k_pcg_update(cx<R>* __restrict__ r, cx<R>* __restrict__ z, const cx<R>* __restri
   }
   __syncthreads();
   const R a = R(s_alpha);
-  R srz = 0, srr = 0;
+  RunSum<R> srz, srr;
   while (i < end) {
     Pack zk[4];
 #pragma unroll
@@ -349,12 +352,15 @@ k_pcg_update(cx<R>* __restrict__ r, cx<R>* __restrict__ z, const cx<R>* __restri
 #pragma unroll
       for (int c = 0; c < kPcSlots; ++c) bl.s[c] = bk[c].e[u];
       mvec4<R>(bl, rv, zv);
+      R trz = 0, trr = 0;
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
         zk[c].e[u] = zv[c];
-        srz += rv[c].x * zv[c].x + rv[c].y * zv[c].y;
-        srr += rv[c].x * rv[c].x + rv[c].y * rv[c].y;
+        trz = rfma(rv[c].x, zv[c].x, rfma(rv[c].y, zv[c].y, trz));
+        trr = rfma(rv[c].x, rv[c].x, rfma(rv[c].y, rv[c].y, trr));
       }
+      srz.add(trz);
+      srr.add(trr);
     }
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
@@ -365,7 +371,7 @@ k_pcg_update(cx<R>* __restrict__ r, cx<R>* __restrict__ z, const cx<R>* __restri
     i += kThreads;
     if (i < end) load(i);
   }
-  double2 s = block_sum2b(make_double2(double(srz), double(srr)));
+  double2 s = block_sum2b(make_double2(srz.value(), srr.value()));
   if (threadIdx.x == 0) *out = s;
 }
 
