@@ -95,8 +95,9 @@ constexpr int kGradThreads = 128;
 // quadratic forms are evaluated once here and only read by k_grad (evaluating
 // them in both took 171 of 300 us per call, 3 vectors at n = 40).
 __global__ void __launch_bounds__(kGradThreads)
-k_quads(const double2* __restrict__ w, const double* __restrict__ fld, PlanData<double> d, VecCtx ctx, int n,
-        GradParams gp, double* __restrict__ quads, double* __restrict__ partial) {
+k_quads(const double2* __restrict__ w, const double* __restrict__ fld, PlanData<double> d,
+        const __grid_constant__ VecCtx ctx, int n, GradParams gp, double* __restrict__ quads,
+        double* __restrict__ partial) {
   const long long Nq = (long long)n * n * n;
   const int vec = blockIdx.y;
   pdl_wait();

@@ -129,7 +129,10 @@ cudaError_t upload_inst(Plan& P, const int* inst_host, int nvec, const int** d_i
     P.inst_cap = nvec;
   }
   *d_inst_out = P.d_inst;
-  return h2d_async(P, P.d_inst, inst_host, sizeof(int) * nvec);
+  // from the caller's memory: a small pageable copy goes through the command stream, where
+  // one from the pinned ring is a DMA transfer that the next kernel waits longer for
+  // (fncA of 64 complex64 vectors at n = 30 28 against 32 us)
+  return cudaMemcpyAsync(P.d_inst, inst_host, sizeof(int) * nvec, cudaMemcpyHostToDevice, P.stream);
 }
 
 cudaError_t ensure_stage(Plan& P, size_t bytes) {

@@ -36,8 +36,12 @@ extern unsigned long long g_host_launches;
 // Which vectors of a batch belong to which k-point instance, and which are
 // still active (converged vectors of a batched solve are skipped).  Up to
 // kSmallInst instance indices travel in the kernel arguments: a device copy
-// costs a call more than its own launches on small grids.
-constexpr int kSmallInst = 32;
+// costs a call more than its own launches on small grids, and the kernel behind it
+// waits some 10 us for it (fncA of 40 complex64 vectors at n = 36 19 us, 29 with a
+// copy from pageable memory, 35 from pinned memory).  Kernels take it as const
+// __grid_constant__: indexing a plain parameter makes every thread copy all of it to
+// its stack first.
+constexpr int kSmallInst = 128;
 struct VecCtx {
   const int* inst = nullptr;    // device [nvec] instance index, or null: small, or (v + vofs) % nk
   const int* active = nullptr;  // device [nvec] 0/1, or null: all active

@@ -274,8 +274,9 @@ template <class R> __device__ __forceinline__ void store_io(cx<R>* p, cx<R> v) {
 // ---------------------------------------------------------------------------
 template <int N, bool PREP>
 __global__ void __launch_bounds__(((3 * N + 31) / 32) * 32, 2)
-k_plane_inv(const float2* __restrict__ x, float2* __restrict__ out, PlanData<float> d, VecCtx ctx,
-            long long in_stride, long long in_side_stride, long long out_stride, int side0) {
+k_plane_inv(const float2* __restrict__ x, float2* __restrict__ out, PlanData<float> d,
+            const __grid_constant__ VecCtx ctx, long long in_stride, long long in_side_stride,
+            long long out_stride, int side0) {
   constexpr int LD = N + 1;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   float2* sm = reinterpret_cast<float2*>(smem_raw);  // [3][N][LD]
@@ -365,7 +366,7 @@ k_plane_inv(const float2* __restrict__ x, float2* __restrict__ out, PlanData<flo
 // else copies the 3 components out.
 template <int N, bool POST>
 __global__ void __launch_bounds__(((3 * N + 31) / 32) * 32, 2)
-k_plane_fwd(const float2* __restrict__ w, float2* __restrict__ y, PlanData<float> d, VecCtx ctx,
+k_plane_fwd(const float2* __restrict__ w, float2* __restrict__ y, PlanData<float> d, const __grid_constant__ VecCtx ctx,
             long long w_stride, long long out_stride, long long out_side_stride, int side0) {
   constexpr int LD = N + 1;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -568,8 +569,9 @@ template <class R, int N, int S> __device__ __forceinline__ void field_rows(cx<R
 // grid: (n / KP, 3 * sides, vectors); blockIdx.y = 3 * (side - side0) + field
 template <class R, int N, bool PREP>
 __global__ void __launch_bounds__(FieldShape<R, N>::TB, FieldShape<R, N>::CTAS)
-k_field_inv(const cx<R>* __restrict__ x, cx<R>* __restrict__ out, PlanData<R> d, VecCtx ctx, long long in_stride,
-            long long in_side_stride, long long out_stride, int side0) {
+k_field_inv(const cx<R>* __restrict__ x, cx<R>* __restrict__ out, PlanData<R> d,
+            const __grid_constant__ VecCtx ctx, long long in_stride, long long in_side_stride,
+            long long out_stride, int side0) {
   using FS = FieldShape<R, N>;
   constexpr int G = FS::G, M = N / G, LD = FS::LD, KP = FS::KP, TB = FS::TB;
   constexpr int NN = N * N, Nq = NN * N;
@@ -644,9 +646,9 @@ k_field_inv(const cx<R>* __restrict__ x, cx<R>* __restrict__ out, PlanData<R> d,
 enum { kCopy = 0, kPi = 1, kPiDot = 2 };
 template <class R, int N, int POST>
 __global__ void __launch_bounds__(FieldShape<R, N>::TB, FieldShape<R, N>::CTAS)
-k_field_fwd(const cx<R>* __restrict__ w, cx<R>* __restrict__ y, PlanData<R> d, VecCtx ctx, long long w_stride,
-            long long out_stride, long long out_side_stride, int side0, const cx<R>* __restrict__ xp,
-            double2* __restrict__ pq) {
+k_field_fwd(const cx<R>* __restrict__ w, cx<R>* __restrict__ y, PlanData<R> d,
+            const __grid_constant__ VecCtx ctx, long long w_stride, long long out_stride,
+            long long out_side_stride, int side0, const cx<R>* __restrict__ xp, double2* __restrict__ pq) {
   using FS = FieldShape<R, N>;
   constexpr int G = FS::G, M = N / G, LD = FS::LD, KP = FS::KP, TB = FS::TB;
   constexpr int NN = N * N, Nq = NN * N;
@@ -776,7 +778,8 @@ k_field_fwd(const cx<R>* __restrict__ w, cx<R>* __restrict__ y, PlanData<R> d, V
 // ---------------------------------------------------------------------------
 template <int N, int DIR, int SMODE>
 __global__ void __launch_bounds__(128, 3)
-k_col(const float2* src, float2* dst, PlanData<float> d, VecCtx ctx, long long stride, float scale) {
+k_col(const float2* src, float2* dst, PlanData<float> d, const __grid_constant__ VecCtx ctx,
+      long long stride, float scale) {
   const int col = blockIdx.x * blockDim.x + threadIdx.x;
   const int f = blockIdx.y;
   const int vec = blockIdx.z;
@@ -818,7 +821,7 @@ template <int N> FAME_HD constexpr int col_width() { return N <= 16 || field_spl
 
 template <class R, int N, int DIR, int SMODE>
 __global__ void __launch_bounds__(((col_width<N>() * field_split(N) + 31) / 32) * 32)
-k_col2(const cx<R>* src, cx<R>* dst, PlanData<R> d, VecCtx ctx, long long stride, R scale) {
+k_col2(const cx<R>* src, cx<R>* dst, PlanData<R> d, const __grid_constant__ VecCtx ctx, long long stride, R scale) {
   constexpr int G = field_split(N);
   using SP = Split<N, G>;
   constexpr int M = SP::M, W = col_width<N>(), LD = W + 1, T = W * G, NN = N * N;

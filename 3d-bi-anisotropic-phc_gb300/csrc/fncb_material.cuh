@@ -139,7 +139,8 @@ __device__ __forceinline__ void shift_phases(const PlanData<R>& d, int inst, boo
 template <class R, int N, int KIND>
 __global__ void __launch_bounds__(512)
 k_vertex(const cx<R>* __restrict__ uv, cx<R>* __restrict__ h, PlanData<R> d,
-         const uint8_t* __restrict__ phase, int nphase, VecCtx ctx, long long stride, bool bloch) {
+         const uint8_t* __restrict__ phase, int nphase, const __grid_constant__ VecCtx ctx, long long stride,
+         bool bloch) {
   constexpr int NN = N * N, Nq = NN * N;
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
   const int vec = blockIdx.y;
@@ -182,7 +183,8 @@ k_vertex(const cx<R>* __restrict__ uv, cx<R>* __restrict__ h, PlanData<R> d,
 template <class R, int N, int KIND>
 __global__ void __launch_bounds__(512)
 k_faceedge(const cx<R>* uv, const cx<R>* __restrict__ h, cx<R>* out, PlanData<R> d,
-           const uint8_t* __restrict__ phase, int nphase, VecCtx ctx, long long stride, bool bloch) {
+           const uint8_t* __restrict__ phase, int nphase, const __grid_constant__ VecCtx ctx, long long stride,
+           bool bloch) {
   constexpr int NN = N * N, Nq = NN * N;
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
   const int vec = blockIdx.y;
@@ -302,7 +304,7 @@ template <int K> __device__ __forceinline__ void cp_async_wait() {
 template <class R, int N, int KIND>
 __global__ void __launch_bounds__(SweepShape<R, N>::TPB, sizeof(R) == 4 && KIND == kMatGeneral ? SweepShape<R, N>::CTAS : 0)
 k_sweep(const cx<R>* __restrict__ uv, cx<R>* __restrict__ out, PlanData<R> d, const uint8_t* __restrict__ phase,
-        int nphase, VecCtx ctx, long long stride, int tz, double2* __restrict__ wdot) {
+        int nphase, const __grid_constant__ VecCtx ctx, long long stride, int tz, double2* __restrict__ wdot) {
   using SH = SweepShape<R, N>;
   constexpr int TY = SH::TY, FR = SH::FR, HR = SH::HR, TPB = SH::TPB, CPR = SH::CPR;
   constexpr int NN = N * N, Nq = NN * N;

@@ -9,8 +9,8 @@ namespace detail {
 
 // fncA.m:3-4: y = [ i/Sigma .* x2 ; -i/Sigma .* x1 ], Sigma = [sqrt(Lq); sqrt(Lq)].
 template <class R>
-__global__ void k_fncA(const cx<R>* __restrict__ x, cx<R>* __restrict__ y, PlanData<R> d, VecCtx ctx,
-                       int n) {
+__global__ void k_fncA(const cx<R>* __restrict__ x, cx<R>* __restrict__ y, PlanData<R> d,
+                       const __grid_constant__ VecCtx ctx, int n) {
   const long long Nq = (long long)n * n * n;
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int vec = blockIdx.y;

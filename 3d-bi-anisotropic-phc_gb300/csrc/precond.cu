@@ -220,7 +220,7 @@ __device__ __forceinline__ double2 block_sum2b(double2 v) {
 template <class R>
 __global__ void __launch_bounds__(kThreads)
 k_pcg_start(const cx<R>* __restrict__ b, cx<R>* __restrict__ x, cx<R>* __restrict__ r, cx<R>* __restrict__ z,
-            cx<R>* __restrict__ p, const cx<R>* __restrict__ pc_all, VecCtx ctx, long long Nq,
+            cx<R>* __restrict__ p, const cx<R>* __restrict__ pc_all, const __grid_constant__ VecCtx ctx, long long Nq,
             double2* __restrict__ partial) {
   const int vec = blockIdx.y;
   const int nblk = gridDim.x;
@@ -270,7 +270,8 @@ k_pcg_start(const cx<R>* __restrict__ b, cx<R>* __restrict__ x, cx<R>* __restric
 template <class R>
 __global__ void __launch_bounds__(kThreads, sizeof(R) == 4 ? 2 : 1)
 k_pcg_update(cx<R>* __restrict__ r, cx<R>* __restrict__ z, const cx<R>* __restrict__ q,
-             const cx<R>* __restrict__ pc_all, VecCtx ctx, long long Nq, double2* __restrict__ partial, CgAlpha ca) {
+             const cx<R>* __restrict__ pc_all, const __grid_constant__ VecCtx ctx, long long Nq,
+             double2* __restrict__ partial, CgAlpha ca) {
   constexpr int U = 16 / sizeof(cx<R>);  // voxels per 16-byte access (n^3 is even)
   struct alignas(16) Pack {
     cx<R> e[U];

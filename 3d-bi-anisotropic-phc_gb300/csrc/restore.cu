@@ -37,7 +37,8 @@ __device__ __forceinline__ double2 field_of(double2 wv) { return cmul_i<-1>(wv);
 // operations per voxel (8 vectors at n = 40: 106 us with the differences scaled
 // one by one, 58 now).
 __global__ void __launch_bounds__(kT)
-k_curl_pair(const double2* __restrict__ w, double2* __restrict__ y, PlanData<double> d, VecCtx ctx, int n) {
+k_curl_pair(const double2* __restrict__ w, double2* __restrict__ y, PlanData<double> d,
+            const __grid_constant__ VecCtx ctx, int n) {
   const long long Nq = (long long)n * n * n;
   const int idx = blockIdx.x * kT + threadIdx.x;
   const int vec = blockIdx.y;
@@ -132,7 +133,7 @@ k_orgsep(const double2* __restrict__ y, const double2* __restrict__ w, const dou
 // E = S .* e, H = S .* h (Bloch frame, the reference's layout: 3Nq each).
 __global__ void __launch_bounds__(kT)
 k_to_bloch(const double2* __restrict__ w, double2* __restrict__ E, double2* __restrict__ H, PlanData<double> d,
-           VecCtx ctx, int n) {
+           const __grid_constant__ VecCtx ctx, int n) {
   const long long Nq = (long long)n * n * n;
   const int idx = blockIdx.x * kT + threadIdx.x;
   const int vec = blockIdx.y;
