@@ -6,7 +6,7 @@
 //                intermediates in L2, and some widths fill the last wave of
 //                CTAs better than others;
 //   stencil_tpb  the material stencil's form: 0 the single-pass k_sweep,
-//                128/256/512 threads per block of the two-kernel form;
+//                128/256/512 threads per block of the two-kernel form.
 // No counterpart in the reference.
 #include <algorithm>
 #include <vector>
@@ -36,7 +36,7 @@ TuneEntry tune_for(const Plan& P, int prec, int nvec) {
   // lose (nine at n = 64 223 -> 227), and thirds lose.
   const long long bytes = 12LL * P.Nq * (long long)sizeof(float2);  // both buffers of a vector
   const int half = (nvec + 1) / 2;
-  if (prec == FAME_C64 && 2 * bytes * nvec > 3LL * P.l2 && bytes * half <= P.l2) d.untuned = half;
+  if (prec == FAME_C64 && 2 * bytes * nvec > 3LL * P.l2 && bytes * half <= P.l2) d.chunk = half;
   return d;
 }
 
@@ -45,7 +45,7 @@ TuneEntry tune_for(const Plan& P, int prec, int nvec) {
 static void put_tune(Plan& P, const TuneEntry& t) {
   for (TuneEntry& u : P.tune)
     if (u.prec == t.prec && u.nvec == t.nvec) {
-      if (u.chunk != t.chunk || u.untuned != t.untuned || u.stencil_tpb != t.stencil_tpb || u.lanes != t.lanes) free_graphs(P);
+      if (u.chunk != t.chunk || u.stencil_tpb != t.stencil_tpb || u.lanes != t.lanes) free_graphs(P);
       u = t;
       return;
     }
@@ -170,7 +170,6 @@ int fame_set_tune(fame_plan_t h, int prec, int nvec, int chunk, int stencil_tpb)
     return fail(&P, FAME_ERR_BAD_ARG, "fame_set_tune: bad argument");
   TuneEntry t = tune_for(P, prec, nvec);  // keeps the width's split
   t.chunk = chunk >= nvec ? 0 : chunk;
-  t.untuned = 0;
   t.stencil_tpb = stencil_tpb;
   put_tune(P, t);
   return FAME_OK;

@@ -85,8 +85,7 @@ FAME_HD constexpr int field_split(int n) {
 // stencil's form (single pass, or threads per block of the two-kernel form).
 struct TuneEntry {
   int prec = 0, nvec = 0;
-  int chunk = 0;         // 0: whole batch, but for untuned batches see untuned
-  int untuned = 0;       // vectors per sequence where nothing was installed (0: whole batch)
+  int chunk = 0;         // vectors per sequence; 0: whole batch
   int stencil_tpb = 0;   // 0: single-pass k_sweep; 128/256/512: two-kernel form
   int lanes = -1;        // kept for its callers (fame_set_tune_lanes); the kernels take one split per size
   double us = 0.0;       // measured time of one fncB on the batch
@@ -189,8 +188,7 @@ struct Plan {
 
 // Vectors per launch sequence of a batch of nvec.
 inline int sub_batch(const TuneEntry& t, int nvec) {
-  const int c = t.chunk > 0 ? t.chunk : t.untuned;
-  return c > 0 && c < nvec ? c : nvec;
+  return t.chunk > 0 && t.chunk < nvec ? t.chunk : nvec;
 }
 // Tuned launch parameters for (prec, nvec), or the defaults.
 TuneEntry tune_for(const Plan& P, int prec, int nvec);

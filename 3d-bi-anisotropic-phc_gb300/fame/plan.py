@@ -307,7 +307,7 @@ class Plan:
         check(self._lib.fame_set_tune_lanes(self._h, pr, int(nvec), int(lanes)), self._h, "fame_set_tune_lanes")
 
     def get_tune(self, prec, nvec):
-        """fame_get_tune: the installed dict(chunk, stencil_tpb, lanes)."""
+        """fame_get_tune: dict(chunk, stencil_tpb, lanes) in force, installed or default."""
         pr = _tune_prec(prec)
         ch, tpb, ln = C.c_int(), C.c_int(), C.c_int()
         check(self._lib.fame_get_tune(self._h, pr, int(nvec), C.byref(ch), C.byref(tpb), C.byref(ln)), self._h,

@@ -163,8 +163,10 @@ int fame_refine_residuals(fame_plan_t plan, double* before, int n);
  * batch), stencil setting and the measured microseconds of one fncB.
  * fame_set_tune installs a chunk and stencil setting directly (e.g. from a
  * cache).  With nothing installed for a width, a complex64 batch whose
- * intermediates exceed 1.5 times the L2 runs as two halves.  fame_set_tune_lanes records a count of threads per FFT pencil
- * (-1 = default) that fame_get_tune returns; every size and precision has one
+ * intermediates exceed 1.5 times the L2, and half of them fits in it, runs as
+ * two halves.  fame_get_tune returns what is in force, installed or default.
+ * fame_set_tune_lanes records a count of threads per FFT pencil (-1 =
+ * default) that fame_get_tune returns; every size and precision has one
  * compiled split, so it has no other effect.
  */
 int fame_autotune(fame_plan_t plan, int prec, int nvec, int* chunk, int* stencil_tpb, double* us);
