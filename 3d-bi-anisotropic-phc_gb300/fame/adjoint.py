@@ -51,10 +51,14 @@ def solve_bands(plan, nbands, tol=1e-10, prec="c128", inner_tol=1e-12, p=None):
     return np.stack(oms), evs
 
 
-# eigenvectors per backward call: one call evaluates the k-points of a group
-# together (four calls of three vectors at n = 40 left the GPU idle for a third
-# of the time), bounded so that the joined copy and the call's scratch stay small
+# One backward call evaluates the k-points of a group together (four calls of three
+# vectors at n = 40 left the GPU idle for a third of the time: 1.76 -> 0.94 ms, at
+# n = 60 4.95 -> 2.58), as many as their joined copy allows; the plan's work arrays,
+# which stay, are three times as large, together less than the basis that a solve
+# of the same pairs holds.  (64 MiB: 2.98 ms at n = 60.)  A k-point beyond the bounds
+# is a call of its own, without a copy.
 GROUP_VECTORS = 32
+GROUP_BYTES = 192 << 20
 
 
 def gradient(plan, evs, omega, weights, cluster_tol=1e-8):
@@ -62,6 +66,7 @@ def gradient(plan, evs, omega, weights, cluster_tol=1e-8):
     g_e = torch.zeros(plan.Nq, dtype=torch.float64, device="cuda")
     g_g = torch.zeros_like(g_e)
     group = []
+    most = min(GROUP_VECTORS, GROUP_BYTES // (16 * 4 * plan.Nq))
 
     def flush():
         if group:
@@ -80,7 +85,7 @@ def gradient(plan, evs, omega, weights, cluster_tol=1e-8):
         nvec = ev.shape[0]
         om, w = (q if q.shape == (nvec,) else np.broadcast_to(q, (nvec,))
                  for q in (np.asarray(omega[k], dtype=np.float64), w))
-        if group and sum(len(g[0]) for g in group) + nvec > GROUP_VECTORS:
+        if group and sum(len(g[0]) for g in group) + nvec > most:
             flush()
         group.append((np.full(nvec, k, dtype=np.int32), ev, om, w))
     flush()
