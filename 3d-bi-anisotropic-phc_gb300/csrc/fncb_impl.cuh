@@ -103,19 +103,25 @@ template <class R, int N> __device__ __forceinline__ R scale3() {
 }
 
 // Component c of Pi1 and Pi2 at a frequency voxel (index vox = k3 n^2 + i2 n +
-// i1) of instance inst, times n^{-3/2}: from the plan's table [6][n^3] when it
-// has one, else evaluated.
+// i1) of instance inst, times n^{-3/2}: from the plan's table [6][n^3], or
+// (pi_comp) evaluated when there is none.
 template <class R> struct PiComp {
   cx<R> p1, p2;
 };
 template <class R, int N>
-__device__ __forceinline__ PiComp<R> pi_comp(const PlanData<R>& d, int inst, int c, int vox, const cx<R>* lam) {
+__device__ __forceinline__ PiComp<R> pi_table(const PlanData<R>& d, int inst, int c, int vox) {
   constexpr int Nq = N * N * N;
+  const cx<R>* t = d.pi + (size_t)inst * 6 * Nq + vox;
+  PiComp<R> P;
+  P.p1 = t[(size_t)c * Nq];
+  P.p2 = t[(size_t)(3 + c) * Nq];
+  return P;
+}
+template <class R, int N>
+__device__ __forceinline__ PiComp<R> pi_comp(const PlanData<R>& d, int inst, int c, int vox, const cx<R>* lam) {
   PiComp<R> P;
   if (d.pi) {
-    const cx<R>* t = d.pi + (size_t)inst * 6 * Nq + vox;
-    P.p1 = t[(size_t)c * Nq];
-    P.p2 = t[(size_t)(3 + c) * Nq];
+    P = pi_table<R, N>(d, inst, c, vox);
   } else {
     const PiBlock<R> B = pi_block<R>(lam[vox % N], lam[N + (vox / N) % N], lam[2 * N + vox / (N * N)]);
     P.p1 = cscale(c == 0 ? B.p1[0] : c == 1 ? B.p1[1] : B.p1[2], scale3<R, N>());
@@ -228,9 +234,13 @@ template <int N> __device__ __forceinline__ PiRow* pi_rows(float2* sm) {
 // operator reads and writes complex128 vectors (the caller's), converting
 // on load and store, so it needs no conversion passes; by bit operations, as
 // an FP64 or conversion instruction takes as long as 64 FP32 ones.
-template <class R> __device__ __forceinline__ cx<R> load_io(const cx<R>* p) {
+// The element type that the caller's vectors have.
+template <class R> using io_t = std::conditional_t<std::is_same_v<R, ff>, double2, cx<R>>;
+template <class R> __device__ __forceinline__ io_t<R> load_raw(const cx<R>* p) {
+  return *reinterpret_cast<const io_t<R>*>(p);
+}
+template <class R> __device__ __forceinline__ cx<R> from_io(io_t<R> v) {
   if constexpr (std::is_same<R, ff>::value) {
-    const double2 v = *reinterpret_cast<const double2*>(p);
     cff c;
     const bool ok = ff_split_bits(__double2hiint(v.x), __double2loint(v.x), c.x) &
                     ff_split_bits(__double2hiint(v.y), __double2loint(v.y), c.y);
@@ -240,9 +250,10 @@ template <class R> __device__ __forceinline__ cx<R> load_io(const cx<R>* p) {
     }
     return c;
   } else {
-    return *p;
+    return v;
   }
 }
+template <class R> __device__ __forceinline__ cx<R> load_io(const cx<R>* p) { return from_io<R>(load_raw<R>(p)); }
 template <class R> __device__ __forceinline__ void store_io(cx<R>* p, cx<R> v) {
   if constexpr (std::is_same<R, ff>::value) {
     uint32_t h[4], l[4];
@@ -566,9 +577,23 @@ template <class R, int N, int S> __device__ __forceinline__ void field_rows(cx<R
   __syncthreads();
 }
 
-// grid: (n / KP, 3 * sides, vectors); blockIdx.y = 3 * (side - side0) + field
-template <class R, int N, bool PREP>
-__global__ void __launch_bounds__(FieldShape<R, N>::TB, FieldShape<R, N>::CTAS)
+// What a field kernel does with Pi: nothing; the product with it; that and the sum of
+// Re(xp^H y) (k_field_fwd); the product with Pi evaluated by the cluster (k_field_inv).
+enum { kCopy = 0, kPi = 1, kPiDot = 2, kPiEval = 3 };
+
+// grid: (n / KP, 3 * sides, vectors); blockIdx.y = 3 * (side - side0) + field.
+// Double-single takes Pi from the plan's table, its loads all issued before the first
+// conversion (8 vectors at n = 40 485 -> 444 us, one at n = 60 268 -> 237), or, for a
+// plan that reads no table, evaluates it in clusters (PREP kPiEval): the three
+// field CTAs of one (plane, side, vector) each take a third of the voxels, whose two
+// square roots and divisions are FP64, and write all three components into each
+// other's shared memory.  fncB without the table of 8 vectors at n = 60: 3110 us with
+// three fields per CTA, 3500 with each field's CTA evaluating its own component,
+// 2660 so.  Complex128, bound by FP64 throughout, tests for the table here
+// (4880 us without it; and a kernel for the table alone was slower, n = 12, ten
+// vectors 38.3 -> 40.1).
+template <class R, int N, int PREP>
+__global__ void __launch_bounds__(FieldShape<R, N>::TB, PREP == kPiEval ? 0 : FieldShape<R, N>::CTAS)
 k_field_inv(const cx<R>* __restrict__ x, cx<R>* __restrict__ out, PlanData<R> d,
             const __grid_constant__ VecCtx ctx, long long in_stride, long long in_side_stride,
             long long out_stride, int side0) {
@@ -586,40 +611,62 @@ k_field_inv(const cx<R>* __restrict__ x, cx<R>* __restrict__ out, PlanData<R> d,
   const int tid = threadIdx.x;
   const cx<R>* lam = d.lam + (long long)inst * 3 * N;
   const cx<R>* xin = x + vec * in_stride + (blockIdx.y / 3) * in_side_stride + k3 * NN;
-  // the loads of U elements issued together
-  constexpr int ITEMS = (KP * NN + TB - 1) / TB;
-  constexpr int UMAX = std::is_same_v<R, ff> ? 2 : 4, U = ITEMS < UMAX ? ITEMS : UMAX;
-  for (int b = 0; b < ITEMS; b += U) {
-    cx<R> in[U][2];
-    PiComp<R> P[U];
+  if constexpr (PREP == kPiEval) {
+    auto cluster = cooperative_groups::this_cluster();
+    cx<R>* f[3];
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int e = tid + (b + u) * TB;
-      if (e < KP * NN) {
-        if constexpr (PREP) {
-          in[u][0] = load_io<R>(xin + e);
-          in[u][1] = load_io<R>(xin + Nq + e);
-          P[u] = pi_comp<R, N>(d, inst, c, k3 * NN + e, lam);
-        } else {
-          in[u][0] = xin[(long long)c * Nq + e];
+    for (int k = 0; k < 3; ++k) f[k] = cluster.map_shared_rank(sm, k);
+    cluster.sync();  // the neighbours run
+    for (int e = c * TB + tid; e < KP * NN; e += 3 * TB) {
+      const int r = e / N, i1 = e - r * N;
+      const cx<R> a = cscale(load_io<R>(xin + e), scale3<R, N>());
+      const cx<R> b = cscale(load_io<R>(xin + Nq + e), scale3<R, N>());
+      const PiBlock<R> P = pi_block<R>(lam[i1], lam[N + r % N], lam[2 * N + k3 + r / N]);
+      // side 1: Pi1 a + Pi2 b; side 0: conj(Pi1) b - conj(Pi2) a (as in k_field_fwd)
+      const cx<R> X = side ? a : b, Y = side ? b : cneg(a);
+#pragma unroll
+      for (int k = 0; k < 3; ++k)
+        f[k][r * LD + i1] = cfma(conj_unless(P.p2[k], side), Y, cmul(conj_unless(P.p1[k], side), X));
+    }
+    cluster.sync();
+  } else {
+    // the loads of U elements issued together
+    constexpr int ITEMS = (KP * NN + TB - 1) / TB;
+    constexpr int UMAX = std::is_same_v<R, ff> ? 2 : 4, U = ITEMS < UMAX ? ITEMS : UMAX;
+    for (int b = 0; b < ITEMS; b += U) {
+      io_t<R> in[U][2];
+      PiComp<R> P[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int e = tid + (b + u) * TB;
+        if (e < KP * NN) {
+          if constexpr (PREP == kPi) {
+            in[u][0] = load_raw<R>(xin + e);
+            in[u][1] = load_raw<R>(xin + Nq + e);
+            if constexpr (std::is_same_v<R, ff>) P[u] = pi_table<R, N>(d, inst, c, k3 * NN + e);
+            else P[u] = pi_comp<R, N>(d, inst, c, k3 * NN + e, lam);
+          } else {
+            in[u][0] = load_raw<R>(xin + (long long)c * Nq + e);
+          }
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int e = tid + (b + u) * TB;
+        if (e < KP * NN) {
+          const int r = e / N, i1 = e - r * N;
+          cx<R> v = from_io<R>(in[u][0]);
+          if constexpr (PREP == kPi) {
+            const cx<R> a = v, b = from_io<R>(in[u][1]);
+            if (side == 0) v = cfmac(P[u].p1, b, cneg(cmulc(P[u].p2, a)));
+            else v = cfma(P[u].p2, b, cmul(P[u].p1, a));
+          }
+          sm[r * LD + i1] = v;
         }
       }
     }
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int e = tid + (b + u) * TB;
-      if (e < KP * NN) {
-        const int r = e / N, i1 = e - r * N;
-        cx<R> v = in[u][0];
-        if constexpr (PREP) {
-          if (side == 0) v = cfmac(P[u].p1, in[u][1], cneg(cmulc(P[u].p2, in[u][0])));
-          else v = cfma(P[u].p2, in[u][1], cmul(P[u].p1, in[u][0]));
-        }
-        sm[r * LD + i1] = v;
-      }
-    }
+    __syncthreads();
   }
-  __syncthreads();
   const int g = tid / FS::NP, p = tid - g * FS::NP;
   const bool act = tid < FS::T;
   field_rows<R, N, +1>(sm, tid, g, p, act);
@@ -643,7 +690,6 @@ k_field_inv(const cx<R>* __restrict__ x, cx<R>* __restrict__ out, PlanData<R> d,
 // its neighbours' shared memory.  POST 2 also sums Re(xp^H y) over the CTA's
 // voxels for xp laid out as y (one partial per CTA): in a CG iteration one
 // pass over p and q less (c128, two vectors at n = 30: a launch of 5.3 us).
-enum { kCopy = 0, kPi = 1, kPiDot = 2 };
 template <class R, int N, int POST>
 __global__ void __launch_bounds__(FieldShape<R, N>::TB, FieldShape<R, N>::CTAS)
 k_field_fwd(const cx<R>* __restrict__ w, cx<R>* __restrict__ y, PlanData<R> d,
@@ -896,8 +942,13 @@ cudaError_t plane_inv(const PlanData<R>& d, const cx<R>* x, cx<R>* out, int nvec
                                             d, ctx, in_stride, in_side_stride, out_stride, side0);
   } else {
     using FS = FieldShape<R, N>;
-    return launch<k_field_inv<R, N, PREP>>(dim3(N / FS::KP, 3 * nside, nvec), FS::TB, FS::SMEM, st, x, out, d, ctx,
-                                               in_stride, in_side_stride, out_stride, side0);
+    const dim3 g(N / FS::KP, 3 * nside, nvec);
+    if constexpr (PREP && std::is_same_v<R, ff>)
+      if (!d.pi)
+        return launch<k_field_inv<R, N, kPiEval>, 3>(g, FS::TB, FS::SMEM, st, x, out, d, ctx, in_stride, in_side_stride,
+                                                     out_stride, side0);
+    return launch<k_field_inv<R, N, PREP ? kPi : kCopy>>(g, FS::TB, FS::SMEM, st, x, out, d, ctx, in_stride,
+                                                         in_side_stride, out_stride, side0);
   }
 }
 
