@@ -39,11 +39,27 @@ enum WsId {
 // elements per thread at least left 28 CTAs for two vectors at n = 30; one
 // element per thread, 212 CTAs on 152 SMs, each with its reduction in FP64: the
 // complex128 update took 71 and 26 us of a CG iteration, 13 with one CTA per SM.)
+// Wide batches have a few CTAs per vector, and their whole number may leave the last
+// round of the SMs largely empty (77 vectors, one CTA each).  Where a quarter or more
+// of it is, up to 16: the count with the least work on the fullest SM, a CTA costing
+// `each` / 2 elements by itself.  A solve's iteration, complex128: 77 vectors at
+// n = 24 1903 -> 1790 us, 100 2360 -> 2268, 153 at n = 16 1066 -> 1008; complex64 153 at
+// n = 30 590 -> 557.  With a smaller part empty the other counts lose as often (complex64
+// 64 vectors at n = 16 49 -> 53).
 static int dot_blocks(const Plan& P, long long len, int nvec, int per_sm = 4, int each = 1024) {
   nvec = std::max(1, nvec);
+  const long long most = (len + 31) / 32;  // a warp's elements at least
   const long long k = std::max(1LL, std::min<long long>(per_sm, len * nvec / ((long long)each * P.sms)));
-  const long long b = std::max(1LL, k * P.sms / nvec);
-  return (int)std::min(512LL, std::min(b, (len + 31) / 32));
+  long long b = std::min(most, std::max(1LL, k * P.sms / nvec));
+  const long long round = k * P.sms;
+  if (4 * b * nvec <= 3 * round * ((b * nvec + round - 1) / round)) {
+    auto fullest = [&](long long c) { return (c * nvec + P.sms - 1) / P.sms * ((len + c - 1) / c + each / 2); };
+    long long best = b;
+    for (long long c = b + 1; c <= std::min(16LL, most); ++c)
+      if (fullest(c) < fullest(best)) best = c;
+    b = best;
+  }
+  return (int)std::min(512LL, b);
 }
 
 // Device scalars of the batched CG, carved from one workspace.  tolv and
