@@ -55,6 +55,12 @@ def _current_stream():
     return raw(torch.cuda.current_device()) if raw is not None else torch.cuda.current_stream().cuda_stream
 
 
+# Generation of the kernels whose launch parameters a tuning cache holds: raised
+# when they change enough that settings measured before no longer hold (1, not
+# written in the keys: three threads per FFT pencil, vertex tensors of 27 entries).
+TUNED_KERNELS = 2
+
+
 def _tune_prec(prec):
     """Tuning key of 'c64', 'c128' or 'c128ds' (complex128 vectors, double-single
     arithmetic: the mixed inner solves' residuals), or the FAME_* code itself."""
@@ -231,7 +237,7 @@ class Plan:
 
     def set_option(self, option, value):
         """fame_set_option: 'precond' (bool), 'tol32' (float), 'graph' (0, 1 or 2), 'itol_floor' (float),
-        'plane_split' (bool), 'sira_nearest' (bool), 'refine' (bool), 'refine_tol' (float),
+        'plane_split' (accepted, without effect), 'sira_nearest' (bool), 'refine' (bool), 'refine_tol' (float),
         'pi_table' (bool), 'c64_round' (bool), 'relax' (float in [0, 1)), 'relax_max' (float >= 1) or
         'ds_residual' (bool)."""
         code = {"precond": L.FAME_OPT_PRECOND, "tol32": L.FAME_OPT_TOL32, "graph": L.FAME_OPT_GRAPH,
@@ -246,8 +252,9 @@ class Plan:
     def autotune(self, nvec=None, prec="c64", cache=None):
         """fame_autotune for batch width `nvec` (default: the plan's instance
         count).  With `cache` (a JSON file path) a setting measured before on
-        the same device, grid, precision and width is installed without
-        re-timing, and new measurements are added to the file.
+        the same device, grid, precision and width and with the same
+        generation of the kernels is installed without re-timing, and new
+        measurements are added to the file.
         Returns dict(chunk, stencil_tpb, lanes, us, cached) (lanes: always -1,
         one split of the FFT pencils is compiled per size and precision)."""
         import json
@@ -255,7 +262,8 @@ class Plan:
         nvec = self.nk if nvec is None else int(nvec)
         pr = _tune_prec(prec)
         dev = torch.cuda.get_device_name() if torch is not None and torch.cuda.is_available() else "gpu"
-        key = f"{dev}|n={self.n}|{ {L.FAME_C64: 'c64', L.FAME_C128: 'c128'}.get(pr, 'c128ds') }|nvec={nvec}"
+        key = f"{dev}|n={self.n}|{ {L.FAME_C64: 'c64', L.FAME_C128: 'c128'}.get(pr, 'c128ds') }|nvec={nvec}" \
+            f"|kernels={TUNED_KERNELS}"
         table = {}
         if cache and os.path.exists(cache):
             with open(cache) as f:
