@@ -74,7 +74,27 @@ inline bool small_inst(VecCtx& ctx, const int* inst, int nvec) {
   return true;
 }
 
-// Threads per FFT pencil of the complex128 / double-single kernels for size n.
+// Threads per FFT pencil of the complex128 / double-single kernels for size n: G with
+// N / G values in each thread's registers, 16 at most but for n = 50, and G
+// coprime to N / G where such a G exists (no twiddles).  fncB of one and of eight
+// complex128 vectors (us) with the count in use and with others:
+//   n = 64   8: 516 3734   4: 504 3532   16: 547 3944
+//   n = 60   4: 408 2721   3: 419 2740    5: 424 2785
+//   n = 50   2: 306 2007   5: 285 1810   10: 298 2027
+//   n = 48   3: 203 1412   4: 193 1397    6: 210 1522    8: 208 1515
+//   n = 40   5: 128  802   4: 134  849    8: 126  796    2: 142  876
+//   n = 36   4: 111  618   3: 116  657    6: 110  621    9: 112  643
+//   n = 32   4:  78  414   8:  81  427    2:  86  437   16: 119  689
+//   n = 30   3:  77  339   2:  78  333    5:  77  336    6:  73  339
+//   n = 24   3:  47  176   4:  47  175    8:  43  177    2:  58  186
+//   n = 20   4:  36  110   5:  33  111    2:  49  136   10:  48  148
+//   n = 18   2:  45  102   3:  39   90    6:  35   94    9:  40  108
+//   n = 16   4:  31   60   2:  42   59    8:  40   64    1:  55   70
+//   n = 12   3:  29   34   4:  26   31    2:  34   37    6:  33   38
+//   n = 10   2:  30   32   5:  27   31    1:  37   38
+//   n = 8    2:  25   26   4:  25   26    1:  29   30
+// (measured after the choice: 3 or 6 at n = 18, 5 at n = 50, 4 at n = 12, 48 and 64 are faster
+// by 1 to 15 % and not in use; in double-single 8 at n = 24 and 40 as well.)
 FAME_HD constexpr int field_split(int n) {
   return n == 64 ? 8 : n == 60 ? 4 : n == 50 ? 2 : n == 48 ? 3 : n == 40 ? 5 : n == 36 ? 4 : n == 32 ? 4 : n == 30 ? 3
        : n == 24 ? 3 : n == 20 ? 4 : n == 18 ? 2 : n == 16 ? 4 : n == 12 ? 3 : n == 10 ? 2 : n == 8 ? 2 : n == 6 ? 2 : 1;

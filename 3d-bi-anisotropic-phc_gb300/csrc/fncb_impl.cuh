@@ -328,7 +328,7 @@ k_plane_inv(const float2* __restrict__ x, float2* __restrict__ out, PlanData<flo
     }
     if constexpr (PREP && decltype(bc)::value == 0) __syncthreads();  // the row table
     if (act) {
-      PiCol pc;
+      [[maybe_unused]] PiCol pc;
       if constexpr (PREP) pc = pi_col<N>(lam, k3, side, i1);
 #pragma unroll
       for (int it = 0; it < PF; ++it) {
@@ -418,7 +418,7 @@ k_plane_fwd(const float2* __restrict__ w, float2* __restrict__ y, PlanData<float
   __syncthreads();
   if (!act) return;
   float2* o = y + vec * out_stride + blockIdx.y * out_side_stride + (long long)k3 * N * N;
-  PiCol pc;
+  [[maybe_unused]] PiCol pc;
   if constexpr (POST) pc = pi_col<N>(lam, k3, side, i1);
 #pragma unroll 4
   for (int i2 = grp; i2 < N; i2 += 3) {
@@ -1108,9 +1108,13 @@ cudaError_t handle_n(const Plan& P, int which, const cx<R>* x, cx<R>* y, int nve
 
 // Grid sizes with a compiled double-single fncB (the residuals b - B x of the
 // mixed inner solves; other sizes take the FP64 fncB), and its declaration.
-// (sizes with a split of the plane kernels: their loads and stores convert the
-// complex128 vectors; at n = 32 the unsplit double-single kernels were no
-// faster than FP64)
+// The grid sizes of the band solves that it was written for.  fncB of one and of eight
+// vectors, double-single against FP64 (us): n = 12 30 33 / 29 34, 24 46 103 / 47 176,
+// 40 78 443 / 128 802, 48 131 838 / 203 1412, 60 242 1640 / 408 2721.  The kernels compile for
+// every size, and measured so it would gain at most of the others too: n = 16 34 48 / 31 60,
+// 18 50 68 / 45 102, 20 40 69 / 36 110, 30 70 224 / 77 340, 32 60 241 / 78 414, 36 74 355 /
+// 111 618, 50 345 1863 / 307 2007, 64 309 2021 / 516 3733; all of them together take the
+// build from 38 to 53 s.
 #define FAME_FOR_EACH_DS_N(X) X(12) X(24) X(40) X(48) X(60)
 #define FAME_DS_SIGS(PFX, NN)                                                                                      \
   PFX cudaError_t fame::detail::fncB_n<fame::ff, NN>(const Plan&, const cx<fame::ff>*, cx<fame::ff>*, int,         \

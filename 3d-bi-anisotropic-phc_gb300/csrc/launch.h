@@ -7,9 +7,10 @@
 // reads or writes anything another kernel touches (active flags and scalars
 // included), on every path, so completion stays transitive along the stream;
 // a kernel launched without the attribute still waits for the whole sequence.
-// fncB of one vector at n = 24 (five kernels of 4-6 us) 26.5 -> 16.2 us, three
-// at n = 50 55 -> 42, ten at n = 60 202 -> 192 (complex64), four at n = 40 434
-// -> 422 (complex128).
+// fncB, called from C one after the other: one vector at n = 24 22.6 -> 11.7 us,
+// three at n = 50 52 -> 39, ten at n = 60 197 -> 175 (complex64), two at n = 16 45.6 -> 31.0,
+// four at n = 40 433 -> 419 (complex128).  (A call from Python has some 10 us of host
+// time more: one vector at n = 24 takes 19.7, none of it waiting for the GPU.)
 // No kernel triggers its successor early: CTAs placed while the previous kernel
 // still runs are spread over the SMs by what is free at that moment, not
 // evenly (complex128 CG of two vectors at n = 30: 10.1 ms with a trigger at

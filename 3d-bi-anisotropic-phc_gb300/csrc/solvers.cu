@@ -2,7 +2,6 @@
 // (fncinvB), the mixed-precision B^{-1} used by the complex64 band solve,
 // and the thick-restart Lanczos band solver of fun_Lanczos/Lanczos.m.
 #include <algorithm>
-#include <atomic>
 #include <chrono>
 #include <cstdio>
 #include <cstdlib>

@@ -48,6 +48,8 @@ enum fame_precision { FAME_C128 = 0, FAME_C64 = 1, FAME_C128_DS = 2 };
 
 enum fame_handle { FAME_PR = 0, FAME_QR = 1, FAME_PRS = 2, FAME_QRS = 3 };
 
+/* x and y of the calls below are device arrays aligned to their elements (8 bytes
+ * complex64, 16 complex128), or host arrays with this flag. */
 #define FAME_HOST_PTR 1
 
 /* Library version string. */
