@@ -1,6 +1,7 @@
 // C ABI of the FAME GB300 library: plan life cycle and operator handles.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <complex>
 #include <cstdio>
@@ -117,6 +118,8 @@ cudaError_t ensure_work(Plan& P, size_t vecs) {
   return e;
 }
 
+constexpr size_t kInstRing = 1 << 16;  // indices of many calls between two waits
+
 cudaError_t upload_inst(Plan& P, const int* inst_host, int nvec, const int** d_inst_out) {
   *d_inst_out = nullptr;
   if (!inst_host) return cudaSuccess;
@@ -129,10 +132,20 @@ cudaError_t upload_inst(Plan& P, const int* inst_host, int nvec, const int** d_i
     P.inst_cap = nvec;
   }
   *d_inst_out = P.d_inst;
-  // from the caller's memory: a small pageable copy goes through the command stream, where
-  // one from the pinned ring is a DMA transfer that the next kernel waits longer for
-  // (fncA of 64 complex64 vectors at n = 30 28 against 32 us)
-  return cudaMemcpyAsync(P.d_inst, inst_host, sizeof(int) * nvec, cudaMemcpyHostToDevice, P.stream);
+  // From pageable memory: such a small copy goes through the command stream, where one
+  // from the pinned ring is a DMA transfer that the next kernel waits longer for (fncA
+  // of 64 complex64 vectors at n = 30 28 against 32 us).  From the plan's own, not the
+  // caller's: whether the driver has read a pageable source when the call returns is its
+  // affair, and the caller's array may be gone by then.
+  if (P.inst_pos + nvec > P.h_inst.size()) {  // wrap only once earlier copies have been consumed
+    if (cudaError_t e = P.inst_pos ? cudaStreamSynchronize(P.stream) : cudaSuccess) return e;
+    P.h_inst.resize(std::max({P.h_inst.size(), (size_t)nvec, kInstRing}));
+    P.inst_pos = 0;
+  }
+  int* src = P.h_inst.data() + P.inst_pos;
+  P.inst_pos += nvec;
+  std::copy(inst_host, inst_host + nvec, src);
+  return cudaMemcpyAsync(P.d_inst, src, sizeof(int) * nvec, cudaMemcpyHostToDevice, P.stream);
 }
 
 cudaError_t ensure_stage(Plan& P, size_t bytes) {

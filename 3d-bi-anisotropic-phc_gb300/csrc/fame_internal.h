@@ -183,6 +183,8 @@ struct Plan {
   // small device buffers
   int* d_inst = nullptr;
   size_t inst_cap = 0;
+  std::vector<int> h_inst;  // what upload_inst copies from, a ring in pageable memory
+  size_t inst_pos = 0;
   double* d_red = nullptr;            // reduction scratch
   size_t red_cap = 0;
   // host staging for FAME_HOST_PTR calls

@@ -37,3 +37,26 @@ def test_indices_in_arguments_and_memory(cuda, fame_lib, nk, dtype):
         one = torch.cat([f(v[k:k + 1], inst[k:k + 1]) for k in range(0, nvec)])
         for width in (33, 128, 129, 140):
             assert torch.equal(f(v[:width], inst[:width]).reshape(width, -1), one.reshape(nvec, -1)[:width]), (j, width)
+
+
+def test_indices_outlive_the_callers_array(cuda, fame_lib):
+    """The library may copy the indices after the call has returned: from memory of
+    its own, with the caller's array overwritten or freed by then, however many
+    calls are under way."""
+    n, nk, nvec = 8, 3, 900
+    rng = np.random.default_rng(5)
+    plan = fame.Plan.from_phases(n, rng.uniform(0.3, 2.5, size=(nk, 3)), rng.integers(0, 2, n ** 3).astype(np.uint8),
+                                 [fame.bi_isotropic(1.0, 0.0), fame.bi_isotropic(13.0, 0.4)])
+    x = torch.randn(nvec, 4 * n ** 3, dtype=torch.complex64, device="cuda")
+    whole = [plan.apply_A(x, inst=k) for k in range(nk)]
+    outs = {}
+    for j in range(200):  # 180000 indices: more than one turn of the library's buffer
+        inst = ((np.arange(nvec) + j) % nk).astype(np.int32)
+        y = plan.apply_A(x, inst=inst)
+        if j % 20 == 0:
+            outs[j] = y
+        inst[:] = 0
+    for j, y in outs.items():
+        want = (np.arange(nvec) + j) % nk
+        for k in range(nk):
+            assert torch.equal(y[torch.from_numpy(want == k).cuda()], whole[k][torch.from_numpy(want == k).cuda()]), (j, k)
